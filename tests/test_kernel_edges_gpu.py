@@ -1,0 +1,52 @@
+"""Edges of the kernels' tiles and of the rules that choose between them: remainders, the smallest and largest sizes of
+a range, against 64-bit (or integer) references."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _rel(got, want):
+    return float((got.detach().double() - want.detach()).norm() / want.detach().norm().clamp_min(1e-30))
+
+
+# ------------------------------------------------------------------------------------------------ norm backward
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 256), (17, 264), (301, 512), (5, 520), (2048, 1024), (77, 1032), (4099, 2048),
+                                    (9, 2056), (1001, 4096), (6, 4104), (613, 8192), (5, 8200)])
+@pytest.mark.parametrize("rms,residual", [(True, False), (False, True)])
+def test_norm_backward_sizes(rows, H, rms, residual, dtype):
+    """Thread groups per row change at hidden 256, 512, 1024, 2048, 4096; the batch of rows per block and the ring of
+    loads end at any row.  Tolerance: results are rounded once to the storage type (2^-9 bf16, 2^-11 fp16), on top of
+    fp32 arithmetic (1e-5)."""
+    from axonn_b200 import ops
+
+    torch.manual_seed(rows + H)
+    x, dl, dy, dh = (torch.randn(rows, H, device=DEV).to(dtype) for _ in range(4))
+    g = (1 + 0.1 * torch.randn(H, device=DEV)).to(dtype).requires_grad_(True)
+    b = None if rms else (0.1 * torch.randn(H, device=DEV)).to(dtype).requires_grad_(True)
+    x.requires_grad_(True)
+    leaves = [x, g] + ([] if rms else [b])
+    if residual:
+        h, y = ops.add_rms_norm(x, dl, g, 1e-5) if rms else ops.add_layer_norm(x, dl, g, b, 1e-5)
+        got = torch.autograd.grad([h, y], leaves, [dh, dy])
+        base = h.detach().double()
+    else:
+        y = ops.rms_norm(x, g, 1e-5) if rms else ops.layer_norm(x, g, b, 1e-5)
+        got = torch.autograd.grad(y, leaves, dy)
+        base = x.detach().double()
+    g64 = g.detach().double()
+    mean = torch.zeros(rows, 1, device=DEV, dtype=torch.float64) if rms else base.mean(-1, keepdim=True)
+    rstd = (base.pow(2).mean(-1, keepdim=True) - mean * mean + 1e-5).rsqrt()
+    xh, d = (base - mean) * rstd, dy.double()
+    gd = d * g64
+    want = [rstd * (gd - (0 if rms else gd.mean(-1, keepdim=True)) - xh * (gd * xh).mean(-1, keepdim=True)), (d * xh).sum(0)]
+    if residual:
+        want[0] = want[0] + dh.double()
+    if not rms:
+        want.append(d.sum(0))
+    tol = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10, torch.float32: 2e-5}[dtype]
+    for a, w in zip(got, want):
+        assert _rel(a, w) < tol, _rel(a, w)
