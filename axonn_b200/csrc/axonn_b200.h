@@ -214,13 +214,16 @@ int axb_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, int T,
 int axb_rope(void* x, const float* cs, long long rows, int S, int nh, int D, int pos_div, long long row_stride,
              int inverse, void* stream);
 
-/* ---- flash attention on the packed projection output [B, S, G, qpk + 2, D] (flash_attn.cu); D 64 or 128, S % 128 == 0 */
+/* ---- flash attention on the packed projection output [B, S, G, qpk + 2, D] (flash_attn.cu); D 64 or 128 */
 int axb_flash_attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int G, int qpk, int D, float scale,
                        int device, void* stream);
 int axb_flash_attn_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta, float* dq_acc,
                        void* dqkv, int B, int S, int G, int qpk, int D, float scale, int device, void* stream);
-/* two-kernel backward without atomics; which: bit 0 = dQ kernel (query slots of dqkv), bit 1 = dK / dV kernel */
-int axb_flash_attn_bwd_split(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta,
+/* (the one-kernel backward: S % 128 == 0) */
+/* two-kernel backward without atomics, any S; which: bit 0 = dQ kernel (query slots of dqkv), bit 1 = dK / dV kernel;
+ * scratch: axb_flash_attn_bwd_scratch() fp32 words */
+long long axb_flash_attn_bwd_scratch(int B, int S, int heads);
+int axb_flash_attn_bwd_split(const void* qkv, const void* out, const void* d_out, const float* lse, float* scratch,
                              void* dqkv, int B, int S, int G, int qpk, int D, float scale, int which, int device,
                              void* stream);
 

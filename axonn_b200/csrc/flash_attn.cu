@@ -1,21 +1,9 @@
-// Causal flash attention forward on tcgen05 tensor cores (sm_100a), grouped-query aware.
+// Causal flash attention on tcgen05 tensor cores (sm_100a), grouped-query aware: the forward kernel and the one-kernel
+// backward (the two-kernel backward is in flash_attn_bwd_split.cu).
 //
-// Input is the fused projection output, packed [B, S, G, q_per_kv + 2, D]: for every KV group its query
-// heads, then its key head, then its value head.  One CTA handles one (batch, query head, 128-row query
-// tile) and walks the KV tiles up to the diagonal:
-//
-//   warp 0   TMA: Q once, then K_j / V_j into a 2-stage shared-memory ring (128-byte swizzle)
-//   warp 1   MMA: S_j = Q K_j^T into one of two TMEM score buffers (issued one tile ahead), then
-//            PV_j = P_j V_j into one of two TMEM output buffers; P_j is read from shared memory
-//            (K-major), V_j is consumed in place as an MN-major operand - no transposes
-//   warps 2-5 softmax: one thread per query row; tcgen05.ld the scores, online max / exp2 / row sum,
-//            write P_j (bf16) into shared memory in the tensor core's canonical swizzled layout,
-//            and fold the previous tile's PV product into the register-resident output row
-//            (o = o * alpha + PV), so score MMAs, exponentials and PV MMAs of neighbouring tiles
-//            overlap.
-//
-// Outputs: O [B, S, heads, D] bf16 and the per-row log-sum-exp (natural log, of the scaled scores)
-// [B, heads, S] fp32 for the backward pass.  All waits are bounded.
+// Input is the fused projection output, packed [B, S, G, q_per_kv + 2, D]: for every KV group its query heads, then
+// its key head, then its value head.  Outputs of the forward: O [B, S, heads, D] bf16 and the per-row log-sum-exp
+// (natural log, of the scaled scores) [B, heads, S] fp32 for the backward pass.  All waits are bounded.
 #include <cstdlib>
 #include <mutex>
 
@@ -25,6 +13,7 @@ namespace axb {
 
 int make_tmap_2d_16bit(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, int dtype);
 int make_tmap_2d_f32(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows);
+int make_tmap_3d_bf16(CUtensorMap* out, const void* ptr, uint64_t batch, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
 struct FaParams {
   __nv_bfloat16* out;
@@ -36,22 +25,7 @@ struct FaParams {
   int debug;   // ablation builds only (-DAXB_ABLATION, read once from AXB_FA_DEBUG; otherwise 0 and compiled out): 4 phase timers of the two-tile forward
 };
 
-constexpr int FA_BQ = 128, FA_BKV = 128, FA_THREADS = 320;   // TMA warp, MMA warp, 8 softmax warps
-
-template <int HD>
-struct FaSmem {
-  static constexpr int TILE = 128 * HD * 2;       // Q, K or V tile bytes
-  static constexpr int P_BYTES = 128 * 128 * 2;
-  static constexpr int Q_OFF = 0;
-  static constexpr int K_OFF = TILE;               // 2 stages
-  static constexpr int V_OFF = 3 * TILE;           // 2 stages
-  static constexpr int P_OFF = 5 * TILE;
-  static constexpr int BAR_OFF = P_OFF + P_BYTES;
-  static constexpr int NBARS = 1 + 2 + 2 + 2 + 2 + 2 + 1 + 1 + 2 + 2;
-  // exchange between the two threads of a query row: maxima [2][2][128], row sums [2][128], sequence tags [2][128]
-  static constexpr int XCH_OFF = BAR_OFF + NBARS * 8 + 16;
-  static constexpr int TOTAL = XCH_OFF + 8 * 128 * 4 + 1024;
-};
+constexpr int FA_BQ = 128;
 
 // Bounded wait until the other thread of a query row has published sequence number `want`.
 __device__ __forceinline__ bool wait_partner(volatile int* flag, int want, volatile int* abort_flag, uint64_t timeout_ns) {
@@ -68,293 +42,15 @@ __device__ __forceinline__ bool wait_partner(volatile int* flag, int want, volat
   return true;
 }
 
-template <int HD>
-__global__ void __launch_bounds__(FA_THREADS, 1)
-fa_fwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams p) {
-  using S_ = FaSmem<HD>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S_::BAR_OFF);
-  uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;
-  uint64_t* v_full = bars + 3;
-  uint64_t* kv_empty = bars + 5;
-  uint64_t* s_full = bars + 7;
-  uint64_t* s_empty = bars + 9;
-  uint64_t* p_full = bars + 11;
-  uint64_t* p_empty = bars + 12;
-  uint64_t* o_full = bars + 13;
-  uint64_t* o_empty = bars + 15;
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + S_::NBARS);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = p.S / FA_BQ;
-  const int qt = nq - 1 - static_cast<int>(blockIdx.z);  // heaviest tiles first, over the whole grid
-  const int head = blockIdx.x;
-  const int b = blockIdx.y;
-  const int g = head / p.qpk, jq = head % p.qpk;
-  const int n_kv = qt + 1;                               // causal: tiles 0..qt
-  const int row0 = b * p.S + qt * FA_BQ;                 // row in the [B*S, G*(qpk+2)*HD] view
-  const int col_q = (g * (p.qpk + 2) + jq) * HD;
-  const int col_k = (g * (p.qpk + 2) + p.qpk) * HD;
-  const int col_v = col_k + HD;
-  const uint64_t timeout = p.timeout_ns;
-
-  if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&kv_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 8);
-      mbar_init(&o_full[i], 1); mbar_init(&o_empty[i], 8);
-    }
-    mbar_init(p_full, 8); mbar_init(p_empty, 1);
-    for (int i = 0; i < 256; ++i) reinterpret_cast<volatile int*>(smem + S_::XCH_OFF + 6 * 128 * 4)[i] = 0;
-    *abort_flag = 0;
-    fence_mbar_init();
-  }
-  if (warp == 0 && lane == 0) tma_prefetch_desc(&tmQKV);
-  if (warp == 1) { tmem_alloc(tmem_ptr_smem, 512); tmem_relinquish(); }
-  tcgen05_fence_before();
-  __syncthreads();
-  tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_ptr_smem;
-  const uint32_t tmem_s = tmem_base;          // 2 x 128 columns
-  const uint32_t tmem_o = tmem_base + 256;    // 2 x HD columns
-
-  if (warp == 0) {
-    if (elect_one()) {
-      bool ok = true;
-      mbar_expect_tx(q_full, S_::TILE);
-#pragma unroll
-      for (int c = 0; c < HD / 64; ++c) tma_load_2d(smem + S_::Q_OFF + c * 16384, &tmQKV, q_full, col_q + 64 * c, row0);
-      for (int j = 0; j < n_kv && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        if (!mbar_wait(&kv_empty[st], ph ^ 1, abort_flag, timeout)) { ok = false; break; }
-        const int krow = b * p.S + j * FA_BKV;
-        mbar_expect_tx(&k_full[st], S_::TILE);
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c)
-          tma_load_2d(smem + S_::K_OFF + st * S_::TILE + c * 16384, &tmQKV, &k_full[st], col_k + 64 * c, krow);
-        mbar_expect_tx(&v_full[st], S_::TILE);
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c)
-          tma_load_2d(smem + S_::V_OFF + st * S_::TILE + c * 16384, &tmQKV, &v_full[st], col_v + 64 * c, krow);
-      }
-      if (!ok) {
-        // drain: give in-flight copies time to land before the CTA exits
-        const uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 200000ull) {}
-        report_status(p.status, 0x401u);
-      }
-    }
-  } else if (warp == 1) {
-    if (elect_one()) {
-      bool ok = true;
-      const uint32_t idesc_s = umma_idesc(1, 0, 0, 128, 128);
-      const uint32_t idesc_o = umma_idesc(1, 0, 1, 128, HD);
-      const uint32_t q_addr = smem_u32(smem + S_::Q_OFF);
-      const uint32_t p_addr = smem_u32(smem + S_::P_OFF);
-      auto issue_s = [&](int j) {
-        const uint32_t k_addr = smem_u32(smem + S_::K_OFF + (j & 1) * S_::TILE);
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_f16(tmem_s + (j & 1) * 128, umma_smem_desc(q_addr + off, 16, 1024), umma_smem_desc(k_addr + off, 16, 1024),
-                   idesc_s, kk != 0 ? 1u : 0u);
-        }
-        umma_commit(&s_full[j & 1]);
-      };
-      ok = mbar_wait(q_full, 0, abort_flag, timeout) && mbar_wait(&k_full[0], 0, abort_flag, timeout);
-      if (ok) { tcgen05_fence_after(); issue_s(0); }
-      for (int j = 0; j < n_kv && ok; ++j) {
-        if (j + 1 < n_kv) {
-          const int u = j + 1;
-          if (!mbar_wait(&k_full[u & 1], (u >> 1) & 1, abort_flag, timeout) ||
-              !mbar_wait(&s_empty[u & 1], ((u >> 1) & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
-          tcgen05_fence_after();
-          issue_s(u);
-        }
-        if (!mbar_wait(p_full, j & 1, abort_flag, timeout) || !mbar_wait(&v_full[j & 1], (j >> 1) & 1, abort_flag, timeout) ||
-            !mbar_wait(&o_empty[j & 1], ((j >> 1) & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
-        tcgen05_fence_after();
-        const uint32_t v_addr = smem_u32(smem + S_::V_OFF + (j & 1) * S_::TILE);
-#pragma unroll
-        for (int kk = 0; kk < FA_BKV / 16; ++kk) {
-          const uint64_t adesc = umma_smem_desc(p_addr + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
-          // V: MN-major, 64-wide column chunks 16 KB apart (leading), 8-row groups 1 KB apart (stride)
-          const uint64_t bdesc = umma_smem_desc(v_addr + kk * 2048, 16384, 1024);
-          umma_f16(tmem_o + (j & 1) * HD, adesc, bdesc, idesc_o, kk != 0 ? 1u : 0u);
-        }
-        umma_commit(&o_full[j & 1]);
-        umma_commit(p_empty);
-        umma_commit(&kv_empty[j & 1]);
-      }
-      if (!ok) report_status(p.status, 0x402u);
-    }
-  } else {
-    // ------------------------------------------------------------------ softmax + output accumulation
-    // Eight warps: two share each TMEM lane quarter; thread = (query row r, column half).  A thread owns 64 of
-    // the 128 score columns of its row and HD/2 of the output columns, so that a KV tile costs it one TMEM
-    // read of the scores (kept in registers between the max and the exponentials) and one of the PV product.
-    // The two threads of a row exchange their partial row maxima through shared memory (one 64-thread named
-    // barrier per tile); the partial row sums are only combined at the end.
-    const int q4 = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int r = q4 * 32 + lane;                 // query row inside the tile
-    const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
-    constexpr int OC = HD / 2;                    // output columns per thread
-    float o[OC];
-#pragma unroll
-    for (int i = 0; i < OC; ++i) o[i] = 0.f;
-    float m = -INFINITY, l = 0.f, alpha_prev = 1.f;
-    bool ok = true;
-    uint8_t* p_row = smem + S_::P_OFF + (r >> 3) * 1024 + (r & 7) * 128 + half * 16384;
-    volatile float* xch = reinterpret_cast<volatile float*>(smem + S_::XCH_OFF);   // [2 tile parities][2 halves][128 rows]
-    volatile int* xflag = reinterpret_cast<volatile int*>(smem + S_::XCH_OFF + 6 * 128 * 4);   // [2 halves][128 rows]
-    for (int j = 0; j < n_kv; ++j) {
-      if (!mbar_wait(&s_full[j & 1], (j >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
-      tcgen05_fence_after();
-      const uint32_t s_addr = tmem_s + lane_base + (j & 1) * 128 + half * 64;
-      const bool diag = (j == qt);
-      uint32_t sv[64];
-      tmem_ld_32x32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&sv[0]));
-      tmem_ld_32x32(s_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&sv[32]));
-      tmem_ld_wait();
-      // the score buffer can be reused by the MMA warp as soon as both halves hold it in registers
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&s_empty[j & 1]);
-      float mx = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < 64; ++i)
-        if (!diag || (half * 64 + i) <= r) mx = fmaxf(mx, __uint_as_float(sv[i]));
-      mx *= p.scale_log2;                       // the scale is positive: scale the maximum once
-      xch[((j & 1) * 2 + half) * 128 + r] = mx;
-      __threadfence_block();
-      xflag[half * 128 + r] = j + 1;
-      if (!wait_partner(xflag + (half ^ 1) * 128 + r, j + 1, abort_flag, timeout)) { ok = false; break; }
-      mx = fmaxf(mx, xch[((j & 1) * 2 + (half ^ 1)) * 128 + r]);
-      const float m_new = fmaxf(m, mx);
-      const float alpha = exp2f(m - m_new);
-      if (!mbar_wait(p_empty, (j & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
-      // exponentials, partial row sum, this thread's half of the P row (bf16, swizzled K-major layout)
-      float rowsum = 0.f;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t packed[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          float e0 = exp2f(__uint_as_float(sv[c * 32 + 2 * i]) * p.scale_log2 - m_new);
-          float e1 = exp2f(__uint_as_float(sv[c * 32 + 2 * i + 1]) * p.scale_log2 - m_new);
-          if (diag) {
-            if (half * 64 + c * 32 + 2 * i > r) e0 = 0.f;
-            if (half * 64 + c * 32 + 2 * i + 1 > r) e1 = 0.f;
-          }
-          const __nv_bfloat162 h = __floats2bfloat162_rn(e0, e1);
-          rowsum += e0 + e1;
-          packed[i] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-        // columns half*64 + [c*32, c*32+32): 16-byte chunks (c * 4 + t), t = 0..3, of the 64-column block
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const int chunk = (c * 4 + t) ^ (r & 7);
-          *reinterpret_cast<uint4*>(p_row + chunk * 16) =
-              make_uint4(packed[4 * t], packed[4 * t + 1], packed[4 * t + 2], packed[4 * t + 3]);
-        }
-      }
-      fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
-      l = l * alpha + rowsum;
-      m = m_new;
-      // fold the previous tile's PV product into the output row
-      if (j > 0) {
-        const int u = j - 1;
-        if (!mbar_wait(&o_full[u & 1], (u >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
-        tcgen05_fence_after();
-        const uint32_t o_addr = tmem_o + lane_base + (u & 1) * HD + half * OC;
-        uint32_t v[OC];
-#pragma unroll
-        for (int c = 0; c < OC / 32; ++c) tmem_ld_32x32(o_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[c * 32]));
-        tmem_ld_wait();
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&o_empty[u & 1]);
-#pragma unroll
-        for (int i = 0; i < OC; ++i) o[i] = o[i] * alpha_prev + __uint_as_float(v[i]);
-      }
-      alpha_prev = alpha;
-    }
-    if (ok) {
-      const int u = n_kv - 1;
-      if (mbar_wait(&o_full[u & 1], (u >> 1) & 1, abort_flag, timeout)) {
-        tcgen05_fence_after();
-        // total row sum = sum of the two halves' partial sums
-        volatile float* lx = xch + 4 * 128;        // [2 halves][128 rows], used once
-        lx[half * 128 + r] = l;
-        __threadfence_block();
-        xflag[half * 128 + r] = n_kv + 1;
-        if (!wait_partner(xflag + (half ^ 1) * 128 + r, n_kv + 1, abort_flag, timeout)) ok = false;
-        l += lx[(half ^ 1) * 128 + r];
-        const uint32_t o_addr = tmem_o + lane_base + (u & 1) * HD + half * OC;
-        const float inv_l = 1.f / l;
-        const size_t heads = static_cast<size_t>(p.G) * p.qpk;
-        __nv_bfloat16* dst = p.out + ((static_cast<size_t>(b) * p.S + qt * FA_BQ + r) * heads + head) * HD + half * OC;
-#pragma unroll
-        for (int c = 0; c < OC / 32; ++c) {
-          uint32_t v[32];
-          tmem_ld_32x32(o_addr + c * 32, v);
-          tmem_ld_wait();
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            uint32_t w[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int e = t * 8 + i * 2;
-              const float a0 = (o[c * 32 + e] * alpha_prev + __uint_as_float(v[e])) * inv_l;
-              const float a1 = (o[c * 32 + e + 1] * alpha_prev + __uint_as_float(v[e + 1])) * inv_l;
-              const __nv_bfloat162 h = __floats2bfloat162_rn(a0, a1);
-              w[i] = *reinterpret_cast<const uint32_t*>(&h);
-            }
-            *reinterpret_cast<uint4*>(dst + c * 32 + t * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-          }
-        }
-        if (half == 0)
-          p.lse[(static_cast<size_t>(b) * heads + head) * p.S + qt * FA_BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
-      } else {
-        ok = false;
-      }
-    }
-    if (!ok && lane == 0) report_status(p.status, 0x404u);
-  }
-  tcgen05_fence_before();
-  __syncthreads();
-  if (warp == 1) { __syncwarp(); tcgen05_fence_after(); tmem_dealloc(tmem_base, 512); }
-}
-
-template <int HD>
-static int fa_launch(const CUtensorMap& tm, const FaParams& p, int device, cudaStream_t s) {
-  using S_ = FaSmem<HD>;
-  static bool configured[64] = {false};
-  auto kern = fa_fwd_kernel<HD>;
-  if (!configured[device & 63]) {
-    AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S_::TOTAL));
-    configured[device & 63] = true;
-  }
-  dim3 grid(p.G * p.qpk, p.B, p.S / FA_BQ);   // z (slowest) = query tile, heaviest tiles first
-  kern<<<grid, FA_THREADS, S_::TOTAL, s>>>(tm, p);
-  AXB_CUDA(cudaGetLastError());
-  return 0;
-}
-
-
 // -----------------------------------------------------------------------------------------------------
 // Forward, two query tiles at a time ("ping-pong"), persistent CTAs.  A work item is the pair of adjacent
 // 128-row query tiles A = 2u and B = 2u + 1 of one (batch, head); they share every K_j / V_j tile that the TMA
 // warp loads.  One CTA per SM walks its share of the items (longest first): the loads and the first score MMAs
 // of the next item overlap the previous item's last softmax steps and its output stores.
+//
+// Any sequence length: rows past S are outside the tensor map and arrive as zeros (keys past S lie to the right of
+// every query that is stored, so the causal mask hides them), and rows past S are not stored.  When S ends inside
+// tile A of the last pair, tile B of that pair is not computed: its warps skip the item and only release the KV ring.
 //
 //   warp 0      TMA: Q_A, Q_B once; K_j and V_j into separate 2-stage rings
 //   warps 1, 2  MMA of tile A and of tile B: S_X = Q_X K^T for 64 keys into one of the two score buffers of tile X, then O_X += P_X V
@@ -399,20 +95,22 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 
 // Work item `idx` of the persistent grid: pairs of query tiles sorted by decreasing length (pair u has 4u + 3 tile
 // steps), dealt to the CTAs in a snake (0..G-1, G-1..0, ...) so that every CTA gets nearly the same total.
-struct Fa2Item { int u, head, b; };
+struct Fa2Item { int u, head, b, has_b; };   // has_b: tile B holds rows of the sequence
+template <bool RAGGED>
 __device__ __forceinline__ bool fa2_item(const FaParams& p, int k, Fa2Item& w) {
   const int G = gridDim.x, c = blockIdx.x;
-  const int heads = p.G * p.qpk, bh = p.B * heads, npairs = p.S / (2 * FA_BQ);
+  const int heads = p.G * p.qpk, bh = p.B * heads, npairs = (p.S + 2 * FA_BQ - 1) / (2 * FA_BQ);
   const int idx = k * G + ((k & 1) ? G - 1 - c : c);
   if (idx >= bh * npairs) return false;
   w.u = npairs - 1 - idx / bh;
+  w.has_b = !RAGGED || (2 * w.u + 1) * FA_BQ < p.S;
   const int rem = idx % bh;
   w.head = rem % heads;
   w.b = rem / heads;
   return true;
 }
 
-template <int HD>
+template <int HD, bool RAGGED>     // RAGGED: S is not a multiple of 256 (the guards cost the even lengths 4 %)
 __global__ void __launch_bounds__(FA2_THREADS, 1)
 fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams p) {
   using S_ = Fa2Smem<HD>;
@@ -460,34 +158,34 @@ fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams
       bool ok = true;
       uint32_t kvc = 0;                                     // KV tiles loaded so far: ring stage and phase
       Fa2Item w;
-      for (int it = 0; ok && fa2_item(p, it, w); ++it) {
+      for (int it = 0; ok && fa2_item<RAGGED>(p, it, w); ++it) {
         const int g = w.head / p.qpk, jq = w.head % p.qpk;
         const int col_q = (g * (p.qpk + 2) + jq) * HD;
         const int col_k = (g * (p.qpk + 2) + p.qpk) * HD;
         const int col_v = col_k + HD;
-        const int row0 = w.b * p.S + 2 * w.u * FA_BQ;
-        const int n_b = 2 * w.u + 2;                         // KV tiles of 128 keys
+        const int row0 = 2 * w.u * FA_BQ;
+        const int n_b = 2 * w.u + 1 + w.has_b;               // KV tiles of 128 keys
         if (!mbar_wait(q_empty, (it & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
         mbar_expect_tx(q_full, 2 * S_::TILE);
 #pragma unroll
         for (int x = 0; x < 2; ++x)
 #pragma unroll
           for (int c = 0; c < HD / 64; ++c)
-            tma_load_2d(smem + S_::Q_OFF + x * S_::TILE + c * 16384, &tmQKV, q_full, col_q + 64 * c, row0 + x * FA_BQ);
+            tma_load_3d(smem + S_::Q_OFF + x * S_::TILE + c * 16384, &tmQKV, q_full, col_q + 64 * c, row0 + x * FA_BQ, w.b);
         for (int j = 0; j < n_b && ok; ++j, ++kvc) {
           const int st = kvc & 1;
           const uint32_t ph = (kvc >> 1) & 1;
-          const int krow = w.b * p.S + j * FA_BKV;
+          const int krow = j * 128;
           if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag, timeout)) { ok = false; break; }
           mbar_expect_tx(&k_full[st], S_::TILE);
 #pragma unroll
           for (int c = 0; c < HD / 64; ++c)
-            tma_load_2d(smem + S_::K_OFF + st * S_::TILE + c * 16384, &tmQKV, &k_full[st], col_k + 64 * c, krow);
+            tma_load_3d(smem + S_::K_OFF + st * S_::TILE + c * 16384, &tmQKV, &k_full[st], col_k + 64 * c, krow, w.b);
           if (!mbar_wait(&v_empty[st], ph ^ 1, abort_flag, timeout)) { ok = false; break; }
           mbar_expect_tx(&v_full[st], S_::TILE);
 #pragma unroll
           for (int c = 0; c < HD / 64; ++c)
-            tma_load_2d(smem + S_::V_OFF + st * S_::TILE + c * 16384, &tmQKV, &v_full[st], col_v + 64 * c, krow);
+            tma_load_3d(smem + S_::V_OFF + st * S_::TILE + c * 16384, &tmQKV, &v_full[st], col_v + 64 * c, krow, w.b);
         }
       }
       if (!ok) {
@@ -528,8 +226,22 @@ fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams
       const bool probe = AXB_DBG(p, 4) && blockIdx.x == 0 && x == 0;
       long long pw_p = 0, pw_kv = 0, p_mark = 0, p_t0 = probe ? clock64() : 0;
       Fa2Item w;
-      for (int it = 0; ok && fa2_item(p, it, w); ++it) {
-        const int n_b = 4 * w.u + 4, n_x = n_b - 2 + 2 * x;     // steps of 64 keys: causal, tiles 2u and 2u + 1
+      for (int it = 0; ok && fa2_item<RAGGED>(p, it, w); ++it) {
+        const int n_t = 2 * w.u + 1 + w.has_b;                  // KV tiles of the item
+        const int n_x = 4 * w.u + 2 + 2 * x;                    // steps of 64 keys: causal, tiles 2u and 2u + 1
+        if (x == 1 && !w.has_b) {
+          // nothing to compute for tile B: release Q and every KV tile once it has been loaded (an earlier arrival
+          // would count for the tile that used the stage before)
+          if (!mbar_wait(q_full, it & 1, abort_flag, timeout)) { ok = false; break; }
+          mbar_arrive(q_empty);
+          for (int t = 0; t < n_t && ok; ++t, ++kvc) {
+            if (!mbar_wait(&k_full[kvc & 1], (kvc >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
+            mbar_arrive(&k_empty[kvc & 1]);
+            if (!mbar_wait(&v_full[kvc & 1], (kvc >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
+            mbar_arrive(&v_empty[kvc & 1]);
+          }
+          continue;
+        }
         if (!mbar_wait(q_full, it & 1, abort_flag, timeout) ||
             !mbar_wait(&k_full[kvc & 1], (kvc >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
         tcgen05_fence_after();
@@ -565,18 +277,18 @@ fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams
             }
           }
         }
-        if (x == 0 && ok) {
+        if (x == 0 && w.has_b && ok) {
           // Tile A does not read the item's last KV tile, but the ring counts two releases per tile.  The release
           // may only be given once that tile has been loaded: before that, the stage still belongs to the tile
           // two steps earlier, and an early arrival would complete that tile's "empty" phase while tile B's warp
           // is still reading it.
-          const uint32_t last = kvc + (n_b >> 1) - 1;
+          const uint32_t last = kvc + n_t - 1;
           if (!mbar_wait(&k_full[last & 1], (last >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
           umma_commit(&k_empty[last & 1]);
           if (!mbar_wait(&v_full[last & 1], (last >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
           umma_commit(&v_empty[last & 1]);
         }
-        kvc += n_b >> 1;
+        kvc += n_t;
       }
       if (probe) {
         volatile unsigned int* wd = reinterpret_cast<volatile unsigned int*>(p.status);
@@ -600,7 +312,8 @@ fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams
     const bool probe = AXB_DBG(p, 4) && blockIdx.x == 0 && warp == 4 && lane == 0;
     long long pw_s = 0, pt_ld = 0, pt_max = 0, pt_exp = 0, pt_epi = 0, p_mark = 0;
     Fa2Item w;
-    for (int it = 0; ok && fa2_item(p, it, w); ++it) {
+    for (int it = 0; ok && fa2_item<RAGGED>(p, it, w); ++it) {
+      if (x == 1 && !w.has_b) continue;
       const int n_x = 4 * w.u + 2 + 2 * x;           // steps of 64 keys; the item's step counts are even, so the
       float m = -INFINITY, l = 0.f;                  // score buffer of a step is also (tc & 1)
       for (int st = 0; st < n_x; ++st, ++tc) {
@@ -708,7 +421,8 @@ fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams
       tcgen05_fence_after();
       const float inv_l = 1.f / l;
       const size_t heads = static_cast<size_t>(p.G) * p.qpk;
-      const size_t qrow = static_cast<size_t>(w.b) * p.S + (2 * w.u + x) * FA_BQ + r;
+      const int qpos = (2 * w.u + x) * FA_BQ + r;
+      const size_t qrow = static_cast<size_t>(w.b) * p.S + qpos;
       __nv_bfloat16* dst = p.out + (qrow * heads + w.head) * HD;
 #pragma unroll
       for (int c = 0; c < HD / 32; ++c) {
@@ -724,10 +438,11 @@ fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams
             const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[e]) * inv_l, __uint_as_float(v[e + 1]) * inv_l);
             wv[i] = *reinterpret_cast<const uint32_t*>(&h);
           }
-          *reinterpret_cast<uint4*>(dst + c * 32 + t * 8) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+          if (!RAGGED || qpos < p.S) *reinterpret_cast<uint4*>(dst + c * 32 + t * 8) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
         }
       }
-      p.lse[(static_cast<size_t>(w.b) * heads + w.head) * p.S + (2 * w.u + x) * FA_BQ + r] = (m + log2f(l)) * 0.6931471805599453f;
+      if (!RAGGED || qpos < p.S)
+        p.lse[(static_cast<size_t>(w.b) * heads + w.head) * p.S + qpos] = (m + log2f(l)) * 0.6931471805599453f;
       // the next item's first PV MMA overwrites O: it waits for this thread's next arrival on p_full, which follows
       // these reads in program order
       tcgen05_fence_before();
@@ -745,29 +460,20 @@ fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams
   if (warp == 1) { __syncwarp(); tcgen05_fence_after(); tmem_dealloc(tmem_base, 512); }
 }
 
-template <int HD>
+template <int HD, bool RAGGED>
 static int fa_launch_pingpong(const CUtensorMap& tm, const FaParams& p, int device, cudaStream_t s) {
   using S_ = Fa2Smem<HD>;
   static bool configured[64] = {false};
-  auto kern = fa_fwd_pingpong_kernel<HD>;
+  auto kern = fa_fwd_pingpong_kernel<HD, RAGGED>;
   if (!configured[device & 63]) {
     AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S_::TOTAL));
     configured[device & 63] = true;
   }
-  const long long items = static_cast<long long>(p.B) * p.G * p.qpk * (p.S / (2 * FA_BQ));
+  const long long items = static_cast<long long>(p.B) * p.G * p.qpk * ((p.S + 2 * FA_BQ - 1) / (2 * FA_BQ));
   const int sms = sm_count(device);
   kern<<<static_cast<int>(items < sms ? items : sms), FA2_THREADS, S_::TOTAL, s>>>(tm, p);   // persistent CTAs
   AXB_CUDA(cudaGetLastError());
   return 0;
-}
-
-// AXONN_FA_FWD=single keeps the one-tile-per-CTA forward for every shape (A/B runs); read once.
-static bool fa_pingpong_enabled() {
-  static const bool on = [] {
-    const char* e = getenv("AXONN_FA_FWD");
-    return !(e && e[0] == 's');
-  }();
-  return on;
 }
 
 }  // namespace axb
@@ -777,10 +483,10 @@ extern "C" int axb_flash_attn_fwd(const void* qkv, void* out, float* lse, int B,
                                   float scale, int device, void* stream) {
   using namespace axb;
   if (D != 64 && D != 128) { set_error("flash attention: head_dim must be 64 or 128"); return -1; }
-  if (S % 128) { set_error("flash attention: sequence length must be a multiple of 128"); return -1; }
+  if (B <= 0 || S <= 0 || G <= 0 || qpk <= 0) { set_error("flash attention: empty problem"); return -1; }
+  if (reinterpret_cast<uintptr_t>(out) & 15) { set_error("flash attention: tensors must be 16-byte aligned"); return -1; }
   CUtensorMap tm;
-  if (make_tmap_2d_16bit(&tm, qkv, static_cast<uint64_t>(B) * S, static_cast<uint64_t>(G) * (qpk + 2) * D, 128, 0))
-    return -1;
+  if (make_tmap_3d_bf16(&tm, qkv, B, S, static_cast<uint64_t>(G) * (qpk + 2) * D, 128)) return -1;
   FaParams p;
   p.out = static_cast<__nv_bfloat16*>(out); p.lse = lse; p.B = B; p.S = S; p.G = G; p.qpk = qpk;
   p.scale_log2 = scale * 1.4426950408889634f;
@@ -791,12 +497,10 @@ extern "C" int axb_flash_attn_fwd(const void* qkv, void* out, float* lse, int B,
 #ifdef AXB_ABLATION
   { static int dbg = -1; if (dbg < 0) { const char* e = getenv("AXB_FA_DEBUG"); dbg = e ? atoi(e) : 0; } p.debug = dbg; }
 #endif
-  if (S % 256 == 0 && fa_pingpong_enabled()) {
-    if (D == 128) return fa_launch_pingpong<128>(tm, p, device, static_cast<cudaStream_t>(stream));
-    return fa_launch_pingpong<64>(tm, p, device, static_cast<cudaStream_t>(stream));
-  }
-  if (D == 128) return fa_launch<128>(tm, p, device, static_cast<cudaStream_t>(stream));
-  return fa_launch<64>(tm, p, device, static_cast<cudaStream_t>(stream));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (S % (2 * FA_BQ) == 0)
+    return D == 128 ? fa_launch_pingpong<128, false>(tm, p, device, s) : fa_launch_pingpong<64, false>(tm, p, device, s);
+  return D == 128 ? fa_launch_pingpong<128, true>(tm, p, device, s) : fa_launch_pingpong<64, true>(tm, p, device, s);
 }
 
 // =====================================================================================================

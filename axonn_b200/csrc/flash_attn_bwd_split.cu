@@ -25,41 +25,72 @@
 
 namespace axb {
 
-int make_tmap_2d_16bit(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows, int dtype);
+int make_tmap_3d_bf16(CUtensorMap* out, const void* ptr, uint64_t batch, uint64_t rows, uint64_t cols, uint32_t box_rows);
 int sm_count(int device);
 
 struct FaSplitParams {
-  const float* lse;      // [B, heads, S], natural log
-  const float* delta;    // [B, heads, S]
+  // per query row, [B, heads, Sp] with Sp = S rounded up to 128: -lse in units of log2 and -delta.  Rows past S have
+  // -inf there, so that their probabilities (and with them every contribution to dK, dV and dQ) are exact zeros.
+  const float* neg_lse2;
+  const float* neg_delta;
   __nv_bfloat16* dqkv;   // [B, S, G, qpk + 2, D]
-  int B, S, G, qpk;
+  int B, S, Sp, G, qpk;
   float scale, scale_log2;
   unsigned int* status;
   unsigned long long timeout_ns;
   int debug;   // ablation builds only (-DAXB_ABLATION, read once from AXB_FA_DEBUG; otherwise 0 and compiled out): 4 phase timers
 };
 
-constexpr int FS_THREADS = 384;   // TMA warp, MMA warp(s), idle warps of the first warpgroup, 8 softmax warps
+// TMA warp, two MMA warps and an idle one (first warpgroup), 16 softmax warps.  The probabilities are what bounds both
+// kernels (one exponential, one conversion and two multiply-adds per score, behind tensor-memory loads); four warps
+// per scheduler with 32 scores per thread hide that latency, two warps with 64 do not.  Registers: 640 threads get 96
+// each at launch, 128 * 64 + 512 * 104 after the split are exactly those.
+// Measured on a B200, dQ / dK+dV kernel, 8 x 2048, 16 heads, head_dim 128 (two warps per scheduler, then four): the pair
+// with its delta kernel 660 - 700 us -> 577 us (247 + 363 + 35 one by one); cuDNN's backward takes 492 us there.
+constexpr int FS_THREADS = 640;
+constexpr int FS_SOFTMAX_WARPS = 16;
+#define FS_REGS_CONTROL "setmaxnreg.dec.sync.aligned.u32 64;"
+#define FS_REGS_SOFTMAX "setmaxnreg.inc.sync.aligned.u32 104;"
 
-// delta[b, h, s] = sum_d dO[b, s, h, d] * O[b, s, h, d]; one warp per (b, s, h) row
-__global__ void fa_split_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                      float* __restrict__ delta, int B, int S, int H, int D) {
-  const long long rows = static_cast<long long>(B) * S * H;
-  const int lane = threadIdx.x & 31;
-  for (long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; row < rows;
-       row += ((long long)gridDim.x * blockDim.x) >> 5) {
-    const __nv_bfloat162* a = reinterpret_cast<const __nv_bfloat162*>(o + row * D);
-    const __nv_bfloat162* c = reinterpret_cast<const __nv_bfloat162*>(d_o + row * D);
+__device__ __forceinline__ uint32_t fs_pack(float2 v) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// neg_delta[b, h, s] = -sum_d dO[b, s, h, d] * O[b, s, h, d] and neg_lse2 = -lse * log2(e); HD / 8 threads per row,
+// 16-byte loads.  Rows S .. Sp - 1 get -inf / 0 (see FaSplitParams).
+template <int HD>
+__global__ void __launch_bounds__(256)
+fa_split_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
+                      const float* __restrict__ lse, float* __restrict__ neg_lse2, float* __restrict__ neg_delta,
+                      int B, int S, int Sp, int H) {
+  constexpr int TPR = HD / 8;
+  const long long rows = static_cast<long long>(B) * Sp * H;
+  const int sub = threadIdx.x % TPR;
+  // all threads of a warp run the same number of rounds: the row's lanes are reduced with full-warp shuffles
+  const long long per_round = static_cast<long long>(gridDim.x) * (256 / TPR);
+  for (long long base = static_cast<long long>(blockIdx.x) * (256 / TPR); base < rows; base += per_round) {
+    const long long row = base + threadIdx.x / TPR;
+    const long long h = row % H, bs = row / H, s = bs % Sp, bb = bs / Sp;
+    const bool live = row < rows && s < S;
     float acc = 0.f;
-    for (int i = lane; i < D / 2; i += 32) {
-      const float2 x = __bfloat1622float2(a[i]), y = __bfloat1622float2(c[i]);
-      acc += x.x * y.x + x.y * y.y;
+    if (live) {
+      const size_t off = (static_cast<size_t>(bb * S + s) * H + h) * HD + sub * 8;
+      const uint4 a = *reinterpret_cast<const uint4*>(o + off), c = *reinterpret_cast<const uint4*>(d_o + off);
+      const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
+      const __nv_bfloat162* c2 = reinterpret_cast<const __nv_bfloat162*>(&c);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(c2[i]);
+        acc += x.x * y.x + x.y * y.y;
+      }
     }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (lane == 0) {
-      const long long h = row % H, bs = row / H, s = bs % S, bb = bs / S;
-      delta[(bb * H + h) * S + s] = acc;
+    for (int off = TPR / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (sub == 0 && row < rows) {
+      const size_t dst = static_cast<size_t>(bb * H + h) * Sp + s;
+      neg_delta[dst] = -acc;
+      neg_lse2[dst] = live ? -lse[static_cast<size_t>(bb * H + h) * S + s] * 1.4426950408889634f : -INFINITY;
     }
   }
 }
@@ -80,10 +111,31 @@ struct DqSmem {
 
 // Work item k of this CTA: query tiles sorted by decreasing length (tile i walks i + 1 key tiles), dealt to the
 // persistent CTAs in a snake.
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      : : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
+// 32 accumulator columns x `scale` -> 32 consecutive bf16 values
+__device__ __forceinline__ void fs_store32(__nv_bfloat16* dst, const uint32_t (&v)[32], float scale) {
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    uint32_t wv[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      wv[i] = fs_pack(make_float2(__uint_as_float(v[t * 8 + 2 * i]) * scale, __uint_as_float(v[t * 8 + 2 * i + 1]) * scale));
+    *reinterpret_cast<uint4*>(dst + t * 8) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+  }
+}
+
 struct DqItem { int i, head, b; };
 __device__ __forceinline__ bool dq_item(const FaSplitParams& p, int k, DqItem& w) {
   const int G = gridDim.x, c = blockIdx.x;
-  const int heads = p.G * p.qpk, bh = p.B * heads, nq = p.S / 128;
+  const int heads = p.G * p.qpk, bh = p.B * heads, nq = p.Sp / 128;
   const int idx = k * G + ((k & 1) ? G - 1 - c : c);
   if (idx >= bh * nq) return false;
   w.i = nq - 1 - idx / bh;
@@ -121,7 +173,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     mbar_init(q_full, 1); mbar_init(q_empty, 1);
     for (int i = 0; i < 3; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 2); }   // released by both MMA warps
     for (int i = 0; i < 2; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
-    mbar_init(sdp_full, 1); mbar_init(sdp_free, 8); mbar_init(ds_full, 8); mbar_init(dq_done, 1);
+    mbar_init(sdp_full, 1); mbar_init(sdp_free, FS_SOFTMAX_WARPS); mbar_init(ds_full, FS_SOFTMAX_WARPS); mbar_init(dq_done, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -135,7 +187,7 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
   const uint32_t tm_s = tmem_base, tm_dp = tmem_base + 128, tm_ds = tmem_base + 256, tm_dq = tmem_base + 384;
 
   if (warp < 4) {
-   asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+   asm volatile(FS_REGS_CONTROL);
    if (warp == 0) {
     if (elect_one()) {
       bool ok = true;
@@ -146,28 +198,28 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
         const int col_q = (g * (p.qpk + 2) + jq) * HD;
         const int col_k = (g * (p.qpk + 2) + p.qpk) * HD;
         const int col_v = col_k + HD;
-        const int row0 = w.b * p.S + w.i * 128;
+        const int row0 = w.i * 128;
         if (!mbar_wait(q_empty, (it & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
         mbar_expect_tx(q_full, 2 * S_::TILE);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c) {
-          tma_load_2d(smem + S_::Q_OFF + c * 16384, &tmQKV, q_full, col_q + 64 * c, row0);
-          tma_load_2d(smem + S_::DO_OFF + c * 16384, &tmDO, q_full, w.head * HD + 64 * c, row0);
+          tma_load_3d(smem + S_::Q_OFF + c * 16384, &tmQKV, q_full, col_q + 64 * c, row0, w.b);
+          tma_load_3d(smem + S_::DO_OFF + c * 16384, &tmDO, q_full, w.head * HD + 64 * c, row0, w.b);
         }
         for (int j = 0; j <= w.i && ok; ++j, ++kvc) {
           const int st = kvc % 3;
           const uint32_t ph = (kvc / 3) & 1;
-          const int krow = w.b * p.S + j * 128;
+          const int krow = j * 128;
           if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag, timeout)) { ok = false; break; }
           mbar_expect_tx(&k_full[st], S_::TILE);
 #pragma unroll
           for (int c = 0; c < HD / 64; ++c)
-            tma_load_2d(smem + S_::K_OFF + st * S_::TILE + c * 16384, &tmQKV, &k_full[st], col_k + 64 * c, krow);
+            tma_load_3d(smem + S_::K_OFF + st * S_::TILE + c * 16384, &tmQKV, &k_full[st], col_k + 64 * c, krow, w.b);
           if (!mbar_wait(&v_empty[kvc & 1], ((kvc >> 1) & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
           mbar_expect_tx(&v_full[kvc & 1], S_::TILE);
 #pragma unroll
           for (int c = 0; c < HD / 64; ++c)
-            tma_load_2d(smem + S_::V_OFF + (kvc & 1) * S_::TILE + c * 16384, &tmQKV, &v_full[kvc & 1], col_v + 64 * c, krow);
+            tma_load_3d(smem + S_::V_OFF + (kvc & 1) * S_::TILE + c * 16384, &tmQKV, &v_full[kvc & 1], col_v + 64 * c, krow, w.b);
         }
       }
       if (!ok) {
@@ -263,12 +315,13 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     }
    }
   } else {
-    // ------------------------------------------------------------------ P, dS: thread = (query row, key half)
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    // ------------------------------------------------------------------ P, dS: thread = (query row, quarter of the keys)
+    asm volatile(FS_REGS_SOFTMAX);
     const int q4 = warp & 3;
-    const int half = (warp - 4) >> 2;
+    const int quarter = (warp - 4) >> 2;
     const int r = q4 * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
+    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     bool ok = true;
     uint32_t c = 0;
     const bool probe = AXB_DBG(p, 4) && blockIdx.x == 0 && warp == 4 && lane == 0;
@@ -276,44 +329,41 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
     DqItem w;
     for (int it = 0; ok && dq_item(p, it, w); ++it) {
       const int n = w.i + 1;
-      const size_t srow = static_cast<size_t>(w.i) * 128 + r;
-      const float lse2 = p.lse[(static_cast<size_t>(w.b) * heads + w.head) * p.S + srow] * 1.4426950408889634f;
-      const float dl = p.delta[(static_cast<size_t>(w.b) * heads + w.head) * p.S + srow];
+      const int srow = w.i * 128 + r;
+      const size_t vec = (static_cast<size_t>(w.b) * heads + w.head) * p.Sp + srow;
+      const float nl = p.neg_lse2[vec], nd = p.neg_delta[vec];
+      const float2 nl2 = make_float2(nl, nl), nd2 = make_float2(nd, nd);
       for (int j = 0; j < n; ++j, ++c) {
         if (probe) p_mark = clock64();
         if (!mbar_wait(sdp_full, c & 1, abort_flag, timeout)) { ok = false; break; }
         if (probe) { const long long now = clock64(); pw_s += now - p_mark; p_mark = now; }
         tcgen05_fence_after();
-        uint32_t sv[64], dv[64];
-        tmem_ld_32x32(tm_s + lane_base + half * 64, *reinterpret_cast<uint32_t(*)[32]>(&sv[0]));
-        tmem_ld_32x32(tm_s + lane_base + half * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&sv[32]));
-        tmem_ld_32x32(tm_dp + lane_base + half * 64, *reinterpret_cast<uint32_t(*)[32]>(&dv[0]));
-        tmem_ld_32x32(tm_dp + lane_base + half * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&dv[32]));
+        uint32_t sv[32], dv[32];
+        tmem_ld_32x32(tm_s + lane_base + quarter * 32, sv);
+        tmem_ld_32x32(tm_dp + lane_base + quarter * 32, dv);
         tmem_ld_wait();
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(sdp_free);          // the MMA warp may issue the next tile's S and dP
         if (probe) { const long long now = clock64(); pt_ld += now - p_mark; p_mark = now; }
-        const bool diag = (j == w.i);
-        uint32_t packed[32];
+        if (j == w.i) {                                // keys to the right of the query: probability 0
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float p0 = exp2f(fmaf(__uint_as_float(sv[2 * i]), p.scale_log2, -lse2));
-          float p1 = exp2f(fmaf(__uint_as_float(sv[2 * i + 1]), p.scale_log2, -lse2));
-          if (diag) {
-            if (half * 64 + 2 * i > r) p0 = 0.f;
-            if (half * 64 + 2 * i + 1 > r) p1 = 0.f;
-          }
-          const float d0 = p0 * (__uint_as_float(dv[2 * i]) - dl) * p.scale;
-          const float d1 = p1 * (__uint_as_float(dv[2 * i + 1]) - dl) * p.scale;
-          const __nv_bfloat162 h = __floats2bfloat162_rn(d0, d1);
-          packed[i] = *reinterpret_cast<const uint32_t*>(&h);
+          for (int i = 0; i < 32; ++i)
+            if (quarter * 32 + i > r) sv[i] = 0xff800000u;
+        }
+        // dS = P (dP - delta); the softmax scale is applied once to the finished dQ and dK
+        uint32_t packed[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), sc2, nl2);
+          const float2 t = __fadd2_rn(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), nd2);
+          packed[i] = fs_pack(__fmul2_rn(make_float2(exp2f(x.x), exp2f(x.y)), t));
         }
         // the previous step's dQ MMA (of this or of the previous item) has read its dS: every phase is observed
         if (probe) { const long long now = clock64(); pt_cmp += now - p_mark; p_mark = now; }
         if (c >= 1 && !mbar_wait(dq_done, (c - 1) & 1, abort_flag, timeout)) { ok = false; break; }
         if (probe) { const long long now = clock64(); pw_dq += now - p_mark; p_mark = now; }
-        tmem_st_32x32(tm_ds + lane_base + half * 32, packed);
+        tmem_st_32x16(tm_ds + lane_base + quarter * 16, packed);
         tmem_st_wait();
         tcgen05_fence_before();
         __syncwarp();
@@ -322,24 +372,15 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
       }
       if (!ok || !mbar_wait(dq_done, (c - 1) & 1, abort_flag, timeout)) { ok = false; break; }
       tcgen05_fence_after();
-      // dQ row r, columns [half * HD/2, +HD/2) -> packed gradient tensor, query slot of this head
+      // dQ row r, 32 columns per quarter -> packed gradient tensor, query slot of this head
       const int g = w.head / p.qpk, jq = w.head % p.qpk;
-      const size_t pos = static_cast<size_t>(w.b) * p.S + srow;
-      __nv_bfloat16* dst = p.dqkv + ((pos * p.G + g) * (p.qpk + 2) + jq) * HD + half * (HD / 2);
-#pragma unroll
-      for (int cc = 0; cc < HD / 64; ++cc) {
+      if (quarter < HD / 32) {
         uint32_t v[32];
-        tmem_ld_32x32(tm_dq + lane_base + half * (HD / 2) + cc * 32, v);
+        tmem_ld_32x32(tm_dq + lane_base + quarter * 32, v);
         tmem_ld_wait();
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          uint32_t wv[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[t * 8 + 2 * i]), __uint_as_float(v[t * 8 + 2 * i + 1]));
-            wv[i] = *reinterpret_cast<const uint32_t*>(&h);
-          }
-          *reinterpret_cast<uint4*>(dst + cc * 32 + t * 8) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+        if (srow < p.S) {
+          const size_t pos = static_cast<size_t>(w.b) * p.S + srow;
+          fs_store32(p.dqkv + ((pos * p.G + g) * (p.qpk + 2) + jq) * HD + quarter * 32, v, p.scale);
         }
       }
       // the next item's first dQ MMA overwrites these columns; it waits for ds_full, which this thread arrives on
@@ -367,7 +408,7 @@ static int dq_launch(const CUtensorMap& tq, const CUtensorMap& td, const FaSplit
     AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S_::TOTAL));
     configured[device & 63] = true;
   }
-  const long long items = static_cast<long long>(p.B) * p.G * p.qpk * (p.S / 128);
+  const long long items = static_cast<long long>(p.B) * p.G * p.qpk * (p.Sp / 128);
   const int sms = sm_count(device);
   kern<<<static_cast<int>(items < sms ? items : sms), FS_THREADS, S_::TOTAL, s>>>(tq, td, p);
   AXB_CUDA(cudaGetLastError());
@@ -383,7 +424,7 @@ struct DkvSmem {
   static constexpr int DO_OFF = 4 * TILE;          // 2 stages
   static constexpr int LSE_OFF = 6 * TILE;         // [2 stages][lse, delta][128] fp32
   static constexpr int BAR_OFF = LSE_OFF + 2048;
-  static constexpr int NBARS = 2 + 4 + 2 + 2 + 1;
+  static constexpr int NBARS = 2 + 4 + 2 + 2 + 2;
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 16 + 1024;
 };
 
@@ -392,7 +433,7 @@ struct DkvSmem {
 struct DkvItem { int jt, g, b; };
 __device__ __forceinline__ bool dkv_item(const FaSplitParams& p, int k, DkvItem& w) {
   const int G = gridDim.x, c = blockIdx.x;
-  const int bg = p.B * p.G, nq = p.S / 128;
+  const int bg = p.B * p.G, nq = p.Sp / 128;
   const int idx = k * G + ((k & 1) ? G - 1 - c : c);
   if (idx >= bg * nq) return false;
   w.jt = idx / bg;
@@ -400,15 +441,6 @@ __device__ __forceinline__ bool dkv_item(const FaSplitParams& p, int k, DkvItem&
   w.g = rem % p.G;
   w.b = rem / p.G;
   return true;
-}
-
-__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-      : : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
 }
 
 // global -> shared bulk copy (16-byte aligned, size a multiple of 16) that completes on an mbarrier
@@ -427,22 +459,24 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
   uint64_t* kv_full = bars;          // K and V of the item
   uint64_t* kv_empty = bars + 1;     // both MMA warps are done with them
   uint64_t* qdo_full = bars + 2;     // [stage]: Q, dO, lse, delta of a query tile
-  uint64_t* qdo_empty = bars + 4;    // [stage]: 2 MMA warps + 8 softmax warps
+  uint64_t* qdo_empty = bars + 4;    // [stage]: 2 MMA warps + 16 softmax warps
   uint64_t* sdp_full = bars + 6;     // [score buffer]: S^T and dP^T of a step (one arrival per MMA warp)
   uint64_t* pds_full = bars + 8;     // [score buffer]: P^T and dS^T of a step are in tensor memory
   uint64_t* acc_done = bars + 10;    // dK and dV of the item are final (one arrival per MMA warp)
+  uint64_t* acc_free = bars + 11;    // ... and have been read: the next item may overwrite them
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + S_::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   float* lse_s = reinterpret_cast<float*>(smem + S_::LSE_OFF);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint64_t timeout = p.timeout_ns;
-  const int heads = p.G * p.qpk, nq = p.S / 128;
+  const int heads = p.G * p.qpk, nq = p.Sp / 128;
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1); mbar_init(kv_empty, 2); mbar_init(acc_done, 2);
+    mbar_init(acc_free, FS_SOFTMAX_WARPS);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 10);
+      mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 2 + FS_SOFTMAX_WARPS);
       mbar_init(&sdp_full[i], 2); mbar_init(&pds_full[i], 8);
     }
     *abort_flag = 0;
@@ -458,7 +492,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
   // [0,32) in its columns [0,16), of queries [32,64) in [32,48)), dK [256,256+HD), dV [384,384+HD)
 
   if (warp < 4) {
-   asm volatile("setmaxnreg.dec.sync.aligned.u32 96;");
+   asm volatile(FS_REGS_CONTROL);
    if (warp == 0) {
     if (elect_one()) {
       bool ok = true;
@@ -466,31 +500,31 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
       DkvItem w;
       for (int it = 0; ok && dkv_item(p, it, w); ++it) {
         const int col_k = (w.g * (p.qpk + 2) + p.qpk) * HD;
-        const int krow = w.b * p.S + w.jt * 128;
+        const int krow = w.jt * 128;
         if (!mbar_wait(kv_empty, (it & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
         mbar_expect_tx(kv_full, 2 * S_::TILE);
 #pragma unroll
         for (int c = 0; c < HD / 64; ++c) {
-          tma_load_2d(smem + S_::K_OFF + c * 16384, &tmQKV, kv_full, col_k + 64 * c, krow);
-          tma_load_2d(smem + S_::V_OFF + c * 16384, &tmQKV, kv_full, col_k + HD + 64 * c, krow);
+          tma_load_3d(smem + S_::K_OFF + c * 16384, &tmQKV, kv_full, col_k + 64 * c, krow, w.b);
+          tma_load_3d(smem + S_::V_OFF + c * 16384, &tmQKV, kv_full, col_k + HD + 64 * c, krow, w.b);
         }
         const int per_head = nq - w.jt;
         for (int t = 0; t < per_head * p.qpk && ok; ++t, ++tq) {
           const int jq = t / per_head, i = w.jt + t % per_head;
           const int head = w.g * p.qpk + jq;
           const int st = tq & 1;
-          const int row0 = w.b * p.S + i * 128;
+          const int row0 = i * 128;
           if (!mbar_wait(&qdo_empty[st], ((tq >> 1) & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
           mbar_expect_tx(&qdo_full[st], 2 * S_::TILE + 1024);
 #pragma unroll
           for (int c = 0; c < HD / 64; ++c) {
-            tma_load_2d(smem + S_::Q_OFF + st * S_::TILE + c * 16384, &tmQKV, &qdo_full[st],
-                        (w.g * (p.qpk + 2) + jq) * HD + 64 * c, row0);
-            tma_load_2d(smem + S_::DO_OFF + st * S_::TILE + c * 16384, &tmDO, &qdo_full[st], head * HD + 64 * c, row0);
+            tma_load_3d(smem + S_::Q_OFF + st * S_::TILE + c * 16384, &tmQKV, &qdo_full[st],
+                        (w.g * (p.qpk + 2) + jq) * HD + 64 * c, row0, w.b);
+            tma_load_3d(smem + S_::DO_OFF + st * S_::TILE + c * 16384, &tmDO, &qdo_full[st], head * HD + 64 * c, row0, w.b);
           }
-          const size_t vec = (static_cast<size_t>(w.b) * heads + head) * p.S + static_cast<size_t>(i) * 128;
-          bulk_load_1d(lse_s + st * 256, p.lse + vec, 512, &qdo_full[st]);
-          bulk_load_1d(lse_s + st * 256 + 128, p.delta + vec, 512, &qdo_full[st]);
+          const size_t vec = (static_cast<size_t>(w.b) * heads + head) * p.Sp + static_cast<size_t>(i) * 128;
+          bulk_load_1d(lse_s + st * 256, p.neg_lse2 + vec, 512, &qdo_full[st]);
+          bulk_load_1d(lse_s + st * 256 + 128, p.neg_delta + vec, 512, &qdo_full[st]);
         }
       }
       if (!ok) {
@@ -543,6 +577,8 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
           const uint32_t tile = tq + (s >> 1);
           const int hq = s & 1;
           if (!mbar_wait(&pds_full[hq], (c >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
+          // the warps of either score buffer read dK / dV of the previous item; only those of buffer 0 are known to be done
+          if (s == 0 && it > 0 && !mbar_wait(acc_free, (it - 1) & 1, abort_flag, timeout)) { ok = false; break; }
           tcgen05_fence_after();
           issue_acc(tile & 1, hq, s == 0);
           if (hq == 1) umma_commit(&qdo_empty[tile & 1]);        // this warp's last read of the tile
@@ -563,89 +599,85 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
    }
   } else {
     // ------------------------------------------------------------------ P^T, dS^T: thread = (key row, 32 of the step's 64 queries)
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 200;");
+    // Warps 4-11 take the steps of score buffer 0 (first 64 queries of every tile), warps 12-19 those of buffer 1.
+    asm volatile(FS_REGS_SOFTMAX);
     const int q4 = warp & 3;
-    const int half = (warp - 4) >> 2;
+    const int hq = (warp - 4) >> 3;
+    const int half = ((warp - 4) >> 2) & 1;
     const int r = q4 * 32 + lane;                     // key row inside the tile
     const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
+    const uint32_t t_s = tmem_base + lane_base + hq * 64 + half * 32, t_dp = t_s + 128;
+    const int qc0 = hq * 64 + half * 32;              // first query column of this thread inside the tile
+    const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     bool ok = true;
-    uint32_t tq = 0, c = 0;
+    uint32_t tq = 0;                                  // query tiles so far: this buffer's steps, ring stage and phases
     DkvItem w;
     for (int it = 0; ok && dkv_item(p, it, w); ++it) {
       const int per_head = nq - w.jt;
-      const int ns = 2 * per_head * p.qpk;
-      for (int s = 0; s < ns; ++s, ++c) {
-        const uint32_t tile = tq + (s >> 1);
-        const int hq = s & 1, st = tile & 1;
-        const int i = w.jt + (s >> 1) % per_head;
-        // lse / delta of the tile arrive with its Q and dO
-        if (hq == 0 && !mbar_wait(&qdo_full[st], (tile >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
-        if (!mbar_wait(&sdp_full[hq], (c >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
+      const int nt = per_head * p.qpk;
+      for (int t = 0; t < nt; ++t, ++tq) {
+        const int st = tq & 1;
+        const bool diag = t % per_head == 0;
+        // -lse and -delta of the tile arrive with its Q and dO
+        if (!mbar_wait(&qdo_full[st], (tq >> 1) & 1, abort_flag, timeout) ||
+            !mbar_wait(&sdp_full[hq], tq & 1, abort_flag, timeout)) { ok = false; break; }
         tcgen05_fence_after();
         uint32_t sv[32], dv[32];
-        tmem_ld_32x32(tmem_base + lane_base + hq * 64 + half * 32, sv);
-        tmem_ld_32x32(tmem_base + lane_base + 128 + hq * 64 + half * 32, dv);
+        tmem_ld_32x32(t_s, sv);
+        tmem_ld_32x32(t_dp, dv);
         tmem_ld_wait();
-        const int qc0 = hq * 64 + half * 32;           // first query column of this thread inside the tile
         const float4* lv = reinterpret_cast<const float4*>(lse_s + st * 256 + qc0);
         const float4* dvv = reinterpret_cast<const float4*>(lse_s + st * 256 + 128 + qc0);
-        const bool diag = (i == w.jt);
+        if (diag) {                                   // the key lies after the query: probability 0
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (r > qc0 + i) sv[i] = 0xff800000u;
+        }
         uint32_t pp[16], pd[16];
 #pragma unroll
         for (int v4 = 0; v4 < 8; ++v4) {
           const float4 l4 = lv[v4], d4 = dvv[v4];
-          const float ls[4] = {l4.x, l4.y, l4.z, l4.w}, ds[4] = {d4.x, d4.y, d4.z, d4.w};
-          float pr[4], dsr[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int col = v4 * 4 + e;
-            float pv = exp2f(fmaf(__uint_as_float(sv[col]), p.scale_log2, -ls[e] * 1.4426950408889634f));
-            if (diag && r > qc0 + col) pv = 0.f;        // the key lies after the query
-            pr[e] = pv;
-            dsr[e] = pv * (__uint_as_float(dv[col]) - ds[e]) * p.scale;
+          for (int e = 0; e < 2; ++e) {
+            const int i = v4 * 2 + e;
+            const float2 nl2 = e ? make_float2(l4.z, l4.w) : make_float2(l4.x, l4.y);
+            const float2 nd2 = e ? make_float2(d4.z, d4.w) : make_float2(d4.x, d4.y);
+            const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), sc2, nl2);
+            const float2 pr = make_float2(exp2f(x.x), exp2f(x.y));
+            const float2 t2 = __fadd2_rn(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), nd2);
+            pp[i] = fs_pack(pr);
+            pd[i] = fs_pack(__fmul2_rn(pr, t2));      // the softmax scale is applied to the finished dK
           }
-          const __nv_bfloat162 a0 = __floats2bfloat162_rn(pr[0], pr[1]), a1 = __floats2bfloat162_rn(pr[2], pr[3]);
-          const __nv_bfloat162 b0 = __floats2bfloat162_rn(dsr[0], dsr[1]), b1 = __floats2bfloat162_rn(dsr[2], dsr[3]);
-          pp[v4 * 2] = *reinterpret_cast<const uint32_t*>(&a0); pp[v4 * 2 + 1] = *reinterpret_cast<const uint32_t*>(&a1);
-          pd[v4 * 2] = *reinterpret_cast<const uint32_t*>(&b0); pd[v4 * 2 + 1] = *reinterpret_cast<const uint32_t*>(&b1);
         }
         // into this thread's own score columns: the other half's thread of the row may not have read its scores yet
-        tmem_st_32x16(tmem_base + lane_base + hq * 64 + half * 32, pp);
-        tmem_st_32x16(tmem_base + lane_base + 128 + hq * 64 + half * 32, pd);
+        tmem_st_32x16(t_s, pp);
+        tmem_st_32x16(t_dp, pd);
         tmem_st_wait();
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(&pds_full[hq]);
-          if (hq == 1) mbar_arrive(&qdo_empty[st]);      // lse / delta of the tile have been read
+          mbar_arrive(&qdo_empty[st]);                // this warp has read its share of -lse / -delta
         }
       }
       if (!ok || !mbar_wait(acc_done, it & 1, abort_flag, timeout)) { ok = false; break; }
       tcgen05_fence_after();
-      // half 0 stores dK row r, half 1 stores dV row r into the key / value slots of the packed gradient tensor
-      const size_t kvpos = static_cast<size_t>(w.b) * p.S + w.jt * 128 + r;
+      // half 0 stores dK row r, half 1 stores dV row r into the key / value slots of the packed gradient tensor; the
+      // warps of buffer 0 take the even, those of buffer 1 the odd 32-column blocks
+      const int krow = w.jt * 128 + r;
+      const size_t kvpos = static_cast<size_t>(w.b) * p.S + krow;
       __nv_bfloat16* dst = p.dqkv + ((kvpos * p.G + w.g) * (p.qpk + 2) + p.qpk + half) * HD;
       const uint32_t src = tmem_base + lane_base + (half ? 384 : 256);
 #pragma unroll
-      for (int cc = 0; cc < HD / 32; ++cc) {
+      for (int cc = hq; cc < HD / 32; cc += 2) {
         uint32_t v[32];
         tmem_ld_32x32(src + cc * 32, v);
         tmem_ld_wait();
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          uint32_t wv[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[t * 8 + 2 * e]), __uint_as_float(v[t * 8 + 2 * e + 1]));
-            wv[e] = *reinterpret_cast<const uint32_t*>(&h);
-          }
-          *reinterpret_cast<uint4*>(dst + cc * 32 + t * 8) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-        }
+        if (krow < p.S) fs_store32(dst + cc * 32, v, half ? 1.f : p.scale);
       }
-      // the next item's first accumulator MMAs overwrite dK / dV; they wait for pds_full, on which this thread
-      // arrives after these reads
       tcgen05_fence_before();
-      tq += ns >> 1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_free);
     }
     if (!ok && lane == 0) report_status(p.status, 0x433u);
   }
@@ -663,7 +695,7 @@ static int dkv_launch(const CUtensorMap& tq, const CUtensorMap& td, const FaSpli
     AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S_::TOTAL));
     configured[device & 63] = true;
   }
-  const long long items = static_cast<long long>(p.B) * p.G * (p.S / 128);
+  const long long items = static_cast<long long>(p.B) * p.G * (p.Sp / 128);
   const int sms = sm_count(device);
   kern<<<static_cast<int>(items < sms ? items : sms), FS_THREADS, S_::TOTAL, s>>>(tq, td, p);
   AXB_CUDA(cudaGetLastError());
@@ -672,28 +704,44 @@ static int dkv_launch(const CUtensorMap& tq, const CUtensorMap& td, const FaSpli
 
 }  // namespace axb
 
+// fp32 words of scratch that axb_flash_attn_bwd_split needs: -lse and -delta of every query row, rows padded to 128
+extern "C" long long axb_flash_attn_bwd_scratch(int B, int S, int heads) {
+  return 2ll * B * heads * ((static_cast<long long>(S) + 127) / 128 * 128);
+}
+
 // which: bit 0 = dQ kernel (writes the query slots of dqkv), bit 1 = dK / dV kernel (writes the key and value slots).
-// qkv [B,S,G,qpk+2,D], out / d_out [B,S,G*qpk,D] bf16; lse [B,G*qpk,S]; delta [B,G*qpk,S] fp32 scratch.
+// qkv [B,S,G,qpk+2,D], out / d_out [B,S,G*qpk,D] bf16; lse [B,G*qpk,S]; scratch: axb_flash_attn_bwd_scratch fp32 words.
 extern "C" int axb_flash_attn_bwd_split(const void* qkv, const void* out, const void* d_out, const float* lse,
-                                        float* delta, void* dqkv, int B, int S, int G, int qpk, int D, float scale,
+                                        float* scratch, void* dqkv, int B, int S, int G, int qpk, int D, float scale,
                                         int which, int device, void* stream) {
   using namespace axb;
   if (D != 64 && D != 128) { set_error("flash attention: head_dim must be 64 or 128"); return -1; }
-  if (S % 128) { set_error("flash attention: sequence length must be a multiple of 128"); return -1; }
+  if (B <= 0 || S <= 0 || G <= 0 || qpk <= 0) { set_error("flash attention: empty problem"); return -1; }
+  if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(d_out) | reinterpret_cast<uintptr_t>(dqkv) |
+       reinterpret_cast<uintptr_t>(scratch)) & 15) {
+    set_error("flash attention: tensors must be 16-byte aligned");
+    return -1;
+  }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int H = G * qpk;
-  const long long rows = static_cast<long long>(B) * S * H;
-  const long long cap = static_cast<long long>(sm_count(device)) * 16;
-  const int blocks = static_cast<int>(rows / 8 < cap ? (rows / 8 < 1 ? 1 : rows / 8) : cap);
-  fa_split_delta_kernel<<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out),
-                                               static_cast<const __nv_bfloat16*>(d_out), delta, B, S, H, D);
+  const int H = G * qpk, Sp = (S + 127) / 128 * 128;
+  // a launch through the runtime comes before the first driver call: on a thread that autograd has just started it is
+  // what binds the device's context
+  const long long row_blocks = (static_cast<long long>(B) * Sp * H + 256 / (D / 8) - 1) / (256 / (D / 8));
+  const long long cap = static_cast<long long>(sm_count(device)) * 8;
+  const int blocks = static_cast<int>(row_blocks < cap ? row_blocks : cap);
+  if (D == 128)
+    fa_split_delta_kernel<128><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out),
+                                                      lse, scratch, scratch + static_cast<size_t>(B) * H * Sp, B, S, Sp, H);
+  else
+    fa_split_delta_kernel<64><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out),
+                                                     lse, scratch, scratch + static_cast<size_t>(B) * H * Sp, B, S, Sp, H);
   AXB_CUDA(cudaGetLastError());
   CUtensorMap tq, td;
-  if (make_tmap_2d_16bit(&tq, qkv, static_cast<uint64_t>(B) * S, static_cast<uint64_t>(G) * (qpk + 2) * D, 128, 0)) return -1;
-  if (make_tmap_2d_16bit(&td, d_out, static_cast<uint64_t>(B) * S, static_cast<uint64_t>(H) * D, 128, 0)) return -1;
+  if (make_tmap_3d_bf16(&tq, qkv, B, S, static_cast<uint64_t>(G) * (qpk + 2) * D, 128)) return -1;
+  if (make_tmap_3d_bf16(&td, d_out, B, S, static_cast<uint64_t>(H) * D, 128)) return -1;
   FaSplitParams p;
-  p.lse = lse; p.delta = delta; p.dqkv = static_cast<__nv_bfloat16*>(dqkv);
-  p.B = B; p.S = S; p.G = G; p.qpk = qpk; p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
+  p.neg_lse2 = scratch; p.neg_delta = scratch + static_cast<size_t>(B) * H * Sp; p.dqkv = static_cast<__nv_bfloat16*>(dqkv);
+  p.B = B; p.S = S; p.Sp = Sp; p.G = G; p.qpk = qpk; p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   unsigned int* st = nullptr;
   if (!device_status_word(device, &st)) { set_error("flash attention: no status word"); return -1; }
   p.status = st; p.timeout_ns = wait_timeout_ns();

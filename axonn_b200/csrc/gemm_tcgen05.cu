@@ -1367,6 +1367,24 @@ int make_tmap_2d_16bit(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_
   return 0;
 }
 
+// [batch, rows, cols] bf16, contiguous; box = 1 x box_rows x 64 columns, 128 B swizzle.  Rows past `rows` of a batch
+// element are outside the tensor and read as zeros (a flat 2-D map would read the next element's rows).
+int make_tmap_3d_bf16(CUtensorMap* out, const void* ptr, uint64_t batch, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  EncodeTiledFn enc = get_encode_fn();
+  if (!enc) { set_error("cuTensorMapEncodeTiled entry point not available"); return -1; }
+  if ((reinterpret_cast<uintptr_t>(ptr) & 15) != 0) { set_error("TMA base address must be 16-byte aligned"); return -1; }
+  if ((cols * 2) % 16 != 0) { set_error("TMA row pitch must be a multiple of 16 bytes (cols=%llu)", (unsigned long long)cols); return -1; }
+  cuuint64_t gdim[3] = {cols, rows, batch};
+  cuuint64_t gstride[2] = {cols * 2, rows * cols * 2};
+  cuuint32_t box[3] = {64, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), gdim, gstride, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (3-D) failed with CUresult %d", (int)r); return -1; }
+  return 0;
+}
+
 // Row-major fp32 [rows, cols] with 32 x `box_rows` boxes (128-byte rows, 128-byte swizzle): destination of
 // bulk tensor reductions.
 int make_tmap_2d_f32(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {

@@ -28,7 +28,7 @@ def _sdpa(q, k, v, causal, scale):
 
 def flash_attention(q, k, v, causal=True, scale=None):
     """Attention of ``q [B, S, heads, D]`` against ``k, v [B, S, kv_heads, D]`` (grouped-query when ``kv_heads <
-    heads``) on the package's tcgen05 kernels (CUDA, D 64 or 128, S a multiple of 128) or through
+    heads``) on the package's tcgen05 kernels (CUDA bf16, D 64 or 128, any S) or through
     ``scaled_dot_product_attention`` otherwise; returns ``[B, S, heads, D]``."""
     if scale is None:
         scale = 1.0 / math.sqrt(q.shape[-1])

@@ -8,10 +8,11 @@ import ctypes
 import os
 
 import torch
+from torch.autograd.function import once_differentiable
 
 from . import _lib
 
-_BWD_DEFAULT = "fused"
+_BWD_DEFAULT = "split"
 
 
 def available():
@@ -19,8 +20,17 @@ def available():
 
 
 def supported(qkv):
+    """Whether the kernels take this packed tensor: bf16, head_dim 64 or 128, dense and 16-byte aligned, any sequence
+    length.  Traced, vmapped or subclassed tensors have no storage that a kernel could be given."""
     B, S, G, n, D = qkv.shape
-    return qkv.dtype == torch.bfloat16 and D in (64, 128) and S % 128 == 0 and qkv.is_contiguous()
+    if qkv.dtype != torch.bfloat16 or D not in (64, 128) or not qkv.is_contiguous() or qkv.numel() == 0 or n < 3:
+        return False
+    if S % 128:
+        if torch.compiler.is_compiling() or torch._C._functorch.peek_interpreter_stack() is not None:
+            return False
+        if type(qkv) not in (torch.Tensor, torch.nn.Parameter):
+            return False
+    return qkv.data_ptr() % 16 == 0
 
 
 def flash_fwd_packed(qkv, scale):
@@ -36,33 +46,39 @@ def flash_fwd_packed(qkv, scale):
     return out, lse
 
 
-def _bwd_split(qkv, out, d_out, lse, delta, dqkv, scale, which):
+def _bwd_split(qkv, out, d_out, lse, dqkv, scale, which):
     B, S, G, n, D = qkv.shape
-    st = _lib.lib().axb_flash_attn_bwd_split(
-        _lib.ptr(qkv), _lib.ptr(out), _lib.ptr(d_out), _lib.ptr(lse), _lib.ptr(delta), _lib.ptr(dqkv),
+    L = _lib.lib()
+    L.axb_flash_attn_bwd_scratch.restype = ctypes.c_longlong
+    words = L.axb_flash_attn_bwd_scratch(ctypes.c_int(B), ctypes.c_int(S), ctypes.c_int(G * (n - 2)))
+    scratch = torch.empty(words, dtype=torch.float32, device=qkv.device)
+    st = L.axb_flash_attn_bwd_split(
+        _lib.ptr(qkv), _lib.ptr(out), _lib.ptr(d_out), _lib.ptr(lse), _lib.ptr(scratch), _lib.ptr(dqkv),
         ctypes.c_int(B), ctypes.c_int(S), ctypes.c_int(G), ctypes.c_int(n - 2), ctypes.c_int(D),
         ctypes.c_float(scale), ctypes.c_int(which), ctypes.c_int(qkv.device.index), _lib.stream_ptr())
     _lib.check(st, "axb_flash_attn_bwd_split")
-    _lib.add_launches(1)
+    _lib.add_launches(1 if which != 3 else 2)
 
 
 def flash_bwd_packed(qkv, out, d_out, lse, scale):
     """Gradient of the packed QKV tensor for ``flash_fwd_packed``.
 
-    ``AXONN_FA_BWD`` selects the implementation: ``split`` - the two-kernel backward without atomics
+    ``AXONN_FA_BWD`` selects the implementation: ``split`` (default) - the two-kernel backward without atomics
     (``csrc/flash_attn_bwd_split.cu``: one kernel for dQ, one for dK and dV); ``fused`` - the one-kernel form
-    (``csrc/flash_attn.cu``) with its fp32 dQ accumulator; ``split_dq`` / ``split_dkv`` take only dQ or only
-    dK, dV from the two-kernel form (A/B runs)."""
+    (``csrc/flash_attn.cu``) with its fp32 dQ accumulator, for sequence lengths that are multiples of 128;
+    ``split_dq`` / ``split_dkv`` take only dQ or only dK, dV from the two-kernel form (A/B runs)."""
     B, S, G, n, D = qkv.shape
     qpk = n - 2
     H = G * qpk
     mode = os.environ.get("AXONN_FA_BWD", _BWD_DEFAULT)
     d_out = d_out if d_out.is_contiguous() else d_out.contiguous()
-    delta = torch.empty((B, H, S), dtype=torch.float32, device=qkv.device)
+    if d_out.data_ptr() % 16:
+        d_out = d_out.clone()
     dqkv = torch.empty_like(qkv)
-    if mode == "split":
-        _bwd_split(qkv, out, d_out, lse, delta, dqkv, scale, 3)
+    if mode == "split" or S % 128:
+        _bwd_split(qkv, out, d_out, lse, dqkv, scale, 3)
         return dqkv
+    delta = torch.empty((B, H, S), dtype=torch.float32, device=qkv.device)
     dq_acc = torch.zeros((B, S, H, D), dtype=torch.float32, device=qkv.device)
     st = _lib.lib().axb_flash_attn_bwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(d_out), _lib.ptr(lse), _lib.ptr(delta),
                                        _lib.ptr(dq_acc), _lib.ptr(dqkv), ctypes.c_int(B), ctypes.c_int(S),
@@ -72,9 +88,9 @@ def flash_bwd_packed(qkv, out, d_out, lse, scale):
     _lib.add_launches(1)
     dqkv[:, :, :, :qpk].copy_(dq_acc.view(B, S, G, qpk, D))
     if mode == "split_dq":
-        _bwd_split(qkv, out, d_out, lse, delta, dqkv, scale, 1)
+        _bwd_split(qkv, out, d_out, lse, dqkv, scale, 1)
     elif mode == "split_dkv":
-        _bwd_split(qkv, out, d_out, lse, delta, dqkv, scale, 2)
+        _bwd_split(qkv, out, d_out, lse, dqkv, scale, 2)
     return dqkv
 
 
@@ -87,6 +103,7 @@ class _FlashPacked(torch.autograd.Function):
         return out
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
         qkv, out, lse = ctx.saved_tensors
         return flash_bwd_packed(qkv, out, g, lse, ctx.scale), None

@@ -1,6 +1,8 @@
 """Edges of the kernels' tiles and of the rules that choose between them: remainders, the smallest and largest sizes of
 a range, against 64-bit (or integer) references."""
 
+import math
+
 import pytest
 import torch
 
@@ -50,3 +52,37 @@ def test_norm_backward_sizes(rows, H, rms, residual, dtype):
     tol = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10, torch.float32: 2e-5}[dtype]
     for a, w in zip(got, want):
         assert _rel(a, w) < tol, _rel(a, w)
+
+
+# ------------------------------------------------------------------------------------------------ attention, any length
+@pytest.mark.parametrize("B,S,G,qpk,D", [(1, 1, 1, 1, 64), (2, 5, 2, 1, 128), (3, 127, 1, 2, 64), (2, 129, 2, 2, 128),
+                                         (2, 255, 1, 4, 128), (1, 257, 2, 1, 64), (3, 300, 2, 2, 128), (2, 511, 1, 1, 128),
+                                         (2, 128, 2, 2, 64), (2, 384, 2, 1, 128), (1, 1531, 2, 4, 128)])
+def test_attention_any_length(B, S, G, qpk, D):
+    """Sequence ends inside either query tile of a pair, on a tile edge, and before the first one.  Rows of the next
+    batch element must not leak in: every element of the batch is compared.  Tolerance: probabilities and score
+    gradients are bf16 MMA operands, results are bf16 (a few 2^-9)."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib, attention_cuda
+
+    torch.manual_seed(S)
+    qkv = torch.randn(B, S, G, qpk + 2, D, device=DEV).bfloat16().requires_grad_(True)
+    dout = torch.randn(B, S, G * qpk, D, device=DEV).bfloat16()
+    assert attention_cuda.supported(qkv)
+    out = ops.flash_attention_packed(qkv)
+    (grad,) = torch.autograd.grad(out, qkv, dout)
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+    x = qkv.detach().double().requires_grad_(True)
+    q = x[:, :, :, :qpk]
+    s = torch.einsum("bsgqd,btgd->bgqst", q, x[:, :, :, qpk]) / math.sqrt(D)
+    s = s.masked_fill(torch.ones(S, S, device=DEV, dtype=torch.bool).triu(1), float("-inf"))
+    ref = torch.einsum("bgqst,btgd->bsgqd", s.softmax(-1), x[:, :, :, qpk + 1]).reshape(B, S, G * qpk, D)
+    (gref,) = torch.autograd.grad(ref, x, dout.double())
+    for bb in range(B):
+        assert _rel(out[bb], ref.detach()[bb]) < 1e-2
+        for sl in (slice(0, qpk), slice(qpk, qpk + 1), slice(qpk + 1, qpk + 2)):
+            want = gref[bb, :, :, sl]
+            err = float((grad[bb, :, :, sl].double() - want).norm())
+            # with one key the score gradients vanish: compare with the size of dV, the gradient that is left
+            assert err < 1.5e-2 * max(float(want.norm()), float(gref[bb].norm()) * 1e-2), (bb, sl, err)
