@@ -31,6 +31,7 @@
 // Every wait is bounded; on expiry the CTA raises an abort flag, records the
 // reason in the device status word, drains its TMA copies, frees TMEM and
 // returns.
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -1330,6 +1331,188 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 1) { tcgen05_fence_after(); tmem_dealloc_pair(tmem_base, 2 * BN); }
 }
 
+// ----------------------------------------------------------------------------- split-K GEMM on clusters
+// Plain GEMM for problems with too few 128x128 tiles to occupy the GPU (a short prompt through a wide layer, weight
+// gradients of narrow layers): a cluster of Z CTAs shares one output tile, CTA z multiplies its part of the K blocks
+// into its own TMEM accumulator, and the fp32 partials are summed through distributed shared memory - every CTA leaves
+// its partial in its (drained) operand ring and finishes 128 / Z columns of the tile from all Z of them, in rank order.
+// No workspace, no atomics, one launch.  Such a problem is bound by reading the weights once; with one CTA per tile
+// the loads of tiles < SMs / 2 CTAs in flight do not fill the memory system.
+// Measured on a B200 (graph replay, bias epilogue): 24 x 8192 x 2048 22.0 -> 12.4 us, 24 x 2048 x 8192 31.7 -> 10.7 us (33.5 MB
+// of weights each).
+constexpr int SK_THREADS = 192;   // TMA warp, MMA warp, 4 epilogue warps
+constexpr int SK_MAX_Z = 8;       // portable cluster size
+struct SplitKSmem {
+  static constexpr int BN = 128;
+  static constexpr int A_BYTES = BM * BK * 2;
+  static constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2;
+  static constexpr int STAGES = 6;
+  static constexpr int PART_LD = BN + 4;           // floats per partial row: 16-byte words of 8 rows hit all banks
+  static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
+  static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 1) * 8 + 16 + 1024 /* alignment slack */;
+  static_assert(BM * PART_LD * 4 <= BAR_OFFSET, "the partial tile lies in the operand ring");
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_smem_addr, uint32_t cta) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_smem_addr), "r"(cta));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+
+template <int A_MN, int B_MN>
+__global__ void __launch_bounds__(SK_THREADS, 1)
+gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p,
+                   int z_ctas) {
+  using S = SplitKSmem;
+  constexpr int BN = S::BN;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::BAR_OFFSET);
+  uint64_t* empty_bar = full_bar + S::STAGES;
+  uint64_t* acc_full = empty_bar + S::STAGES;
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(acc_full + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int z = static_cast<int>(cluster_cta_rank());
+  const int tile = blockIdx.x / z_ctas;
+  const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
+  const int num_kb = (p.K + BK - 1) / BK;
+  const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * z / z_ctas);
+  const int kb1 = static_cast<int>(static_cast<long long>(num_kb) * (z + 1) / z_ctas);
+  const uint64_t timeout = p.timeout_ns;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S::STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 0 && lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); }
+  if (warp == 1) { tmem_alloc(tmem_ptr_smem, BN); tmem_relinquish(); }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_ptr_smem;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int stage = 0; uint32_t phase = 0;
+      bool ok = true;
+      const int m0 = tm * BM, n0 = tn * BN;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, timeout)) { ok = false; break; }
+        uint8_t* sA = smem + stage * S::STAGE_BYTES;
+        uint8_t* sB = sA + S::A_BYTES;
+        mbar_expect_tx(&full_bar[stage], S::STAGE_BYTES);
+        const int k0 = kb * BK;
+        if (A_MN == 0) {
+          tma_load_2d(sA, &tmA, &full_bar[stage], k0, m0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < BM / 64; ++j) tma_load_2d(sA + j * (BK * 128), &tmA, &full_bar[stage], m0 + 64 * j, k0);
+        }
+        if (B_MN == 0) {
+          tma_load_2d(sB, &tmB, &full_bar[stage], k0, n0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j) tma_load_2d(sB + j * (BK * 128), &tmB, &full_bar[stage], n0 + 64 * j, k0);
+        }
+        if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (!ok) {
+        const uint64_t t0 = globaltimer_ns();     // give in-flight copies time to land before the CTA exits
+        while (globaltimer_ns() - t0 < 200000ull) {}
+        report_status(p.status, 0x151u);
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      const uint32_t idesc = umma_idesc(p.in_dtype == 0 ? 1 : 0, A_MN, B_MN, BM, BN);
+      const uint32_t a_lbo = A_MN ? BK * 128 : 16, a_kstep = A_MN ? UMMA_K * 128 : UMMA_K * 2;
+      const uint32_t b_lbo = B_MN ? BK * 128 : 16, b_kstep = B_MN ? UMMA_K * 128 : UMMA_K * 2;
+      int stage = 0; uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&full_bar[stage], phase, abort_flag, timeout)) { ok = false; break; }
+        tcgen05_fence_after();
+        const uint32_t a_addr = smem_u32(smem + stage * S::STAGE_BYTES), b_addr = a_addr + S::A_BYTES;
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          umma_f16(tmem_base, umma_smem_desc(a_addr + k * a_kstep, a_lbo, 1024), umma_smem_desc(b_addr + k * b_kstep, b_lbo, 1024),
+                   idesc, (kb == kb0 && k == 0) ? 0u : 1u);
+        umma_commit(&empty_bar[stage]);
+        if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (ok) umma_commit(acc_full);
+      else {
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 50000ull) {}   // let MMAs in flight finish before TMEM is released
+        report_status(p.status, 0x152u);
+      }
+    }
+  } else {
+    // the accumulator is complete: every MMA has read its operands, the ring now holds this CTA's partial tile
+    const int q = warp & 3;
+    const int row = q * 32 + lane;
+    if (!mbar_wait(acc_full, 0, abort_flag, timeout)) {
+      if (lane == 0) report_status(p.status, 0x154u);
+    } else {
+      tcgen05_fence_after();
+      if (tm * BM + q * 32 < p.M) {
+        float* part = reinterpret_cast<float*>(smem) + row * S::PART_LD;
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<uint4*>(part + c * 32 + i * 4) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+        }
+      }
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) { __syncwarp(); tcgen05_fence_after(); tmem_dealloc(tmem_base, BN); }
+  __syncwarp();
+  cluster_sync_all();                 // all partials of the tile are in shared memory
+  if (*abort_flag == 0) {
+    const int groups = BN / 8 / z_ctas;                       // 8-column groups finished by this CTA
+    const int rows = min(BM, p.M - tm * BM);
+    const uint32_t base = smem_u32(smem);
+    for (int u = threadIdx.x; u < rows * groups; u += SK_THREADS) {
+      const int row = u / groups, cg = z * groups + u % groups;
+      const int col = tn * BN + cg * 8;
+      if (col >= p.N) continue;                               // N is a multiple of 8
+      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int j = 0; j < z_ctas; ++j) {
+        const uint32_t addr = base + (row * S::PART_LD + cg * 8) * 4;
+        const float4 a = ld_cluster_f4(addr, j), b = ld_cluster_f4(addr + 16, j);
+        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+      }
+      if (p.epilogue == 1 || p.epilogue == 2) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          v[i] += (p.in_dtype == 0) ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[col + i])
+                                    : __half2float(reinterpret_cast<const __half*>(p.bias)[col + i]);
+      }
+      const size_t off = static_cast<size_t>(tm * BM + row) * p.N + col;
+      if (p.epilogue >= 2) {
+        if (p.aux != nullptr) store_vec8(p.aux, p.out_dtype, off, v, false);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = gelu_tanh(v[i]);
+      }
+      store_vec8(p.C, p.out_dtype, off, v, p.accumulate != 0);
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();                 // a CTA's partial stays valid until its peers have read it
+}
+
 // ----------------------------------------------------------------------------- host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1502,6 +1685,62 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParam
   return 0;
 }
 
+// Clusters of z split-K CTAs that the device holds at once (one CTA per SM; a cluster does not cross a GPC, so this is
+// less than SMs / z), cached per device.
+static int splitk_max_clusters(int z, int device) {
+  static std::atomic<int> cached[64][4];
+  const int i = z == 8 ? 3 : (z == 4 ? 2 : 1);
+  int n = cached[device & 63][i].load(std::memory_order_relaxed);
+  if (n == 0) {
+    auto kern = gemm_splitk_kernel<0, 0>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(z); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = SplitKSmem::TOTAL;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = z; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitKSmem::TOTAL) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = -1;                                           // not available: never split
+    }
+    cached[device & 63][i].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// CTAs per output tile of the split-K kernel: the largest power of two with which all tiles are in flight at once and
+// every CTA still has 4 K blocks of work; 1 = do not split.
+static int splitk_ctas(int M, int N, int K, int sms, int device) {
+  const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + SplitKSmem::BN - 1) / SplitKSmem::BN);
+  const int num_kb = (K + BK - 1) / BK;
+  for (int z = SK_MAX_Z; z > 1; z /= 2)
+    if (num_kb >= 4 * z && tiles * z <= sms && tiles <= splitk_max_clusters(z, device)) return z;
+  return 1;
+}
+
+template <int A_MN, int B_MN>
+static int launch_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int z, int device, cudaStream_t stream) {
+  using S = SplitKSmem;
+  static bool configured[64] = {false};
+  auto kern = gemm_splitk_kernel<A_MN, B_MN>;
+  if (!configured[device & 63]) {
+    AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
+    configured[device & 63] = true;
+  }
+  p.tiles_m = (p.M + BM - 1) / BM;
+  p.tiles_n = (p.N + S::BN - 1) / S::BN;
+  p.gemm_ctas = p.tiles_m * p.tiles_n * z;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.gemm_ctas); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = S::TOTAL; cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = z; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  AXB_CUDA(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, z));
+  return 0;
+}
+
 // Tiles per system-scope fence in the fused reductions (AXONN_FLAG_BATCH, default 4, 1..16).
 static int flag_batch_setting() {
   static int v = -1;
@@ -1553,6 +1792,7 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
   if (a_mn == 0) { if (make_tmap_2d_16bit(&tmA, A, M, K, BM, in_dtype)) return -1; }
   else           { if (make_tmap_2d_16bit(&tmA, A, K, M, BK, in_dtype)) return -1; }
   const bool pair = !comm && BN == 256 && pair_mode_enabled() && enough_pairs;
+  const int splitk = (comm || pair || BN != 128) ? 1 : splitk_ctas(M, N, K, usable_sms(device), device);
   if (b_mn == 0) { if (make_tmap_2d_16bit(&tmB, B, N, K, (pair || comm_pair) ? BN / 2 : BN, in_dtype)) return -1; }
   else           { if (make_tmap_2d_16bit(&tmB, B, K, N, BK, in_dtype)) return -1; }
 
@@ -1613,6 +1853,11 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
     if (layout == 0) return launch_pair<0, 0>(tmA, tmB, p, device, s);
     if (layout == 1) return launch_pair<0, 1>(tmA, tmB, p, device, s);
     return launch_pair<1, 1>(tmA, tmB, p, device, s);
+  }
+  if (splitk > 1) {
+    if (layout == 0) return launch_splitk<0, 0>(tmA, tmB, p, splitk, device, s);
+    if (layout == 1) return launch_splitk<0, 1>(tmA, tmB, p, splitk, device, s);
+    return launch_splitk<1, 1>(tmA, tmB, p, splitk, device, s);
   }
 #define AXB_DISPATCH(BN_, A_, B_) return launch<BN_, A_, B_>(tmA, tmB, p, device, s)
   if (BN == 256) {

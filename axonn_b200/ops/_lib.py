@@ -124,6 +124,9 @@ _STATUS_NAMES = {
     0x411: "flash attention backward: producer timed out",
     0x412: "flash attention backward: MMA issuer timed out",
     0x414: "flash attention backward: softmax / reduction warps timed out",
+    0x151: "split-K GEMM producer timed out",
+    0x152: "split-K GEMM MMA issuer timed out",
+    0x154: "split-K GEMM epilogue timed out",
     0x141: "CTA-pair GEMM producer timed out",
     0x142: "CTA-pair GEMM MMA issuer timed out",
     0x144: "CTA-pair GEMM epilogue timed out",

@@ -86,3 +86,38 @@ def test_attention_any_length(B, S, G, qpk, D):
             err = float((grad[bb, :, :, sl].double() - want).norm())
             # with one key the score gradients vanish: compare with the size of dV, the gradient that is left
             assert err < 1.5e-2 * max(float(want.norm()), float(gref[bb].norm()) * 1e-2), (bb, sl, err)
+
+
+# ------------------------------------------------------------------------------------------------ split-K GEMM
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("M,N,K", [(8, 128, 256), (24, 2048, 8192), (24, 8192, 2048), (120, 136, 1000), (136, 264, 520),
+                                   (128, 1024, 4096), (256, 256, 16384), (1, 512, 2048), (33, 40, 4104)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gemm_few_tiles(layout, M, N, K, dtype):
+    """Problems of few tiles (K split over a cluster), rows and columns that end inside a tile, K blocks that do not
+    divide evenly; bias, GELU, accumulation and fp32 output go through the shared epilogue."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib
+
+    if layout == "tn" and M % 8:
+        M = 8 * ((M + 7) // 8)
+    torch.manual_seed(M + N + K)
+    a = torch.randn((M, K) if layout != "tn" else (K, M), device=DEV).to(dtype)
+    b = torch.randn((N, K) if layout == "nt" else (K, N), device=DEV).to(dtype)
+    want = (a.double() if layout != "tn" else a.double().t()) @ (b.double().t() if layout == "nt" else b.double())
+    f = {"nt": ops.matmul_nt, "nn": ops.matmul_nn, "tn": ops.matmul_tn}[layout]
+    one = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10
+    assert _rel(f(a, b), want) < one
+    got = f(a, b, out_dtype=torch.float32)
+    assert got.dtype == torch.float32 and _rel(got, want) < 1e-5
+    base = torch.randn(M, N, device=DEV)
+    assert _rel(f(a, b, out=base.clone(), accumulate=True), want + base.double()) < 1e-5
+    if layout == "nt":
+        bias = torch.randn(N, device=DEV).to(dtype)
+        pre = torch.empty(M, N, device=DEV, dtype=dtype)
+        act = ops.matmul_nt(a, b, bias=bias, epilogue=ops.EPI_BIAS_GELU, aux=pre)
+        w = want + bias.double()
+        assert _rel(pre, w) < one
+        assert _rel(act, torch.nn.functional.gelu(w, approximate="tanh")) < 2 * one
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
