@@ -27,18 +27,6 @@ class _CrossEntropyFn(torch.autograd.Function):
                 raise TypeError("cross-entropy kernel needs bf16 logits")
             z = z.contiguous()
             stats = torch.empty((rows, 3), dtype=torch.float32, device=z.device)
-            if n == 1 and rows > 0:
-                lse = torch.empty(rows, dtype=torch.float32, device=z.device)
-                # two tensors: the loss is returned, and a view made in here could not be modified in place later
-                mean, kept = (torch.empty((), dtype=torch.float32, device=z.device) for _ in range(2))
-                _lib.check(_lib.lib().axb_ce_fwd_mean(_lib.addr(z), _lib.addr(t), _lib.addr(stats), _lib.addr(lse),
-                                                      _lib.addr(mean), _lib.addr(kept), rows, V,
-                                                      ignore_index, _lib.stream()),
-                           "axb_ce_fwd_mean")
-                _lib.add_launches(1)
-                ctx.save_for_backward(z, t, lse, kept)
-                ctx.start, ctx.ignore_index, ctx.shape = start, ignore_index, logits.shape
-                return mean
             _lib.check(_lib.lib().axb_ce_fwd(_lib.ptr(z), _lib.ptr(t), _lib.ptr(stats), ctypes.c_int(rows),
                                              ctypes.c_int(V), ctypes.c_int(start), _lib.stream_ptr()), "axb_ce_fwd")
             m, s, tl = stats[:, 0], stats[:, 1], stats[:, 2]
@@ -69,9 +57,9 @@ class _CrossEntropyFn(torch.autograd.Function):
         V = z.shape[-1]
         scale = (g.float() / count).reshape(1).contiguous()
         if z.is_cuda:
-            _lib.check(_lib.lib().axb_ce_bwd(_lib.addr(z), _lib.addr(t), _lib.addr(lse), _lib.addr(scale),
-                                             z.shape[0], V, ctx.start,
-                                             ctx.ignore_index, _lib.stream()), "axb_ce_bwd")
+            _lib.check(_lib.lib().axb_ce_bwd(_lib.ptr(z), _lib.ptr(t), _lib.ptr(lse), _lib.ptr(scale),
+                                             ctypes.c_int(z.shape[0]), ctypes.c_int(V), ctypes.c_int(ctx.start),
+                                             ctypes.c_longlong(ctx.ignore_index), _lib.stream_ptr()), "axb_ce_bwd")
             return z.reshape(ctx.shape), None, None, None
         p = (z.float() - lse[:, None]).exp()
         loc = t - ctx.start
