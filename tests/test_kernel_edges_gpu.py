@@ -121,3 +121,20 @@ def test_gemm_few_tiles(layout, M, N, K, dtype):
         assert _rel(act, torch.nn.functional.gelu(w, approximate="tanh")) < 2 * one
     torch.cuda.synchronize()
     assert _lib.device_status() == 0
+
+
+# ------------------------------------------------------------------------------------------------ in-place scale
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_scale_sizes_and_offsets(dtype):
+    """Chunk edges, vector remainders and tensors that do not start on a 16-byte boundary; one is the identity."""
+    from axonn_b200 import ops
+
+    torch.manual_seed(1)
+    sizes = [1, 7, 8, 9, 65535, 65536, 65537, 200003]
+    base = [torch.randn(n + 1, device=DEV).to(dtype) for n in sizes]
+    tensors = [t[:-1] for t in base] + [t[1:] for t in base]
+    for s in (0.37, 1.0):
+        work = [t.clone() if t.data_ptr() % 16 == 0 else torch.cat([t[:1], t])[1:] for t in tensors]
+        want = [(t.float() * s).to(dtype) for t in work]
+        ops.multi_tensor_scale_(work, s)
+        assert all(torch.equal(a, b) for a, b in zip(work, want))
