@@ -133,6 +133,14 @@ int axb_moe_signal(const AxbMoeCtx* ctx, int device, void* stream);
 int axb_copy_publish(const void* src, void* dst, long long nbytes, const AxbMoeCtx* ctx, int device, void* stream);
 int axb_moe_wait(const AxbMoeCtx* ctx, int device, void* stream);
 
+/* Experts that all live on this GPU (moe_local.cu): routing slots, row dispatch (gate null) or gate-scaled rows with
+ * the gate's gradient, and the weighted sum of a token's rows */
+int axb_moe_slots(const long long* idx, long long n, int E, int C, int Cp, int* dest, int* inverse, int* counts,
+                  float* assigned, void* stream);
+int axb_moe_rows(const void* x, const int* inverse, void* out, const float* gate, const void* other, float* dgate,
+                 int rows, int k, int H, void* stream);
+int axb_moe_tokens(const void* buf, const int* dest, const float* gate, void* out, int T, int k, int H, void* stream);
+
 /* Peer-memory context of the gradient all-reduce kernels (see AxbMoeCtx for the flag conventions). */
 typedef struct AxbCommCtx {
   int n, rank;

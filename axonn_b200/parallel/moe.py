@@ -22,15 +22,18 @@ tensor-parallelises every expert
 extension required for the Mixtral-style configuration.
 """
 
+import ctypes
 import math
 
 import torch
 import torch.distributed as dist
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd.function import once_differentiable
 
 from .. import axonn as ax
 from .. import ops
+from ..ops import _lib
 
 
 class _AllToAll(torch.autograd.Function):
@@ -54,6 +57,66 @@ class _AllToAll(torch.autograd.Function):
         out = torch.empty_like(g)
         dist.all_to_all_single(out, g, group=ctx.group)
         return out, None
+
+
+class _LocalDispatch(torch.autograd.Function):
+    """Token rows ``[T, H]`` into the experts' capacity buffers ``[E, rows, H]`` (zeros where no token is), and the
+    adjoint: the sum of a token's rows (``csrc/moe_local.cu``)."""
+
+    @staticmethod
+    def forward(ctx, x2, dest, inverse, E, rows, k):
+        x2 = _dense(x2)
+        ctx.save_for_backward(dest)
+        ctx.T, ctx.k = x2.shape[0], k
+        out = torch.empty((E, rows, x2.shape[1]), dtype=x2.dtype, device=x2.device)
+        _rows_kernel(x2, inverse, out, None, None, None, k)
+        return out
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, g):
+        (dest,) = ctx.saved_tensors
+        return _tokens_kernel(_dense(g), dest, None, ctx.T, ctx.k), None, None, None, None, None
+
+
+class _LocalCombine(torch.autograd.Function):
+    """``y[t] = sum_j gate[t, j] * out[dest[t, j]]`` over the kept assignments, fp32 sums; the adjoint gives the
+    experts' output gradient and the gate's in one pass."""
+
+    @staticmethod
+    def forward(ctx, out, gate, dest, inverse, T, k):
+        ctx.save_for_backward(out, gate, dest, inverse)
+        ctx.k = k
+        return _tokens_kernel(out, dest, gate, T, k)
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, g):
+        out, gate, dest, inverse = ctx.saved_tensors
+        dout = torch.empty_like(out)
+        dgate = torch.zeros_like(gate)                   # dropped assignments keep zero
+        _rows_kernel(_dense(g), inverse, dout, gate, out, dgate, ctx.k)
+        return dout, dgate, None, None, None, None
+
+
+def _dense(t):
+    """Contiguous and 16-byte aligned (the kernels use 16-byte accesses)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _rows_kernel(x, inverse, out, gate, other, dgate, k):
+    _lib.check(_lib.lib().axb_moe_rows(_lib.ptr(x), _lib.ptr(inverse), _lib.ptr(out), _lib.ptr(gate), _lib.ptr(other),
+                                       _lib.ptr(dgate), ctypes.c_int(inverse.numel()), ctypes.c_int(k),
+                                       ctypes.c_int(x.shape[1]), _lib.stream_ptr()), "axb_moe_rows")
+
+
+def _tokens_kernel(buf, dest, gate, T, k):
+    H = buf.shape[-1]
+    y = torch.empty((T, H), dtype=buf.dtype, device=buf.device)
+    _lib.check(_lib.lib().axb_moe_tokens(_lib.ptr(buf), _lib.ptr(dest), _lib.ptr(gate), _lib.ptr(y), ctypes.c_int(T),
+                                         ctypes.c_int(k), ctypes.c_int(H), _lib.stream_ptr()), "axb_moe_tokens")
+    return y
 
 
 def route_top_k(logits, top_k, capacity):
@@ -151,6 +214,31 @@ class ExpertParallelMoE(nn.Module):
         h = ops.swiglu(ops.linear_batched(x, self.w1, seg, seg_rows))
         return ops.linear_batched(h, self.w2, seg, seg_rows)
 
+    def _forward_local(self, x2, logits, C):
+        """The layer when every expert is on this GPU: same routing, capacity and statistics as the general path; the
+        permutations are one kernel each, the expert GEMMs skip the rows of the buffers that hold no token, and
+        nothing waits for the host.  The buffers are padded to 64 rows per expert, which the weight-gradient GEMM
+        needs of its reduction dimension."""
+        T, E, k = x2.shape[0], self.n_experts, self.top_k
+        rows = (C + 63) // 64 * 64
+        probs = F.softmax(logits.float(), dim=-1)
+        gate, idx = probs.topk(k, dim=-1)
+        gate = gate / gate.sum(-1, keepdim=True)
+        idx = idx.contiguous()
+        dest, inverse, counts = (torch.empty(n, dtype=torch.int32, device=x2.device) for n in (T * k, E * rows, E))
+        assigned = torch.empty(E, dtype=torch.float32, device=x2.device)
+        _lib.check(_lib.lib().axb_moe_slots(_lib.ptr(idx), ctypes.c_longlong(T * k), ctypes.c_int(E), ctypes.c_int(C),
+                                            ctypes.c_int(rows), _lib.ptr(dest), _lib.ptr(inverse), _lib.ptr(counts),
+                                            _lib.ptr(assigned), _lib.stream_ptr()), "axb_moe_slots")
+        self.last_aux_loss = E * (assigned / (T * k) * probs.mean(0)).sum()
+        kept = counts.float()
+        self.last_drop_fraction = 1.0 - kept.sum() / (T * k)
+        self.last_assignments_per_expert = assigned
+        self.last_dropped_per_expert = assigned - kept
+        xin = _LocalDispatch.apply(x2, dest, inverse, E, rows, k)
+        out = self._experts(xin, counts.view(E, 1), rows)
+        return _LocalCombine.apply(out, gate.contiguous(), dest, inverse, T, k)
+
     def forward(self, x):
         shape = x.shape
         x2 = x.reshape(-1, self.hidden)
@@ -158,6 +246,9 @@ class ExpertParallelMoE(nn.Module):
         C = self.capacity(T)
         E, k = self.n_experts, self.top_k
         logits = ops.linear(x2, self.router)
+        if (self.ep == 1 and T > 0 and x2.is_cuda and x2.dtype == torch.bfloat16 and self.w1.dtype == x2.dtype
+                and self.hidden % 8 == 0):
+            return self._forward_local(x2, logits, C).reshape(shape)
         idx, gate, slot, keep, aux = route_top_k(logits, k, C)
         self.last_aux_loss = aux
         self.last_drop_fraction = 1.0 - keep.float().mean().detach()

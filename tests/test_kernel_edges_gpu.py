@@ -138,3 +138,69 @@ def test_scale_sizes_and_offsets(dtype):
         want = [(t.float() * s).to(dtype) for t in work]
         ops.multi_tensor_scale_(work, s)
         assert all(torch.equal(a, b) for a, b in zip(work, want))
+
+
+# ------------------------------------------------------------------------------------------------ local experts
+@pytest.mark.parametrize("T,E,k,C", [(1, 4, 2, 8), (5, 8, 2, 8), (1000, 8, 2, 312), (4097, 4, 2, 2048), (8192, 8, 2, 2560),
+                                     (3000, 5, 1, 64)])
+def test_moe_slots(T, E, k, C):
+    """Slots are running counts per expert in assignment order (integers: exact), also past one chunk of the scan and
+    for experts that overflow their capacity."""
+    import ctypes
+
+    from axonn_b200.ops import _lib
+
+    torch.manual_seed(T)
+    idx = torch.rand(T, E, device=DEV).mul_(torch.linspace(0.5, 1.5, E, device=DEV)).topk(k, -1)[1].contiguous()
+    n, rows = T * k, (C + 63) // 64 * 64
+    dest, inv, cnt = (torch.full((m,), -7, dtype=torch.int32, device=DEV) for m in (n, E * rows, E))
+    assigned = torch.empty(E, device=DEV)
+    _lib.check(_lib.lib().axb_moe_slots(_lib.ptr(idx), ctypes.c_longlong(n), ctypes.c_int(E), ctypes.c_int(C),
+                                        ctypes.c_int(rows), _lib.ptr(dest), _lib.ptr(inv), _lib.ptr(cnt),
+                                        _lib.ptr(assigned), _lib.stream_ptr()), "axb_moe_slots")
+    flat = idx.reshape(-1).tolist()
+    seen, want, winv = [0] * E, [], [-1] * (E * rows)
+    for a, e in enumerate(flat):
+        ok = seen[e] < C
+        want.append(e * rows + seen[e] if ok else -1)
+        if ok:
+            winv[e * rows + seen[e]] = a
+        seen[e] += 1
+    assert dest.tolist() == want and inv.tolist() == winv
+    assert cnt.tolist() == [min(s, C) for s in seen] and assigned.tolist() == [float(s) for s in seen]
+
+
+@pytest.mark.parametrize("T,k,rows,H", [(1, 1, 64, 8), (77, 2, 128, 264), (500, 3, 512, 2048)])
+def test_moe_permutations(T, k, rows, H):
+    """Dispatch, combine and their adjoints against indexing in 64 bits, with dropped assignments and empty rows."""
+    from axonn_b200.parallel import moe
+
+    torch.manual_seed(H)
+    E = 4
+    n = T * k
+    perm = torch.randperm(E * rows, device=DEV)[:n].int()
+    dest = torch.where(torch.rand(n, device=DEV) < 0.2, torch.full_like(perm, -1), perm)
+    inv = torch.full((E * rows,), -1, dtype=torch.int32, device=DEV)
+    kept = dest >= 0
+    inv[dest[kept].long()] = torch.arange(n, device=DEV, dtype=torch.int32)[kept]
+    x = torch.randn(T, H, device=DEV).bfloat16().requires_grad_(True)
+    gate = torch.rand(T, k, device=DEV).requires_grad_(True)
+    buf = moe._LocalDispatch.apply(x, dest, inv, E, rows, k)
+    ref = torch.zeros(E * rows, H, device=DEV, dtype=torch.bfloat16)
+    tok = torch.arange(T, device=DEV).repeat_interleave(k)
+    ref[dest[kept].long()] = x.detach()[tok[kept]]
+    assert torch.equal(buf.detach().view(-1, H), ref)
+    gbuf = torch.randn_like(buf)
+    (dx,) = torch.autograd.grad(buf, x, gbuf)
+    rows64 = gbuf.double().view(-1, H)
+    want = torch.zeros(T, H, device=DEV, dtype=torch.float64).index_add(0, tok[kept], rows64[dest[kept].long()])
+    assert _rel(dx, want) < 2.0 ** -8
+    out = torch.randn(E, rows, H, device=DEV).bfloat16().requires_grad_(True)
+    y = moe._LocalCombine.apply(out, gate, dest, inv, T, k)
+    o64, g64 = out.detach().double().requires_grad_(True), gate.detach().double().requires_grad_(True)
+    y64 = torch.zeros(T, H, device=DEV, dtype=torch.float64).index_add(
+        0, tok[kept], o64.view(-1, H)[dest[kept].long()] * g64.view(-1)[kept][:, None])
+    assert _rel(y.detach(), y64.detach()) < 2.0 ** -8
+    dy = torch.randn_like(y)
+    got, want = torch.autograd.grad(y, [out, gate], dy), torch.autograd.grad(y64, [o64, g64], dy.double())
+    assert _rel(got[0], want[0]) < 2.0 ** -8 and _rel(got[1], want[1]) < 1e-5
