@@ -1,13 +1,11 @@
 // Gradient pruning: keep the k largest-magnitude entries of a tensor, zero the rest.
 //
-// The threshold (k-th largest |g|) comes from a radix select on the magnitude
-// bits instead of a sort: one histogram pass over the top 15 magnitude bits
-// (block-private shared-memory histograms, flushed with atomics), a one-block
-// suffix scan that finds the bin holding the k-th element, for fp32 a second
-// histogram over the next 16 bits restricted to that bin, then one masking
-// pass.  bf16 tensors (15 magnitude bits in total) need exactly two passes
-// over the data.  Ties at the threshold are all kept (|g| >= threshold), the
-// same rule as thresholding with the k-th value of a sort.
+// The threshold (k-th largest |g|) comes from a radix select on the magnitude bits instead of a sort: one histogram
+// pass over the top 15 magnitude bits (block-private shared-memory histograms, flushed with atomics; the last block to
+// finish scans the bins for the one that holds the k-th element), for fp32 a second histogram over the next 16 bits
+// restricted to that bin, then one masking pass.  bf16 tensors (15 magnitude bits in total) need exactly two passes
+// over the data.  Ties at the threshold are all kept (|g| >= threshold), the same rule as thresholding with the k-th
+// value of a sort.
 //
 // Scratch: 32768 + 65536 + 8 32-bit words, supplied by the caller.
 #include <mutex>
@@ -28,104 +26,173 @@ __device__ __forceinline__ uint32_t mag_bits(const void* g, long long i, int dty
   return (static_cast<uint32_t>(reinterpret_cast<const uint16_t*>(g)[i]) & 0x7FFFu) << 16;
 }
 
-// level 1: histogram of the top 15 magnitude bits
-__global__ void __launch_bounds__(PR_THREADS)
-prune_hist1_kernel(const void* __restrict__ g, long long n, int dtype, unsigned int* __restrict__ hist) {
-  extern __shared__ unsigned int sh[];
-  for (int i = threadIdx.x; i < PR_BINS1; i += blockDim.x) sh[i] = 0;
-  __syncthreads();
-  if (dtype != PR_F32 && (reinterpret_cast<uintptr_t>(g) & 15) == 0) {
-    const long long nv = n / 8;
-    const uint4* q = reinterpret_cast<const uint4*>(g);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
-      const uint4 u = q[i];
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        atomicAdd(&sh[w[k] & 0x7FFFu], 1u);
-        atomicAdd(&sh[(w[k] >> 16) & 0x7FFFu], 1u);
-      }
-    }
-    for (long long i = nv * 8 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-      atomicAdd(&sh[mag_bits(g, i, dtype) >> 16], 1u);
-  } else {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-      atomicAdd(&sh[mag_bits(g, i, dtype) >> 16], 1u);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < PR_BINS1; i += blockDim.x)
-    if (sh[i]) atomicAdd(&hist[i], sh[i]);
-}
+// the last 8 words of the scratch
+struct PruneMeta {
+  long long bin1, rank1;      // bin of the threshold's top 15 bits, rank of the threshold inside it
+  long long bin2;             // fp32: the next 16 bits
+  unsigned int blocks_done;   // zero between kernels
+  unsigned int pad;
+};
+static_assert(sizeof(PruneMeta) == 32, "scratch layout");
 
-// One block: find the largest bin b with  count(bins > b) < k <= count(bins >= b).
-// meta_out[0] = b, meta_out[1] = k - count(bins > b)  (rank of the target inside bin b)
+// Called by all threads of the block that finishes last: the largest bin b with count(bins > b) < k <= count(bins >= b).
+// Every thread sums its bins with 16-byte loads and the block scans the sums in registers: a one-block kernel of its own
+// with a word-wise sum and a log-step scan in shared memory took 21 us per tensor.
 template <int BINS>
-__global__ void __launch_bounds__(PR_THREADS)
-prune_select_kernel(const unsigned int* __restrict__ hist, const long long* __restrict__ k_in, long long k_const,
-                    long long* __restrict__ meta_out) {
-  __shared__ unsigned long long part[PR_THREADS];
+__device__ void prune_select(const unsigned int* __restrict__ hist, long long k, long long* bin, long long* rank) {
+  __shared__ unsigned long long warp_sum[PR_THREADS / 32];
   constexpr int PER = BINS / PR_THREADS;
-  const long long k = k_in ? *k_in : k_const;
   // thread t owns bins [BINS - (t+1)*PER, BINS - t*PER): thread 0 holds the largest magnitudes
-  const int hi = BINS - threadIdx.x * PER;
+  const int hi = BINS - threadIdx.x * PER, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   unsigned long long mine = 0;
-  for (int b = hi - PER; b < hi; ++b) mine += hist[b];
-  part[threadIdx.x] = mine;
-  __syncthreads();
-  // inclusive prefix over threads (Hillis-Steele)
-  for (int off = 1; off < PR_THREADS; off <<= 1) {
-    unsigned long long v = threadIdx.x >= off ? part[threadIdx.x - off] : 0;
-    __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
+#pragma unroll 8
+  for (int i = 0; i < PER / 4; ++i) {
+    const uint4 u = __ldcg(reinterpret_cast<const uint4*>(hist + hi - PER) + i);
+    mine += static_cast<unsigned long long>(u.x) + u.y + u.z + u.w;
   }
-  const unsigned long long incl = part[threadIdx.x], excl = incl - mine;
+  unsigned long long incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+  if (lane == 31) warp_sum[w] = incl;
+  __syncthreads();
+  if (w == 0) {
+    const unsigned long long v = warp_sum[lane];
+    unsigned long long pre = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const unsigned long long u = __shfl_up_sync(0xffffffffu, pre, o); if (lane >= o) pre += u; }
+    warp_sum[lane] = pre - v;
+  }
+  __syncthreads();
+  incl += warp_sum[w];
+  const unsigned long long excl = incl - mine;
   if (excl < (unsigned long long)k && (unsigned long long)k <= incl) {
     unsigned long long above = excl;
     for (int b = hi - 1; b >= hi - PER; --b) {
-      const unsigned long long c = hist[b];
-      if (above + c >= (unsigned long long)k) { meta_out[0] = b; meta_out[1] = k - (long long)above; return; }
+      const unsigned long long c = __ldcg(hist + b);
+      if (above + c >= (unsigned long long)k) { *bin = b; if (rank) *rank = k - (long long)above; return; }
       above += c;
     }
   }
-  if (threadIdx.x == PR_THREADS - 1 && incl < (unsigned long long)k) { meta_out[0] = 0; meta_out[1] = 1; }  // k > n: keep all
+  if (threadIdx.x == PR_THREADS - 1 && incl < (unsigned long long)k) { *bin = 0; if (rank) *rank = 1; }  // k > n: keep all
 }
 
-// level 2 (fp32 only): histogram of the next 16 bits among elements whose top bits equal meta[0]
-__global__ void prune_hist2_kernel(const void* __restrict__ g, long long n, const long long* __restrict__ meta,
-                                   unsigned int* __restrict__ hist2) {
-  const uint32_t top = (uint32_t)meta[0];
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const uint32_t m = reinterpret_cast<const uint32_t*>(g)[i] & 0x7FFFFFFFu;
-    if ((m >> 16) == top) atomicAdd(&hist2[m & 0xFFFFu], 1u);
+// True in every thread of the block that arrives last (its predecessors' histogram updates are visible to it).
+__device__ __forceinline__ bool prune_last_block(unsigned int* counter) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    if (last) { *counter = 0; __threadfence(); }
   }
+  __syncthreads();
+  return last;
 }
 
-// thr = 31-bit magnitude threshold: keep |g| bits >= thr
-__global__ void prune_mask_kernel(void* __restrict__ g, long long n, int dtype, const long long* __restrict__ meta1,
-                                  const long long* __restrict__ meta2) {
-  const uint32_t thr = ((uint32_t)meta1[0] << 16) | (dtype == PR_F32 ? (uint32_t)meta2[0] : 0u);
-  if (dtype != PR_F32 && (reinterpret_cast<uintptr_t>(g) & 15) == 0) {
-    const long long nv = n / 8;
+// level 1: histogram of the top 15 magnitude bits, then (last block) the threshold's bin.  Four 16-byte loads per thread
+// are in flight; they are ordinary loads, so that a tensor that fits the L2 is still there for the masking pass.
+__global__ void __launch_bounds__(PR_THREADS)
+prune_hist1_kernel(const void* __restrict__ g, long long n, int dtype, long long k, unsigned int* __restrict__ hist,
+                   PruneMeta* __restrict__ meta) {
+  extern __shared__ unsigned int sh[];
+  for (int i = threadIdx.x; i < PR_BINS1; i += PR_THREADS) sh[i] = 0;
+  __syncthreads();
+  auto count = [&](uint32_t key) { atomicAdd(&sh[key], 1u); };
+  long long tail = 0;
+  const long long first = blockIdx.x * (long long)PR_THREADS + threadIdx.x, step = (long long)gridDim.x * PR_THREADS;
+  if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+    const int per_vec = dtype == PR_F32 ? 4 : 8;
+    const long long nv = n / per_vec;
+    const uint4* q = reinterpret_cast<const uint4*>(g);
+    for (long long i = first; i < nv; i += 4 * step) {
+      uint4 u[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) if (i + v * step < nv) u[v] = q[i + v * step];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        if (i + v * step >= nv) break;
+        const uint32_t w[4] = {u[v].x, u[v].y, u[v].z, u[v].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          count((w[j] >> 16) & 0x7FFFu);
+          if (dtype != PR_F32) count(w[j] & 0x7FFFu);
+        }
+      }
+    }
+    tail = nv * per_vec;
+  }
+  for (long long i = tail + first; i < n; i += step) count(mag_bits(g, i, dtype) >> 16);
+  __syncthreads();
+  for (int i = threadIdx.x; i < PR_BINS1; i += PR_THREADS)
+    if (sh[i]) atomicAdd(&hist[i], sh[i]);
+  if (!prune_last_block(&meta->blocks_done)) return;
+  prune_select<PR_BINS1>(hist, k, &meta->bin1, &meta->rank1);
+}
+
+// level 2 (fp32 only): histogram of the next 16 bits among elements whose top bits equal the threshold's, and its bin
+__global__ void __launch_bounds__(PR_THREADS)
+prune_hist2_kernel(const void* __restrict__ g, long long n, PruneMeta* __restrict__ meta, unsigned int* __restrict__ hist2) {
+  const uint32_t top = static_cast<uint32_t>(meta->bin1);
+  auto count = [&](uint32_t w) { if (((w >> 16) & 0x7FFFu) == top) atomicAdd(&hist2[w & 0xFFFFu], 1u); };
+  const uint32_t* f = reinterpret_cast<const uint32_t*>(g);
+  const long long first = blockIdx.x * (long long)PR_THREADS + threadIdx.x, step = (long long)gridDim.x * PR_THREADS;
+  long long tail = 0;
+  if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+    const long long nv = n / 4;
+    const uint4* q = reinterpret_cast<const uint4*>(g);
+    for (long long i = first; i < nv; i += 4 * step) {
+      uint4 u[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) if (i + v * step < nv) u[v] = q[i + v * step];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        if (i + v * step >= nv) break;
+        count(u[v].x); count(u[v].y); count(u[v].z); count(u[v].w);
+      }
+    }
+    tail = nv * 4;
+  }
+  for (long long i = tail + first; i < n; i += step) count(f[i]);
+  if (!prune_last_block(&meta->blocks_done)) return;
+  prune_select<PR_BINS2>(hist2, meta->rank1, &meta->bin2, nullptr);
+}
+
+// thr = 31-bit magnitude threshold: keep |g| bits >= thr.  Bound by one read and one write of the tensor.
+__global__ void __launch_bounds__(512)
+prune_mask_kernel(void* __restrict__ g, long long n, int dtype, const PruneMeta* __restrict__ meta) {
+  const uint32_t thr = ((uint32_t)meta->bin1 << 16) | (dtype == PR_F32 ? (uint32_t)meta->bin2 : 0u);
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  long long tail = 0;
+  if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+    const int per_vec = dtype == PR_F32 ? 4 : 8;
+    const long long nv = n / per_vec;
     uint4* q = reinterpret_cast<uint4*>(g);
     const uint32_t t16 = thr >> 16;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv; i += (long long)gridDim.x * blockDim.x) {
-      uint4 u = q[i];
-      uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    for (long long i = first; i < nv; i += 4 * step) {
+      uint4 u[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if ((w[k] & 0x7FFFu) < t16) w[k] &= 0xFFFF0000u;
-        if (((w[k] >> 16) & 0x7FFFu) < t16) w[k] &= 0x0000FFFFu;
+      for (int v = 0; v < 4; ++v) if (i + v * step < nv) u[v] = q[i + v * step];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        if (i + v * step >= nv) break;
+        uint32_t w[4] = {u[v].x, u[v].y, u[v].z, u[v].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (dtype == PR_F32) {
+            if ((w[j] & 0x7FFFFFFFu) < thr) w[j] = 0u;
+          } else {
+            if ((w[j] & 0x7FFFu) < t16) w[j] &= 0xFFFF0000u;
+            if (((w[j] >> 16) & 0x7FFFu) < t16) w[j] &= 0x0000FFFFu;
+          }
+        }
+        q[i + v * step] = make_uint4(w[0], w[1], w[2], w[3]);
       }
-      q[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    for (long long i = nv * 8 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-      if (mag_bits(g, i, dtype) < thr) reinterpret_cast<uint16_t*>(g)[i] = 0;
-  } else {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-      if (mag_bits(g, i, dtype) < thr) {
-        if (dtype == PR_F32) reinterpret_cast<uint32_t*>(g)[i] = 0; else reinterpret_cast<uint16_t*>(g)[i] = 0;
-      }
+    tail = nv * per_vec;
+  }
+  for (long long i = tail + first; i < n; i += step) {
+    if (mag_bits(g, i, dtype) < thr) {
+      if (dtype == PR_F32) reinterpret_cast<uint32_t*>(g)[i] = 0; else reinterpret_cast<uint16_t*>(g)[i] = 0;
     }
   }
 }
@@ -139,7 +206,8 @@ int prune_topk_launch(void* g, long long n, int dtype, long long k, unsigned int
   if (k >= n) return 0;
   unsigned int* hist1 = work;
   unsigned int* hist2 = work + PR_BINS1;
-  long long* meta = reinterpret_cast<long long*>(work + PR_BINS1 + PR_BINS2);  // meta1 = meta[0..1], meta2 = meta[2..3]
+  PruneMeta* meta = reinterpret_cast<PruneMeta*>(work + PR_BINS1 + PR_BINS2);
+  // one memset: for 16-bit tensors it covers the second level's bins too, which costs less than a second launch
   AXB_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned int) * PR_WORK_WORDS, s));
   static bool configured[64] = {false};
   if (!configured[device & 63]) {
@@ -147,17 +215,13 @@ int prune_topk_launch(void* g, long long n, int dtype, long long k, unsigned int
     configured[device & 63] = true;
   }
   const int sms = sm_count(device);
-  prune_hist1_kernel<<<sms, PR_THREADS, PR_BINS1 * 4, s>>>(g, n, dtype, hist1);
-  AXB_CUDA(cudaGetLastError());
-  prune_select_kernel<PR_BINS1><<<1, PR_THREADS, 0, s>>>(hist1, nullptr, k, meta);
+  prune_hist1_kernel<<<sms, PR_THREADS, PR_BINS1 * 4, s>>>(g, n, dtype, k, hist1, meta);
   AXB_CUDA(cudaGetLastError());
   if (dtype == PR_F32) {
-    prune_hist2_kernel<<<sms * 4, 512, 0, s>>>(g, n, meta, hist2);
-    AXB_CUDA(cudaGetLastError());
-    prune_select_kernel<PR_BINS2><<<1, PR_THREADS, 0, s>>>(hist2, meta + 1, 0, meta + 2);
+    prune_hist2_kernel<<<sms * 2, PR_THREADS, 0, s>>>(g, n, meta, hist2);
     AXB_CUDA(cudaGetLastError());
   }
-  prune_mask_kernel<<<sms * 4, 512, 0, s>>>(g, n, dtype, meta, meta + 2);
+  prune_mask_kernel<<<sms * 4, 512, 0, s>>>(g, n, dtype, meta);
   AXB_CUDA(cudaGetLastError());
   return 0;
 }
