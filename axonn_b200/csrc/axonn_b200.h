@@ -237,6 +237,9 @@ int axb_flash_attn_bwd_split(const void* qkv, const void* out, const void* d_out
 
 /* ---- cross entropy on a vocabulary shard of bf16 logits (loss.cu); backward overwrites the logits with their gradient */
 int axb_ce_fwd(const void* logits, const long long* targets, float* stats, int rows, int V, int vocab_start, void* stream);
+/* whole vocabulary on this GPU: also lse [rows], the mean loss and kept = max(rows not ignored, 1) */
+int axb_ce_fwd_mean(const void* logits, const long long* targets, float* stats, float* lse, float* mean, float* kept,
+                    int rows, int V, long long ignore_index, void* stream);
 int axb_ce_bwd(void* logits, const long long* targets, const float* lse, const float* scale, int rows, int V,
                int vocab_start, long long ignore_index, void* stream);
 

@@ -1,9 +1,9 @@
 // Softmax cross-entropy over (possibly vocabulary-sharded) logits.
 //
 // forward statistics, one block per row:  m = max_j z_j, s = sum_j exp(z_j - m),
-// t = z_target when the target lies in this shard (else 0).  The caller turns
-// (m, s, t) — all-reduced over the vocabulary shards when there are several —
-// into lse = m + log s and loss = lse - t.
+// t = z_target when the target lies in this shard (else 0), in one pass over the row (running maximum per thread).
+// With the whole vocabulary on this GPU the kernel also writes lse = m + log s, and a one-block kernel turns the rows
+// into the mean loss; otherwise the caller all-reduces (m, s, t) over the vocabulary shards first.
 // backward, in place: z_j <- (exp(z_j - lse) - [j == target]) * scale.
 #include "common.cuh"
 
@@ -43,34 +43,92 @@ __device__ __forceinline__ void ld8bf(const __nv_bfloat16* p, float (&f)[8]) {
   for (int i = 0; i < 4; ++i) { float2 t = __bfloat1622float2(h[i]); f[2 * i] = t.x; f[2 * i + 1] = t.y; }
 }
 
-// stats: [rows, 3] = (max, sumexp, target logit)
-__global__ void __launch_bounds__(CE_THREADS)
+// stats: [rows, 3] = (max, sumexp, target logit); lse: [rows] or null.  The row is read once: every thread keeps its own
+// running maximum and rescales its sum when the maximum of the next CE_UNROLL vectors raises it.  The next vectors are
+// loaded before the current ones are used, and many small blocks (one row each) share an SM, so that the reductions at
+// the end of one row run under the loads of others.
+constexpr int CE_FWD_THREADS = 256, CE_UNROLL = 4;
+__global__ void __launch_bounds__(CE_FWD_THREADS)
 ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
-              float* __restrict__ stats, int rows, int V, int vocab_start) {
+              float* __restrict__ stats, float* __restrict__ lse, int rows, int V, int vocab_start) {
   __shared__ float red[32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const __nv_bfloat16* z = logits + (size_t)row * V;
     const int nchunk = V / 8;
-    float m = -INFINITY;
-    for (int c = threadIdx.x; c < nchunk; c += blockDim.x) {
-      float f[8]; ld8bf(z + c * 8, f);
+    uint4 next[CE_UNROLL];
+    auto fetch = [&](int c) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) m = fmaxf(m, f[i]);
-    }
-    m = block_max(m, red);
-    float s = 0.f;
-    for (int c = threadIdx.x; c < nchunk; c += blockDim.x) {
-      float f[8]; ld8bf(z + c * 8, f);
+      for (int k = 0; k < CE_UNROLL; ++k) {
+        const int cc = c + k * CE_FWD_THREADS;
+        // vectors past the row: -inf, which adds exactly nothing
+        next[k] = cc < nchunk ? __ldg(reinterpret_cast<const uint4*>(z) + cc)
+                              : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);
+      }
+    };
+    float m = -INFINITY, s = 0.f;
+    fetch(threadIdx.x);
+    for (int c = threadIdx.x; c < nchunk; c += CE_FWD_THREADS * CE_UNROLL) {
+      uint4 u[CE_UNROLL];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) s += __expf(f[i] - m);
+      for (int k = 0; k < CE_UNROLL; ++k) u[k] = next[k];
+      if (c + CE_FWD_THREADS * CE_UNROLL < nchunk) fetch(c + CE_FWD_THREADS * CE_UNROLL);
+      __nv_bfloat162 m2 = *reinterpret_cast<const __nv_bfloat162*>(&u[0].x);
+#pragma unroll
+      for (int k = 0; k < CE_UNROLL; ++k) {
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[k]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m2 = __hmax2(m2, h[i]);
+      }
+      const float2 mf = __bfloat1622float2(m2);
+      const float mx = fmaxf(m, fmaxf(mf.x, mf.y));
+      // nothing but -inf so far: keep the sum at zero (a NaN among them must still reach it)
+      const float ref = mx == -INFINITY ? 0.f : mx;
+      s *= __expf((m == -INFINITY ? ref : m) - ref);
+      m = mx;
+      float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < CE_UNROLL; ++k) {
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[k]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 d = __fadd2_rn(__bfloat1622float2(h[i]), make_float2(-ref, -ref));
+          acc = __fadd2_rn(acc, make_float2(__expf(d.x), __expf(d.y)));
+        }
+      }
+      s += acc.x + acc.y;
     }
+    const float mrow = block_max(m, red);
+    s *= __expf((m == -INFINITY && mrow != -INFINITY ? mrow : m) - mrow);   // a row of -inf only: NaN, as its softmax is
     s = block_sum(s, red);
     if (threadIdx.x == 0) {
       const long long t = targets[row] - vocab_start;
-      stats[3 * row] = m;
+      stats[3 * row] = mrow;
       stats[3 * row + 1] = s;
       stats[3 * row + 2] = (t >= 0 && t < V) ? __bfloat162float(z[t]) : 0.f;
+      if (lse) lse[row] = mrow + logf(s);
     }
+  }
+}
+
+// mean = mean over the rows whose target is not ignore_index of lse - target logit, kept = max(number of them, 1).
+// One block: the rows' losses are a few hundred KB at most, and the fixed order keeps the result reproducible.
+__global__ void __launch_bounds__(1024)
+ce_mean_kernel(const float* __restrict__ stats, const float* __restrict__ lse, const long long* __restrict__ targets,
+               float* __restrict__ mean, float* __restrict__ kept, int rows, long long ignore_index) {
+  __shared__ float red[32];
+  float loss = 0.f, count = 0.f;                     // counts stay below 2^24 per thread
+#pragma unroll 4
+  for (int r = threadIdx.x; r < rows; r += 1024) {
+    const float valid = targets[r] != ignore_index ? 1.f : 0.f;
+    loss += (lse[r] - stats[3 * (size_t)r + 2]) * valid;
+    count += valid;
+  }
+  loss = block_sum(loss, red);
+  count = block_sum(count, red);
+  if (threadIdx.x == 0) {
+    count = fmaxf(count, 1.f);
+    *mean = loss / count;
+    *kept = count;
   }
 }
 
@@ -108,15 +166,27 @@ ce_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ 
 
 using namespace axb;
 
-extern "C" int axb_ce_fwd(const void* logits, const long long* targets, float* stats, int rows, int V, int vocab_start,
-                          void* stream) {
+// lse null: statistics of a vocabulary shard only; otherwise also lse [rows], the mean loss and the rows that count
+static int ce_fwd(const void* logits, const long long* targets, float* stats, float* lse, float* mean, float* kept,
+                  int rows, int V, int vocab_start, long long ignore_index, void* stream) {
   if (V % 8) { set_error("cross entropy: vocab shard %d must be a multiple of 8", V); return -1; }
-  const int cap = sm_count_current() * 8;
-  const int grid = rows < cap ? rows : cap;
-  ce_fwd_kernel<<<grid, CE_THREADS, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, targets, stats, rows, V,
+  // one block per row (a block that walked several rows would leave the last round of a capped grid half empty)
+  ce_fwd_kernel<<<rows, CE_FWD_THREADS, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, targets, stats, lse, rows, V,
                                                              vocab_start);
   AXB_CUDA(cudaGetLastError());
+  if (mean) {
+    ce_mean_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(stats, lse, targets, mean, kept, rows, ignore_index);
+    AXB_CUDA(cudaGetLastError());
+  }
   return 0;
+}
+extern "C" int axb_ce_fwd(const void* logits, const long long* targets, float* stats, int rows, int V, int vocab_start,
+                          void* stream) {
+  return ce_fwd(logits, targets, stats, nullptr, nullptr, nullptr, rows, V, vocab_start, 0, stream);
+}
+extern "C" int axb_ce_fwd_mean(const void* logits, const long long* targets, float* stats, float* lse, float* mean,
+                               float* kept, int rows, int V, long long ignore_index, void* stream) {
+  return ce_fwd(logits, targets, stats, lse, mean, kept, rows, V, 0, ignore_index, stream);
 }
 extern "C" int axb_ce_bwd(void* logits, const long long* targets, const float* lse, const float* scale, int rows, int V,
                           int vocab_start, long long ignore_index, void* stream) {

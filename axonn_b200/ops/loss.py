@@ -27,6 +27,18 @@ class _CrossEntropyFn(torch.autograd.Function):
                 raise TypeError("cross-entropy kernel needs bf16 logits")
             z = z.contiguous()
             stats = torch.empty((rows, 3), dtype=torch.float32, device=z.device)
+            if n == 1 and rows > 0:
+                lse = torch.empty(rows, dtype=torch.float32, device=z.device)
+                # two tensors: the loss is returned, and a view made in here could not be modified in place later
+                mean, kept = (torch.empty((), dtype=torch.float32, device=z.device) for _ in range(2))
+                _lib.check(_lib.lib().axb_ce_fwd_mean(_lib.ptr(z), _lib.ptr(t), _lib.ptr(stats), _lib.ptr(lse),
+                                                      _lib.ptr(mean), _lib.ptr(kept), ctypes.c_int(rows), ctypes.c_int(V),
+                                                      ctypes.c_longlong(ignore_index), _lib.stream_ptr()),
+                           "axb_ce_fwd_mean")
+                _lib.add_launches(1)
+                ctx.save_for_backward(z, t, lse, kept)
+                ctx.start, ctx.ignore_index, ctx.shape = start, ignore_index, logits.shape
+                return mean
             _lib.check(_lib.lib().axb_ce_fwd(_lib.ptr(z), _lib.ptr(t), _lib.ptr(stats), ctypes.c_int(rows),
                                              ctypes.c_int(V), ctypes.c_int(start), _lib.stream_ptr()), "axb_ce_fwd")
             m, s, tl = stats[:, 0], stats[:, 1], stats[:, 2]

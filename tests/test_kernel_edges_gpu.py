@@ -123,6 +123,29 @@ def test_gemm_few_tiles(layout, M, N, K, dtype):
     assert _lib.device_status() == 0
 
 
+# ------------------------------------------------------------------------------------------------ cross-entropy
+@pytest.mark.parametrize("rows,V", [(1, 8), (3, 4096), (5, 4104), (7, 16384), (2, 16392), (1030, 50304)])
+def test_cross_entropy_rows(rows, V):
+    """Rows shorter than one batch of vectors, exactly one, one more; ignored targets, a row whose first vectors are all
+    -inf, maxima that grow along the row.  Tolerance: fp32 sums."""
+    from axonn_b200 import ops
+
+    torch.manual_seed(V)
+    z = (torch.randn(rows, V, device=DEV) * 3 + torch.linspace(-20, 20, V, device=DEV)).bfloat16()
+    z[0, : V // 2] = float("-inf")
+    t = torch.randint(V // 2, V, (rows,), device=DEV)
+    if rows > 2:
+        t[1] = -100
+    ref = torch.nn.functional.cross_entropy(z.double(), t)
+    x = z.clone().requires_grad_(True)
+    loss = ops.cross_entropy(x, t)
+    assert abs(float(loss) - float(ref)) < 1e-5 * abs(float(ref)) + 1e-6
+    (g,) = torch.autograd.grad(loss * 2.0, x)
+    zr = z.double().requires_grad_(True)
+    (gr,) = torch.autograd.grad(torch.nn.functional.cross_entropy(zr, t) * 2.0, zr)
+    assert _rel(g, gr) < 2.0 ** -8
+
+
 # ------------------------------------------------------------------------------------------------ in-place scale
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_scale_sizes_and_offsets(dtype):
