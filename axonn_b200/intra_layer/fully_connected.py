@@ -42,7 +42,7 @@ from .asym_communication import (
     Gatherv,
     gather_batch_sizes,
 )
-from .communication import Drop, GatherSumBackward, _drop, _gather, _reduce_scatter
+from .communication import Drop, GatherSumBackward, _drop, _gather, _reduce_scatter, _size
 
 
 @torch.no_grad()
@@ -123,8 +123,8 @@ class AsyncLinear(Function):
             compute_dtype = torch.get_autocast_dtype(input_.device.type)
             input_ = input_.to(compute_dtype)
         x2 = input_.reshape(-1, input_.shape[-1])
-        inner_n = dist.get_world_size(forward_all_reduce_group)
-        depth_n = dist.get_world_size(depth_parallel_group)
+        inner_n = _size(forward_all_reduce_group)
+        depth_n = _size(depth_parallel_group)
         b = None if bias is None else bias.to(compute_dtype)
         pre_act = None
         if activation not in (None, "gelu"):
@@ -201,8 +201,8 @@ class AsyncLinear(Function):
         x2 = input_.reshape(-1, input_.shape[-1])
         overlap_rs = oc.OVERLAP_REDUCE_SCATTER
         overlap_ar = oc.OVERLAP_ALL_REDUCE
-        outer_n = dist.get_world_size(ctx.backward_all_reduce_group)
-        depth_n = dist.get_world_size(ctx.depth_parallel_group)
+        outer_n = _size(ctx.backward_all_reduce_group)
+        depth_n = _size(ctx.depth_parallel_group)
         grad_input = grad_weight = grad_bias = None
         handle = None
 

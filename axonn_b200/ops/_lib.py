@@ -32,6 +32,37 @@ class KernelError(RuntimeError):
     pass
 
 
+# Argument types of the launchers that run once per layer (i int, l long long, f float, p pointer).  With them declared,
+# plain Python numbers and addresses are converted by ctypes itself; without, every call builds an object per argument
+# (some fifteen of them for a GEMM).
+_SIGNATURES = {
+    "axb_gemm": "ippppp" "iiiiiiii" "p",
+    "axb_norm_fwd": "ppppp" "iii" "f" "iiii" "p",
+    "axb_norm_bwd": "pppppppppp" "iiiiiiii" "p",
+    "axb_add_norm_fwd": "ppppppp" "iii" "f" "iiii" "p",
+    "axb_add_norm_bwd": "ppppppppppp" "iiiiiiii" "p",
+    "axb_norm_grid": "ii",
+    "axb_colsum_splits": "iii",
+    "axb_colsum": "ppp" "iiiii" "p",
+    "axb_gelu_bwd_colsum": "ppppp" "iiiii" "p",
+    "axb_gelu_fwd": "pplp",
+    "axb_gelu_bwd": "ppplp",
+    "axb_swiglu_fwd": "ppiip",
+    "axb_swiglu_bwd": "pppiip",
+    "axb_rope": "pp" "l" "iiii" "l" "i" "p",
+    "axb_flash_attn_fwd": "ppp" "iiiii" "f" "i" "p",
+    "axb_flash_attn_bwd_split": "pppppp" "iiiii" "f" "ii" "p",
+    "axb_flash_attn_bwd_scratch": "iii",
+    "axb_ce_fwd_mean": "pppppp" "ii" "l" "p",
+    "axb_ce_bwd": "pppp" "iii" "l" "p",
+    "axb_multi_l2norm_sq": "p" "il" "pp",
+    "axb_multi_scale": "p" "il" "pp",
+    "axb_multi_adamw": "p" "il" "fffffff" "ppp",
+    "axb_prune_topk": "p" "lil" "p" "i" "p",
+}
+_CTYPES = {"i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float, "p": ctypes.c_void_p}
+
+
 def available() -> bool:
     return os.path.exists(LIB_PATH)
 
@@ -48,11 +79,16 @@ def lib():
                 from ..utils import build
 
                 build.build_library(verbose=False)
-            _LIB = ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)
-            _LIB.axb_last_error.restype = ctypes.c_char_p
+            L = ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)
+            L.axb_last_error.restype = ctypes.c_char_p
+            for name, sig in _SIGNATURES.items():
+                if hasattr(L, name):
+                    getattr(L, name).argtypes = [_CTYPES[c] for c in sig]
+            L.axb_flash_attn_bwd_scratch.restype = ctypes.c_longlong
             ms = os.environ.get("AXONN_COMM_TIMEOUT_MS")
             if ms:
-                _LIB.axb_set_wait_timeout_ms(ctypes.c_uint(int(ms)))
+                L.axb_set_wait_timeout_ms(ctypes.c_uint(int(ms)))
+            _LIB = L      # published when complete: another thread may be waiting for it without the lock
     return _LIB
 
 
@@ -71,6 +107,16 @@ def use_cuda_kernels(*tensors) -> bool:
 
 def stream_ptr() -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def stream() -> int:
+    """Address of the current CUDA stream of the current device, for launchers with declared argument types."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def addr(t):
+    """Device address of ``t`` (``None``: null), for launchers with declared argument types."""
+    return None if t is None else t.data_ptr()
 
 
 def ptr(t) -> ctypes.c_void_p:

@@ -1,7 +1,5 @@
 """GELU (tanh form) and SwiGLU (``csrc/elementwise.cu``)."""
 
-import ctypes
-
 import torch
 import torch.nn.functional as F
 
@@ -15,8 +13,8 @@ class _GeluFn(torch.autograd.Function):
         if x.is_cuda and x.dtype == torch.bfloat16 and x.numel() % 8 == 0:
             x = x.contiguous()
             y = torch.empty_like(x)
-            _lib.check(_lib.lib().axb_gelu_fwd(_lib.ptr(x), _lib.ptr(y), ctypes.c_longlong(x.numel()),
-                                               _lib.stream_ptr()), "axb_gelu_fwd")
+            _lib.check(_lib.lib().axb_gelu_fwd(_lib.addr(x), _lib.addr(y), x.numel(),
+                                               _lib.stream()), "axb_gelu_fwd")
             return y
         if x.is_cuda:
             raise TypeError("gelu kernel needs bf16 input with numel % 8 == 0")
@@ -38,15 +36,15 @@ def gelu_backward_colsum(dy, x, out_dtype=torch.float32):
         rows, n = x.shape
         L = _lib.lib()
         dev = x.device.index
-        splits = L.axb_colsum_splits(ctypes.c_int(dev), ctypes.c_int(rows), ctypes.c_int(n))
+        splits = L.axb_colsum_splits(dev, rows, n)
         part = torch.empty((splits, n), dtype=torch.float32, device=x.device)
         colsum = torch.empty(n, dtype=out_dtype, device=x.device)
         dx = torch.empty_like(x)
-        _lib.check(L.axb_gelu_bwd_colsum(_lib.ptr(dy), _lib.ptr(x), _lib.ptr(dx), _lib.ptr(part), _lib.ptr(colsum),
-                                         ctypes.c_int(rows), ctypes.c_int(n),
-                                         ctypes.c_int(0 if x.dtype == torch.bfloat16 else 1),
-                                         ctypes.c_int({torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}[out_dtype]),
-                                         ctypes.c_int(dev), _lib.stream_ptr()), "axb_gelu_bwd_colsum")
+        _lib.check(L.axb_gelu_bwd_colsum(_lib.addr(dy), _lib.addr(x), _lib.addr(dx), _lib.addr(part), _lib.addr(colsum),
+                                         rows, n,
+                                         0 if x.dtype == torch.bfloat16 else 1,
+                                         {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}[out_dtype],
+                                         dev, _lib.stream()), "axb_gelu_bwd_colsum")
         _lib.add_launches(1)
         return dx, colsum
     dx = gelu_backward(dy, x)
@@ -58,8 +56,8 @@ def gelu_backward(dy, x):
     if x.is_cuda:
         x, dy = x.contiguous(), dy.contiguous()
         dx = torch.empty_like(x)
-        _lib.check(_lib.lib().axb_gelu_bwd(_lib.ptr(dy), _lib.ptr(x), _lib.ptr(dx),
-                                           ctypes.c_longlong(x.numel()), _lib.stream_ptr()), "axb_gelu_bwd")
+        _lib.check(_lib.lib().axb_gelu_bwd(_lib.addr(dy), _lib.addr(x), _lib.addr(dx),
+                                           x.numel(), _lib.stream()), "axb_gelu_bwd")
         return dx
     xf = x.float()
     k0, k1 = 0.7978845608028654, 0.044715
@@ -89,8 +87,8 @@ class _SwiGLUFn(torch.autograd.Function):
                 raise TypeError("swiglu kernel needs bf16 input with F % 8 == 0")
             g2 = gu.reshape(-1, F2).contiguous()
             out = torch.empty((g2.shape[0], Fh), dtype=gu.dtype, device=gu.device)
-            _lib.check(_lib.lib().axb_swiglu_fwd(_lib.ptr(g2), _lib.ptr(out), ctypes.c_int(g2.shape[0]),
-                                                 ctypes.c_int(Fh), _lib.stream_ptr()), "axb_swiglu_fwd")
+            _lib.check(_lib.lib().axb_swiglu_fwd(_lib.addr(g2), _lib.addr(out), g2.shape[0],
+                                                 Fh, _lib.stream()), "axb_swiglu_fwd")
             return out.reshape(*gu.shape[:-1], Fh)
         g, u = _split_gu(gu)
         return F.silu(g) * u
@@ -104,9 +102,9 @@ class _SwiGLUFn(torch.autograd.Function):
             g2 = gu.reshape(-1, F2).contiguous()
             d2 = dout.reshape(-1, Fh).contiguous()
             dgu = torch.empty_like(g2)
-            _lib.check(_lib.lib().axb_swiglu_bwd(_lib.ptr(d2), _lib.ptr(g2), _lib.ptr(dgu),
-                                                 ctypes.c_int(g2.shape[0]), ctypes.c_int(Fh),
-                                                 _lib.stream_ptr()), "axb_swiglu_bwd")
+            _lib.check(_lib.lib().axb_swiglu_bwd(_lib.addr(d2), _lib.addr(g2), _lib.addr(dgu),
+                                                 g2.shape[0], Fh,
+                                                 _lib.stream()), "axb_swiglu_bwd")
             return dgu.reshape(gu.shape)
         g, u = (t.float() for t in _split_gu(gu))
         s = torch.sigmoid(g)

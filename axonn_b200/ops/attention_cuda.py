@@ -39,9 +39,9 @@ def flash_fwd_packed(qkv, scale):
     qpk = n - 2
     out = torch.empty((B, S, G * qpk, D), dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty((B, G * qpk, S), dtype=torch.float32, device=qkv.device)
-    st = _lib.lib().axb_flash_attn_fwd(_lib.ptr(qkv), _lib.ptr(out), _lib.ptr(lse), ctypes.c_int(B), ctypes.c_int(S),
-                                       ctypes.c_int(G), ctypes.c_int(qpk), ctypes.c_int(D), ctypes.c_float(scale),
-                                       ctypes.c_int(qkv.device.index), _lib.stream_ptr())
+    st = _lib.lib().axb_flash_attn_fwd(_lib.addr(qkv), _lib.addr(out), _lib.addr(lse), B, S,
+                                       G, qpk, D, scale,
+                                       qkv.device.index, _lib.stream())
     _lib.check(st, "axb_flash_attn_fwd")
     return out, lse
 
@@ -49,13 +49,12 @@ def flash_fwd_packed(qkv, scale):
 def _bwd_split(qkv, out, d_out, lse, dqkv, scale, which):
     B, S, G, n, D = qkv.shape
     L = _lib.lib()
-    L.axb_flash_attn_bwd_scratch.restype = ctypes.c_longlong
-    words = L.axb_flash_attn_bwd_scratch(ctypes.c_int(B), ctypes.c_int(S), ctypes.c_int(G * (n - 2)))
+    words = L.axb_flash_attn_bwd_scratch(B, S, G * (n - 2))
     scratch = torch.empty(words, dtype=torch.float32, device=qkv.device)
     st = L.axb_flash_attn_bwd_split(
-        _lib.ptr(qkv), _lib.ptr(out), _lib.ptr(d_out), _lib.ptr(lse), _lib.ptr(scratch), _lib.ptr(dqkv),
-        ctypes.c_int(B), ctypes.c_int(S), ctypes.c_int(G), ctypes.c_int(n - 2), ctypes.c_int(D),
-        ctypes.c_float(scale), ctypes.c_int(which), ctypes.c_int(qkv.device.index), _lib.stream_ptr())
+        _lib.addr(qkv), _lib.addr(out), _lib.addr(d_out), _lib.addr(lse), _lib.addr(scratch), _lib.addr(dqkv),
+        B, S, G, n - 2, D,
+        scale, which, qkv.device.index, _lib.stream())
     _lib.check(st, "axb_flash_attn_bwd_split")
     _lib.add_launches(1 if which != 3 else 2)
 

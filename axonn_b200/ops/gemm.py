@@ -45,11 +45,11 @@ def _launch(layout, a, b, M, N, K, out, bias=None, epilogue=EPI_NONE, accumulate
         raise ValueError(f"gemm dims must be multiples of 8 for 16-byte TMA strides, got M={M} N={N} K={K}")
     L = _lib.lib()
     st = L.axb_gemm(
-        ctypes.c_int(layout), _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), _lib.ptr(bias), _lib.ptr(aux),
-        ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
-        ctypes.c_int(_DT[a.dtype]), ctypes.c_int(_DT[out.dtype]),
-        ctypes.c_int(epilogue), ctypes.c_int(1 if accumulate else 0),
-        ctypes.c_int(a.device.index), _lib.stream_ptr())
+        layout, _lib.addr(a), _lib.addr(b), _lib.addr(out), _lib.addr(bias), _lib.addr(aux),
+        M, N, K,
+        _DT[a.dtype], _DT[out.dtype],
+        epilogue, 1 if accumulate else 0,
+        a.device.index, _lib.stream())
     _lib.check(st, "axb_gemm")
     return out
 

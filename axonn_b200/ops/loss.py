@@ -31,9 +31,9 @@ class _CrossEntropyFn(torch.autograd.Function):
                 lse = torch.empty(rows, dtype=torch.float32, device=z.device)
                 # two tensors: the loss is returned, and a view made in here could not be modified in place later
                 mean, kept = (torch.empty((), dtype=torch.float32, device=z.device) for _ in range(2))
-                _lib.check(_lib.lib().axb_ce_fwd_mean(_lib.ptr(z), _lib.ptr(t), _lib.ptr(stats), _lib.ptr(lse),
-                                                      _lib.ptr(mean), _lib.ptr(kept), ctypes.c_int(rows), ctypes.c_int(V),
-                                                      ctypes.c_longlong(ignore_index), _lib.stream_ptr()),
+                _lib.check(_lib.lib().axb_ce_fwd_mean(_lib.addr(z), _lib.addr(t), _lib.addr(stats), _lib.addr(lse),
+                                                      _lib.addr(mean), _lib.addr(kept), rows, V,
+                                                      ignore_index, _lib.stream()),
                            "axb_ce_fwd_mean")
                 _lib.add_launches(1)
                 ctx.save_for_backward(z, t, lse, kept)
@@ -69,9 +69,9 @@ class _CrossEntropyFn(torch.autograd.Function):
         V = z.shape[-1]
         scale = (g.float() / count).reshape(1).contiguous()
         if z.is_cuda:
-            _lib.check(_lib.lib().axb_ce_bwd(_lib.ptr(z), _lib.ptr(t), _lib.ptr(lse), _lib.ptr(scale),
-                                             ctypes.c_int(z.shape[0]), ctypes.c_int(V), ctypes.c_int(ctx.start),
-                                             ctypes.c_longlong(ctx.ignore_index), _lib.stream_ptr()), "axb_ce_bwd")
+            _lib.check(_lib.lib().axb_ce_bwd(_lib.addr(z), _lib.addr(t), _lib.addr(lse), _lib.addr(scale),
+                                             z.shape[0], V, ctx.start,
+                                             ctx.ignore_index, _lib.stream()), "axb_ce_bwd")
             return z.reshape(ctx.shape), None, None, None
         p = (z.float() - lse[:, None]).exp()
         loc = t - ctx.start

@@ -63,8 +63,8 @@ def multi_tensor_l2norm_sq(tensors):
     if tensors[0].is_cuda:
         tab = _cached_table(tensors)
         out = torch.zeros((), dtype=torch.float32, device=tensors[0].device)
-        st = _lib.lib().axb_multi_l2norm_sq(_lib.ptr(tab.dev), ctypes.c_int(tab.n),
-                                            ctypes.c_longlong(tab.total_chunks), _lib.ptr(out), _lib.stream_ptr())
+        st = _lib.lib().axb_multi_l2norm_sq(_lib.addr(tab.dev), tab.n,
+                                            tab.total_chunks, _lib.addr(out), _lib.stream())
         _lib.check(st, "axb_multi_l2norm_sq")
         return out
     return torch.stack([t.detach().float().pow(2).sum() for t in tensors]).sum()
@@ -82,8 +82,8 @@ def multi_tensor_scale_(tensors, scale):
             scale = torch.full((), float(scale), dtype=torch.float32, device=tensors[0].device)   # no host sync
         else:
             scale = scale.to(device=tensors[0].device, dtype=torch.float32)
-        st = _lib.lib().axb_multi_scale(_lib.ptr(tab.dev), ctypes.c_int(tab.n),
-                                        ctypes.c_longlong(tab.total_chunks), _lib.ptr(scale), _lib.stream_ptr())
+        st = _lib.lib().axb_multi_scale(_lib.addr(tab.dev), tab.n,
+                                        tab.total_chunks, _lib.addr(scale), _lib.stream())
         _lib.check(st, "axb_multi_scale")
         return
     for t in tensors:

@@ -8,8 +8,6 @@ reference's models rely on (``external/models/nvidia_transformer.py:57-95``,
 ``axonn/models/transformers/modify_llama.py``).
 """
 
-import ctypes
-
 import torch
 import torch.distributed as dist
 
@@ -19,7 +17,7 @@ _DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
 def _group_size(group):
-    return 1 if group is None else dist.get_world_size(group)
+    return 1 if group is None else (group.size() if isinstance(group, dist.ProcessGroup) else dist.get_world_size(group))
 
 
 def _torch_norm_fwd(x, gamma, beta, eps, rms, group):
@@ -62,10 +60,10 @@ class _NormFn(torch.autograd.Function):
         b = None if beta is None else (beta.to(x2.dtype) if beta.dtype != x2.dtype else beta)
 
         def call(mode):
-            st = L.axb_norm_fwd(_lib.ptr(x2), _lib.ptr(g), _lib.ptr(b), _lib.ptr(y), _lib.ptr(stats),
-                                ctypes.c_int(rows), ctypes.c_int(H), ctypes.c_int(H * n), ctypes.c_float(eps),
-                                ctypes.c_int(1 if rms else 0), ctypes.c_int(mode), ctypes.c_int(_DT[x2.dtype]),
-                                ctypes.c_int(dev), _lib.stream_ptr())
+            st = L.axb_norm_fwd(_lib.addr(x2), _lib.addr(g), _lib.addr(b), _lib.addr(y), _lib.addr(stats),
+                                rows, H, H * n, eps,
+                                1 if rms else 0, mode, _DT[x2.dtype],
+                                dev, _lib.stream())
             _lib.check(st, "axb_norm_fwd")
 
         if n == 1:
@@ -101,18 +99,19 @@ class _NormFn(torch.autograd.Function):
         rows = x2.shape[0]
         L = _lib.lib()
         dev = x2.device.index
-        grid = L.axb_norm_grid(ctypes.c_int(dev), ctypes.c_int(rows))
+        grid = L.axb_norm_grid(dev, rows)
         dx = torch.empty_like(x2)
         sums = torch.empty((rows, 2), dtype=torch.float32, device=x2.device) if n > 1 else None
         part = torch.empty((2, grid, H), dtype=torch.float32, device=x2.device)
-        dgb = torch.empty((2, H), dtype=g.dtype, device=x2.device)   # written in the parameter's dtype: no cast kernel
+        pa = part.data_ptr()
+        # written in the parameter's dtype: no cast kernel
+        dg, db = torch.empty_like(g), (None if rms else torch.empty_like(g))
 
         def call(mode):
-            st = L.axb_norm_bwd(_lib.ptr(dy2), _lib.ptr(x2), _lib.ptr(g), _lib.ptr(stats), _lib.ptr(dx),
-                                _lib.ptr(sums), _lib.ptr(part[0]), _lib.ptr(part[1]), _lib.ptr(dgb[0]),
-                                _lib.ptr(dgb[1]), ctypes.c_int(rows), ctypes.c_int(H), ctypes.c_int(H * n),
-                                ctypes.c_int(1 if rms else 0), ctypes.c_int(mode), ctypes.c_int(_DT[x2.dtype]),
-                                ctypes.c_int(_DT[g.dtype]), ctypes.c_int(dev), _lib.stream_ptr())
+            st = L.axb_norm_bwd(_lib.addr(dy2), _lib.addr(x2), _lib.addr(g), _lib.addr(stats), _lib.addr(dx),
+                                _lib.addr(sums), pa, pa + grid * H * 4, _lib.addr(dg), _lib.addr(db), rows, H, H * n,
+                                1 if rms else 0, mode, _DT[x2.dtype],
+                                _DT[g.dtype], dev, _lib.stream())
             _lib.check(st, "axb_norm_bwd")
             if mode != 1:
                 _lib.add_launches(1)
@@ -123,9 +122,7 @@ class _NormFn(torch.autograd.Function):
             call(1)
             dist.all_reduce(sums, group=group)
             call(2)
-        dgamma = dgb[0]
-        dbeta = dgb[1] if ctx.has_beta else None
-        return dx.reshape(ctx.shape), dgamma, dbeta, None, None, None
+        return dx.reshape(ctx.shape), dg, (db if ctx.has_beta else None), None, None, None
 
 
 class _AddNormFn(torch.autograd.Function):
@@ -156,10 +153,10 @@ class _AddNormFn(torch.autograd.Function):
         b = None if beta is None else (beta.to(x2.dtype) if beta.dtype != x2.dtype else beta)
 
         def call(mode, src, dl):
-            st = L.axb_add_norm_fwd(_lib.ptr(src), _lib.ptr(dl), _lib.ptr(h if dl is not None else None), _lib.ptr(g),
-                                    _lib.ptr(b), _lib.ptr(y), _lib.ptr(stats), ctypes.c_int(rows), ctypes.c_int(H),
-                                    ctypes.c_int(H * n), ctypes.c_float(eps), ctypes.c_int(1 if rms else 0),
-                                    ctypes.c_int(mode), ctypes.c_int(_DT[x2.dtype]), ctypes.c_int(dev), _lib.stream_ptr())
+            st = L.axb_add_norm_fwd(_lib.addr(src), _lib.addr(dl), _lib.addr(h if dl is not None else None), _lib.addr(g),
+                                    _lib.addr(b), _lib.addr(y), _lib.addr(stats), rows, H,
+                                    H * n, eps, 1 if rms else 0,
+                                    mode, _DT[x2.dtype], dev, _lib.stream())
             _lib.check(st, "axb_add_norm_fwd")
 
         if n == 1:
@@ -199,18 +196,18 @@ class _AddNormFn(torch.autograd.Function):
         rows = x2.shape[0]
         L = _lib.lib()
         dev = x2.device.index
-        grid = L.axb_norm_grid(ctypes.c_int(dev), ctypes.c_int(rows))
+        grid = L.axb_norm_grid(dev, rows)
         dx = torch.empty_like(x2)
         sums = torch.empty((rows, 2), dtype=torch.float32, device=x2.device) if n > 1 else None
         part = torch.empty((2, grid, H), dtype=torch.float32, device=x2.device)
-        dgb = torch.empty((2, H), dtype=g.dtype, device=x2.device)
+        pa = part.data_ptr()
+        dg, db = torch.empty_like(g), (None if rms else torch.empty_like(g))
 
         def call(mode):
-            st = L.axb_add_norm_bwd(_lib.ptr(dy2), _lib.ptr(dh2), _lib.ptr(x2), _lib.ptr(g), _lib.ptr(stats), _lib.ptr(dx),
-                                    _lib.ptr(sums), _lib.ptr(part[0]), _lib.ptr(part[1]), _lib.ptr(dgb[0]),
-                                    _lib.ptr(dgb[1]), ctypes.c_int(rows), ctypes.c_int(H), ctypes.c_int(H * n),
-                                    ctypes.c_int(1 if rms else 0), ctypes.c_int(mode), ctypes.c_int(_DT[x2.dtype]),
-                                    ctypes.c_int(_DT[g.dtype]), ctypes.c_int(dev), _lib.stream_ptr())
+            st = L.axb_add_norm_bwd(_lib.addr(dy2), _lib.addr(dh2), _lib.addr(x2), _lib.addr(g), _lib.addr(stats), _lib.addr(dx),
+                                    _lib.addr(sums), pa, pa + grid * H * 4, _lib.addr(dg), _lib.addr(db), rows, H, H * n,
+                                    1 if rms else 0, mode, _DT[x2.dtype],
+                                    _DT[g.dtype], dev, _lib.stream())
             _lib.check(st, "axb_add_norm_bwd")
             if mode != 1:
                 _lib.add_launches(1)
@@ -222,7 +219,7 @@ class _AddNormFn(torch.autograd.Function):
             dist.all_reduce(sums, group=group)
             call(2)
         dx = dx.reshape(ctx.shape)
-        return dx, dx, dgb[0], (dgb[1] if ctx.has_beta else None), None, None, None
+        return dx, dx, dg, (db if ctx.has_beta else None), None, None, None
 
 
 def add_layer_norm(x, delta, gamma, beta, eps=1e-5, group=None):
@@ -258,11 +255,11 @@ def column_sum(x, out_dtype=torch.float32):
     rows, n = x.shape
     L = _lib.lib()
     dev = x.device.index
-    splits = L.axb_colsum_splits(ctypes.c_int(dev), ctypes.c_int(rows), ctypes.c_int(n))
+    splits = L.axb_colsum_splits(dev, rows, n)
     part = torch.empty((splits, n), dtype=torch.float32, device=x.device)
     out = torch.empty(n, dtype=out_dtype, device=x.device)
-    _lib.check(L.axb_colsum(_lib.ptr(x), _lib.ptr(part), _lib.ptr(out), ctypes.c_int(rows), ctypes.c_int(n),
-                            ctypes.c_int(_DT[x.dtype]), ctypes.c_int(_DT[out_dtype]), ctypes.c_int(dev),
-                            _lib.stream_ptr()), "axb_colsum")
+    _lib.check(L.axb_colsum(_lib.addr(x), _lib.addr(part), _lib.addr(out), rows, n,
+                            _DT[x.dtype], _DT[out_dtype], dev,
+                            _lib.stream()), "axb_colsum")
     _lib.add_launches(1)
     return out

@@ -35,9 +35,9 @@ def multi_tensor_adamw(table, lr, beta1, beta2, eps, weight_decay, step, grad_sc
     bc1 = 1.0 - beta1 ** step
     bc2 = 1.0 - beta2 ** step
     st = _lib.lib().axb_multi_adamw(
-        _lib.ptr(table.dev), ctypes.c_int(table.n), ctypes.c_longlong(table.total_chunks), ctypes.c_float(lr),
-        ctypes.c_float(beta1), ctypes.c_float(beta2), ctypes.c_float(eps), ctypes.c_float(weight_decay),
-        ctypes.c_float(bc1), ctypes.c_float(bc2), _lib.ptr(grad_scale), _lib.ptr(found_inf), _lib.stream_ptr())
+        _lib.addr(table.dev), table.n, table.total_chunks, lr,
+        beta1, beta2, eps, weight_decay,
+        bc1, bc2, _lib.addr(grad_scale), _lib.addr(found_inf), _lib.stream())
     _lib.check(st, "axb_multi_adamw")
 
 
@@ -70,8 +70,8 @@ def prune_topk_(grad, keep_fraction):
         if ws is None:
             ws = torch.empty(L.axb_prune_workspace_words(), dtype=torch.int32, device=dev)
             _prune_ws[dev] = ws
-        st = L.axb_prune_topk(_lib.ptr(grad), ctypes.c_longlong(n), ctypes.c_int(_LIB_DTYPE[grad.dtype]),
-                              ctypes.c_longlong(k), _lib.ptr(ws), ctypes.c_int(dev.index), _lib.stream_ptr())
+        st = L.axb_prune_topk(_lib.addr(grad), n, _LIB_DTYPE[grad.dtype],
+                              k, _lib.addr(ws), dev.index, _lib.stream())
         _lib.check(st, "axb_prune_topk")
         _lib.add_launches(2)
         return grad

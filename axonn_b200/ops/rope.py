@@ -1,8 +1,6 @@
 """Rotary position embedding, applied in place to ``[B, S, heads, D]`` tensors
 (rotate-half convention, pairs ``(i, i + D/2)``; kernel in ``csrc/elementwise.cu``)."""
 
-import ctypes
-
 import torch
 
 from . import _lib
@@ -48,9 +46,9 @@ def _rope_apply(x, table, inverse):
         G = x.shape[2]
         rows, pos_div, row_stride = x.shape[0] * S * G, G, x.stride(2)
         assert x.stride(1) == G * x.stride(2) and x.stride(0) == S * x.stride(1)
-    st = _lib.lib().axb_rope(_lib.ptr(x), _lib.ptr(table), ctypes.c_longlong(rows), ctypes.c_int(S),
-                             ctypes.c_int(nh), ctypes.c_int(D), ctypes.c_int(pos_div),
-                             ctypes.c_longlong(row_stride), ctypes.c_int(1 if inverse else 0), _lib.stream_ptr())
+    st = _lib.lib().axb_rope(_lib.addr(x), _lib.addr(table), rows, S,
+                             nh, D, pos_div,
+                             row_stride, 1 if inverse else 0, _lib.stream())
     _lib.check(st, "axb_rope")
     return x
 
