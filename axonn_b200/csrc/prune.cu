@@ -41,6 +41,8 @@ static_assert(sizeof(PruneMeta) == 32, "scratch layout");
 template <int BINS>
 __device__ void prune_select(const unsigned int* __restrict__ hist, long long k, long long* bin, long long* rank) {
   __shared__ unsigned long long warp_sum[PR_THREADS / 32];
+  __shared__ unsigned long long found_above;
+  __shared__ int found_hi;
   constexpr int PER = BINS / PR_THREADS;
   // thread t owns bins [BINS - (t+1)*PER, BINS - t*PER): thread 0 holds the largest magnitudes
   const int hi = BINS - threadIdx.x * PER, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -65,15 +67,29 @@ __device__ void prune_select(const unsigned int* __restrict__ hist, long long k,
   __syncthreads();
   incl += warp_sum[w];
   const unsigned long long excl = incl - mine;
-  if (excl < (unsigned long long)k && (unsigned long long)k <= incl) {
-    unsigned long long above = excl;
-    for (int b = hi - 1; b >= hi - PER; --b) {
-      const unsigned long long c = __ldcg(hist + b);
-      if (above + c >= (unsigned long long)k) { *bin = b; if (rank) *rank = k - (long long)above; return; }
-      above += c;
-    }
+  if (threadIdx.x == 0) found_hi = 0;
+  __syncthreads();
+  if (excl < (unsigned long long)k && (unsigned long long)k <= incl) { found_hi = hi; found_above = excl; }
+  __syncthreads();
+  if (w != 0) return;
+  if (found_hi == 0) {                                     // k > n: keep all
+    if (lane == 0) { *bin = 0; if (rank) *rank = 1; }
+    return;
   }
-  if (threadIdx.x == PR_THREADS - 1 && incl < (unsigned long long)k) { *bin = 0; if (rank) *rank = 1; }  // k > n: keep all
+  // one warp looks through that thread's bins, 32 at a time from the top
+  unsigned long long above = found_above;
+  for (int top = found_hi; top > found_hi - PER; top -= 32) {
+    const unsigned long long c = __ldcg(hist + top - 1 - lane);
+    unsigned long long upto = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const unsigned long long u = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += u; }
+    const unsigned hit = __ballot_sync(0xffffffffu, above + upto >= (unsigned long long)k);
+    if (hit) {
+      if (lane == __ffs(hit) - 1) { *bin = top - 1 - lane; if (rank) *rank = k - (long long)(above + upto - c); }
+      return;
+    }
+    above += __shfl_sync(0xffffffffu, upto, 31);
+  }
 }
 
 // True in every thread of the block that arrives last (its predecessors' histogram updates are visible to it).
