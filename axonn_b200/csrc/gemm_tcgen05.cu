@@ -1804,7 +1804,17 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
   // K-major operand [R, K]: box 64(K) x tile rows.  MN-major operand [K, R]: box 64(R) x 64(K).
   if (a_mn == 0) { if (make_tmap_2d_16bit(&tmA, A, M, K, BM, in_dtype)) return -1; }
   else           { if (make_tmap_2d_16bit(&tmA, A, K, M, BK, in_dtype)) return -1; }
-  const bool pair = !comm && BN == 256 && pair_mode_enabled() && enough_pairs;
+  // Plain GEMMs run on CTA pairs whenever those need less time than single CTAs with 128x128 tiles.  A pair's 256x256
+  // tile is twice the work per SM, but single CTAs reach only 0.6 of its rate (their operands exceed the shared-memory
+  // bandwidth), so the pairs win as long as they need at most 5 waves where single CTAs need 6 of half the size - in
+  // particular with one wave of pairs against two, which the demand for a full wave of pairs used to rule out.  One B200,
+  // bf16: 2048 x 2048 x 16384 119.8 -> 97.0 us, 777 x 4096 x 4096 30.1 -> 26.7 us, 1000 x 1024 x 4096 16.6 -> 14.1 us.
+  const long long pair_tiles = static_cast<long long>((tiles_m + 1) / 2) * ((N + 255) / 256);
+  const long long single_tiles = static_cast<long long>(tiles_m) * ((N + 127) / 128);
+  const int sms = usable_sms(device);
+  const long long pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2), single_waves = (single_tiles + sms - 1) / sms;
+  const bool pair = !comm && pair_mode_enabled() && ((BN == 256 && enough_pairs) || 6 * pair_waves <= 5 * single_waves);
+  if (pair) BN = 256;
   const int splitk = (comm || pair || BN != 128) ? 1 : splitk_ctas(M, N, K, usable_sms(device), device);
   if (b_mn == 0) { if (make_tmap_2d_16bit(&tmB, B, N, K, (pair || comm_pair) ? BN / 2 : BN, in_dtype)) return -1; }
   else           { if (make_tmap_2d_16bit(&tmB, B, K, N, BK, in_dtype)) return -1; }
