@@ -1175,6 +1175,14 @@ __device__ __forceinline__ bool pair_tile_computed(const GemmParams& p, int e, i
   return true;
 }
 
+// K blocks of problem e that the kernel walks.  With one segment per problem (all tokens of an expert come from this
+// rank) the blocks with data are the first ones, and the producer and the MMA issuer loop over just those instead of
+// asking for every block: the question was a dependent global load in front of every MMA.
+__device__ __forceinline__ int pair_kb_count(const GemmParams& p, int e, int num_kb) {
+  if (p.mask_mode != 2 || p.nseg != 1) return num_kb;
+  return min(num_kb, (__ldg(p.seg_counts + e) + BK - 1) / BK);
+}
+
 template <int A_MN, int B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -1229,8 +1237,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // row coordinate of problem e in the stacked operands (rows = M or N for a K-major operand, K otherwise)
         const int a_r = e * p.a_batch_rows, b_r = e * p.b_batch_rows;
         if (p.mask_mode == 1 && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, tm2 * 2 * BM, 2 * BM)) continue;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (p.mask_mode == 2 && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, kb * BK, BK)) continue;
+        const int kb_end = pair_kb_count(p, e, num_kb);
+        for (int kb = 0; kb < kb_end; ++kb) {
+          if (p.mask_mode == 2 && p.nseg > 1 && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, kb * BK, BK)) continue;
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, timeout)) { ok = false; break; }
           uint8_t* sA = smem + stage * S::STAGE_BYTES;
           uint8_t* sB = sA + S::A_BYTES;
@@ -1276,8 +1285,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tcgen05_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
         bool first = true;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (p.mask_mode == 2 && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, kb * BK, BK)) continue;
+        const int kb_end = pair_kb_count(p, e, num_kb);
+        for (int kb = 0; kb < kb_end; ++kb) {
+          if (p.mask_mode == 2 && p.nseg > 1 && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, kb * BK, BK)) continue;
           if (!mbar_wait(&full_bar[stage], phase, abort_flag, timeout)) { ok = false; break; }
           tcgen05_fence_after();
           const uint32_t a_addr = smem_u32(smem + stage * S::STAGE_BYTES);
