@@ -420,11 +420,15 @@ template <int HD>
 struct DkvSmem {
   static constexpr int TILE = 128 * HD * 2;
   static constexpr int K_OFF = 0, V_OFF = TILE;
+  // Q / dO: two query tiles of two halves (64 queries) each.  A half is loaded and released by itself: its step's
+  // accumulator MMAs free it a whole tile before its successor is needed, which hides the load; a ring of whole tiles
+  // got half a tile's time for that and the MMA warps waited for it in every tile.
+  // dK / dV kernel on a B200: 8 x 2048, 16 heads, head_dim 128 338 -> 318 us; head_dim 64 285 -> 244 us.
   static constexpr int Q_OFF = 2 * TILE;           // 2 stages
   static constexpr int DO_OFF = 4 * TILE;          // 2 stages
   static constexpr int LSE_OFF = 6 * TILE;         // [2 stages][lse, delta][128] fp32
   static constexpr int BAR_OFF = LSE_OFF + 2048;
-  static constexpr int NBARS = 2 + 4 + 2 + 2 + 2;
+  static constexpr int NBARS = 2 + 8 + 2 + 2 + 2;
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 16 + 1024;
 };
 
@@ -458,12 +462,12 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S_::BAR_OFF);
   uint64_t* kv_full = bars;          // K and V of the item
   uint64_t* kv_empty = bars + 1;     // both MMA warps are done with them
-  uint64_t* qdo_full = bars + 2;     // [stage]: Q, dO, lse, delta of a query tile
-  uint64_t* qdo_empty = bars + 4;    // [stage]: 2 MMA warps + 16 softmax warps
-  uint64_t* sdp_full = bars + 6;     // [score buffer]: S^T and dP^T of a step (one arrival per MMA warp)
-  uint64_t* pds_full = bars + 8;     // [score buffer]: P^T and dS^T of a step are in tensor memory
-  uint64_t* acc_done = bars + 10;    // dK and dV of the item are final (one arrival per MMA warp)
-  uint64_t* acc_free = bars + 11;    // ... and have been read: the next item may overwrite them
+  uint64_t* qdo_full = bars + 2;     // [stage][half]: Q, dO, lse, delta of 64 queries
+  uint64_t* qdo_empty = bars + 6;    // [stage][half]: 2 MMA warps + the half's 8 softmax warps
+  uint64_t* sdp_full = bars + 10;    // [score buffer]: S^T and dP^T of a step (one arrival per MMA warp)
+  uint64_t* pds_full = bars + 12;    // [score buffer]: P^T and dS^T of a step are in tensor memory
+  uint64_t* acc_done = bars + 14;    // dK and dV of the item are final (one arrival per MMA warp)
+  uint64_t* acc_free = bars + 15;    // ... and have been read: the next item may overwrite them
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + S_::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   float* lse_s = reinterpret_cast<float*>(smem + S_::LSE_OFF);
@@ -475,10 +479,8 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1); mbar_init(kv_empty, 2); mbar_init(acc_done, 2);
     mbar_init(acc_free, FS_SOFTMAX_WARPS);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 2 + FS_SOFTMAX_WARPS);
-      mbar_init(&sdp_full[i], 2); mbar_init(&pds_full[i], 8);
-    }
+    for (int i = 0; i < 4; ++i) { mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 2 + FS_SOFTMAX_WARPS / 2); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&sdp_full[i], 2); mbar_init(&pds_full[i], FS_SOFTMAX_WARPS / 2); }
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -504,27 +506,31 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
         if (!mbar_wait(kv_empty, (it & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
         mbar_expect_tx(kv_full, 2 * S_::TILE);
 #pragma unroll
-        for (int c = 0; c < HD / 64; ++c) {
-          tma_load_3d(smem + S_::K_OFF + c * 16384, &tmQKV, kv_full, col_k + 64 * c, krow, w.b);
-          tma_load_3d(smem + S_::V_OFF + c * 16384, &tmQKV, kv_full, col_k + HD + 64 * c, krow, w.b);
+        for (int c = 0; c < 2 * (HD / 64); ++c) {            // boxes of 64 rows x 64 columns
+          const int at = (c >> 1) * 16384 + (c & 1) * 8192, col = col_k + 64 * (c >> 1), row = krow + (c & 1) * 64;
+          tma_load_3d(smem + S_::K_OFF + at, &tmQKV, kv_full, col, row, w.b);
+          tma_load_3d(smem + S_::V_OFF + at, &tmQKV, kv_full, col + HD, row, w.b);
         }
         const int per_head = nq - w.jt;
         for (int t = 0; t < per_head * p.qpk && ok; ++t, ++tq) {
           const int jq = t / per_head, i = w.jt + t % per_head;
           const int head = w.g * p.qpk + jq;
           const int st = tq & 1;
-          const int row0 = i * 128;
-          if (!mbar_wait(&qdo_empty[st], ((tq >> 1) & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
-          mbar_expect_tx(&qdo_full[st], 2 * S_::TILE + 1024);
-#pragma unroll
-          for (int c = 0; c < HD / 64; ++c) {
-            tma_load_3d(smem + S_::Q_OFF + st * S_::TILE + c * 16384, &tmQKV, &qdo_full[st],
-                        (w.g * (p.qpk + 2) + jq) * HD + 64 * c, row0, w.b);
-            tma_load_3d(smem + S_::DO_OFF + st * S_::TILE + c * 16384, &tmDO, &qdo_full[st], head * HD + 64 * c, row0, w.b);
-          }
           const size_t vec = (static_cast<size_t>(w.b) * heads + head) * p.Sp + static_cast<size_t>(i) * 128;
-          bulk_load_1d(lse_s + st * 256, p.neg_lse2 + vec, 512, &qdo_full[st]);
-          bulk_load_1d(lse_s + st * 256 + 128, p.neg_delta + vec, 512, &qdo_full[st]);
+          for (int hq = 0; hq < 2; ++hq) {
+            uint64_t* full = &qdo_full[st * 2 + hq];
+            const int row0 = i * 128 + hq * 64;
+            if (!mbar_wait(&qdo_empty[st * 2 + hq], ((tq >> 1) & 1) ^ 1, abort_flag, timeout)) { ok = false; break; }
+            mbar_expect_tx(full, S_::TILE + 512);
+#pragma unroll
+            for (int c = 0; c < HD / 64; ++c) {
+              const int at = st * S_::TILE + c * 16384 + hq * 8192;
+              tma_load_3d(smem + S_::Q_OFF + at, &tmQKV, full, (w.g * (p.qpk + 2) + jq) * HD + 64 * c, row0, w.b);
+              tma_load_3d(smem + S_::DO_OFF + at, &tmDO, full, head * HD + 64 * c, row0, w.b);
+            }
+            bulk_load_1d(lse_s + st * 256 + hq * 64, p.neg_lse2 + vec + hq * 64, 256, full);
+            bulk_load_1d(lse_s + st * 256 + 128 + hq * 64, p.neg_delta + vec + hq * 64, 256, full);
+          }
         }
       }
       if (!ok) {
@@ -567,12 +573,13 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
       DkvItem w;
       for (int it = 0; ok && dkv_item(p, it, w); ++it) {
         const int ns = 2 * (nq - w.jt) * p.qpk;
-        if (!mbar_wait(kv_full, it & 1, abort_flag, timeout) ||
-            !mbar_wait(&qdo_full[tq & 1], (tq >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
-        tcgen05_fence_after();
+        if (!mbar_wait(kv_full, it & 1, abort_flag, timeout)) { ok = false; break; }
         // both buffers are free: the previous item's accumulator MMAs, which read them, were issued earlier
-        issue_t(tq & 1, 0); umma_commit(&sdp_full[0]);
-        issue_t(tq & 1, 1); umma_commit(&sdp_full[1]);
+        for (int hq = 0; hq < 2 && ok; ++hq) {
+          if (!mbar_wait(&qdo_full[(tq & 1) * 2 + hq], (tq >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
+          tcgen05_fence_after();
+          issue_t(tq & 1, hq); umma_commit(&sdp_full[hq]);
+        }
         for (int s = 0; s < ns && ok; ++s, ++c) {
           const uint32_t tile = tq + (s >> 1);
           const int hq = s & 1;
@@ -581,10 +588,10 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
           if (s == 0 && it > 0 && !mbar_wait(acc_free, (it - 1) & 1, abort_flag, timeout)) { ok = false; break; }
           tcgen05_fence_after();
           issue_acc(tile & 1, hq, s == 0);
-          if (hq == 1) umma_commit(&qdo_empty[tile & 1]);        // this warp's last read of the tile
+          umma_commit(&qdo_empty[(tile & 1) * 2 + hq]);          // this warp's last read of the half
           if (s + 2 < ns) {
             const uint32_t tn = tile + 1;
-            if (!mbar_wait(&qdo_full[tn & 1], (tn >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
+            if (!mbar_wait(&qdo_full[(tn & 1) * 2 + hq], (tn >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
             tcgen05_fence_after();
             issue_t(tn & 1, hq);
             umma_commit(&sdp_full[hq]);
@@ -619,7 +626,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
         const int st = tq & 1;
         const bool diag = t % per_head == 0;
         // -lse and -delta of the tile arrive with its Q and dO
-        if (!mbar_wait(&qdo_full[st], (tq >> 1) & 1, abort_flag, timeout) ||
+        if (!mbar_wait(&qdo_full[st * 2 + hq], (tq >> 1) & 1, abort_flag, timeout) ||
             !mbar_wait(&sdp_full[hq], tq & 1, abort_flag, timeout)) { ok = false; break; }
         tcgen05_fence_after();
         uint32_t sv[32], dv[32];
@@ -657,7 +664,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
         __syncwarp();
         if (lane == 0) {
           mbar_arrive(&pds_full[hq]);
-          mbar_arrive(&qdo_empty[st]);                // this warp has read its share of -lse / -delta
+          mbar_arrive(&qdo_empty[st * 2 + hq]);       // this warp has read its share of -lse / -delta
         }
       }
       if (!ok || !mbar_wait(acc_done, it & 1, abort_flag, timeout)) { ok = false; break; }
@@ -736,9 +743,11 @@ extern "C" int axb_flash_attn_bwd_split(const void* qkv, const void* out, const 
     fa_split_delta_kernel<64><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out),
                                                      lse, scratch, scratch + static_cast<size_t>(B) * H * Sp, B, S, Sp, H);
   AXB_CUDA(cudaGetLastError());
-  CUtensorMap tq, td;
-  if (make_tmap_3d_bf16(&tq, qkv, B, S, static_cast<uint64_t>(G) * (qpk + 2) * D, 128)) return -1;
-  if (make_tmap_3d_bf16(&td, d_out, B, S, static_cast<uint64_t>(H) * D, 128)) return -1;
+  CUtensorMap tq, td, tq64, td64;                     // dQ kernel: 128-row boxes, dK / dV kernel: 64-row boxes
+  const uint64_t cols = static_cast<uint64_t>(G) * (qpk + 2) * D, do_cols = static_cast<uint64_t>(H) * D;
+  if (make_tmap_3d_bf16(&tq, qkv, B, S, cols, 128) || make_tmap_3d_bf16(&td, d_out, B, S, do_cols, 128) ||
+      make_tmap_3d_bf16(&tq64, qkv, B, S, cols, 64) || make_tmap_3d_bf16(&td64, d_out, B, S, do_cols, 64))
+    return -1;
   FaSplitParams p;
   p.neg_lse2 = scratch; p.neg_delta = scratch + static_cast<size_t>(B) * H * Sp; p.dqkv = static_cast<__nv_bfloat16*>(dqkv);
   p.B = B; p.S = S; p.Sp = Sp; p.G = G; p.qpk = qpk; p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
@@ -750,8 +759,8 @@ extern "C" int axb_flash_attn_bwd_split(const void* qkv, const void* out, const 
   { static int dbg = -1; if (dbg < 0) { const char* e = getenv("AXB_FA_DEBUG"); dbg = e ? atoi(e) : 0; } p.debug = dbg; }
 #endif
   if (which & 2) {
-    if (D == 128) { if (dkv_launch<128>(tq, td, p, device, s)) return -1; }
-    else          { if (dkv_launch<64>(tq, td, p, device, s)) return -1; }
+    if (D == 128) { if (dkv_launch<128>(tq64, td64, p, device, s)) return -1; }
+    else          { if (dkv_launch<64>(tq64, td64, p, device, s)) return -1; }
   }
   if (which & 1) {
     if (D == 128) { if (dq_launch<128>(tq, td, p, device, s)) return -1; }
