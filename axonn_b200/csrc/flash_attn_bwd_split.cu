@@ -57,41 +57,53 @@ __device__ __forceinline__ uint32_t fs_pack(float2 v) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// neg_delta[b, h, s] = -sum_d dO[b, s, h, d] * O[b, s, h, d] and neg_lse2 = -lse * log2(e); HD / 8 threads per row,
-// 16-byte loads.  Rows S .. Sp - 1 get -inf / 0 (see FaSplitParams).
+// neg_delta[b, h, s] = -sum_d dO[b, s, h, d] * O[b, s, h, d] and neg_lse2 = -lse * log2(e); HD / 8 threads per row, four
+// rows per thread with all their 16-byte loads in flight.  Rows S .. Sp - 1 get -inf / 0 (see FaSplitParams).  The grid's
+// y dimension is the batch, so that a row's data lies at its index and the only division is by the head count.  One B200,
+// 262144 rows: head_dim 128 (134 MB) 35 -> 31 us, head_dim 64 20 -> 11 us (64-bit divisions for every 16 bytes before).
+constexpr int FS_DELTA_ROWS = 4;
 template <int HD>
 __global__ void __launch_bounds__(256)
 fa_split_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                       const float* __restrict__ lse, float* __restrict__ neg_lse2, float* __restrict__ neg_delta,
-                      int B, int S, int Sp, int H) {
-  constexpr int TPR = HD / 8;
-  const long long rows = static_cast<long long>(B) * Sp * H;
-  const int sub = threadIdx.x % TPR;
+                      int B, int S, int Sp, unsigned H) {
+  constexpr unsigned TPR = HD / 8, RPT = 256 / TPR;          // threads per row, rows per step of the block
+  const unsigned rows = static_cast<unsigned>(Sp) * H, live_rows = static_cast<unsigned>(S) * H, sub = threadIdx.x % TPR;
+  for (unsigned b = blockIdx.y; b < static_cast<unsigned>(B); b += gridDim.y) {
+  const size_t base = static_cast<size_t>(b) * live_rows * HD, vec = static_cast<size_t>(b) * H;
   // all threads of a warp run the same number of rounds: the row's lanes are reduced with full-warp shuffles
-  const long long per_round = static_cast<long long>(gridDim.x) * (256 / TPR);
-  for (long long base = static_cast<long long>(blockIdx.x) * (256 / TPR); base < rows; base += per_round) {
-    const long long row = base + threadIdx.x / TPR;
-    const long long h = row % H, bs = row / H, s = bs % Sp, bb = bs / Sp;
-    const bool live = row < rows && s < S;
-    float acc = 0.f;
-    if (live) {
-      const size_t off = (static_cast<size_t>(bb * S + s) * H + h) * HD + sub * 8;
-      const uint4 a = *reinterpret_cast<const uint4*>(o + off), c = *reinterpret_cast<const uint4*>(d_o + off);
-      const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a);
-      const __nv_bfloat162* c2 = reinterpret_cast<const __nv_bfloat162*>(&c);
+  for (unsigned r0 = blockIdx.x * (RPT * FS_DELTA_ROWS); r0 < rows; r0 += gridDim.x * (RPT * FS_DELTA_ROWS)) {
+    uint4 a[FS_DELTA_ROWS], c[FS_DELTA_ROWS];
+#pragma unroll
+    for (int u = 0; u < FS_DELTA_ROWS; ++u) {
+      const unsigned row = r0 + u * RPT + threadIdx.x / TPR;
+      a[u] = c[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (row < live_rows) {
+        a[u] = __ldg(reinterpret_cast<const uint4*>(o + base + static_cast<size_t>(row) * HD + sub * 8));
+        c[u] = __ldg(reinterpret_cast<const uint4*>(d_o + base + static_cast<size_t>(row) * HD + sub * 8));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < FS_DELTA_ROWS; ++u) {
+      const unsigned row = r0 + u * RPT + threadIdx.x / TPR;
+      const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&a[u]);
+      const __nv_bfloat162* c2 = reinterpret_cast<const __nv_bfloat162*>(&c[u]);
+      float acc = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(c2[i]);
         acc += x.x * y.x + x.y * y.y;
       }
-    }
 #pragma unroll
-    for (int off = TPR / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (sub == 0 && row < rows) {
-      const size_t dst = static_cast<size_t>(bb * H + h) * Sp + s;
-      neg_delta[dst] = -acc;
-      neg_lse2[dst] = live ? -lse[static_cast<size_t>(bb * H + h) * S + s] * 1.4426950408889634f : -INFINITY;
+      for (unsigned off = TPR / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+      if (sub == 0 && row < rows) {
+        const unsigned s = row / H, h = row - s * H;
+        const size_t dst = (vec + h) * Sp + s;
+        neg_delta[dst] = -acc;
+        neg_lse2[dst] = row < live_rows ? -lse[(vec + h) * S + s] * 1.4426950408889634f : -INFINITY;
+      }
     }
+  }
   }
 }
 
@@ -733,15 +745,17 @@ extern "C" int axb_flash_attn_bwd_split(const void* qkv, const void* out, const 
   const int H = G * qpk, Sp = (S + 127) / 128 * 128;
   // a launch through the runtime comes before the first driver call: on a thread that autograd has just started it is
   // what binds the device's context
-  const long long row_blocks = (static_cast<long long>(B) * Sp * H + 256 / (D / 8) - 1) / (256 / (D / 8));
-  const long long cap = static_cast<long long>(sm_count(device)) * 8;
-  const int blocks = static_cast<int>(row_blocks < cap ? row_blocks : cap);
+  const int rows_per_block = 256 / (D / 8) * FS_DELTA_ROWS;
+  const long long rows = static_cast<long long>(Sp) * H;
+  if (rows > 0x7fffffffll) { set_error("flash attention: too many rows"); return -1; }
+  const dim3 dgrid(static_cast<unsigned>((rows + rows_per_block - 1) / rows_per_block), B < 65535 ? B : 65535);
+  float* neg_delta = scratch + static_cast<size_t>(B) * H * Sp;
   if (D == 128)
-    fa_split_delta_kernel<128><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out),
-                                                      lse, scratch, scratch + static_cast<size_t>(B) * H * Sp, B, S, Sp, H);
+    fa_split_delta_kernel<128><<<dgrid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out),
+                                                     lse, scratch, neg_delta, B, S, Sp, H);
   else
-    fa_split_delta_kernel<64><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out),
-                                                     lse, scratch, scratch + static_cast<size_t>(B) * H * Sp, B, S, Sp, H);
+    fa_split_delta_kernel<64><<<dgrid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(d_out),
+                                                    lse, scratch, neg_delta, B, S, Sp, H);
   AXB_CUDA(cudaGetLastError());
   CUtensorMap tq, td, tq64, td64;                     // dQ kernel: 128-row boxes, dK / dV kernel: 64-row boxes
   const uint64_t cols = static_cast<uint64_t>(G) * (qpk + 2) * D, do_cols = static_cast<uint64_t>(H) * D;
