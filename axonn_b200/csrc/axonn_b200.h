@@ -222,7 +222,7 @@ int axb_swiglu_bwd(const void* dout, const void* gate_up, void* dgate_up, int T,
 int axb_rope(void* x, const float* cs, long long rows, int S, int nh, int D, int pos_div, long long row_stride,
              int inverse, void* stream);
 
-/* ---- flash attention on the packed projection output [B, S, G, qpk + 2, D] (flash_attn.cu); D 64 or 128 */
+/* ---- flash attention on the packed projection output [B, S, G, qpk + 2, D] (flash_attn.cu); D 64 or 128, scale > 0 */
 int axb_flash_attn_fwd(const void* qkv, void* out, float* lse, int B, int S, int G, int qpk, int D, float scale,
                        int device, void* stream);
 int axb_flash_attn_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, float* delta, float* dq_acc,

@@ -484,6 +484,7 @@ extern "C" int axb_flash_attn_fwd(const void* qkv, void* out, float* lse, int B,
   using namespace axb;
   if (D != 64 && D != 128) { set_error("flash attention: head_dim must be 64 or 128"); return -1; }
   if (B <= 0 || S <= 0 || G <= 0 || qpk <= 0) { set_error("flash attention: empty problem"); return -1; }
+  if (!(scale > 0.f)) { set_error("flash attention: the scale must be positive"); return -1; }   // see the masks and maxima above
   if (reinterpret_cast<uintptr_t>(out) & 15) { set_error("flash attention: tensors must be 16-byte aligned"); return -1; }
   CUtensorMap tm;
   if (make_tmap_3d_bf16(&tm, qkv, B, S, static_cast<uint64_t>(G) * (qpk + 2) * D, 128)) return -1;

@@ -736,6 +736,7 @@ extern "C" int axb_flash_attn_bwd_split(const void* qkv, const void* out, const 
   using namespace axb;
   if (D != 64 && D != 128) { set_error("flash attention: head_dim must be 64 or 128"); return -1; }
   if (B <= 0 || S <= 0 || G <= 0 || qpk <= 0) { set_error("flash attention: empty problem"); return -1; }
+  if (!(scale > 0.f)) { set_error("flash attention: the scale must be positive"); return -1; }   // masked scores are -inf before it
   if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(d_out) | reinterpret_cast<uintptr_t>(dqkv) |
        reinterpret_cast<uintptr_t>(scratch)) & 15) {
     set_error("flash attention: tensors must be 16-byte aligned");

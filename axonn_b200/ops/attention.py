@@ -28,7 +28,7 @@ def _sdpa(q, k, v, causal, scale):
 
 def flash_attention(q, k, v, causal=True, scale=None):
     """Attention of ``q [B, S, heads, D]`` against ``k, v [B, S, kv_heads, D]`` (grouped-query when ``kv_heads <
-    heads``) on the package's tcgen05 kernels (CUDA bf16, D 64 or 128, any S) or through
+    heads``) on the package's tcgen05 kernels (CUDA bf16, D 64 or 128, any S, positive ``scale``) or through
     ``scaled_dot_product_attention`` otherwise; returns ``[B, S, heads, D]``."""
     if scale is None:
         scale = 1.0 / math.sqrt(q.shape[-1])
@@ -39,7 +39,7 @@ def flash_attention(q, k, v, causal=True, scale=None):
             B, S, hq, D = q.shape
             G = k.shape[2]
             qkv = torch.cat([q.reshape(B, S, G, hq // G, D), k.unsqueeze(3), v.unsqueeze(3)], 3)
-            if attention_cuda.supported(qkv):
+            if attention_cuda.supported(qkv, scale):
                 return attention_cuda.flash_attention_packed_cuda(qkv, causal, scale)
     return _sdpa(q, k, v, causal, scale)
 
@@ -54,7 +54,7 @@ def flash_attention_packed(qkv, causal=True, scale=None):
     if qkv.is_cuda and not _IMPL["force_torch"]:
         from . import attention_cuda
 
-        if attention_cuda.available() and attention_cuda.supported(qkv) and causal:
+        if attention_cuda.available() and attention_cuda.supported(qkv, scale) and causal:
             return attention_cuda.flash_attention_packed_cuda(qkv, causal, scale)
     q = qkv[:, :, :, :qpk].reshape(B, S, G * qpk, D)
     return _sdpa(q, qkv[:, :, :, qpk], qkv[:, :, :, qpk + 1], causal, scale)

@@ -19,10 +19,15 @@ def available():
     return hasattr(_lib.lib(), "axb_flash_attn_fwd") and os.environ.get("AXONN_FLASH", "1") == "1"
 
 
-def supported(qkv):
+def supported(qkv, scale=1.0):
     """Whether the kernels take this packed tensor: bf16, head_dim 64 or 128, dense and 16-byte aligned, any sequence
-    length.  Traced, vmapped or subclassed tensors have no storage that a kernel could be given."""
+    length, a positive softmax scale.  Traced, vmapped or subclassed tensors have no storage that a kernel could be
+    given.  The scale: masked scores are -inf before they are multiplied by it and the row maximum is taken before the
+    multiplication, so it has to be positive, and a normal fp32 number after the change to base 2 (the kernels flush
+    denormals)."""
     B, S, G, n, D = qkv.shape
+    if not 2.0 ** -100 < scale < 2.0 ** 100:
+        return False
     if qkv.dtype != torch.bfloat16 or D not in (64, 128) or not qkv.is_contiguous() or qkv.numel() == 0 or n < 3:
         return False
     if S % 128:

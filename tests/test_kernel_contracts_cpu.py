@@ -1,0 +1,35 @@
+"""What the kernels' entry points accept and refuse, checked on the host before anything is launched."""
+
+import ctypes
+import shutil
+
+import pytest
+import torch
+
+from axonn_b200.ops import _lib
+
+native = pytest.mark.skipif(not (_lib.available() or shutil.which("nvcc")), reason="native library not built")
+
+
+def _error():
+    return _lib.lib().axb_last_error().decode()
+
+
+@pytest.mark.parametrize("scale,ok", [(0.125, True), (1e-20, True), (0.0, False), (-0.125, False), (float("nan"), False),
+                                      (float("inf"), False), (1e-42, False)])
+@pytest.mark.parametrize("S", [77, 128])
+def test_attention_kernels_take_positive_scales_only(S, scale, ok):
+    """Masked scores are -inf before the softmax scale multiplies them: with zero the product is NaN and with a negative
+    scale +inf.  Such calls belong to the general path, at every sequence length."""
+    from axonn_b200.ops import attention_cuda
+
+    qkv = torch.randn(1, S, 1, 3, 64).bfloat16()
+    assert attention_cuda.supported(qkv, scale) is ok
+
+
+@native
+@pytest.mark.parametrize("scale", [0.0, -0.125, float("nan")])
+def test_attention_entry_points_refuse_other_scales(scale):
+    L, p = _lib.lib(), 4096                       # never dereferenced: the call is refused on the host
+    assert L.axb_flash_attn_fwd(p, p, p, 1, 128, 1, 1, 64, scale, 0, None) == -1 and "scale" in _error()
+    assert L.axb_flash_attn_bwd_split(p, p, p, p, p, p, 1, 128, 1, 1, 64, scale, 3, 0, None) == -1 and "scale" in _error()

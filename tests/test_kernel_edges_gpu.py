@@ -88,6 +88,27 @@ def test_attention_any_length(B, S, G, qpk, D):
             assert err < 1.5e-2 * max(float(want.norm()), float(gref[bb].norm()) * 1e-2), (bb, sl, err)
 
 
+@pytest.mark.parametrize("S", [77, 128, 256])
+@pytest.mark.parametrize("scale", [0.0, -0.3])
+def test_attention_other_scales(S, scale):
+    """A scale that is not positive takes the general path: forward and backward against 64 bits (bf16 results and
+    probabilities, as above)."""
+    from axonn_b200 import ops
+
+    torch.manual_seed(S)
+    B, G, qpk, D = 2, 2, 2, 64
+    qkv = torch.randn(B, S, G, qpk + 2, D, device=DEV).bfloat16().requires_grad_(True)
+    dout = torch.randn(B, S, G * qpk, D, device=DEV).bfloat16()
+    out = ops.flash_attention_packed(qkv, scale=scale)
+    (grad,) = torch.autograd.grad(out, qkv, dout)
+    x = qkv.detach().double().requires_grad_(True)
+    s = torch.einsum("bsgqd,btgd->bgqst", x[:, :, :, :qpk], x[:, :, :, qpk]) * scale
+    s = s.masked_fill(torch.ones(S, S, device=DEV, dtype=torch.bool).triu(1), float("-inf"))
+    ref = torch.einsum("bgqst,btgd->bsgqd", s.softmax(-1), x[:, :, :, qpk + 1]).reshape(B, S, G * qpk, D)
+    (gref,) = torch.autograd.grad(ref, x, dout.double())
+    assert _rel(out, ref) < 1e-2 and _rel(grad, gref) < 1.5e-2
+
+
 # ------------------------------------------------------------------------------------------------ split-K GEMM
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("M,N,K", [(8, 128, 256), (24, 2048, 8192), (24, 8192, 2048), (120, 136, 1000), (136, 264, 520),
