@@ -293,7 +293,7 @@ unsigned long long axb_heap_info(void* heap, int what);
 int axb_heap_destroy(void* heap);
 
 /* ---- top-k gradient pruning (prune.cu): keep the k largest |g|, zero the rest, in place.
- * dtype: the codes above (0 bf16, 1 fp16, 2 fp32).  `work`: device scratch of axb_prune_workspace_words() 32-bit words. */
+ * dtype: the codes above (0 bf16, 1 fp16, 2 fp32).  `work`: device scratch of axb_prune_workspace_words() 32-bit words, 8-byte aligned. */
 int axb_prune_workspace_words(void);
 int axb_prune_topk(void* g, long long n, int dtype, long long k, void* work, int device, void* stream);
 

@@ -36,8 +36,9 @@ struct PruneMeta {
 static_assert(sizeof(PruneMeta) == 32, "scratch layout");
 
 // Called by all threads of the block that finishes last: the largest bin b with count(bins > b) < k <= count(bins >= b).
-// Every thread sums its bins with 16-byte loads and the block scans the sums in registers: a one-block kernel of its own
-// with a word-wise sum and a log-step scan in shared memory took 21 us per tensor.
+// Every thread sums its bins with 8-byte loads (the caller's scratch need not be aligned to more) and the block scans the
+// sums in registers: a one-block kernel of its own with a word-wise sum and a log-step scan in shared memory took 21 us
+// per tensor.
 template <int BINS>
 __device__ void prune_select(const unsigned int* __restrict__ hist, long long k, long long* bin, long long* rank) {
   __shared__ unsigned long long warp_sum[PR_THREADS / 32];
@@ -48,9 +49,9 @@ __device__ void prune_select(const unsigned int* __restrict__ hist, long long k,
   const int hi = BINS - threadIdx.x * PER, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   unsigned long long mine = 0;
 #pragma unroll 8
-  for (int i = 0; i < PER / 4; ++i) {
-    const uint4 u = __ldcg(reinterpret_cast<const uint4*>(hist + hi - PER) + i);
-    mine += static_cast<unsigned long long>(u.x) + u.y + u.z + u.w;
+  for (int i = 0; i < PER / 2; ++i) {
+    const uint2 u = __ldcg(reinterpret_cast<const uint2*>(hist + hi - PER) + i);
+    mine += static_cast<unsigned long long>(u.x) + u.y;
   }
   unsigned long long incl = mine;
 #pragma unroll
@@ -250,6 +251,7 @@ extern "C" int axb_prune_workspace_words(void) { return axb::PR_WORK_WORDS; }
 // work: device scratch of axb_prune_workspace_words() 32-bit words (8-byte aligned).
 extern "C" int axb_prune_topk(void* g, long long n, int dtype, long long k, void* work, int device, void* stream) {
   if (!work) { axb::set_error("prune: workspace is null"); return -1; }
+  if (reinterpret_cast<uintptr_t>(work) & 7) { axb::set_error("prune: the workspace must be 8-byte aligned"); return -1; }
   if (dtype < 0 || dtype > 2) { axb::set_error("prune: bad dtype %d (0 bf16, 1 fp16, 2 fp32)", dtype); return -1; }
   return axb::prune_topk_launch(g, n, dtype, k, static_cast<unsigned int*>(work), device, (cudaStream_t)stream);
 }

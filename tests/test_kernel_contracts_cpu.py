@@ -33,3 +33,10 @@ def test_attention_entry_points_refuse_other_scales(scale):
     L, p = _lib.lib(), 4096                       # never dereferenced: the call is refused on the host
     assert L.axb_flash_attn_fwd(p, p, p, 1, 128, 1, 1, 64, scale, 0, None) == -1 and "scale" in _error()
     assert L.axb_flash_attn_bwd_split(p, p, p, p, p, p, 1, 128, 1, 1, 64, scale, 3, 0, None) == -1 and "scale" in _error()
+
+
+@native
+def test_prune_refuses_an_unaligned_workspace():
+    """The scratch holds 64-bit words: 8-byte alignment is what the interface asks for (and all it needs)."""
+    L = _lib.lib()
+    assert L.axb_prune_topk(4096, 1 << 20, 0, 1000, 4096 + 4, 0, None) == -1 and "aligned" in _error()

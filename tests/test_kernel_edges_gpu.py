@@ -184,6 +184,25 @@ def test_scale_sizes_and_offsets(dtype):
         assert all(torch.equal(a, b) for a, b in zip(work, want))
 
 
+# ------------------------------------------------------------------------------------------------ gradient pruning
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("offset", [0, 2, 4])
+def test_prune_workspace_of_8_byte_alignment(offset, dtype):
+    """The C entry point takes scratch at any 8-byte boundary (``offset``: 32-bit words); values are kept or zeroed, so
+    the comparison is exact."""
+    from axonn_b200.ops import _lib
+    from axonn_b200.ops.optim_step import _LIB_DTYPE
+
+    torch.manual_seed(offset)
+    L = _lib.lib()
+    g = torch.randn(300_001, device=DEV).to(dtype)
+    k = 30_000
+    ws = torch.empty(L.axb_prune_workspace_words() + 4, dtype=torch.int32, device=DEV)[offset:]
+    want = torch.where(g.abs().float() >= g.abs().float().sort(descending=True)[0][k - 1], g, torch.zeros_like(g))
+    _lib.check(L.axb_prune_topk(_lib.addr(g), g.numel(), _LIB_DTYPE[dtype], k, _lib.addr(ws), 0, _lib.stream()), "axb_prune_topk")
+    assert torch.equal(g, want)
+
+
 # ------------------------------------------------------------------------------------------------ local experts
 @pytest.mark.parametrize("T,E,k,C", [(1, 4, 2, 8), (5, 8, 2, 8), (1000, 8, 2, 312), (4097, 4, 2, 2048), (8192, 8, 2, 2560),
                                      (3000, 5, 1, 64)])
