@@ -51,7 +51,6 @@ def adamw_reference_(p, g, m, v, lr, beta1, beta2, eps, weight_decay, step, grad
     p.mul_(1 - lr * weight_decay).addcdiv_(m, denom, value=-lr / bc1)
 
 
-_prune_ws = {}
 # dtype codes of the C interface (csrc/axonn_b200.h)
 _LIB_DTYPE = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
@@ -66,10 +65,9 @@ def prune_topk_(grad, keep_fraction):
         assert grad.is_contiguous()
         L = _lib.lib()
         dev = grad.device
-        ws = _prune_ws.get(dev)
-        if ws is None:
-            ws = torch.empty(L.axb_prune_workspace_words(), dtype=torch.int32, device=dev)
-            _prune_ws[dev] = ws
+        # scratch of this call (393 KB): calls on other streams or threads may overlap with it, and the allocator hands
+        # the block on in the order of this stream
+        ws = torch.empty(L.axb_prune_workspace_words(), dtype=torch.int32, device=dev)
         st = L.axb_prune_topk(_lib.addr(grad), n, _LIB_DTYPE[grad.dtype],
                               k, _lib.addr(ws), dev.index, _lib.stream())
         _lib.check(st, "axb_prune_topk")

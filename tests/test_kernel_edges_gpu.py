@@ -203,6 +203,27 @@ def test_prune_workspace_of_8_byte_alignment(offset, dtype):
     assert torch.equal(g, want)
 
 
+def test_prune_on_two_streams():
+    """Calls that overlap on two streams have their own scratch: histograms, ranks and the block counter of one are not
+    touched by the other.  Exact."""
+    from axonn_b200 import ops
+
+    torch.manual_seed(0)
+    new = [torch.randn(n, device=DEV).bfloat16() * s for n, s in ((24_000_000, 1.0), (16_000_003, 1e-3))]
+    want = [torch.where(g.abs().float() >= g.abs().float().sort(descending=True)[0][g.numel() // 10 - 1], g,
+                        torch.zeros_like(g)) for g in (t[: t.numel() // 10 * 10] for t in new)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    work = [[t[: t.numel() // 10 * 10].clone() for _ in range(8)] for t in new]
+    torch.cuda.synchronize()
+    for i in range(8):
+        for st, ts in zip(streams, work):
+            with torch.cuda.stream(st):
+                ops.prune_topk_(ts[i], 0.1)
+    torch.cuda.synchronize()
+    for w, ts in zip(want, work):
+        assert all(torch.equal(t, w) for t in ts)
+
+
 # ------------------------------------------------------------------------------------------------ local experts
 @pytest.mark.parametrize("T,E,k,C", [(1, 4, 2, 8), (5, 8, 2, 8), (1000, 8, 2, 312), (4097, 4, 2, 2048), (8192, 8, 2, 2560),
                                      (3000, 5, 1, 64)])
