@@ -22,6 +22,9 @@ def _sdpa(q, k, v, causal, scale):
     if rep > 1:
         kh = kh.repeat_interleave(rep, dim=1)
         vh = vh.repeat_interleave(rep, dim=1)
+    if scale <= 0:
+        # the sign goes into the queries: fused backends of the library call give NaN for a scale of zero
+        qh, scale = (qh * 0, 1.0) if scale == 0 else (-qh, -scale)
     o = F.scaled_dot_product_attention(qh, kh, vh, is_causal=causal, scale=scale)
     return o.transpose(1, 2)
 
