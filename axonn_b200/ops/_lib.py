@@ -164,12 +164,19 @@ _STATUS_NAMES = {
     0x701: "bounds check (debug build): inbox slot outside the peer's inbox",
     0x702: "bounds check (debug build): output element outside C",
     0x703: "bounds check (debug build): flag index outside the flag array",
-    0x401: "flash attention forward: producer timed out",
-    0x402: "flash attention forward: MMA issuer timed out",
-    0x404: "flash attention forward: softmax warps timed out",
-    0x411: "flash attention backward: producer timed out",
-    0x412: "flash attention backward: MMA issuer timed out",
-    0x414: "flash attention backward: softmax / reduction warps timed out",
+    0x405: "flash attention forward: producer timed out",
+    0x406: "flash attention forward: MMA issuer timed out",
+    0x407: "flash attention forward: softmax warps timed out",
+    0x411: "flash attention backward (one kernel): producer timed out",
+    0x412: "flash attention backward (one kernel): MMA issuer timed out",
+    0x414: "flash attention backward (one kernel): softmax / reduction warps timed out",
+    0x421: "flash attention backward, dQ kernel: producer timed out",
+    0x422: "flash attention backward, dQ kernel: score MMA issuer timed out",
+    0x423: "flash attention backward, dQ kernel: softmax warps timed out",
+    0x424: "flash attention backward, dQ kernel: dQ MMA issuer timed out",
+    0x431: "flash attention backward, dK / dV kernel: producer timed out",
+    0x432: "flash attention backward, dK / dV kernel: MMA issuer timed out",
+    0x433: "flash attention backward, dK / dV kernel: softmax warps timed out",
     0x151: "split-K GEMM producer timed out",
     0x152: "split-K GEMM MMA issuer timed out",
     0x154: "split-K GEMM epilogue timed out",

@@ -1,6 +1,8 @@
 """What the kernels' entry points accept and refuse, checked on the host before anything is launched."""
 
-import ctypes
+import glob
+import os
+import re
 import shutil
 
 import pytest
@@ -40,3 +42,13 @@ def test_prune_refuses_an_unaligned_workspace():
     """The scratch holds 64-bit words: 8-byte alignment is what the interface asks for (and all it needs)."""
     L = _lib.lib()
     assert L.axb_prune_topk(4096, 1 << 20, 0, 1000, 4096 + 4, 0, None) == -1 and "aligned" in _error()
+
+
+def test_every_status_code_of_the_kernels_has_a_name():
+    """A wait that gave up is reported by name: every code that a kernel writes, and no code of a kernel that is gone."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(_lib.__file__))), "csrc")
+    text = "\n".join(open(f).read() for f in glob.glob(os.path.join(csrc, "*.cu*")))
+    written = {int(c, 16) for c in re.findall(r"report_status\([^;]*?(0x[0-9a-f]{3})u\)", text)}
+    assert len(written) > 20 and not written - set(_lib._STATUS_NAMES)
+    mentioned = {int(c, 16) for c in re.findall(r"\b(0x[0-9a-f]{3})u?\b", text)}
+    assert not set(_lib._STATUS_NAMES) - mentioned
