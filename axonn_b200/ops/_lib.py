@@ -10,6 +10,7 @@ never a silent fallback.
 import ctypes
 import os
 import threading
+import warnings
 
 import torch
 
@@ -60,6 +61,12 @@ _SIGNATURES = {
     "axb_multi_adamw": "p" "il" "fffffff" "ppp",
     "axb_prune_topk": "p" "lil" "p" "i" "p",
 }
+# Switches of kernels that are gone.  The one kernel that is left covers what they selected; a program that still sets
+# one is told so instead of being ignored.
+_REMOVED_SWITCHES = {
+    "AXONN_FA_FWD": "the two-tile attention forward serves every sequence length",
+    "AXONN_NORM_WARP": "the ring kernel is the norm forward for every hidden size up to 8192",
+}
 _CTYPES = {"i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float, "p": ctypes.c_void_p}
 
 
@@ -89,6 +96,9 @@ def lib():
             if ms:
                 L.axb_set_wait_timeout_ms(ctypes.c_uint(int(ms)))
             _LIB = L      # published when complete: another thread may be waiting for it without the lock
+            for name, why in _REMOVED_SWITCHES.items():
+                if name in os.environ:
+                    warnings.warn(f"{name} has no effect: {why}", stacklevel=2)
     return _LIB
 
 

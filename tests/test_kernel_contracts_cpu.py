@@ -52,3 +52,12 @@ def test_every_status_code_of_the_kernels_has_a_name():
     assert len(written) > 20 and not written - set(_lib._STATUS_NAMES)
     mentioned = {int(c, 16) for c in re.findall(r"\b(0x[0-9a-f]{3})u?\b", text)}
     assert not set(_lib._STATUS_NAMES) - mentioned
+
+
+@native
+@pytest.mark.parametrize("name", ["AXONN_FA_FWD", "AXONN_NORM_WARP"])
+def test_removed_switches_are_reported(name, monkeypatch):
+    monkeypatch.setattr(_lib, "_LIB", None)
+    monkeypatch.setenv(name, "0")
+    with pytest.warns(UserWarning, match=name):
+        _lib.lib()
