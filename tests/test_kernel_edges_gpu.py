@@ -144,6 +144,40 @@ def test_gemm_few_tiles(layout, M, N, K, dtype):
     assert _lib.device_status() == 0
 
 
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(777, 4104, 1000), (1500, 2056, 520), (136, 16136, 512)])
+def test_gemm_one_wave_of_pairs(M, N, K, dtype, layout):
+    """Two waves of single tiles that one wave of CTA pairs replaces: rows, columns and K blocks end inside a tile, the
+    last column chunk of a row is 8 wide, and the bias starts off a 16-byte boundary.  Tolerance: one rounding to the
+    storage type; fp32 sums."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib
+
+    if layout == "tn":
+        M = M // 8 * 8
+    torch.manual_seed(M + N + K)
+    a = torch.randn((M, K) if layout != "tn" else (K, M), device=DEV).to(dtype)
+    b = torch.randn((N, K) if layout == "nt" else (K, N), device=DEV).to(dtype)
+    want = (a.double() if layout != "tn" else a.double().t()) @ (b.double().t() if layout == "nt" else b.double())
+    f = {"nt": ops.matmul_nt, "nn": ops.matmul_nn, "tn": ops.matmul_tn}[layout]
+    one = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10
+    assert _rel(f(a, b), want) < one
+    base = torch.randn(M, N, device=DEV)
+    assert _rel(f(a, b, out=base.clone(), accumulate=True), want + base.double()) < 1e-5
+    if layout == "nt":
+        for off in (0, 1):
+            bias = torch.randn(N + 1, device=DEV).to(dtype)[off:N + off]
+            pre = torch.empty(M, N, device=DEV, dtype=dtype)
+            act = ops.matmul_nt(a, b, bias=bias, epilogue=ops.EPI_BIAS_GELU, aux=pre)
+            w = want + bias.double()
+            assert _rel(pre, w) < one
+            assert _rel(act, torch.nn.functional.gelu(w, approximate="tanh")) < 2 * one
+            assert _rel(ops.matmul_nt(a, b, bias=bias, epilogue=ops.EPI_BIAS), w) < one
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+
+
 # ------------------------------------------------------------------------------------------------ cross-entropy
 @pytest.mark.parametrize("rows,V", [(1, 8), (3, 4096), (5, 4104), (7, 16384), (2, 16392), (1030, 50304)])
 def test_cross_entropy_rows(rows, V):
