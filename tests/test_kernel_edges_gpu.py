@@ -88,6 +88,40 @@ def test_attention_any_length(B, S, G, qpk, D):
             assert err < 1.5e-2 * max(float(want.norm()), float(gref[bb].norm()) * 1e-2), (bb, sl, err)
 
 
+@pytest.mark.parametrize("B,S,G,qpk,D", [(2, 777, 4, 2, 128), (4, 640, 4, 1, 64), (2, 1531, 4, 1, 128), (2, 896, 2, 2, 128)])
+def test_attention_precision_off_256(B, S, G, qpk, D):
+    """Lengths that are not multiples of 256: the log-sum-exp to fp32 rounding (sums of at most 1531 positive terms and
+    two logarithms of magnitude 10: below 1e-5), and outputs no further from 64 bits than the library's attention,
+    which rounds the same probabilities to bf16 (0.3 % for the sampling of the rounding errors)."""
+    from axonn_b200.ops.attention_cuda import flash_fwd_packed
+
+    torch.manual_seed(S)
+    qkv = torch.randn(B, S, G, qpk + 2, D, device=DEV).bfloat16()
+    out, lse = flash_fwd_packed(qkv, 1 / math.sqrt(D))
+    x = qkv.double()
+    s = torch.einsum("bsgqd,btgd->bgqst", x[:, :, :, :qpk], x[:, :, :, qpk]) / math.sqrt(D)
+    s = s.masked_fill(torch.ones(S, S, device=DEV, dtype=torch.bool).triu(1), float("-inf"))
+    assert float((lse.double() - s.logsumexp(-1).reshape(B, G * qpk, S)).abs().max()) < 1e-5
+    ref = torch.einsum("bgqst,btgd->bsgqd", s.softmax(-1), x[:, :, :, qpk + 1]).reshape(B, S, G * qpk, D)
+    q, k, v = qkv[:, :, :, :qpk].reshape(B, S, G * qpk, D), qkv[:, :, :, qpk], qkv[:, :, :, qpk + 1]
+    k, v = (t.repeat_interleave(qpk, 2) for t in (k, v))
+    lib = torch.nn.functional.scaled_dot_product_attention(*(t.transpose(1, 2) for t in (q, k, v)), is_causal=True).transpose(1, 2)
+    assert _rel(out, ref) < 1.003 * _rel(lib, ref)
+
+
+@pytest.mark.parametrize("S", [77, 300, 384])
+def test_attention_lets_nan_through(S):
+    """A NaN key reaches every query that sees it, and no other."""
+    from axonn_b200 import ops
+
+    for at in (0, 2, 9, S - 1):
+        qkv = torch.randn(1, S, 2, 3, 64, device=DEV).bfloat16()
+        qkv[0, at, 0, 1, 5] = float("nan")
+        out = ops.flash_attention_packed(qkv)
+        assert bool(out[0, at:, 0].isnan().all()) and bool(out[0, :at, 0].isfinite().all())
+        assert bool(out[0, :, 1].isfinite().all())
+
+
 @pytest.mark.parametrize("S", [77, 128, 256])
 @pytest.mark.parametrize("scale", [0.0, -0.3])
 def test_attention_other_scales(S, scale):
