@@ -1,12 +1,22 @@
 // Multi-tensor kernels: fused AdamW step, squared L2 norm, in-place scale.
 //
 // A launch covers a whole list of tensors through a device table; work is cut
-// into fixed-size chunks (the table holds their prefix sums), every chunk into
-// MT_PARTS units, and a grid-stride loop maps unit -> (tensor, offset), so one
-// launch replaces hundreds of per-parameter launches.  The units are small
-// because every kernel here is bound by memory and ends with its last unit.
-// One B200, the 50 M bf16 parameters of a GPT-1.3B block: scale 133 -> 28 us
-// (2-byte accesses before), squared norm 32 -> 24 us, AdamW 278 -> 241 us.
+// into fixed-size chunks (the table holds their prefix sums), and a grid-stride
+// loop maps units of work -> (tensor, offset), so one launch replaces hundreds
+// of per-parameter launches.  A unit is a quarter of a chunk for the
+// optimizers, whose 28 bytes per element make a whole chunk too long a last
+// unit; squared norm and scale take whole chunks for tables of small tensors,
+// where three of four quarters would be empty.  One B200, us, inputs warm in
+// the L2 where they fit; a: whole chunks found by binary search, b: quarters
+// found by a linear search, c: now
+//                                       AdamW            scale          norm
+//                                       a    b    c      a    b   c    a    b   c
+//   12 tensors of 4 M (bf16)            288  238  237    130  29  30   20   19  20
+//   a 300-tensor model, 315 M           1650 1409 1409   671  190 188  110  135 96
+//   1500 tensors of 32768               282  261  239    110  90  32   22   91  18
+//   3000 tensors of 4096                109  328  80     29   272 20   19   279 18
+//   300 tensors of 2048                 13   12   10     5.3  8.3 4.3  5.8  9.5 5.1
+// (the scale used 2-byte accesses in a)
 #include <mutex>
 
 #include "common.cuh"
@@ -14,7 +24,7 @@
 namespace axb {
 
 constexpr int MT_CHUNK = 1 << 16;
-constexpr int MT_PARTS = 4;                      // units per chunk
+constexpr int MT_PARTS = 4;                      // units per chunk of the optimizer kernels (and of the scale of long tensors)
 constexpr int MT_UNIT = MT_CHUNK / MT_PARTS;
 constexpr int MT_THREADS = 512;
 constexpr int ADAM_THREADS = 256;
@@ -22,18 +32,20 @@ constexpr int ADAM_UNROLL = 2;
 
 // table row for norm/scale: {ptr, numel, dtype (0 fp32, 1 bf16, 2 fp16), chunk_prefix}
 // table row for adamw:      {master fp32, model bf16 or 0, grad, exp_avg, exp_avg_sq, numel, grad dtype, chunk_prefix}
-// Row of the tensor that holds `chunk`: the last one whose prefix is <= chunk.  Whole warps call it; the lanes look at 32
-// rows at a time (one load latency for up to 32 tensors where a binary search has five in series).
+// Row of the tensor that holds `chunk`: the last one whose prefix is <= chunk (tensors without elements share the prefix of
+// their successor).  Whole warps call it; every round the 32 lanes look at 32 evenly spaced rows of what is left, so
+// 32 tensors take one load latency, 1024 two.
 __device__ __forceinline__ int find_tensor(const long long* table, int width, int prefix_col, int n, long long chunk) {
   const int lane = threadIdx.x & 31;
-  int found = 0;
-  for (int base = 0; base < n; base += 32) {
-    const bool le = base + lane < n && __ldg(table + (size_t)(base + lane) * width + prefix_col) <= chunk;
-    const int c = __popc(__ballot_sync(0xffffffffu, le));      // prefixes are sorted
-    if (c > 0) found = base + c - 1;
-    if (c < 32) break;
+  int lo = 0, len = n;
+  while (len > 1) {
+    const int step = (len + 31) / 32, at = lane * step;
+    const bool le = at < len && (at == 0 || __ldg(table + static_cast<size_t>(lo + at) * width + prefix_col) <= chunk);
+    const int c = __popc(__ballot_sync(0xffffffffu, le)) - 1;      // prefixes are sorted, and the first is taken
+    lo += c * step;
+    len = min(step, len - c * step);
   }
-  return found;
+  return lo;
 }
 
 __device__ __forceinline__ float load_as_f32(const void* p, long long i, int dtype) {
@@ -47,19 +59,21 @@ __device__ __forceinline__ void store_from_f32(void* p, long long i, int dtype, 
   else reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
 }
 
+template <int PARTS>      // units per chunk
 __global__ void __launch_bounds__(MT_THREADS)
 multi_l2norm_sq_kernel(const long long* __restrict__ table, int n, long long total_chunks, float* __restrict__ out) {
   __shared__ float red[32];
   float acc = 0.f;
-  for (long long unit = blockIdx.x; unit < total_chunks * MT_PARTS; unit += gridDim.x) {
-    const long long chunk = unit / MT_PARTS;
+  constexpr int UNIT = MT_CHUNK / PARTS;
+  for (long long unit = blockIdx.x; unit < total_chunks * PARTS; unit += gridDim.x) {
+    const long long chunk = unit / PARTS;
     const int t = find_tensor(table, 4, 3, n, chunk);
     const long long* row = table + (size_t)t * 4;
     const void* p = reinterpret_cast<const void*>(row[0]);
     const long long numel = row[1];
     const int dtype = (int)row[2];
-    const long long begin = (chunk - row[3]) * MT_CHUNK + (unit % MT_PARTS) * MT_UNIT;
-    const long long end = begin + MT_UNIT < numel ? begin + MT_UNIT : numel;
+    const long long begin = (chunk - row[3]) * MT_CHUNK + (unit % PARTS) * UNIT;
+    const long long end = begin + UNIT < numel ? begin + UNIT : numel;
     if (begin >= numel) continue;
     const bool vec = (reinterpret_cast<uintptr_t>(p) & 15) == 0;
     if (vec && dtype == 1) {
@@ -119,19 +133,21 @@ __device__ __forceinline__ uint32_t scale_word(uint32_t w, int dtype, float s) {
 // In-place scale, bound by one read and one write of the tensors: 16-byte accesses with SCALE_UNROLL of them in flight
 // per thread.  A factor of exactly one (a gradient norm below the clipping limit) leaves every value as it is.
 constexpr int SCALE_UNROLL = 4;
+template <int PARTS>      // units per chunk
 __global__ void __launch_bounds__(MT_THREADS)
 multi_scale_kernel(const long long* __restrict__ table, int n, long long total_chunks, const float* __restrict__ scale_ptr) {
   const float s = *scale_ptr;
   if (s == 1.f) return;
-  for (long long unit = blockIdx.x; unit < total_chunks * MT_PARTS; unit += gridDim.x) {
-    const long long chunk = unit / MT_PARTS;
+  constexpr int UNIT = MT_CHUNK / PARTS;
+  for (long long unit = blockIdx.x; unit < total_chunks * PARTS; unit += gridDim.x) {
+    const long long chunk = unit / PARTS;
     const int t = find_tensor(table, 4, 3, n, chunk);
     const long long* row = table + (size_t)t * 4;
     void* p = reinterpret_cast<void*>(row[0]);
     const long long numel = row[1];
     const int dtype = (int)row[2];
-    const long long begin = (chunk - row[3]) * MT_CHUNK + (unit % MT_PARTS) * MT_UNIT;
-    const long long end = begin + MT_UNIT < numel ? begin + MT_UNIT : numel;
+    const long long begin = (chunk - row[3]) * MT_CHUNK + (unit % PARTS) * UNIT;
+    const long long end = begin + UNIT < numel ? begin + UNIT : numel;
     if (begin >= numel) continue;
     long long scalar_from = begin;
     if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {      // chunks start at multiples of 65536 elements
@@ -162,13 +178,15 @@ multi_scale_kernel(const long long* __restrict__ table, int n, long long total_c
 // SGD with momentum (torch.optim.SGD semantics without dampening / Nesterov): g' = g * grad_scale + wd * p,
 // buf = mu * buf + g', p -= lr * buf.  Table rows: {param, grad, momentum buffer (fp32), numel, param dtype,
 // grad dtype, chunk prefix, -}.
+template <int PARTS>      // units per chunk
 __global__ void __launch_bounds__(MT_THREADS)
 multi_sgd_kernel(const long long* __restrict__ table, int n, long long total_chunks, float lr, float momentum,
                  float weight_decay, const float* __restrict__ grad_scale, const unsigned int* __restrict__ status) {
   if (status && *reinterpret_cast<const volatile unsigned int*>(status) != 0u) return;
   const float gs = grad_scale ? *grad_scale : 1.f;
-  for (long long unit = blockIdx.x; unit < total_chunks * MT_PARTS; unit += gridDim.x) {
-    const long long chunk = unit / MT_PARTS;
+  constexpr int UNIT = MT_CHUNK / PARTS;
+  for (long long unit = blockIdx.x; unit < total_chunks * PARTS; unit += gridDim.x) {
+    const long long chunk = unit / PARTS;
     const int t = find_tensor(table, 8, 6, n, chunk);
     const long long* row = table + (size_t)t * 8;
     void* p = reinterpret_cast<void*>(row[0]);
@@ -176,8 +194,8 @@ multi_sgd_kernel(const long long* __restrict__ table, int n, long long total_chu
     float* buf = reinterpret_cast<float*>(row[2]);
     const long long numel = row[3];
     const int pdtype = (int)row[4], gdtype = (int)row[5];
-    const long long begin = (chunk - row[6]) * MT_CHUNK + (unit % MT_PARTS) * MT_UNIT;
-    const long long end = begin + MT_UNIT < numel ? begin + MT_UNIT : numel;
+    const long long begin = (chunk - row[6]) * MT_CHUNK + (unit % PARTS) * UNIT;
+    const long long end = begin + UNIT < numel ? begin + UNIT : numel;
     if (begin >= numel) continue;
     for (long long i = begin + threadIdx.x; i < end; i += blockDim.x) {
       const float w = load_as_f32(p, i, pdtype);
@@ -302,24 +320,36 @@ __global__ void status_gate_kernel(const unsigned int* __restrict__ status, unsi
 }
 
 int sm_count(int device);
-static inline int mt_grid(long long chunks) {
-  const long long units = chunks * MT_PARTS, cap = static_cast<long long>(sm_count_current()) * 64;
+// blocks for `units` of work: at most `per_sm` per SM
+static inline int mt_grid(long long units, int per_sm = 64) {
+  const long long cap = static_cast<long long>(sm_count_current()) * per_sm;
   return (int)(units < cap ? (units < 1 ? 1 : units) : cap);
 }
+// at least 8 chunks per tensor on average: few quarters of a chunk are empty
+static inline bool mt_long_tensors(int n, long long total_chunks) { return total_chunks >= 8ll * n; }
 
 }  // namespace axb
 
 using namespace axb;
 
 extern "C" int axb_multi_l2norm_sq(const long long* table, int n, long long total_chunks, float* out, void* stream) {
-  // every block ends with an atomic: few blocks, each over many units
-  const int grid = min(mt_grid(total_chunks), sm_count_current() * 4);
-  multi_l2norm_sq_kernel<<<grid, MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, out);
+  // Every block ends with an atomic: few blocks.  Whole chunks, unless there are so few of them that the last wave counts
+  // and the tensors are long and found in one round of the search.  From DRAM, whole / quarters: 12 tensors of 64 chunks
+  // 30.8 / 28.7 us, 8 of 10 12.3 / 10.2; 33 of 16 22.6 / 22.6, 300 of 16 121 / 127, 1500 of one half 31 / 45.
+  if (n <= 32 && mt_long_tensors(n, total_chunks) && total_chunks < 16ll * sm_count_current())
+    multi_l2norm_sq_kernel<MT_PARTS><<<mt_grid(total_chunks * MT_PARTS, 4), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, out);
+  else
+    multi_l2norm_sq_kernel<1><<<mt_grid(total_chunks, 8), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, out);
   AXB_CUDA(cudaGetLastError());
   return 0;
 }
 extern "C" int axb_multi_scale(const long long* table, int n, long long total_chunks, const float* scale, void* stream) {
-  multi_scale_kernel<<<mt_grid(total_chunks), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, scale);
+  // quarters of a chunk where tensors are long: 29 against 30 us for 12 tensors of 64 chunks, 188 against 194 for 300 of 16,
+  // but 104 against 96 for 1500 of 2
+  if (mt_long_tensors(n, total_chunks))
+    multi_scale_kernel<MT_PARTS><<<mt_grid(total_chunks * MT_PARTS), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, scale);
+  else
+    multi_scale_kernel<1><<<mt_grid(total_chunks), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, scale);
   AXB_CUDA(cudaGetLastError());
   return 0;
 }
@@ -347,8 +377,9 @@ extern "C" int axb_multi_sgd(const long long* table, int n, long long total_chun
                              float weight_decay, const float* grad_scale, void* stream) {
   unsigned int* gate = refreshed_status_gate((cudaStream_t)stream);
   AXB_CUDA(cudaGetLastError());
-  multi_sgd_kernel<<<mt_grid(total_chunks), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, lr, momentum,
-                                                                                weight_decay, grad_scale, gate);
+  const bool parts = mt_long_tensors(n, total_chunks);
+  auto kern = parts ? multi_sgd_kernel<MT_PARTS> : multi_sgd_kernel<1>;
+  kern<<<mt_grid(total_chunks * (parts ? MT_PARTS : 1)), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, lr, momentum, weight_decay, grad_scale, gate);
   AXB_CUDA(cudaGetLastError());
   return 0;
 }
@@ -361,7 +392,7 @@ extern "C" int axb_multi_adamw(const long long* table, int n, long long total_ch
   unsigned int* gate = refreshed_status_gate((cudaStream_t)stream);
   AXB_CUDA(cudaGetLastError());
   AdamArgs a{lr, beta1, beta2, eps, weight_decay, bias_c1, bias_c2, grad_scale, found_inf, gate};
-  multi_adamw_kernel<<<mt_grid(total_chunks), ADAM_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, a);
+  multi_adamw_kernel<<<mt_grid(total_chunks * MT_PARTS), ADAM_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, a);
   AXB_CUDA(cudaGetLastError());
   return 0;
 }

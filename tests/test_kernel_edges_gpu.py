@@ -252,6 +252,42 @@ def test_scale_sizes_and_offsets(dtype):
         assert all(torch.equal(a, b) for a, b in zip(work, want))
 
 
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 1023, 1024, 1025, 2500])
+def test_tables_of_many_tensors(n):
+    """The search for a unit's tensor narrows 32-fold per round: table lengths around powers of 32, tensors without
+    elements, of less than a unit, of exactly one chunk and of several.  Scale: each product rounded once (exact).  Norm:
+    fp32 sums.  AdamW: fp32 arithmetic against the plain update (5e-6 of the size of a parameter and its step)."""
+    from axonn_b200.ops import _lib
+    from axonn_b200.ops.multi_tensor import _PtrTable
+    from axonn_b200.ops.optim_step import adamw_reference_
+    from axonn_b200.optim import FusedAdamW
+
+    torch.manual_seed(n)
+    kinds = [5, 16384, 0, 16385, 3, 65536, 0, 0, 70001, 1]
+    sizes = [kinds[(i * 7 + i // 10) % 10] if n < 1000 or i % 50 == 0 else (i * 37) % 3000 for i in range(n)]
+    sizes[0] = sizes[0] or 9
+    ts = [torch.randn(m, device=DEV) for m in sizes]
+    want = [t * 0.37 for t in ts]
+    tab = _PtrTable(ts)
+    norm = torch.zeros((), device=DEV)
+    L = _lib.lib()
+    _lib.check(L.axb_multi_l2norm_sq(_lib.addr(tab.dev), tab.n, tab.total_chunks, _lib.addr(norm), _lib.stream()), "norm")
+    ref = sum(float(t.double().pow(2).sum()) for t in ts)
+    assert abs(float(norm) - ref) < 1e-5 * ref
+    s = torch.full((), 0.37, device=DEV)
+    _lib.check(L.axb_multi_scale(_lib.addr(tab.dev), tab.n, tab.total_chunks, _lib.addr(s), _lib.stream()), "scale")
+    assert all(torch.equal(a, b) for a, b in zip(ts, want))
+    ps = [torch.nn.Parameter(t.clone()) for t in ts if t.numel()]
+    for p in ps:
+        p.grad = torch.randn_like(p)
+    ref = [(p.detach().clone(), torch.zeros_like(p), torch.zeros_like(p)) for p in ps]
+    FusedAdamW(ps, lr=1e-2, betas=(0.9, 0.95), eps=1e-8, weight_decay=0.1).step()
+    for p, (w, m, v) in zip(ps, ref):
+        adamw_reference_(w, p.grad, m, v, 1e-2, 0.9, 0.95, 1e-8, 0.1, 1)
+    got, ref = torch.cat([p.detach() for p in ps]), torch.cat([r[0] for r in ref])
+    assert float((got - ref).abs().max()) < 5e-6 * max(1.0, float(ref.abs().max()))
+
+
 # ------------------------------------------------------------------------------------------------ gradient pruning
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("offset", [0, 2, 4])
