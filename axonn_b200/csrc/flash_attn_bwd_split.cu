@@ -744,8 +744,6 @@ extern "C" int axb_flash_attn_bwd_split(const void* qkv, const void* out, const 
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int H = G * qpk, Sp = (S + 127) / 128 * 128;
-  // a launch through the runtime comes before the first driver call: on a thread that autograd has just started it is
-  // what binds the device's context
   const int rows_per_block = 256 / (D / 8) * FS_DELTA_ROWS;
   const long long rows = static_cast<long long>(Sp) * H;
   if (rows > 0x7fffffffll) { set_error("flash attention: too many rows"); return -1; }

@@ -212,6 +212,30 @@ def test_gemm_one_wave_of_pairs(M, N, K, dtype, layout):
     assert _lib.device_status() == 0
 
 
+# ------------------------------------------------------------------------------------------------ threads
+@pytest.mark.parametrize("op", ["gemm", "batched", "attention"])
+def test_first_call_of_a_thread(op):
+    """A new thread (autograd's worker at the start of a backward, for one) has no context before its first runtime call;
+    the tensor maps of these kernels are encoded before anything is launched."""
+    import threading
+
+    from axonn_b200 import ops
+    from axonn_b200.ops.gemm import bmm_nt
+
+    a, b = (torch.randn(2, 256, 256, device=DEV).bfloat16() for _ in range(2))
+    qkv = torch.randn(1, 256, 2, 3, 64, device=DEV).bfloat16()
+    call = {"gemm": lambda: ops.matmul_nt(a[0], b[0]), "batched": lambda: bmm_nt(a, b),
+            "attention": lambda: ops.flash_attention_packed(qkv)}[op]
+    want, got = call(), []                        # the allocator holds blocks of the sizes that the thread will ask for
+    torch.cuda.synchronize()
+    keep = want.clone()
+    del want
+    th = threading.Thread(target=lambda: got.append(call()))
+    th.start()
+    th.join()
+    assert got and torch.equal(got[0], keep)
+
+
 # ------------------------------------------------------------------------------------------------ cross-entropy
 @pytest.mark.parametrize("rows,V", [(1, 8), (3, 4096), (5, 4104), (7, 16384), (2, 16392), (1030, 50304)])
 def test_cross_entropy_rows(rows, V):
