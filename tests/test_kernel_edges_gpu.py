@@ -54,6 +54,33 @@ def test_norm_backward_sizes(rows, H, rms, residual, dtype):
         assert _rel(a, w) < tol, _rel(a, w)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,H", [(1, 8), (17, 264), (301, 512), (5, 520), (77, 1032), (4099, 2048), (9, 2056), (1001, 4096),
+                                    (6, 4104), (613, 8192), (5, 8200)])
+@pytest.mark.parametrize("rms", [True, False])
+@pytest.mark.parametrize("residual", [True, False])
+def test_norm_forward_sizes(rows, H, rms, residual, dtype):
+    """Outputs of the forward at the sizes where its thread groups, rings and kernels change.  The residual sum is exact
+    (one rounding of an fp32 sum); the normalised rows are rounded once to the storage type (2^-9 bf16, 2^-11 fp16) on
+    top of fp32 arithmetic (1e-5), row by row."""
+    from axonn_b200 import ops
+
+    torch.manual_seed(rows + H)
+    x, dl = (torch.randn(rows, H, device=DEV).to(dtype) for _ in range(2))
+    g = (1 + 0.1 * torch.randn(H, device=DEV)).to(dtype)
+    b = None if rms else (0.1 * torch.randn(H, device=DEV)).to(dtype)
+    if residual:
+        h, y = ops.add_rms_norm(x, dl, g, 1e-5) if rms else ops.add_layer_norm(x, dl, g, b, 1e-5)
+        assert torch.equal(h, (x.float() + dl.float()).to(dtype))
+    else:
+        h, y = x, (ops.rms_norm(x, g, 1e-5) if rms else ops.layer_norm(x, g, b, 1e-5))
+    z = h.double()
+    mean = 0 if rms else z.mean(-1, keepdim=True)
+    want = (z - mean) * ((z - mean).pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt() * g.double() + (0 if rms else b.double())
+    tol = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10, torch.float32: 2e-5}[dtype]
+    assert float(((y.double() - want).norm(dim=-1) / want.norm(dim=-1)).max()) < tol
+
+
 # ------------------------------------------------------------------------------------------------ attention, any length
 @pytest.mark.parametrize("B,S,G,qpk,D", [(1, 1, 1, 1, 64), (2, 5, 2, 1, 128), (3, 127, 1, 2, 64), (2, 129, 2, 2, 128),
                                          (2, 255, 1, 4, 128), (1, 257, 2, 1, 64), (3, 300, 2, 2, 128), (2, 511, 1, 1, 128),
@@ -208,6 +235,32 @@ def test_gemm_one_wave_of_pairs(M, N, K, dtype, layout):
             assert _rel(pre, w) < one
             assert _rel(act, torch.nn.functional.gelu(w, approximate="tanh")) < 2 * one
             assert _rel(ops.matmul_nt(a, b, bias=bias, epilogue=ops.EPI_BIAS), w) < one
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,N,K", [(192, 320, 328), (512, 264, 128)])
+def test_batched_gemm_one_segment(rows, N, K):
+    """One segment per problem: the weight gradient loops over the K blocks with data only.  Counts at the edges of a
+    block, none and all; rows past a count are zero and stay so."""
+    from axonn_b200.ops import _lib, gemm
+
+    torch.manual_seed(rows)
+    counts = [0, 1, 63, 64, 65, 128, rows - 1, rows]
+    seg = torch.tensor(counts, dtype=torch.int32, device=DEV).view(-1, 1)
+    live = torch.arange(rows, device=DEV)[None, :] < seg.long()
+    E = len(counts)
+    a = torch.randn(E, rows, K, device=DEV).bfloat16() * live[:, :, None]
+    b = torch.randn(E, N, K, device=DEV).bfloat16()
+    g = torch.randn(E, rows, N, device=DEV).bfloat16() * live[:, :, None]
+    y, gx = gemm.bmm_nt(a, b, seg=seg, seg_rows=rows), gemm.bmm_nn(g, b, seg=seg, seg_rows=rows)
+    gw = gemm.bmm_tn(g, a, out_dtype=torch.float32, seg=seg, seg_rows=rows)
+    assert bool((y[~live] == 0).all()) and bool((gx[~live] == 0).all()) and bool((gw[0] == 0).all())
+    for e in range(1, E):
+        a64, b64, g64 = a[e].double(), b[e].double(), g[e].double()
+        assert _rel(y[e], a64 @ b64.t()) < 2.0 ** -8
+        assert _rel(gx[e], g64 @ b64) < 2.0 ** -8
+        assert _rel(gw[e], g64.t() @ a64) < 1e-5
     torch.cuda.synchronize()
     assert _lib.device_status() == 0
 
@@ -416,3 +469,61 @@ def test_moe_permutations(T, k, rows, H):
     dy = torch.randn_like(y)
     got, want = torch.autograd.grad(y, [out, gate], dy), torch.autograd.grad(y64, [o64, g64], dy.double())
     assert _rel(got[0], want[0]) < 2.0 ** -8 and _rel(got[1], want[1]) < 1e-5
+
+
+def _local_moe(rank, world, T, hidden, ffn, E, k):
+    from axonn_b200 import axonn as ax
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib
+    from axonn_b200.parallel.moe import ExpertParallelMoE, route_top_k
+
+    ax.init(G_inter=1, G_data=world)
+    torch.manual_seed(T)
+    layer = ExpertParallelMoE(hidden, ffn, n_experts=E, top_k=k, dtype=torch.bfloat16)
+    with torch.no_grad():                          # the first expert overflows, the last one is never chosen
+        layer.router[0, 0], layer.router[-1, 0] = 0.5, -50.0
+    x = torch.randn(T, hidden, device=DEV).bfloat16()
+    x[:, 0] = 1.0
+    x.requires_grad_(True)
+    y = layer(x)
+    dy = torch.randn_like(y)
+    params = [x, layer.router, layer.w1, layer.w2]
+    got = torch.autograd.grad([y, layer.last_aux_loss], params, [dy, torch.full((), 0.02, device=DEV)])
+    assert _lib.device_status() == 0
+
+    C = layer.capacity(T)
+    with torch.no_grad():
+        idx, _, slot, keep, aux = route_top_k(ops.linear(x, layer.router), k, C)
+    per = torch.zeros(E, device=DEV).index_add(0, idx.reshape(-1), torch.ones(T * k, device=DEV))
+    assert float(per.max()) > C and float(per[-1]) == 0
+    assert torch.equal(layer.last_assignments_per_expert, per)
+    assert torch.equal(layer.last_dropped_per_expert, (per - C).clamp_min(0))
+    assert abs(float(layer.last_drop_fraction) - float((~keep).float().mean())) < 1e-6
+    x64, r64, w1, w2 = (p.detach().double().requires_grad_(True) for p in params)
+    z = x64 @ r64.t()
+    z = z + (z.to(torch.bfloat16).double() - z).detach()          # the router's logits are bf16 values
+    probs = z.softmax(-1)
+    gate = probs.gather(1, idx)
+    gate = gate / gate.sum(-1, keepdim=True)
+    ref = torch.zeros(T, hidden, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        tok, which = ((idx == e) & keep).nonzero(as_tuple=True)
+        v = (x64[tok] @ w1[e].t()).reshape(-1, ffn // 8, 2, 8)    # gate and up rows interleave in blocks of 8
+        h = (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(-1, ffn)
+        ref = ref.index_add(0, tok, (h @ w2[e].t()) * gate[tok, which][:, None])
+    aux64 = E * (per.double() / (T * k) * probs.mean(0)).sum()
+    want = torch.autograd.grad([ref, aux64], [x64, r64, w1, w2], [dy.double(), torch.full((), 0.02, dtype=torch.float64, device=DEV)])
+    assert abs(float(layer.last_aux_loss) - float(aux64)) < 1e-4 * abs(float(aux64))
+    return [_rel(y, ref)] + [_rel(a, b) for a, b in zip(got, want)], bool((got[3][-1] == 0).all() and (got[2][-1] == 0).all())
+
+
+@pytest.mark.parametrize("T,hidden,ffn,E,k", [(517, 256, 512, 4, 2), (96, 136, 72, 5, 1), (2000, 512, 1024, 8, 2)])
+def test_local_moe_layer(T, hidden, ffn, E, k):
+    """The whole layer with all experts on one GPU, an expert past its capacity and one without tokens, against routing in
+    torch and 64-bit experts.  Tolerance: the layer's intermediates are bf16 (four roundings of 2^-9 forward, twice as
+    many backward; the router's gradient is a difference of such sums)."""
+    from _dist import run_distributed
+
+    errors, empty = run_distributed(_local_moe, 1, T, hidden, ffn, E, k, backend="nccl", timeout=300)[0]
+    assert empty
+    assert errors[0] < 1e-2 and max(errors[1], errors[3], errors[4]) < 1.5e-2 and errors[2] < 2e-2, errors
