@@ -251,7 +251,7 @@ __device__ __forceinline__ void store_row32(void* base, int out_dtype, size_t ro
 }
 
 // Bias of 32 consecutive output columns as four 16-byte words (the columns past N stay undefined and are not stored).
-// Every lane reads the same words.  They are requested before the accumulator columns they belong to are waited for;
+// Every lane reads the same words.  They are requested ahead of the arithmetic that needs them;
 // read one 2-byte element at a time, inside the arithmetic, they took longer than the matrix product itself: 16384 x 8192 x
 // 2048 bf16 on a B200 took 358 us without bias, 560 - 620 us with it, 670 - 750 us with GELU; now 366, 375 and 492 us.
 __device__ __forceinline__ void load_bias32(const GemmParams& p, int col, uint4 (&b)[4]) {
@@ -285,41 +285,36 @@ __device__ __forceinline__ void add_bias32(const uint4 (&b)[4], int dtype, float
 }
 
 // Plain epilogue of one accumulator row (this thread's TMEM lane): columns col0 .. col0 + BN of row `row` in chunks of 32,
-// bias / GELU / accumulation.  The accumulator and bias words of a chunk are requested before the previous chunk is
-// converted and stored.  To the compiler the load's registers are written as soon as it is issued, so the wait has them as
-// operands and comes before the loop's back edge, and the load itself is predicated instead of branched around: nowhere
-// can a copy of them be due before they have arrived.  The same loop with the wait at its top, where the registers cross
-// the back edge in flight, takes as long: 777 x 4096 x 4096 bf16 on a B200 26.1 us without epilogue (now 26.5), 27.5 with
-// bias (27.4), 30.9 with bias, GELU and the saved pre-activation (30.6).
+// bias / GELU / accumulation.  The bias words of a chunk are requested when those of the previous one have been used, under
+// its GELU and stores; the accumulator columns are loaded, waited for and used in one round (to the compiler a load's
+// registers are written as soon as it is issued, so the wait has them as operands).  Loading the accumulator a chunk ahead
+// as well costs registers and gains nothing: one B200, bf16, ahead / now: 24 x 1024 x 256 6.0 / 5.8 us, with bias 7.0 / 6.7;
+// 777 x 4096 x 4096 26.1 / 25.5, 27.8 / 27.7, with GELU and the saved pre-activation 30.7 / 30.4.
 template <int BN>
 __device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t taddr, size_t row, bool row_ok, int col0) {
   const bool biased = p.epilogue == 1 || p.epilogue == 2;
-  uint32_t r[32];
   uint4 bn[4] = {};
-  tmem_ld_32x32(taddr, r);
   if (biased) load_bias32(p, col0, bn);
-  tmem_ld_wait(r);
 #pragma unroll 1
   for (int c = 0; c < BN / 32; ++c) {
     const int col = col0 + c * 32;
     if (col >= p.N) break;  // uniform across the warp
+    uint32_t r[32];
+    tmem_ld_32x32(taddr + c * 32, r);
+    tmem_ld_wait(r);
     float v[32];
-    uint4 b[4];
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-#pragma unroll
-    for (int g = 0; g < 4; ++g) b[g] = bn[g];
-    const bool more = c + 1 < BN / 32 && col + 32 < p.N;
-    tmem_ld_32x32_if(more, taddr + (c + 1) * 32, r);
-    if (biased && more) load_bias32(p, col + 32, bn);
-    if (biased) add_bias32(b, p.in_dtype, v);
+    if (biased) {
+      add_bias32(bn, p.in_dtype, v);
+      if (c + 1 < BN / 32 && col + 32 < p.N) load_bias32(p, col + 32, bn);
+    }
     if (p.epilogue >= 2) {
       if (p.aux != nullptr && row_ok) store_row32(p.aux, p.out_dtype, row, p.N, col, p.N, v, false);
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
     }
     if (row_ok) store_row32(p.C, p.out_dtype, row, p.N, col, p.N, v, p.accumulate != 0);
-    tmem_ld_wait(r);
   }
 }
 
