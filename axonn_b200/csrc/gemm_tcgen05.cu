@@ -1362,7 +1362,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // Measured on a B200 (graph replay, bias epilogue): 24 x 8192 x 2048 22.0 -> 12.4 us, 24 x 2048 x 8192 31.7 -> 10.7 us (33.5 MB
 // of weights each).
 constexpr int SK_THREADS = 192;   // TMA warp, MMA warp, 4 epilogue warps
-constexpr int SK_MAX_Z = 8;       // portable cluster size
 struct SplitKSmem {
   static constexpr int BN = 128;
   static constexpr int A_BYTES = BM * BK * 2;
@@ -1745,14 +1744,27 @@ static int splitk_max_clusters(int z, int device) {
   return n;
 }
 
-// CTAs per output tile of the split-K kernel: the largest power of two with which all tiles are in flight at once and
-// every CTA still has 4 K blocks of work; 1 = do not split.
+// CTAs per output tile of the split-K kernel, 1 = do not split.  All tiles have to be in flight at once and every CTA needs
+// 4 K blocks to work on; among 2, 4 and 8 CTAs the one that saves most wins, if any saves at all: a K block that a CTA does
+// not walk saves 0.16 us, and the exchange of the partial tiles costs as much as a number of K blocks that grows with
+// the rows in the tile.  Measured on a B200 for z = 1, 2, 4, 8 over M 1 .. 512, N 128 .. 8192, K 512 .. 16384, warm and cold
+// weights (us, one CTA / split): 24 x 1024 x 1024 7.7 / 6.3 (z 4), 128 x 1024 x 1024 7.8 / 9.1 (z 2, not taken), 128 x 1024 x
+// 4096 16.0 / 11.2 (z 4), 1000 x 1024 x 4096 16.5 / 14.3 (z 2).  Nothing in that range is slower than one CTA by more
+// than 2 %; splitting whenever every CTA had its 4 K blocks was, by up to 37 % (512 x 2048 x 512).
 static int splitk_ctas(int M, int N, int K, int sms, int device) {
+  static constexpr struct { int z; float per_row; } kCost[3] = {{2, 0.14f}, {4, 0.18f}, {8, 0.29f}};
   const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + SplitKSmem::BN - 1) / SplitKSmem::BN);
-  const int num_kb = (K + BK - 1) / BK;
-  for (int z = SK_MAX_Z; z > 1; z /= 2)
-    if (num_kb >= 4 * z && tiles * z <= sms && tiles <= splitk_max_clusters(z, device)) return z;
-  return 1;
+  const int num_kb = (K + BK - 1) / BK, rows = M < BM ? M : BM;
+  int best = 1;
+  float best_gain = 0.f;
+  for (const auto& c : kCost) {
+    const float gain = static_cast<float>(num_kb) * (c.z - 1) / c.z - (1.f + c.per_row * rows);
+    if (num_kb >= 4 * c.z && tiles * c.z <= sms && gain > best_gain && tiles <= splitk_max_clusters(c.z, device)) {
+      best = c.z;
+      best_gain = gain;
+    }
+  }
+  return best;
 }
 
 template <int A_MN, int B_MN>

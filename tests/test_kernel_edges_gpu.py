@@ -173,7 +173,8 @@ def test_attention_other_scales(S, scale):
 # ------------------------------------------------------------------------------------------------ split-K GEMM
 @pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
 @pytest.mark.parametrize("M,N,K", [(8, 128, 256), (24, 2048, 8192), (24, 8192, 2048), (120, 136, 1000), (136, 264, 520),
-                                   (128, 1024, 4096), (256, 256, 16384), (1, 512, 2048), (33, 40, 4104)])
+                                   (128, 1024, 4096), (256, 256, 16384), (1, 512, 2048), (33, 40, 4104),
+                                   (120, 136, 8200), (100, 264, 3080), (128, 2056, 2568), (40, 8200, 1544)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_gemm_few_tiles(layout, M, N, K, dtype):
     """Problems of few tiles (K split over a cluster), rows and columns that end inside a tile, K blocks that do not
