@@ -228,6 +228,241 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
   }
 }
 
+// ---- fp32, hidden 1032 .. 4096, local statistics: a block handles R rows per iteration with one 8-element chunk per thread
+// and CH, keeps the rows in registers between the statistics and the apply step (one global read per element) and needs
+// a single block barrier per iteration.  In fp32 the rings below take twice the shared memory and leave two blocks on an
+// SM; these kernels keep eight (norm_fwd_path, norm_bwd_path: where which is faster).
+template <int NV>
+__device__ __forceinline__ void block_sum_n(float (&v)[NV], float* red /* [2][NV][8] */, int it) {
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+  float* buf = red + (it & 1) * NV * 8;     // double-buffered by iteration: one barrier per iteration
+  if (l == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) buf[k * 8 + w] = v[k];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    float t = 0.f;
+    for (int i = 0; i < nw; ++i) t += buf[k * 8 + i];
+    v[k] = t;
+  }
+}
+
+template <typename T, bool RMS, int CH, int R>
+__global__ void __launch_bounds__(NORM_THREADS)
+norm_fwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta,
+                     T* __restrict__ y, float* __restrict__ stats, int rows, int H, float eps,
+                     const T* __restrict__ delta, T* __restrict__ hout) {
+  __shared__ float red[2 * 2 * R * 8];
+  const int nchunk = H / 8;
+  float g[CH][8], b[CH][8];
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    const int c = threadIdx.x + k * blockDim.x;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { g[k][i] = 0.f; b[k][i] = 0.f; }
+    if (c < nchunk) {
+      Vec8<T>::load(gamma + c * 8, g[k]);
+      if (!RMS && beta) Vec8<T>::load(beta + c * 8, b[k]);
+    }
+  }
+  int it = 0;
+  for (int row0 = blockIdx.x * R; row0 < rows; row0 += gridDim.x * R, ++it) {
+    float f[R][CH][8];
+    float sm[2 * R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      sm[2 * r] = 0.f; sm[2 * r + 1] = 0.f;
+#pragma unroll
+      for (int k = 0; k < CH; ++k) {
+        const int c = threadIdx.x + k * blockDim.x;
+        if (row0 + r < rows && c < nchunk) {
+          Vec8<T>::load(x + static_cast<size_t>(row0 + r) * H + c * 8, f[r][k]);
+          if (delta) {
+            add_rounded<T>(f[r][k], delta + static_cast<size_t>(row0 + r) * H + c * 8);
+            Vec8<T>::store(hout + static_cast<size_t>(row0 + r) * H + c * 8, f[r][k]);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) f[r][k][i] = 0.f;
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int k = 0; k < CH; ++k)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) { sm[2 * r] += f[r][k][i]; sm[2 * r + 1] += f[r][k][i] * f[r][k][i]; }
+    block_sum_n<2 * R>(sm, red, it);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (row0 + r >= rows) break;
+      float mean, rstd;
+      if (RMS) { mean = 0.f; rstd = rsqrtf(sm[2 * r + 1] / H + eps); }
+      else { mean = sm[2 * r] / H; rstd = rsqrtf(fmaxf(sm[2 * r + 1] / H - mean * mean, 0.f) + eps); }
+      if (threadIdx.x == 0) { stats[2 * (row0 + r)] = mean; stats[2 * (row0 + r) + 1] = rstd; }
+#pragma unroll
+      for (int k = 0; k < CH; ++k) {
+        const int c = threadIdx.x + k * blockDim.x;
+        if (c >= nchunk) continue;
+        float o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = (f[r][k][i] - mean) * rstd * g[k][i] + b[k][i];
+        Vec8<T>::store(y + static_cast<size_t>(row0 + r) * H + c * 8, o);
+      }
+    }
+  }
+}
+
+// Forward with one warp per row (hidden = 256 * VPL elements, the whole row in registers): the statistics need only
+// warp shuffles, so there is no block barrier between the load and the store phase and the eight warps of a block
+// run their rows independently - their loads stay in flight continuously.  gamma / beta are re-read per row (they
+// stay in L1).  It wants many rows (see norm_fwd_path).
+template <typename T, bool RMS, int VPL>
+__global__ void __launch_bounds__(256)
+norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta,
+                     T* __restrict__ y, float* __restrict__ stats, int rows, int H, float eps,
+                     const T* __restrict__ delta, T* __restrict__ hout) {
+  const int lane = threadIdx.x & 31;
+  const long long nwarps = static_cast<long long>(gridDim.x) * 8;
+  for (long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5); row < rows; row += nwarps) {
+    const size_t base = static_cast<size_t>(row) * H;
+    float f[VPL][8];
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+      const int c = (lane + 32 * k) * 8;
+      Vec8<T>::load(x + base + c, f[k]);
+      if (delta) {
+        add_rounded<T>(f[k], delta + base + c);
+        Vec8<T>::store(hout + base + c, f[k]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < VPL; ++k)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) { s1 += f[k][i]; s2 += f[k][i] * f[k][i]; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    }
+    float mean, rstd;
+    if (RMS) { mean = 0.f; rstd = rsqrtf(s2 / H + eps); }
+    else { mean = s1 / H; rstd = rsqrtf(fmaxf(s2 / H - mean * mean, 0.f) + eps); }
+    if (lane == 0) { stats[2 * row] = mean; stats[2 * row + 1] = rstd; }
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) {
+      const int c = (lane + 32 * k) * 8;
+      float g[8], b[8], o[8];
+      Vec8<T>::load(gamma + c, g);
+      if (!RMS && beta) Vec8<T>::load(beta + c, b);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float v = (f[k][i] - mean) * rstd * g[i];
+        if (!RMS && beta) v += b[i];
+        o[i] = v;
+      }
+      Vec8<T>::store(y + base + c, o);
+    }
+  }
+}
+
+template <typename T, bool RMS, int CH, int R>
+__global__ void __launch_bounds__(NORM_THREADS)
+norm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
+                     const float* __restrict__ stats, T* __restrict__ dx, float* __restrict__ dgamma_part,
+                     float* __restrict__ dbeta_part, int rows, int H, const T* __restrict__ dres) {
+  __shared__ float red[2 * 2 * R * 8];
+  const int nchunk = H / 8;
+  float g[CH][8], ag[CH][8], ab[CH][8];
+#pragma unroll
+  for (int k = 0; k < CH; ++k) {
+    const int c = threadIdx.x + k * blockDim.x;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { g[k][i] = 0.f; ag[k][i] = 0.f; ab[k][i] = 0.f; }
+    if (c < nchunk) Vec8<T>::load(gamma + c * 8, g[k]);
+  }
+  int it = 0;
+  for (int row0 = blockIdx.x * R; row0 < rows; row0 += gridDim.x * R, ++it) {
+    float xh[R][CH][8], d[R][CH][8];
+    float rstd[R];
+    float sm[2 * R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const bool live = row0 + r < rows;
+      const float mean = live ? stats[2 * (row0 + r)] : 0.f;
+      rstd[r] = live ? stats[2 * (row0 + r) + 1] : 0.f;
+      sm[2 * r] = 0.f; sm[2 * r + 1] = 0.f;
+#pragma unroll
+      for (int k = 0; k < CH; ++k) {
+        const int c = threadIdx.x + k * blockDim.x;
+        if (live && c < nchunk) {
+          Vec8<T>::load(x + static_cast<size_t>(row0 + r) * H + c * 8, xh[r][k]);
+          Vec8<T>::load(dy + static_cast<size_t>(row0 + r) * H + c * 8, d[r][k]);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) xh[r][k][i] = (xh[r][k][i] - mean) * rstd[r];
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) { xh[r][k][i] = 0.f; d[r][k][i] = 0.f; }
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int k = 0; k < CH; ++k)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float gd = g[k][i] * d[r][k][i];
+          sm[2 * r] += gd; sm[2 * r + 1] += gd * xh[r][k][i];
+          ag[k][i] += d[r][k][i] * xh[r][k][i]; ab[k][i] += d[r][k][i];
+        }
+    block_sum_n<2 * R>(sm, red, it);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (row0 + r >= rows) break;
+      const float m1 = RMS ? 0.f : sm[2 * r] / H, m2 = sm[2 * r + 1] / H;
+#pragma unroll
+      for (int k = 0; k < CH; ++k) {
+        const int c = threadIdx.x + k * blockDim.x;
+        if (c >= nchunk) continue;
+        float o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = rstd[r] * (g[k][i] * d[r][k][i] - m1 - xh[r][k][i] * m2);
+        if (dres) {
+          float r8[8];
+          Vec8<T>::load(dres + static_cast<size_t>(row0 + r) * H + c * 8, r8);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] += r8[i];
+        }
+        Vec8<T>::store(dx + static_cast<size_t>(row0 + r) * H + c * 8, o);
+      }
+    }
+  }
+  if (dgamma_part) {
+#pragma unroll
+    for (int k = 0; k < CH; ++k) {
+      const int c = threadIdx.x + k * blockDim.x;
+      if (c >= nchunk) continue;
+      float4* pg = reinterpret_cast<float4*>(dgamma_part + static_cast<size_t>(blockIdx.x) * H + c * 8);
+      pg[0] = make_float4(ag[k][0], ag[k][1], ag[k][2], ag[k][3]);
+      pg[1] = make_float4(ag[k][4], ag[k][5], ag[k][6], ag[k][7]);
+      if (!RMS && dbeta_part) {
+        float4* pb = reinterpret_cast<float4*>(dbeta_part + static_cast<size_t>(blockIdx.x) * H + c * 8);
+        pb[0] = make_float4(ab[k][0], ab[k][1], ab[k][2], ab[k][3]);
+        pb[1] = make_float4(ab[k][4], ab[k][5], ab[k][6], ab[k][7]);
+      }
+    }
+  }
+}
+
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -409,8 +644,8 @@ static int norm_fwd_ring(const T* x, const T* gamma, const T* beta, T* y, float*
 // cp.async: the ring needs no barrier, and the loads of the next STAGES - 1 row batches run under the reduction of the
 // current one.  One block barrier per batch of R rows combines the row sums (none when a warp holds the row); the
 // column sums for dgamma / dbeta stay in registers until the end, one partial row per block.
-// Two blocks per SM, so a quarter of the partial rows that one block per visiting row batch wrote.  Measured on a B200,
-// kernel + fold: LayerNorm with residual, 16384 x 2048 bf16 (268 MB) 94.8 + 10.0 -> 50.4 + 4.0 us; RMSNorm, 4099 x 4096
+// One or two blocks per SM (NormBwdRing::MINB: two in 16 bits up to hidden 4096), so a quarter of the partial rows that one
+// block per visiting row batch wrote.  Measured on a B200, kernel + fold: LayerNorm with residual, 16384 x 2048 bf16 (268 MB) 94.8 + 10.0 -> 50.4 + 4.0 us; RMSNorm, 4099 x 4096
 // bf16 (101 MB) 38.7 + 10.1 -> 20.9 + 4.1 us.  The kernel before it loaded a batch, reduced and stored it in turn.
 template <typename T, int NT, int CH, int R>
 struct NormBwdRing {
@@ -739,15 +974,87 @@ gelu_bwd_colsum_kernel(const T* __restrict__ dy, const T* __restrict__ x, T* __r
 
 int sm_count(int device);
 
+// Which kernel takes a norm with local statistics (the split-hidden modes have the general kernel only).  All of them were
+// measured on a B200 over 1 .. 16384 rows and hidden 128 .. 8192, with inputs in the L2 and from DRAM; the rings win where
+// nothing is said.  Times in us, the ring's first.
+enum class NormPath { RING, WARP, ROWS, GENERAL };
+
+// Forward.
+//   16 bits: a warp per row at hidden 1024 and 2048 with many rows and no residual (4096 x 2048 9.2 / 7.4, 16384 x 1024 14.6 /
+//     11.7; with few rows 1000 x 2048 3.7 / 4.2).  Above 4096 the ring has one block per SM: with a residual it pays for
+//     at most a row per SM (128 x 5120 2.7 / 3.4, 1000 x 5120 8.6 / 6.7) or many wide rows (8192 x 6144 0.9 of the general
+//     kernel's time), without one not at all.
+//   fp32: the ring's shared memory leaves two blocks per SM.  Without a residual the general kernel is faster for few narrow
+//     rows (16 x 512 2.6 / 2.2) and a warp per row for many at 1024, 2048 and 4096 (16384 x 1024 32.9 / 25.7).  With one
+//     only the narrowest rows keep the ring: general kernel up to 1024 and for few rows (16384 x 768 45.0 / 36.2, 128 x 2048
+//     3.3 / 2.5), a warp per row or a block of rows for many (16384 x 2048 115 / 91, 16384 x 1536 85 / 65).
+template <typename T>
+static NormPath norm_fwd_path(int rows, int H, bool residual, int sms) {
+  const int nchunk = H / 8;
+  const bool warp_width = H == 1024 || H == 2048 || H == 4096;
+  if (sizeof(T) == 2) {
+    if (nchunk <= 512)
+      return !residual && (H == 1024 || H == 2048) && rows >= 13 * sms ? NormPath::WARP : NormPath::RING;
+    return residual && nchunk <= 1024 && (rows <= sms || (nchunk > 640 && rows >= 20 * sms)) ? NormPath::RING : NormPath::GENERAL;
+  }
+  if (nchunk > 512) return NormPath::GENERAL;
+  if (residual) {
+    if (nchunk <= 16 && rows >= 6 * sms) return NormPath::RING;
+    if (nchunk <= 128 || rows < 4 * sms) return NormPath::GENERAL;
+    return warp_width ? NormPath::WARP : NormPath::ROWS;
+  }
+  if (nchunk > 32 && nchunk < 128 && rows < 6 * sms) return NormPath::GENERAL;
+  return warp_width && rows >= 4 * sms ? NormPath::WARP : NormPath::RING;
+}
+
+// Backward.
+//   16 bits: the general kernel for few narrow rows (16 x 512 4.6 / 4.0), which it gives a block each.
+//   fp32: up to 1024 the general kernel for few rows (16 x 512 6.0 / 4.0) and for very many of the wider ones (16384 x 1024
+//     74 / 61, 4096 x 1024 21.7 / 27.8); above, a block of rows for both (128 x 4096 7.8 / 6.7, 16384 x 2048 138 / 115; 1000 x 4096
+//     22 / 29).
+template <typename T>
+static NormPath norm_bwd_path(int rows, int H, int sms) {
+  const int nchunk = H / 8;
+  if (sizeof(T) == 2) {
+    if (nchunk > 1024) return NormPath::GENERAL;
+    return nchunk <= 96 && rows <= 128 ? NormPath::GENERAL : NormPath::RING;
+  }
+  if (nchunk > 512) return NormPath::GENERAL;
+  if (nchunk <= 128) return rows < 3 * sms || (nchunk >= 96 && rows > 55 * sms) ? NormPath::GENERAL : NormPath::RING;
+  return rows < 4 * sms || rows > 40 * sms ? NormPath::ROWS : NormPath::RING;
+}
+
 template <typename T>
 static int norm_fwd_t(const void* x, const void* gamma, const void* beta, void* y, float* stats, int rows, int H,
                       int H_total, float eps, int rms, int mode, int grid, cudaStream_t s, const void* delta, void* hout) {
   const int threads = (H / 8 <= 128) ? 128 : NORM_THREADS;  // no idle threads for narrow (sharded) rows
-  // local statistics: the ring kernel, hidden 8192 at most.  Split-hidden modes and wider rows take the general kernel, and
-  // so do rows above 4096 without a residual, where the ring's one block per SM brings nothing (3000 x 8192: 22.5 against
-  // 23.3 us; with the residual 38 against 33.5 us).
   const int nchunk = H / 8;
-  if (mode == 0 && H == H_total && nchunk <= (delta ? 1024 : 512)) {
+  const NormPath path = mode == 0 && H == H_total ? norm_fwd_path<T>(rows, H, delta != nullptr, sm_count_current()) : NormPath::GENERAL;
+  if (path == NormPath::WARP) {
+    const int wgrid = min((rows + 7) / 8, grid * 2);
+#define AXB_NORM_FWD_WARP(RMS_, VPL_)                                                                           \
+  norm_fwd_warp_kernel<T, RMS_, VPL_><<<wgrid, 256, 0, s>>>((const T*)x, (const T*)gamma, (const T*)beta, (T*)y, \
+                                                           stats, rows, H, eps, (const T*)delta, (T*)hout)
+    if (H == 1024) { if (rms) AXB_NORM_FWD_WARP(true, 4); else AXB_NORM_FWD_WARP(false, 4); }
+    else if (H == 2048) { if (rms) AXB_NORM_FWD_WARP(true, 8); else AXB_NORM_FWD_WARP(false, 8); }
+    else if constexpr (sizeof(T) == 4) { if (rms) AXB_NORM_FWD_WARP(true, 16); else AXB_NORM_FWD_WARP(false, 16); }
+#undef AXB_NORM_FWD_WARP
+    AXB_CUDA(cudaGetLastError());
+    return 0;
+  }
+  if constexpr (sizeof(T) == 4) {
+    if (path == NormPath::ROWS) {
+#define AXB_NORM_FWD_ROWS(RMS_, CH_, R_)                                                                         \
+  norm_fwd_rows_kernel<T, RMS_, CH_, R_><<<min(grid, (rows + R_ - 1) / R_), NORM_THREADS, 0, s>>>(              \
+      (const T*)x, (const T*)gamma, (const T*)beta, (T*)y, stats, rows, H, eps, (const T*)delta, (T*)hout)
+      if (nchunk <= NORM_THREADS) { if (rms) AXB_NORM_FWD_ROWS(true, 1, 4); else AXB_NORM_FWD_ROWS(false, 1, 4); }
+      else { if (rms) AXB_NORM_FWD_ROWS(true, 2, 2); else AXB_NORM_FWD_ROWS(false, 2, 2); }
+#undef AXB_NORM_FWD_ROWS
+      AXB_CUDA(cudaGetLastError());
+      return 0;
+    }
+  }
+  if (path == NormPath::RING) {
 #define AXB_NORM_FWD_RING(NT_, TPR_, CH_, R_)                                                                        \
   return rms ? norm_fwd_ring<T, true, NT_, TPR_, CH_, R_>((const T*)x, (const T*)gamma, (const T*)beta, (T*)y, stats, \
                                                           rows, H, eps, (const T*)delta, (T*)hout, s)                \
@@ -758,7 +1065,7 @@ static int norm_fwd_t(const void* x, const void* gamma, const void* beta, void* 
     if (nchunk <= 128) AXB_NORM_FWD_RING(256, 128, 1, 2);
     if (nchunk <= 256) AXB_NORM_FWD_RING(256, 256, 1, 2);
     if (nchunk <= 512) AXB_NORM_FWD_RING(256, 256, 2, 1);
-    AXB_NORM_FWD_RING(512, 512, 2, 1);
+    if constexpr (sizeof(T) == 2) AXB_NORM_FWD_RING(512, 512, 2, 1);
 #undef AXB_NORM_FWD_RING
   }
   if (rms)
@@ -779,9 +1086,21 @@ static int norm_bwd_t(const void* dy, const void* x, const void* gamma, const fl
   const int nchunk = H / 8;
   const int threads = (nchunk <= 128) ? 128 : NORM_THREADS;
   const int ch = (nchunk + threads - 1) / threads;
-  // local statistics: the ring kernel up to the widest row whose ring fits the shared memory (hidden 8192 in 16 bits,
-  // 4096 in fp32); the split-hidden modes and wider rows take the general kernel below
-  if (mode == 0 && H == H_total && nchunk <= (sizeof(T) == 4 ? 512 : 1024)) {
+  const NormPath path = mode == 0 && H == H_total ? norm_bwd_path<T>(rows, H, sm_count_current()) : NormPath::GENERAL;
+  if constexpr (sizeof(T) == 4) {
+    if (path == NormPath::ROWS) {
+#define AXB_NORM_BWD_ROWS(RMS_, CH_, R_)                                                                       \
+  *blocks_launched = min(grid, (rows + R_ - 1) / R_);                                                          \
+  norm_bwd_rows_kernel<T, RMS_, CH_, R_><<<*blocks_launched, NORM_THREADS, 0, s>>>(                            \
+      (const T*)dy, (const T*)x, (const T*)gamma, stats, (T*)dx, dgp, dbp, rows, H, (const T*)dres)
+      if (nchunk <= NORM_THREADS) { if (rms) { AXB_NORM_BWD_ROWS(true, 1, 2); } else { AXB_NORM_BWD_ROWS(false, 1, 2); } }
+      else { if (rms) { AXB_NORM_BWD_ROWS(true, 2, 1); } else { AXB_NORM_BWD_ROWS(false, 2, 1); } }
+#undef AXB_NORM_BWD_ROWS
+      AXB_CUDA(cudaGetLastError());
+      return 0;
+    }
+  }
+  if (path == NormPath::RING) {
 #define AXB_NORM_BWD_RING(NT_, TPR_, CH_, R_)                                                                       \
   return rms ? norm_bwd_ring<T, true, NT_, TPR_, CH_, R_>((const T*)dy, (const T*)x, (const T*)gamma, stats, (T*)dx, \
                                                           dgp, dbp, rows, H, (const T*)dres, grid, blocks_launched, s) \

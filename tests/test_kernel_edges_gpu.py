@@ -17,7 +17,8 @@ def _rel(got, want):
 # ------------------------------------------------------------------------------------------------ norm backward
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("rows,H", [(1, 8), (3, 256), (17, 264), (301, 512), (5, 520), (2048, 1024), (77, 1032), (4099, 2048),
-                                    (9, 2056), (1001, 4096), (6, 4104), (613, 8192), (5, 8200)])
+                                    (9, 2056), (1001, 4096), (6, 4104), (613, 8192), (5, 8200), (128, 768), (129, 768), (443, 512),
+                                    (445, 512), (591, 2056), (593, 1032), (5921, 1536), (8141, 1024)])
 @pytest.mark.parametrize("rms,residual", [(True, False), (False, True)])
 def test_norm_backward_sizes(rows, H, rms, residual, dtype):
     """Thread groups per row change at hidden 256, 512, 1024, 2048, 4096; the batch of rows per block and the ring of
@@ -56,7 +57,8 @@ def test_norm_backward_sizes(rows, H, rms, residual, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("rows,H", [(1, 8), (17, 264), (301, 512), (5, 520), (77, 1032), (4099, 2048), (9, 2056), (1001, 4096),
-                                    (6, 4104), (613, 8192), (5, 8200)])
+                                    (6, 4104), (613, 8192), (5, 8200), (2500, 1024), (887, 520), (889, 520), (591, 1032), (593, 1032),
+                                    (601, 2056), (601, 2048), (148, 5120), (149, 5120), (2963, 6144)])
 @pytest.mark.parametrize("rms", [True, False])
 @pytest.mark.parametrize("residual", [True, False])
 def test_norm_forward_sizes(rows, H, rms, residual, dtype):
