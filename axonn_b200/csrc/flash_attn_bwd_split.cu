@@ -8,8 +8,8 @@
 //   fa_bwd_dq_kernel   one 128-row query tile per work item, walks the key tiles up to the diagonal:
 //                      S = Q K^T and dP = dO V^T (128 x 128 each) into tensor memory, the softmax threads read
 //                      them into registers (the MMA warp then already issues the next tile's S and dP),
-//                      dS = P (dP - delta) scale goes back as bf16 and dQ += dS K accumulates in tensor memory.
-//                      dQ is written once, as bf16, into the packed gradient tensor.
+//                      dS = P (dP - delta) goes back as bf16 and dQ += dS K accumulates in tensor memory.
+//                      dQ is scaled and written once, as bf16, into the packed gradient tensor.
 //   fa_bwd_dkv_kernel  one 128-row key tile per work item, walks the query tiles from the diagonal down (and the
 //                      query heads of the group) in steps of 64 queries: S^T = K Q^T and dP^T = V dO^T into
 //                      double-buffered 64-column score buffers (a thread owns a key row), P^T and dS^T go back as
@@ -45,8 +45,8 @@ struct FaSplitParams {
 // kernels (one exponential, one conversion and two multiply-adds per score, behind tensor-memory loads); four warps
 // per scheduler with 32 scores per thread hide that latency, two warps with 64 do not.  Registers: 640 threads get 96
 // each at launch, 128 * 64 + 512 * 104 after the split are exactly those.
-// Measured on a B200, dQ / dK+dV kernel, 8 x 2048, 16 heads, head_dim 128 (two warps per scheduler, then four): the pair
-// with its delta kernel 660 - 700 us -> 577 us (247 + 363 + 35 one by one); cuDNN's backward takes 492 us there.
+// Measured on a B200, 8 x 2048, 16 heads, head_dim 128, back to back in one graph: dQ, dK / dV and delta kernel together 660 -
+// 700 us with two warps per scheduler, 584 - 599 us now (the library's backward 492 us).
 constexpr int FS_THREADS = 640;
 constexpr int FS_SOFTMAX_WARPS = 16;
 #define FS_REGS_CONTROL "setmaxnreg.dec.sync.aligned.u32 64;"
@@ -121,8 +121,6 @@ struct DqSmem {
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 16 + 1024;
 };
 
-// Work item k of this CTA: query tiles sorted by decreasing length (tile i walks i + 1 key tiles), dealt to the
-// persistent CTAs in a snake.
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
@@ -144,6 +142,8 @@ __device__ __forceinline__ void fs_store32(__nv_bfloat16* dst, const uint32_t (&
   }
 }
 
+// Work item k of this CTA: query tiles sorted by decreasing length (tile i walks i + 1 key tiles), dealt to the
+// persistent CTAs in a snake.
 struct DqItem { int i, head, b; };
 __device__ __forceinline__ bool dq_item(const FaSplitParams& p, int k, DqItem& w) {
   const int G = gridDim.x, c = blockIdx.x;
@@ -435,7 +435,7 @@ struct DkvSmem {
   // Q / dO: two query tiles of two halves (64 queries) each.  A half is loaded and released by itself: its step's
   // accumulator MMAs free it a whole tile before its successor is needed, which hides the load; a ring of whole tiles
   // got half a tile's time for that and the MMA warps waited for it in every tile.
-  // dK / dV kernel on a B200: 8 x 2048, 16 heads, head_dim 128 338 -> 318 us; head_dim 64 285 -> 244 us.
+  // dK / dV kernel by itself on a B200: 8 x 2048, 16 heads, head_dim 128 338 -> 318 us; head_dim 64 285 -> 244 us.
   static constexpr int Q_OFF = 2 * TILE;           // 2 stages
   static constexpr int DO_OFF = 4 * TILE;          // 2 stages
   static constexpr int LSE_OFF = 6 * TILE;         // [2 stages][lse, delta][128] fp32

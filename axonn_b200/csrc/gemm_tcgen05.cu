@@ -251,9 +251,10 @@ __device__ __forceinline__ void store_row32(void* base, int out_dtype, size_t ro
 }
 
 // Bias of 32 consecutive output columns as four 16-byte words (the columns past N stay undefined and are not stored).
-// Every lane reads the same words.  They are requested ahead of the arithmetic that needs them;
-// read one 2-byte element at a time, inside the arithmetic, they took longer than the matrix product itself: 16384 x 8192 x
-// 2048 bf16 on a B200 took 358 us without bias, 560 - 620 us with it, 670 - 750 us with GELU; now 366, 375 and 492 us.
+// Every lane reads the same words.  They are requested ahead of the arithmetic that needs them; read one 2-byte element at a
+// time, inside the arithmetic, they took longer than the matrix product itself: 16384 x 8192 x 2048 bf16 on a B200 took 359
+// us without bias, 538 - 620 us with it, 670 - 780 us with GELU and the saved pre-activation; now 359, 355 - 375 and 434 - 492
+// us (the clock under the power cap moves them).
 __device__ __forceinline__ void load_bias32(const GemmParams& p, int col, uint4 (&b)[4]) {
   const uint16_t* src = reinterpret_cast<const uint16_t*>(p.bias) + col;
   if ((reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {      // N and col are multiples of 8: whole words inside the vector
@@ -1360,7 +1361,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // No workspace, no atomics, one launch.  Such a problem is bound by reading the weights once; with one CTA per tile
 // the loads of tiles < SMs / 2 CTAs in flight do not fill the memory system.
 // Measured on a B200 (graph replay, bias epilogue): 24 x 8192 x 2048 22.0 -> 12.4 us, 24 x 2048 x 8192 31.7 -> 10.7 us (33.5 MB
-// of weights each).
+// of weights each).  splitk_ctas says when it is taken.
 constexpr int SK_THREADS = 192;   // TMA warp, MMA warp, 4 epilogue warps
 struct SplitKSmem {
   static constexpr int BN = 128;
@@ -1748,8 +1749,8 @@ static int splitk_max_clusters(int z, int device) {
 // 4 K blocks to work on; among 2, 4 and 8 CTAs the one that saves most wins, if any saves at all: a K block that a CTA does
 // not walk saves 0.16 us, and the exchange of the partial tiles costs as much as a number of K blocks that grows with
 // the rows in the tile.  Measured on a B200 for z = 1, 2, 4, 8 over M 1 .. 512, N 128 .. 8192, K 512 .. 16384, warm and cold
-// weights (us, one CTA / split): 24 x 1024 x 1024 7.7 / 6.3 (z 4), 128 x 1024 x 1024 7.8 / 9.1 (z 2, not taken), 128 x 1024 x
-// 4096 16.0 / 11.2 (z 4), 1000 x 1024 x 4096 16.5 / 14.3 (z 2).  Nothing in that range is slower than one CTA by more
+// weights (us, one CTA / split): 24 x 1024 x 1024 7.6 / 6.1 (z 4), 128 x 1024 x 1024 8.0 / 9.0 (z 2, not taken), 128 x 1024 x
+// 4096 15.7 / 10.9 (z 4), 1000 x 1024 x 4096 16.5 / 14.3 (z 2).  Nothing in that range is slower than one CTA by more
 // than 2 %; splitting whenever every CTA had its 4 K blocks was, by up to 37 % (512 x 2048 x 512).
 static int splitk_ctas(int M, int N, int K, int sms, int device) {
   static constexpr struct { int z; float per_row; } kCost[3] = {{2, 0.14f}, {4, 0.18f}, {8, 0.29f}};
@@ -1843,7 +1844,9 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
   // tile is twice the work per SM, but single CTAs reach only 0.6 of its rate (their operands exceed the shared-memory
   // bandwidth), so the pairs win as long as they need at most 5 waves where single CTAs need 6 of half the size - in
   // particular with one wave of pairs against two, which the demand for a full wave of pairs used to rule out.  One B200,
-  // bf16: 2048 x 2048 x 16384 119.8 -> 97.0 us, 777 x 4096 x 4096 30.1 -> 26.7 us, 1000 x 1024 x 4096 16.6 -> 14.1 us.
+  // bf16 (M x N x K): 2048 x 2048 x 16384 119 -> 96 us, 777 x 4096 x 4096 29.7 -> 26.2, 640 x 4096 x 1024 13.3 -> 11.9.  Over the
+  // 40 shapes of M 129 .. 8192, N 512 .. 16384 that only this clause sends to pairs, their time is 0.80 - 0.94 of the
+  // single CTAs' at K 4096, 0.89 - 1.01 at K 1024 and 0.88 - 1.03 (N 3072 and 5120) at K 128 .. 768.
   const long long pair_tiles = static_cast<long long>((tiles_m + 1) / 2) * ((N + 255) / 256);
   const long long single_tiles = static_cast<long long>(tiles_m) * ((N + 127) / 128);
   const int sms = usable_sms(device);

@@ -10,8 +10,6 @@
 // All three are bound by memory traffic: every row is read and written once with 16-byte accesses, sums are fp32.
 // One B200, 8192 tokens x 2048, 8 experts, top 2: slots 7 us (a running count through torch.cumsum over 16384 x 8 took
 // 3454 us, one thread per column), dispatch 17 us, combine 21 us, adjoint with the gate's gradient 35 us.
-// One B200, 8192 tokens x 2048, 8 experts, top 2: slots 7 us (a running count through torch.cumsum over 16384 x 8 took
-// 3454 us, one thread per column), dispatch 17 us, combine 21 us, adjoint with the gate's gradient 35 us.
 #include "common.cuh"
 
 namespace axb {
