@@ -1,0 +1,36 @@
+"""GEMM epilogues at the edges of their rules: alignment of the output, remainders of tiles, masked rows."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF16 = torch.bfloat16
+
+
+def _rel(got, want):
+    return float((got.detach().double() - want.detach().double()).norm() / want.detach().double().norm().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(1, 16, 64), (77, 264, 128), (130, 1048, 72), (1031, 2064, 256), (2500, 4104, 192),
+                                   (2500, 4112, 192), (2049, 4096, 64)])
+@pytest.mark.parametrize("shift", [0, 8])
+def test_gemm_store_alignment(M, N, K, shift, dtype):
+    """Outputs whose rows start on a 32-byte boundary and ones that do not (N = 8 mod 16, or a base 16 bytes off), the
+    last chunk of 32 columns cut at 8, 16 and 24.  Tolerance: one rounding of the result (2^-9 / 2^-11) after fp32 sums;
+    the saved pre-activation has the same, and nothing outside the output is written."""
+    from axonn_b200 import ops
+
+    torch.manual_seed(M + N)
+    a, b = torch.randn(M, K, device=DEV).to(dtype), torch.randn(N, K, device=DEV).to(dtype)
+    bias = torch.randn(N, device=DEV).to(dtype)
+    bufs = [torch.full((M * N + 64,), 7.0, device=DEV, dtype=dtype) for _ in range(2)]
+    out, aux = (t[shift:shift + M * N].view(M, N) for t in bufs)
+    ops.matmul_nt(a, b, bias=bias, epilogue=ops.EPI_BIAS_GELU, out=out, aux=aux)
+    z = a.double() @ b.double().t() + bias.double()
+    tol = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10}[dtype]
+    assert _rel(aux, z) < tol
+    assert _rel(out, torch.nn.functional.gelu(z, approximate="tanh")) < tol
+    for t in bufs:
+        assert bool((t[:shift] == 7).all()) and bool((t[shift + M * N:] == 7).all())
