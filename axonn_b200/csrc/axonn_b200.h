@@ -265,6 +265,8 @@ int axb_gelu_bwd_colsum(const void* dy, const void* x, void* dx, float* part, vo
 
 /* ---- multi-tensor kernels over a device table of tensor pointers (optim.cu) */
 int axb_multi_l2norm_sq(const long long* table, int n, long long total_chunks, float* out, void* stream);
+// words[4], the first two zero on entry: squared norm, block counter, norm, min(1, max_norm / (norm + 1e-6))
+int axb_multi_clip_factor(const long long* table, int n, long long total_chunks, float max_norm, float* words, void* stream);
 int axb_multi_scale(const long long* table, int n, long long total_chunks, const float* scale, void* stream);
 /* SGD with momentum over a pointer table (rows {param, grad, fp32 momentum buffer, numel, param dtype, grad dtype,
    chunk prefix, 0}; dtype codes 0 fp32, 1 bf16, 2 fp16) */

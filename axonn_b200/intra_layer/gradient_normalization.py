@@ -30,6 +30,13 @@ def _local_norm_pow(grads, norm_type):
                         for g in grads]).sum()
 
 
+def _one_table(grads):
+    """Do all gradients lie on one GPU, in types and layouts that a pointer table takes, with an element among them?"""
+    return (any(g.numel() > 0 for g in grads)
+            and all(g.is_cuda and g.device == grads[0].device and g.is_contiguous()
+                    and g.dtype in (torch.float32, torch.bfloat16, torch.float16) for g in grads))
+
+
 def clip_grad_norm_(parameters, max_norm, norm_type=2.0, error_if_nonfinite=False):
     """``torch.nn.utils.clip_grad_norm_`` for sharded parameters: the local norms of tensor-parallel parameters
     are reduced over ``param.process_group_for_norm_reduction`` (replicas counted once), combined with the norm
@@ -53,6 +60,13 @@ def clip_grad_norm_(parameters, max_norm, norm_type=2.0, error_if_nonfinite=Fals
             by_group[(p.process_group_for_norm_reduction, replicas)].append(p.grad)
         else:
             plain.append(p.grad)
+    all_grads = plain + [g for gs in by_group.values() for g in gs]
+    if norm_type == 2.0 and not error_if_nonfinite and _one_table(all_grads) and all(
+            replicas == 1 and dist.get_world_size(group) == 1 for group, replicas in by_group):
+        # nothing to reduce over ranks: norm and factor come from one kernel over all gradients
+        total_norm, clip = ops.multi_tensor_clip_factor(all_grads, max_norm)
+        ops.multi_tensor_scale_(all_grads, clip)
+        return total_norm
     pieces = []
     for (group, replicas), grads in by_group.items():
         v = _local_norm_pow(grads, norm_type)
@@ -80,6 +94,5 @@ def clip_grad_norm_(parameters, max_norm, norm_type=2.0, error_if_nonfinite=Fals
         raise RuntimeError(f"The total norm of order {norm_type} for gradients is non-finite, "
                            "so it cannot be clipped.")
     clip = torch.clamp(max_norm / (total_norm + 1e-6), max=1.0)
-    all_grads = plain + [g for gs in by_group.values() for g in gs]
     ops.multi_tensor_scale_(all_grads, clip)
     return total_norm

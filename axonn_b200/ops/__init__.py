@@ -20,6 +20,7 @@ from .linear import linear, linear_batched  # noqa: F401
 from .loss import cross_entropy  # noqa: F401
 from .multi_tensor import (  # noqa: F401
     all_reduce_bucketed_,
+    multi_tensor_clip_factor,
     multi_tensor_l2norm_sq,
     multi_tensor_scale_,
 )

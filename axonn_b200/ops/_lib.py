@@ -57,6 +57,7 @@ _SIGNATURES = {
     "axb_ce_fwd_mean": "pppppp" "ii" "l" "p",
     "axb_ce_bwd": "pppp" "iii" "l" "p",
     "axb_multi_l2norm_sq": "p" "il" "pp",
+    "axb_multi_clip_factor": "p" "il" "f" "pp",
     "axb_multi_scale": "p" "il" "pp",
     "axb_multi_adamw": "p" "il" "fffffff" "ppp",
     "axb_prune_topk": "p" "lil" "p" "i" "p",

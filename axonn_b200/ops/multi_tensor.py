@@ -70,6 +70,17 @@ def multi_tensor_l2norm_sq(tensors):
     return torch.stack([t.detach().float().pow(2).sum() for t in tensors]).sum()
 
 
+def multi_tensor_clip_factor(tensors, max_norm):
+    """``(norm, min(1, max_norm / (norm + 1e-6)))`` of the L2 norm over all elements of CUDA tensors of one device, as
+    0-d fp32 tensors: one launch, the block that finishes last does the arithmetic."""
+    tab = _cached_table([t for t in tensors if t.numel() > 0])
+    words = torch.zeros(4, dtype=torch.float32, device=tensors[0].device)
+    st = _lib.lib().axb_multi_clip_factor(_lib.addr(tab.dev), tab.n, tab.total_chunks, max_norm, _lib.addr(words),
+                                          _lib.stream())
+    _lib.check(st, "axb_multi_clip_factor")
+    return words[2], words[3]
+
+
 def multi_tensor_scale_(tensors, scale):
     """``t *= scale`` for every tensor; ``scale`` is a float or a 0-d tensor
     (kept on device: no host synchronisation)."""
