@@ -60,6 +60,8 @@ _SIGNATURES = {
     "axb_multi_clip_factor": "p" "il" "f" "pp",
     "axb_multi_scale": "p" "il" "pp",
     "axb_multi_adamw": "p" "il" "fffffff" "ppp",
+    "axb_moe_route": "piiiii" "pppppppppp" "p",
+    "axb_moe_route_bwd": "piii" "pppppp" "p",
     "axb_prune_topk": "p" "lil" "p" "i" "p",
 }
 # Switches of kernels that are gone.  The one kernel that is left covers what they selected; a program that still sets

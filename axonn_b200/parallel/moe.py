@@ -59,6 +59,49 @@ class _AllToAll(torch.autograd.Function):
         return out, None
 
 
+class _LocalRoute(torch.autograd.Function):
+    """Top-``k`` softmax routing of ``logits [T, E]`` (bf16) into capacity buffers of ``rows`` rows per expert, ``C`` of them in
+    use: ``(gate [T, k], balance loss, dest, inverse, counts, statistics)``; two launches forward and one backward
+    (``csrc/moe_local.cu``).  Statistics: ``[assignments per expert | dropped per expert | dropped fraction]``."""
+
+    @staticmethod
+    def forward(ctx, logits, k, C, rows):
+        logits = logits.contiguous()
+        T, E = logits.shape
+        dev = logits.device
+        idx, dest, inverse, counts = (torch.empty(n, dtype=torch.int32, device=dev) for n in (T * k, T * k, E * rows, E))
+        gate, aux, stats, scratch = (torch.empty(n, dtype=torch.float32, device=dev)
+                                     for n in ((T, k), (), 2 * E + 1, ((T + 127) // 128 + 1) * E + 1))
+        word = stats.data_ptr()
+        _lib.check(_lib.lib().axb_moe_route(_lib.addr(logits), T, E, k, C, rows, _lib.addr(idx), _lib.addr(gate),
+                                            _lib.addr(dest), _lib.addr(inverse), _lib.addr(counts), word, word + 4 * E,
+                                            _lib.addr(aux), word + 8 * E, _lib.addr(scratch), _lib.stream()), "axb_moe_route")
+        _lib.add_launches(1)
+        ctx.save_for_backward(logits, idx, gate, stats)
+        ctx.mark_non_differentiable(dest, inverse, counts, stats)
+        ctx.set_materialize_grads(False)
+        ctx.k = k
+        return gate, aux, dest, inverse, counts, stats
+
+    @staticmethod
+    @once_differentiable
+    def backward(ctx, dgate, daux, *_):
+        logits, idx, gate, stats = ctx.saved_tensors
+        if dgate is None and daux is None:
+            return None, None, None, None
+        T, E = logits.shape
+        dgate = None if dgate is None else dgate.float().contiguous()
+        daux = None if daux is None else daux.float()
+        dlogits = torch.empty_like(logits)
+        _lib.check(_lib.lib().axb_moe_route_bwd(_lib.addr(logits), T, E, ctx.k, _lib.addr(idx), _lib.addr(gate), _lib.addr(dgate),
+                                                _lib.addr(daux), _lib.addr(stats), _lib.addr(dlogits), _lib.stream()),
+                   "axb_moe_route_bwd")
+        return dlogits, None, None, None
+
+
+_ROUTE_MAX_EXPERTS = 32       # AXB_MOE_MAX_EXPERTS: the routing kernel holds a token's logits in registers
+
+
 class _LocalDispatch(torch.autograd.Function):
     """Token rows ``[T, H]`` into the experts' capacity buffers ``[E, rows, H]`` (zeros where no token is), and the
     adjoint: the sum of a token's rows (``csrc/moe_local.cu``)."""
@@ -221,20 +264,25 @@ class ExpertParallelMoE(nn.Module):
         needs of its reduction dimension."""
         T, E, k = x2.shape[0], self.n_experts, self.top_k
         rows = (C + 63) // 64 * 64
-        probs = F.softmax(logits.float(), dim=-1)
-        gate, idx = probs.topk(k, dim=-1)
-        gate = gate / gate.sum(-1, keepdim=True)
-        idx = idx.contiguous()
-        dest, inverse, counts = (torch.empty(n, dtype=torch.int32, device=x2.device) for n in (T * k, E * rows, E))
-        assigned = torch.empty(E, dtype=torch.float32, device=x2.device)
-        _lib.check(_lib.lib().axb_moe_slots(_lib.ptr(idx), ctypes.c_longlong(T * k), ctypes.c_int(E), ctypes.c_int(C),
-                                            ctypes.c_int(rows), _lib.ptr(dest), _lib.ptr(inverse), _lib.ptr(counts),
-                                            _lib.ptr(assigned), _lib.stream_ptr()), "axb_moe_slots")
-        self.last_aux_loss = E * (assigned / (T * k) * probs.mean(0)).sum()
-        kept = counts.float()
-        self.last_drop_fraction = 1.0 - kept.sum() / (T * k)
-        self.last_assignments_per_expert = assigned
-        self.last_dropped_per_expert = assigned - kept
+        if E <= _ROUTE_MAX_EXPERTS:
+            gate, self.last_aux_loss, dest, inverse, counts, stats = _LocalRoute.apply(logits, k, C, rows)
+            self.last_assignments_per_expert, self.last_dropped_per_expert = stats[:E], stats[E:2 * E]
+            self.last_drop_fraction = stats[2 * E]
+        else:
+            probs = F.softmax(logits.float(), dim=-1)
+            gate, idx = probs.topk(k, dim=-1)
+            gate = gate / gate.sum(-1, keepdim=True)
+            idx = idx.contiguous()
+            dest, inverse, counts = (torch.empty(n, dtype=torch.int32, device=x2.device) for n in (T * k, E * rows, E))
+            assigned = torch.empty(E, dtype=torch.float32, device=x2.device)
+            _lib.check(_lib.lib().axb_moe_slots(_lib.ptr(idx), ctypes.c_longlong(T * k), ctypes.c_int(E), ctypes.c_int(C),
+                                                ctypes.c_int(rows), _lib.ptr(dest), _lib.ptr(inverse), _lib.ptr(counts),
+                                                _lib.ptr(assigned), _lib.stream_ptr()), "axb_moe_slots")
+            self.last_aux_loss = E * (assigned / (T * k) * probs.mean(0)).sum()
+            kept = counts.float()
+            self.last_drop_fraction = 1.0 - kept.sum() / (T * k)
+            self.last_assignments_per_expert = assigned
+            self.last_dropped_per_expert = assigned - kept
         xin = _LocalDispatch.apply(x2, dest, inverse, E, rows, k)
         out = self._experts(xin, counts.view(E, 1), rows)
         return _LocalCombine.apply(out, gate.contiguous(), dest, inverse, T, k)
