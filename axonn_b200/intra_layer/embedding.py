@@ -19,6 +19,7 @@ import torch.distributed as dist
 import torch.nn.functional as F
 
 from .. import axonn as ax
+from ..ops.direct import no_graph
 from ..utils import divide
 from .communication import ForwardGather_BackwardReduceScatter, Gather, _gather
 
@@ -149,8 +150,10 @@ class Embedding(torch.nn.Module):
             if not self.expert_mode:
                 x = Gather.apply(x, self.hidden_group)
             return x
-        weight = ForwardGather_BackwardReduceScatter.apply(self.weight, self.depth_group).reshape(
-            self.local_in_features, self.local_out_features)
+        weight = self.weight
+        if self.depth_group_size > 1 or not no_graph(weight):
+            weight = ForwardGather_BackwardReduceScatter.apply(weight, self.depth_group)
+        weight = weight.reshape(self.local_in_features, self.local_out_features)
         x = F.embedding(x, weight, self.padding_idx, self.max_norm, self.norm_type,
                         self.scale_grad_by_freq, self.sparse)
         if not self.expert_mode:

@@ -32,6 +32,7 @@ from torch.autograd import Function
 from .. import axonn as ax
 from .. import ops
 from ..ops import _lib
+from ..ops.direct import no_graph
 from ..parallel import fused
 from ..utils import divide
 from . import overlap_communication as oc
@@ -349,6 +350,9 @@ class Linear(torch.nn.Module):
         """``activation="gelu"`` fuses bias + GELU (tanh form) into the layer; only
         meaningful when the bias is added inside the layer (expert mode, no
         ``skip_bias_add``)."""
+        y = self._forward_direct(x, activation)
+        if y is not None:
+            return y
         lead_shape = x.shape[:-1]
         x = x.reshape(-1, x.shape[-1])
         switch_layout = (not self.expert_mode) and self.inner_group_size * self.outer_group_size > 1
@@ -375,6 +379,28 @@ class Linear(torch.nn.Module):
         if self.skip_bias_add:
             return x, bias
         return x + bias.to(x.dtype)
+
+    def _forward_direct(self, x, activation):
+        """The layer as one GEMM launch, when it needs no gradient and no collective; ``None`` when the general path has to
+        run.  One B200 (host-bound): 24 tokens through 2048 -> 8192 -> 2048 78 -> 31 us; the saved pre-activation
+        of a GELU layer is not written either."""
+        w, b = self.weight, self.bias
+        if self.inner_group_size * self.depth_group_size != 1 or (activation is not None and activation != "gelu"):
+            return None
+        if b is not None and (not self.expert_mode or self.skip_bias_add or b.dtype != w.dtype):
+            return None
+        n, k = self.local_out_features, self.local_in_features
+        if (n % 8 or k % 8 or x.dtype != w.dtype or w.dtype not in (torch.bfloat16, torch.float16) or x.dim() == 0
+                or x.shape[-1] != k or w.shape != (n * k,) or x.numel() == 0 or not no_graph(x, w, b)
+                or not x.is_contiguous() or not w.is_contiguous() or torch.is_autocast_enabled("cuda")):
+            return None
+        out = x.new_empty(x.shape[:-1] + (n,))
+        epilogue = (ops.EPI_NONE if b is None else ops.EPI_BIAS) if activation is None else (
+            ops.EPI_GELU if b is None else ops.EPI_BIAS_GELU)
+        code = 0 if w.dtype == torch.bfloat16 else 1
+        _lib.check(_lib.lib().axb_gemm(0, x.data_ptr(), w.data_ptr(), out.data_ptr(), _lib.addr(b), None, x.numel() // k, n, k,
+                                       code, code, epilogue, 0, x.device.index, _lib.stream()), "axb_gemm")
+        return out
 
     # ---------------------------------------------------------------- state dict
     def _is_full_weight_matrix(self, w):

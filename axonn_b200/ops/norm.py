@@ -12,12 +12,22 @@ import torch
 import torch.distributed as dist
 
 from . import _lib
+from .direct import no_graph
 
 _DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
 def _group_size(group):
     return 1 if group is None else (group.size() if isinstance(group, dist.ProcessGroup) else dist.get_world_size(group))
+
+
+def _dense_rows(t, H):
+    """``t`` itself when it is dense (the kernels see rows of ``H``), otherwise a dense copy of its rows."""
+    return t if t.is_contiguous() else t.reshape(-1, H).contiguous()
+
+
+def _shaped(t, shape):
+    return t if t.shape == shape else t.reshape(shape)
 
 
 def _torch_norm_fwd(x, gamma, beta, eps, rms, group):
@@ -44,14 +54,15 @@ class _NormFn(torch.autograd.Function):
     def forward(ctx, x, gamma, beta, eps, rms, group):
         shape = x.shape
         H = shape[-1]
-        x2 = x.reshape(-1, H).contiguous()
-        rows = x2.shape[0]
         n = _group_size(group)
         ctx.rms, ctx.group, ctx.n, ctx.shape, ctx.has_beta = rms, group, n, shape, beta is not None
-        if not x2.is_cuda:
+        if not x.is_cuda:
+            x2 = x.reshape(-1, H).contiguous()
             y, mean, rstd = _torch_norm_fwd(x2, gamma, beta, eps, rms, group)
             ctx.save_for_backward(x2, gamma, mean, rstd)
             return y.reshape(shape)
+        x2 = _dense_rows(x, H)
+        rows = x2.numel() // H
         L = _lib.lib()
         dev = x2.device.index
         y = torch.empty_like(x2)
@@ -73,14 +84,14 @@ class _NormFn(torch.autograd.Function):
             dist.all_reduce(stats, group=group)
             call(3)                              # finishes (mean, rstd) in place and applies them
         ctx.save_for_backward(x2, g, stats)
-        return y.reshape(shape)
+        return _shaped(y, shape)
 
     @staticmethod
     def backward(ctx, dy):
         rms, group, n = ctx.rms, ctx.group, ctx.n
         H = ctx.shape[-1]
-        dy2 = dy.reshape(-1, H).contiguous()
-        if not dy2.is_cuda:
+        if not dy.is_cuda:
+            dy2 = dy.reshape(-1, H).contiguous()
             x2, gamma, mean, rstd = ctx.saved_tensors
             xh = (x2.float() - mean) * rstd
             gd = dy2.float() * gamma.float()
@@ -96,7 +107,8 @@ class _NormFn(torch.autograd.Function):
             dbeta = dy2.float().sum(0).to(gamma.dtype) if ctx.has_beta else None
             return dx.to(dy.dtype).reshape(ctx.shape), dgamma, dbeta, None, None, None
         x2, g, stats = ctx.saved_tensors
-        rows = x2.shape[0]
+        dy2 = _dense_rows(dy, H)
+        rows = stats.shape[0]
         L = _lib.lib()
         dev = x2.device.index
         grid = L.axb_norm_grid(dev, rows)
@@ -122,7 +134,7 @@ class _NormFn(torch.autograd.Function):
             call(1)
             dist.all_reduce(sums, group=group)
             call(2)
-        return dx.reshape(ctx.shape), dg, (db if ctx.has_beta else None), None, None, None
+        return _shaped(dx, ctx.shape), dg, (db if ctx.has_beta else None), None, None, None
 
 
 class _AddNormFn(torch.autograd.Function):
@@ -136,14 +148,15 @@ class _AddNormFn(torch.autograd.Function):
         H = shape[-1]
         n = _group_size(group)
         ctx.rms, ctx.group, ctx.n, ctx.shape, ctx.has_beta = rms, group, n, shape, beta is not None
-        x2 = x.reshape(-1, H).contiguous()
-        d2 = delta.reshape(-1, H).contiguous()
-        rows = x2.shape[0]
-        if not x2.is_cuda:
+        if not x.is_cuda:
+            x2 = x.reshape(-1, H).contiguous()
+            d2 = delta.reshape(-1, H).contiguous()
             h = x2 + d2
             y, mean, rstd = _torch_norm_fwd(h, gamma, beta, eps, rms, group)
             ctx.save_for_backward(h, gamma, mean, rstd)
             return h.reshape(shape), y.reshape(shape)
+        x2, d2 = _dense_rows(x, H), _dense_rows(delta, H)
+        rows = x2.numel() // H
         L = _lib.lib()
         dev = x2.device.index
         h = torch.empty_like(x2)
@@ -166,15 +179,15 @@ class _AddNormFn(torch.autograd.Function):
             dist.all_reduce(stats, group=group)
             call(3, h, None)                     # finishes (mean, rstd) in place and applies them
         ctx.save_for_backward(h, g, stats)
-        return h.reshape(shape), y.reshape(shape)
+        return _shaped(h, shape), _shaped(y, shape)
 
     @staticmethod
     def backward(ctx, dh, dy):
         rms, group, n = ctx.rms, ctx.group, ctx.n
         H = ctx.shape[-1]
-        dy2 = dy.reshape(-1, H).contiguous()
-        dh2 = None if dh is None else dh.reshape(-1, H).contiguous()
-        if not dy2.is_cuda:
+        if not dy.is_cuda:
+            dy2 = dy.reshape(-1, H).contiguous()
+            dh2 = None if dh is None else dh.reshape(-1, H).contiguous()
             x2, gamma, mean, rstd = ctx.saved_tensors
             xh = (x2.float() - mean) * rstd
             gd = dy2.float() * gamma.float()
@@ -193,7 +206,9 @@ class _AddNormFn(torch.autograd.Function):
             dx = dx.to(dy.dtype).reshape(ctx.shape)
             return dx, dx, dgamma, dbeta, None, None, None
         x2, g, stats = ctx.saved_tensors
-        rows = x2.shape[0]
+        dy2 = _dense_rows(dy, H)
+        dh2 = None if dh is None else _dense_rows(dh, H)
+        rows = stats.shape[0]
         L = _lib.lib()
         dev = x2.device.index
         grid = L.axb_norm_grid(dev, rows)
@@ -218,30 +233,56 @@ class _AddNormFn(torch.autograd.Function):
             call(1)
             dist.all_reduce(sums, group=group)
             call(2)
-        dx = dx.reshape(ctx.shape)
+        dx = _shaped(dx, ctx.shape)
         return dx, dx, dg, (db if ctx.has_beta else None), None, None, None
+
+
+def _norm_direct(x, delta, gamma, beta, eps, rms, group):
+    """``(h, norm(h))`` with ``h = x + delta`` (``delta`` None: ``h = x``) as one launch, when neither a gradient nor a
+    reduction over ``group`` is needed; ``None`` when the general path has to run."""
+    H = x.shape[-1] if x.dim() else 0
+    if (not no_graph(x, delta, gamma, beta) or x.dtype not in _DT or gamma.dtype != x.dtype or gamma.shape != (H,)
+            or (beta is not None and (beta.dtype != x.dtype or beta.shape != (H,) or not beta.is_contiguous()))
+            or x.numel() == 0 or _group_size(group) != 1 or not x.is_contiguous() or not gamma.is_contiguous()
+            or (delta is not None and (delta.shape != x.shape or delta.dtype != x.dtype or not delta.is_contiguous()))):
+        return None
+    rows = x.numel() // H
+    y = torch.empty_like(x)
+    stats = torch.empty((rows, 2), dtype=torch.float32, device=x.device)
+    if delta is None:
+        _lib.check(_lib.lib().axb_norm_fwd(x.data_ptr(), gamma.data_ptr(), _lib.addr(beta), y.data_ptr(), stats.data_ptr(), rows,
+                                           H, H, eps, 1 if rms else 0, 0, _DT[x.dtype], x.device.index, _lib.stream()),
+                   "axb_norm_fwd")
+        return x, y
+    h = torch.empty_like(x)
+    _lib.check(_lib.lib().axb_add_norm_fwd(x.data_ptr(), delta.data_ptr(), h.data_ptr(), gamma.data_ptr(), _lib.addr(beta),
+                                           y.data_ptr(), stats.data_ptr(), rows, H, H, eps, 1 if rms else 0, 0, _DT[x.dtype],
+                                           x.device.index, _lib.stream()), "axb_add_norm_fwd")
+    return h, y
 
 
 def add_layer_norm(x, delta, gamma, beta, eps=1e-5, group=None):
     """``h = x + delta; y = LayerNorm(h)`` in one kernel; returns ``(h, y)``."""
-    return _AddNormFn.apply(x, delta, gamma, beta, eps, False, group)
+    return _norm_direct(x, delta, gamma, beta, eps, False, group) or _AddNormFn.apply(x, delta, gamma, beta, eps, False, group)
 
 
 def add_rms_norm(x, delta, gamma, eps=1e-6, group=None):
     """``h = x + delta; y = RMSNorm(h)`` in one kernel; returns ``(h, y)``."""
-    return _AddNormFn.apply(x, delta, gamma, None, eps, True, group)
+    return _norm_direct(x, delta, gamma, None, eps, True, group) or _AddNormFn.apply(x, delta, gamma, None, eps, True, group)
 
 
 def layer_norm(x, gamma, beta, eps=1e-5, group=None):
     """LayerNorm over the last dimension; with ``group`` the last dimension is one
     shard of a hidden dimension split over that process group."""
-    return _NormFn.apply(x, gamma, beta, eps, False, group)
+    direct = _norm_direct(x, None, gamma, beta, eps, False, group)
+    return _NormFn.apply(x, gamma, beta, eps, False, group) if direct is None else direct[1]
 
 
 def rms_norm(x, gamma, eps=1e-6, group=None):
     """RMSNorm over the last dimension; with ``group`` the last dimension is one shard of a hidden dimension
     split over that process group."""
-    return _NormFn.apply(x, gamma, None, eps, True, group)
+    direct = _norm_direct(x, None, gamma, None, eps, True, group)
+    return _NormFn.apply(x, gamma, None, eps, True, group) if direct is None else direct[1]
 
 
 def column_sum(x, out_dtype=torch.float32):

@@ -4,13 +4,14 @@
 import torch
 
 from . import _lib
+from .direct import no_graph
 
 _tables = {}
 
 
 def rope_table(seq_len, head_dim, theta, device):
     """``[S, D/2, 2]`` fp32 table of (cos, sin)."""
-    key = (seq_len, head_dim, float(theta), str(device))
+    key = (seq_len, head_dim, float(theta), device)
     t = _tables.get(key)
     if t is None:
         inv = 1.0 / (theta ** (torch.arange(0, head_dim, 2, dtype=torch.float64) / head_dim))
@@ -71,4 +72,8 @@ class _RopeFn(torch.autograd.Function):
 def apply_rope(x, table):
     """Rotate ``x`` (``[B, S, heads, D]`` or ``[B, S, groups, heads, D]``).  On GPU ``x``
     must be a non-leaf tensor (it is updated in place)."""
+    if no_graph(x, table):
+        if not x.is_inference():
+            torch.autograd.graph.increment_version(x)  # as any in-place operation does: x may be saved in a graph elsewhere
+        return _rope_apply(x, table, False)
     return _RopeFn.apply(x, table)

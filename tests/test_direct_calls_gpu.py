@@ -1,0 +1,133 @@
+"""Layers that launch their kernel without an autograd function when no gradient can be asked for: the same results as with
+one, and the general path wherever something else looks at the operation."""
+
+import pytest
+import torch
+import torch.distributed as dist
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+BF16 = torch.bfloat16
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _grid():
+    from axonn_b200 import axonn as ax
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    if not ax.is_initialized:
+        ax.init(G_inter=1, G_data=1, G_intra_r=1, G_intra_c=1, G_intra_d=1)
+
+
+def _views(shape, dtype):
+    """A dense tensor, one 16 bytes into a buffer, one with gaps, one with permuted dimensions."""
+    n = 1
+    for d in shape:
+        n *= d
+    base = torch.randn(n + 8, device=DEV).to(dtype)
+    wide = torch.randn(*shape[:-1], shape[-1] * 2, device=DEV).to(dtype)
+    out = [base[:n].view(shape), base[8:].view(shape), wide[..., :shape[-1]]]
+    if len(shape) == 3:
+        out.append(torch.randn(shape[1], shape[0], shape[2], device=DEV).to(dtype).transpose(0, 1))
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(16,), (5, 16), (2, 3, 264), (0, 16)])
+def test_norms(shape, dtype):
+    from axonn_b200 import ops
+
+    H = shape[-1]
+    g, b = torch.randn(H, device=DEV).to(dtype), torch.randn(H, device=DEV).to(dtype)
+    gg = g.clone().requires_grad_(True)
+    for x, d in zip(_views(shape, dtype), reversed(_views(shape, dtype))):
+        if x.numel() == 0:
+            continue
+        for rms in (False, True):
+            norm = (lambda t, w: ops.rms_norm(t, w)) if rms else (lambda t, w: ops.layer_norm(t, w, b))
+            add = (lambda t, w: ops.add_rms_norm(t, d, w)) if rms else (lambda t, w: ops.add_layer_norm(t, d, w, b))
+            ref, ref_h, ref_y = norm(x, gg), *add(x, gg)
+            assert ref.requires_grad
+            with torch.no_grad():
+                got, (h, y) = norm(x, gg), add(x, gg)
+            assert not got.requires_grad and torch.equal(got, ref) and torch.equal(h, ref_h) and torch.equal(y, ref_y)
+            assert got.shape == h.shape == y.shape == x.shape
+            h2, y2 = add(x, g)                       # grad mode on, nothing requires a gradient
+            assert torch.equal(h2, ref_h) and not y2.requires_grad
+            x3 = x.detach().clone().requires_grad_(True)
+            h3, y3 = add(x3, gg)
+            (gx,) = torch.autograd.grad([h3, y3], x3, [torch.ones_like(h3), torch.ones_like(y3)])
+            assert gx.shape == x.shape
+
+
+@pytest.mark.parametrize("expert,bias,skip", [(True, True, False), (True, False, False), (False, True, False), (True, True, True)])
+@pytest.mark.parametrize("k,n,dtype", [(64, 24, BF16), (264, 520, torch.float16), (24, 20, BF16), (32, 32, torch.float32)])
+def test_linear(expert, bias, skip, k, n, dtype):
+    from axonn_b200.intra_layer import Linear
+
+    torch.manual_seed(k)
+    layer = Linear(k, n, bias=bias, skip_bias_add=skip, expert_mode=expert, dtype=dtype)
+    if bias:
+        with torch.no_grad():
+            layer.bias.normal_()
+    for shape in [(k,), (3, k), (2, 5, k), (200, k)]:
+        for x in _views(shape, dtype):
+            for act in (None, "gelu"):
+                if act and (not expert or skip or (not bias and n % 8) or dtype == torch.float32):
+                    continue
+                try:
+                    ref = layer(x, activation=act)
+                except Exception as e:               # what the general path refuses stays refused
+                    with torch.no_grad(), pytest.raises(type(e)):
+                        layer(x, activation=act)
+                    continue
+                with torch.no_grad():
+                    got = layer(x, activation=act)
+                for a, r in zip(got, ref) if skip and bias else [(got, ref)]:
+                    assert a.shape == r.shape and torch.equal(a, r)
+    with torch.no_grad(), torch.autocast("cuda", dtype=BF16):
+        assert (layer(torch.randn(4, k, device=DEV))[0] if skip and bias else layer(torch.randn(4, k, device=DEV))).dtype == BF16
+    with torch.no_grad(), pytest.raises(Exception):
+        layer(torch.randn(4, k + 8, device=DEV).to(dtype))
+
+
+def test_general_path_is_kept():
+    """Forward-mode tangents, function transforms and tracing reach the autograd function, as before."""
+    import torch.autograd.forward_ad as fw
+
+    from axonn_b200 import ops
+    from axonn_b200.ops.direct import no_graph
+
+    x, w = torch.randn(4, 64, device=DEV, dtype=BF16), torch.ones(64, device=DEV, dtype=BF16)
+    assert no_graph(x, w, None) and not no_graph(x.cpu()) and not no_graph(x, w.clone().requires_grad_(True))
+    with torch.no_grad():
+        assert no_graph(x, w.clone().requires_grad_(True))
+        with fw.dual_level():
+            assert not no_graph(fw.make_dual(x, torch.ones_like(x)))
+            with pytest.raises(RuntimeError):
+                ops.rms_norm(fw.make_dual(x, torch.ones_like(x)), w)
+        with pytest.raises(RuntimeError):
+            torch.func.vmap(lambda t: ops.rms_norm(t, w))(x[None])
+
+    class Sub(torch.Tensor):
+        pass
+
+    assert not no_graph(x.as_subclass(Sub))
+
+
+def test_rope_counts_as_in_place():
+    """A tensor saved for a backward and then rotated without a graph is noticed."""
+    from axonn_b200 import ops
+
+    table = ops.rope_table(8, 64, 1e4, torch.device("cuda", 0))
+    x = torch.randn(1, 8, 2, 64, device=DEV, dtype=BF16, requires_grad=True)
+    y = x * 1
+    z = y * y
+    with torch.no_grad():
+        out = ops.apply_rope(y.detach(), table)
+    assert out.shape == y.shape
+    with pytest.raises(RuntimeError, match="modified by an inplace"):
+        z.sum().backward()
+    with torch.inference_mode():
+        ops.apply_rope(torch.randn(1, 8, 2, 64, device=DEV, dtype=BF16), table)
