@@ -75,6 +75,7 @@ struct GemmParams {
   // (mode 2) without a data row are not computed; a skipped tile is stored as zeros.
   const int* seg_counts;
   int seg_rows, nseg, mask_mode;
+  int whole_tiles;   // plain CTA-pair kernel: tiles from this one on are computed as two halves of their columns (PairWalk)
   int debug;      // ablation builds only (-DAXB_ABLATION, then read once from AXB_AR_DEBUG; otherwise 0 and every branch on it is compiled out): 1 no flagger fence, 2 no peer stores, 4 no reducer fence, 8 no reduction, 16 no partial stores, 128 register-path reducer instead of the shared-memory ring
 };
 
@@ -1203,10 +1204,32 @@ __device__ __forceinline__ int pair_kb_count(const GemmParams& p, int e, int num
   return min(num_kb, (__ldg(p.seg_counts + e) + BK - 1) / BK);
 }
 
+// Work of a CTA pair: tiles, dealt in turn.  When the last wave would leave half of the pairs or more without a tile, its tiles
+// are cut into two halves of 128 columns, one for each of two pairs: the same MMAs with N = 128, half the time.
+// One B200, bf16, whole tiles / with halves: 777 x 6144 x 4096 (96 tiles on 74 pairs) 46.7 / 38.8 us, 1024 x 6144 x 2048 26.9 /
+// 22.3, 1024 x 6144 x 512 14.8 / 10.5, 8192 x 2048 x 4096 111 / 103; no difference within the noise of the power cap for the
+// weight gradients 8192 x 2048 x 16384.  More than half of the pairs busy: halves would need a second round, nothing gained.
+// (Sharing the K blocks of the last wave between all pairs, partial sums through global memory, was 20 - 30 us slower.)
+struct PairWalk {
+  int it;
+  int tile, col, cols;                   // the current item: tile, first column inside it, columns
+  __device__ __forceinline__ PairWalk() : it(blockIdx.x >> 1) {}
+  __device__ __forceinline__ bool next(const GemmParams& p, int total) {
+    const int h = it - p.whole_tiles;
+    if (h < 0) {
+      tile = it; col = 0; cols = PAIR_BN;
+    } else {
+      tile = p.whole_tiles + (h >> 1); col = (h & 1) * (PAIR_BN / 2); cols = PAIR_BN / 2;
+    }
+    it += gridDim.x >> 1;
+    return tile < total;
+  }
+};
+
 template <int A_MN, int B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const GemmParams p) {
+                 const __grid_constant__ CUtensorMap tmBh, const GemmParams p) {
   using S = PairSmem;
   constexpr int BN = PAIR_BN;
   extern __shared__ uint8_t smem_raw[];
@@ -1221,8 +1244,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();         // 0: leader (issues the MMAs), 1: peer
-  const int pair_id = blockIdx.x >> 1;
-  const int num_pairs = gridDim.x >> 1;
   const int num_kb = (p.K + BK - 1) / BK;
   const int tiles_m2 = (p.tiles_m + 1) >> 1;         // 256-row tile rows
   const int per_batch = tiles_m2 * p.tiles_n;
@@ -1249,11 +1270,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (elect_one()) {
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
-      for (int it = pair_id; it < total && ok; it += num_pairs) {
-        const int e = it / per_batch;
-        int tm2, tn; tile_coords(it - e * per_batch, tiles_m2, p.tiles_n, 8, tm2, tn);
+      PairWalk walk;
+      while (ok && walk.next(p, total)) {
+        const int e = walk.tile / per_batch;
+        int tm2, tn; tile_coords(walk.tile - e * per_batch, tiles_m2, p.tiles_n, 8, tm2, tn);
         const int m0 = (2 * tm2 + static_cast<int>(rank)) * BM;
-        const int n0 = tn * BN + static_cast<int>(rank) * (BN / 2);   // this CTA's half of the B tile
+        const bool whole = walk.cols == BN;
+        const int n0 = tn * BN + walk.col + static_cast<int>(rank) * (walk.cols / 2);   // this CTA's half of the B tile
+        const uint32_t stage_bytes = 2 * (S::A_BYTES + (whole ? S::B_BYTES : S::B_BYTES / 2));
         // row coordinate of problem e in the stacked operands (rows = M or N for a K-major operand, K otherwise)
         const int a_r = e * p.a_batch_rows, b_r = e * p.b_batch_rows;
         if (p.mask_mode == 1 && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, tm2 * 2 * BM, 2 * BM)) continue;
@@ -1264,7 +1288,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           uint8_t* sA = smem + stage * S::STAGE_BYTES;
           uint8_t* sB = sA + S::A_BYTES;
           // the leader's barrier counts the bytes of both CTAs' loads of this stage
-          if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * S::STAGE_BYTES);
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], stage_bytes);
           const int k0 = kb * BK;
           if (A_MN == 0) {
             tma_load_2d_pair(sA, &tmA, &full_bar[stage], k0, m0 + a_r);
@@ -1273,10 +1297,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sA + j * (BK * 128), &tmA, &full_bar[stage], m0 + 64 * j, k0 + a_r);
           }
           if (B_MN == 0) {
-            tma_load_2d_pair(sB, &tmB, &full_bar[stage], k0, n0 + b_r);
+            tma_load_2d_pair(sB, whole ? &tmB : &tmBh, &full_bar[stage], k0, n0 + b_r);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(sB + j * (BK * 128), &tmB, &full_bar[stage], n0 + 64 * j, k0 + b_r);
+            for (int j = 0; j < BN / 128; ++j) if (j == 0 || whole) tma_load_2d_pair(sB + j * (BK * 128), &tmB, &full_bar[stage], n0 + 64 * j, k0 + b_r);
           }
           if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
         }
@@ -1286,16 +1310,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
     if (rank == 0 && elect_one()) {
-      const uint32_t idesc = umma_idesc(p.in_dtype == 0 ? 1 : 0, A_MN, B_MN, 2 * BM, BN);
+      const uint32_t idesc_whole = umma_idesc(p.in_dtype == 0 ? 1 : 0, A_MN, B_MN, 2 * BM, BN);
+      const uint32_t idesc_half = umma_idesc(p.in_dtype == 0 ? 1 : 0, A_MN, B_MN, 2 * BM, BN / 2);
       const uint32_t a_lbo = A_MN ? BK * 128 : 16, a_sbo = 1024, a_kstep = A_MN ? UMMA_K * 128 : UMMA_K * 2;
       const uint32_t b_lbo = B_MN ? BK * 128 : 16, b_sbo = 1024, b_kstep = B_MN ? UMMA_K * 128 : UMMA_K * 2;
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       int t = 0;
-      for (int it = pair_id; it < total && ok; it += num_pairs) {
-        const int e = it / per_batch;
+      PairWalk walk;
+      while (ok && walk.next(p, total)) {
+        const int e = walk.tile / per_batch;
+        const uint32_t idesc = walk.cols == BN ? idesc_whole : idesc_half;
         if (p.mask_mode != 0) {
-          int tm2, tn; tile_coords(it - e * per_batch, tiles_m2, p.tiles_n, 8, tm2, tn);
+          int tm2, tn; tile_coords(walk.tile - e * per_batch, tiles_m2, p.tiles_n, 8, tm2, tn);
           if (!pair_tile_computed(p, e, tm2, num_kb)) continue;      // no accumulator buffer is used for it
         }
         const int buf = t & 1;
@@ -1335,9 +1362,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int q = warp & 3;
     bool ok = true;
     int t = 0;
-    for (int it = pair_id; it < total && ok; it += num_pairs) {
-      const int e = it / per_batch;
-      int tm2, tn; tile_coords(it - e * per_batch, tiles_m2, p.tiles_n, 8, tm2, tn);
+    PairWalk walk;
+    while (ok && walk.next(p, total)) {
+      const int e = walk.tile / per_batch;
+      int tm2, tn; tile_coords(walk.tile - e * per_batch, tiles_m2, p.tiles_n, 8, tm2, tn);
       const int tm = 2 * tm2 + static_cast<int>(rank);
       const size_t local_row = static_cast<size_t>(tm) * BM + q * 32 + lane;
       const bool row_ok = local_row < static_cast<size_t>(p.M);     // rows past M belong to the next problem
@@ -1359,7 +1387,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!mbar_wait(&tmem_full[buf], acc_phase, abort_flag, timeout)) { ok = false; break; }
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
-      epilogue_row<BN>(p, taddr, row, row_ok, tn * BN);
+      if (walk.cols == BN) epilogue_row<BN>(p, taddr, row, row_ok, tn * BN);
+      else if (tn * BN + walk.col < p.N) epilogue_row<BN / 2>(p, taddr, row, row_ok, tn * BN + walk.col);
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_leader(&tmem_empty[buf]);   // 8 arrivals (4 warps x 2 CTAs) free the buffer
@@ -1722,8 +1751,16 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p,
   return 0;
 }
 
+// Tiles of a plain GEMM on `pairs` CTA pairs that are computed whole: all, unless the last wave is at most half full.
+static int pair_whole_tiles(long long total, int pairs) {
+  const long long rest = total % pairs;
+  return static_cast<int>(rest != 0 && 2 * rest <= pairs ? total - rest : total);
+}
+
+// tmBh: B with boxes of half as many rows, for the halves of tiles (any map for an MN-major B); null: whole tiles only
 template <int A_MN, int B_MN>
-static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int device, cudaStream_t stream) {
+static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap* tmBh, GemmParams& p, int device,
+                       cudaStream_t stream) {
   using S = PairSmem;
   static bool configured[64] = {false};
   auto kern = gemm_pair_kernel<A_MN, B_MN>;
@@ -1735,9 +1772,11 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParam
   p.tiles_n = (p.N + PAIR_BN - 1) / PAIR_BN;
   const int total = ((p.tiles_m + 1) / 2) * p.tiles_n * p.nb;
   const int pairs = usable_sms(device) / 2;
-  const int grid = 2 * (total < pairs ? total : pairs);
+  p.whole_tiles = tmBh ? pair_whole_tiles(total, pairs) : total;
+  const int items = p.whole_tiles + 2 * (total - p.whole_tiles);
+  const int grid = 2 * (items < pairs ? items : pairs);
   p.gemm_ctas = grid;
-  kern<<<grid, PAIR_THREADS, S::TOTAL, stream>>>(tmA, tmB, p);
+  kern<<<grid, PAIR_THREADS, S::TOTAL, stream>>>(tmA, tmB, tmBh ? *tmBh : tmB, p);
   AXB_CUDA(cudaGetLastError());
   return 0;
 }
@@ -1932,9 +1971,11 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
     return launch_comm_pair<1, 1>(tmA, tmB, p, device, s);
   }
   if (pair) {
-    if (layout == 0) return launch_pair<0, 0>(tmA, tmB, p, device, s);
-    if (layout == 1) return launch_pair<0, 1>(tmA, tmB, p, device, s);
-    return launch_pair<1, 1>(tmA, tmB, p, device, s);
+    CUtensorMap tmBh = tmB;
+    if (b_mn == 0 && pair_whole_tiles(pair_tiles, sms / 2) != pair_tiles && make_tmap_2d_16bit(&tmBh, B, N, K, BN / 4, in_dtype)) return -1;
+    if (layout == 0) return launch_pair<0, 0>(tmA, tmB, &tmBh, p, device, s);
+    if (layout == 1) return launch_pair<0, 1>(tmA, tmB, &tmBh, p, device, s);
+    return launch_pair<1, 1>(tmA, tmB, &tmBh, p, device, s);
   }
   if (splitk > 1) {
     if (layout == 0) return launch_splitk<0, 0>(tmA, tmB, p, splitk, device, s);
@@ -2021,9 +2062,9 @@ extern "C" int axb_gemm_batched(int layout, const void* A, const void* B, void* 
     p.seg_counts = seg_counts; p.seg_rows = seg_rows; p.nseg = nseg; p.mask_mode = (layout == 2) ? 2 : 1;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (layout == 0) return launch_pair<0, 0>(tmA, tmB, p, device, s);
-  if (layout == 1) return launch_pair<0, 1>(tmA, tmB, p, device, s);
-  return launch_pair<1, 1>(tmA, tmB, p, device, s);
+  if (layout == 0) return launch_pair<0, 0>(tmA, tmB, nullptr, p, device, s);
+  if (layout == 1) return launch_pair<0, 1>(tmA, tmB, nullptr, p, device, s);
+  return launch_pair<1, 1>(tmA, tmB, nullptr, p, device, s);
 }
 
 extern "C" int axb_gemm(int layout, const void* A, const void* B, void* C, const void* bias, void* aux, int M, int N,

@@ -34,3 +34,34 @@ def test_gemm_store_alignment(M, N, K, shift, dtype):
     assert _rel(out, torch.nn.functional.gelu(z, approximate="tanh")) < tol
     for t in bufs:
         assert bool((t[:shift] == 7).all()) and bool((t[shift + M * N:] == 7).all())
+
+
+@pytest.mark.parametrize("layout", ["nt", "nn", "tn"])
+@pytest.mark.parametrize("M,N,K", [(776, 6144, 512), (1032, 4616, 136), (1000, 5656, 1992), (1024, 4872, 264), (3000, 1560, 72)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gemm_halved_tiles(layout, M, N, K, dtype):
+    """A last wave of a few tiles, which are computed as halves of their columns: N that ends inside the first half, the
+    second one, and on the seam; a ragged M and K; every epilogue.  Tolerance: one rounding of the result (2^-9 / 2^-11)."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib
+
+    torch.manual_seed(M)
+    a, b = torch.randn(M, K, device=DEV).to(dtype), torch.randn(N, K, device=DEV).to(dtype)
+    z = a.double() @ b.double().t()
+    tol = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10}[dtype]
+    fn, x, y = {"nt": (ops.matmul_nt, a, b), "nn": (ops.matmul_nn, a, b.t().contiguous()),
+                "tn": (ops.matmul_tn, a.t().contiguous(), b.t().contiguous())}[layout]
+    got = fn(x, y)
+    assert _lib.device_status() == 0
+    for r in range(0, M, 128):                       # a wrong tile must not hide in the norm of the whole
+        for c in range(0, N, 128):
+            assert _rel(got[r:r + 128, c:c + 128], z[r:r + 128, c:c + 128]) < tol, (r, c)
+    acc = torch.randn(M, N, device=DEV, dtype=torch.float32)
+    want = acc.double() + z
+    assert _rel(fn(x, y, out=acc, accumulate=True), want) < 1e-5
+    if layout == "nt":
+        bias = torch.randn(N, device=DEV).to(dtype)
+        aux = torch.empty(M, N, device=DEV, dtype=dtype)
+        out = ops.matmul_nt(x, y, bias=bias, epilogue=ops.EPI_BIAS_GELU, aux=aux)
+        assert _rel(aux, z + bias.double()) < tol
+        assert _rel(out, torch.nn.functional.gelu(z + bias.double(), approximate="tanh")) < tol
