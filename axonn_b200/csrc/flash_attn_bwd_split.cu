@@ -440,7 +440,7 @@ struct DkvSmem {
   static constexpr int DO_OFF = 4 * TILE;          // 2 stages
   static constexpr int LSE_OFF = 6 * TILE;         // [2 stages][lse, delta][128] fp32
   static constexpr int BAR_OFF = LSE_OFF + 2048;
-  static constexpr int NBARS = 2 + 8 + 2 + 2 + 2;
+  static constexpr int NBARS = 2 + 8 + 4 + 4 + 2;
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 16 + 1024;
 };
 
@@ -476,10 +476,10 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
   uint64_t* kv_empty = bars + 1;     // both MMA warps are done with them
   uint64_t* qdo_full = bars + 2;     // [stage][half]: Q, dO, lse, delta of 64 queries
   uint64_t* qdo_empty = bars + 6;    // [stage][half]: 2 MMA warps + the half's 8 softmax warps
-  uint64_t* sdp_full = bars + 10;    // [score buffer]: S^T and dP^T of a step (one arrival per MMA warp)
-  uint64_t* pds_full = bars + 12;    // [score buffer]: P^T and dS^T of a step are in tensor memory
-  uint64_t* acc_done = bars + 14;    // dK and dV of the item are final (one arrival per MMA warp)
-  uint64_t* acc_free = bars + 15;    // ... and have been read: the next item may overwrite them
+  uint64_t* t_full = bars + 10;      // [S^T, dP^T][score buffer]: complete
+  uint64_t* a_full = bars + 14;      // [P^T, dS^T][score buffer]: in tensor memory
+  uint64_t* acc_done = bars + 18;    // dK and dV of the item are final (one arrival per MMA warp)
+  uint64_t* acc_free = bars + 19;    // ... and have been read: the next item may overwrite them
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(bars + S_::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   float* lse_s = reinterpret_cast<float*>(smem + S_::LSE_OFF);
@@ -492,7 +492,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
     mbar_init(kv_full, 1); mbar_init(kv_empty, 2); mbar_init(acc_done, 2);
     mbar_init(acc_free, FS_SOFTMAX_WARPS);
     for (int i = 0; i < 4; ++i) { mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 2 + FS_SOFTMAX_WARPS / 2); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&sdp_full[i], 2); mbar_init(&pds_full[i], FS_SOFTMAX_WARPS / 2); }
+    for (int i = 0; i < 4; ++i) { mbar_init(&t_full[i], 1); mbar_init(&a_full[i], FS_SOFTMAX_WARPS / 2); }
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -590,12 +590,12 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
         for (int hq = 0; hq < 2 && ok; ++hq) {
           if (!mbar_wait(&qdo_full[(tq & 1) * 2 + hq], (tq >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
           tcgen05_fence_after();
-          issue_t(tq & 1, hq); umma_commit(&sdp_full[hq]);
+          issue_t(tq & 1, hq); umma_commit(&t_full[which * 2 + hq]);
         }
         for (int s = 0; s < ns && ok; ++s, ++c) {
           const uint32_t tile = tq + (s >> 1);
           const int hq = s & 1;
-          if (!mbar_wait(&pds_full[hq], (c >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
+          if (!mbar_wait(&a_full[which * 2 + hq], (c >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
           // the warps of either score buffer read dK / dV of the previous item; only those of buffer 0 are known to be done
           if (s == 0 && it > 0 && !mbar_wait(acc_free, (it - 1) & 1, abort_flag, timeout)) { ok = false; break; }
           tcgen05_fence_after();
@@ -606,7 +606,7 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
             if (!mbar_wait(&qdo_full[(tn & 1) * 2 + hq], (tn >> 1) & 1, abort_flag, timeout)) { ok = false; break; }
             tcgen05_fence_after();
             issue_t(tn & 1, hq);
-            umma_commit(&sdp_full[hq]);
+            umma_commit(&t_full[which * 2 + hq]);
           }
         }
         umma_commit(acc_done);
@@ -619,6 +619,10 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
   } else {
     // ------------------------------------------------------------------ P^T, dS^T: thread = (key row, 32 of the step's 64 queries)
     // Warps 4-11 take the steps of score buffer 0 (first 64 queries of every tile), warps 12-19 those of buffer 1.
+    // P^T is handed on before dP^T is waited for: the first MMA warp then issues dV and the next scores while the threads
+    // still work on dS^T, and each warp's chain (scores -> P -> dV, dP -> dS -> dK) is its own.  One B200, this kernel with the
+    // delta kernel, both handed on together / one by one: 1 x 4096, 32 heads over 8, head_dim 128 258 / 229 us, 1 x 777 62.3 /
+    // 55, 8 x 2048, 16 heads, head_dim 64 252 / 244.  The dQ kernel gains nothing from the same split (22.0 / 21.9, 176 / 176).
     asm volatile(FS_REGS_SOFTMAX);
     const int q4 = warp & 3;
     const int hq = (warp - 4) >> 3;
@@ -639,12 +643,11 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
         const bool diag = t % per_head == 0;
         // -lse and -delta of the tile arrive with its Q and dO
         if (!mbar_wait(&qdo_full[st * 2 + hq], (tq >> 1) & 1, abort_flag, timeout) ||
-            !mbar_wait(&sdp_full[hq], tq & 1, abort_flag, timeout)) { ok = false; break; }
+            !mbar_wait(&t_full[hq], tq & 1, abort_flag, timeout)) { ok = false; break; }
         tcgen05_fence_after();
-        uint32_t sv[32], dv[32];
+        uint32_t sv[32];
         tmem_ld_32x32(t_s, sv);
-        tmem_ld_32x32(t_dp, dv);
-        tmem_ld_wait();
+        tmem_ld_wait(sv);
         const float4* lv = reinterpret_cast<const float4*>(lse_s + st * 256 + qc0);
         const float4* dvv = reinterpret_cast<const float4*>(lse_s + st * 256 + 128 + qc0);
         if (diag) {                                   // the key lies after the query: probability 0
@@ -652,30 +655,48 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
           for (int i = 0; i < 32; ++i)
             if (r > qc0 + i) sv[i] = 0xff800000u;
         }
-        uint32_t pp[16], pd[16];
+        float2 pr[16];
+        uint32_t pk[16];
 #pragma unroll
         for (int v4 = 0; v4 < 8; ++v4) {
-          const float4 l4 = lv[v4], d4 = dvv[v4];
+          const float4 l4 = lv[v4];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int i = v4 * 2 + e;
             const float2 nl2 = e ? make_float2(l4.z, l4.w) : make_float2(l4.x, l4.y);
-            const float2 nd2 = e ? make_float2(d4.z, d4.w) : make_float2(d4.x, d4.y);
             const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), sc2, nl2);
-            const float2 pr = make_float2(exp2f(x.x), exp2f(x.y));
-            const float2 t2 = __fadd2_rn(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), nd2);
-            pp[i] = fs_pack(pr);
-            pd[i] = fs_pack(__fmul2_rn(pr, t2));      // the softmax scale is applied to the finished dK
+            pr[i] = make_float2(exp2f(x.x), exp2f(x.y));
+            pk[i] = fs_pack(pr[i]);
           }
         }
         // into this thread's own score columns: the other half's thread of the row may not have read its scores yet
-        tmem_st_32x16(t_s, pp);
-        tmem_st_32x16(t_dp, pd);
+        tmem_st_32x16(t_s, pk);
+        tmem_st_wait();
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&a_full[hq]);      // dV and the next scores need not wait for dS
+        if (!mbar_wait(&t_full[2 + hq], tq & 1, abort_flag, timeout)) { ok = false; break; }
+        tcgen05_fence_after();
+        uint32_t dv[32];
+        tmem_ld_32x32(t_dp, dv);
+        tmem_ld_wait(dv);
+#pragma unroll
+        for (int v4 = 0; v4 < 8; ++v4) {
+          const float4 d4 = dvv[v4];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int i = v4 * 2 + e;
+            const float2 nd2 = e ? make_float2(d4.z, d4.w) : make_float2(d4.x, d4.y);
+            const float2 t2 = __fadd2_rn(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), nd2);
+            pk[i] = fs_pack(__fmul2_rn(pr[i], t2));   // the softmax scale is applied to the finished dK
+          }
+        }
+        tmem_st_32x16(t_dp, pk);
         tmem_st_wait();
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive(&pds_full[hq]);
+          mbar_arrive(&a_full[2 + hq]);
           mbar_arrive(&qdo_empty[st * 2 + hq]);       // this warp has read its share of -lse / -delta
         }
       }
