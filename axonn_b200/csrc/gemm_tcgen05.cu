@@ -341,6 +341,86 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t taddr
   }
 }
 
+// ---- epilogues of a gated feed-forward layer (bf16, CTA-pair kernel only); gate and up columns alternate in blocks of 8
+enum PairAct {
+  ACT_NONE = 0,
+  ACT_SWIGLU = 1,     // C [rows, N / 2] = silu(gate) * up of the product; aux [rows, N] receives the product, unless null
+  ACT_DSWIGLU = 2,    // the product is the gradient of that result; aux [rows, 2N] the saved product, C [rows, 2N] its gradient
+};
+
+__device__ __forceinline__ void ld_global_32b(const void* p, uint32_t* w) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(p));
+}
+
+// The 64 saved gate and up values that belong to 32 columns of the gradient.
+__device__ __forceinline__ void load_gate_up(const GemmParams& p, size_t row, bool row_ok, int col, uint32_t (&z)[32]) {
+  const uint16_t* src = reinterpret_cast<const uint16_t*>(p.aux) + row * (2 * static_cast<size_t>(p.N)) + 2 * col;
+#pragma unroll
+  for (int g = 0; g < 4; ++g)
+    if (row_ok && col + g * 8 < p.N) ld_global_32b(src + g * 16, z + g * 8);
+}
+
+__device__ __forceinline__ float2 bf16x2_f32(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
+
+// One row of the tile like epilogue_row.  The activations are computed from the rounded product that is stored (SwiGLU), and
+// from the fp32 gradient (its adjoint).  Saved values are requested a chunk ahead; those of the first chunk (`z`) before
+// the accumulator is waited for.
+template <int BN, int ACT>
+__device__ __forceinline__ void epilogue_act(const GemmParams& p, uint32_t taddr, size_t row, bool row_ok, int col0, uint32_t (&z)[32]) {
+#pragma unroll 1
+  for (int c = 0; c < BN / 32; ++c) {
+    const int col = col0 + c * 32;
+    if (col >= p.N) break;  // uniform across the warp
+    uint32_t r[32];
+    tmem_ld_32x32(taddr + c * 32, r);
+    if (ACT == ACT_SWIGLU) {
+      tmem_ld_wait(r);
+      uint32_t w[16], h[8];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) w[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]), 0);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int g = (i >> 2) * 8 + (i & 3);            // word of the gates; the ups lie 4 words behind
+        const float2 a = bf16x2_f32(w[g]), b = bf16x2_f32(w[g + 4]);
+        h[i] = pack2(a.x * sigmoidf_(a.x) * b.x, a.y * sigmoidf_(a.y) * b.y, 0);
+      }
+      if (row_ok) {
+        uint16_t* dst = reinterpret_cast<uint16_t*>(p.C) + row * (p.N / 2) + col / 2;
+        uint16_t* sav = reinterpret_cast<uint16_t*>(p.aux) + row * p.N + col;
+        const bool all = col + 32 <= p.N;                // otherwise 16 columns: N is a multiple of 16
+        if (p.aux != nullptr) {
+          st_global_32b(sav, *reinterpret_cast<uint32_t (*)[8]>(w));
+          if (all) st_global_32b(sav + 16, *reinterpret_cast<uint32_t (*)[8]>(w + 8));
+        }
+        *reinterpret_cast<uint4*>(dst) = make_uint4(h[0], h[1], h[2], h[3]);
+        if (all) *reinterpret_cast<uint4*>(dst + 8) = make_uint4(h[4], h[5], h[6], h[7]);
+      }
+    } else {
+      uint32_t zc[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) zc[i] = z[i];
+      if (c + 1 < BN / 32 && col + 32 < p.N) load_gate_up(p, row, row_ok, col + 32, z);
+      tmem_ld_wait(r);
+      uint16_t* dst = reinterpret_cast<uint16_t*>(p.C) + row * (2 * static_cast<size_t>(p.N)) + 2 * col;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        if (!row_ok || col + g * 8 >= p.N) continue;
+        uint32_t o[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 a = bf16x2_f32(zc[g * 8 + i]), b = bf16x2_f32(zc[g * 8 + 4 + i]);
+          const float d0 = __uint_as_float(r[g * 8 + 2 * i]), d1 = __uint_as_float(r[g * 8 + 2 * i + 1]);
+          const float s0 = sigmoidf_(a.x), s1 = sigmoidf_(a.y), l0 = a.x * s0, l1 = a.y * s1;
+          o[i] = pack2(d0 * b.x * (s0 + l0 * (1.f - s0)), d1 * b.y * (s1 + l1 * (1.f - s1)), 0);
+          o[4 + i] = pack2(d0 * l0, d1 * l1, 0);
+        }
+        st_global_32b(dst + g * 16, o);
+      }
+    }
+  }
+}
+
 // Named-barrier OR-reduction over the 128 epilogue threads (barrier 1): returns true if all passed true.
 __device__ __forceinline__ bool __syncthreads_or_named(bool ok) {
   __shared__ int sh_fail;
@@ -1226,7 +1306,7 @@ struct PairWalk {
   }
 };
 
-template <int A_MN, int B_MN>
+template <int A_MN, int B_MN, int ACT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmBh, const GemmParams p) {
@@ -1371,6 +1451,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const bool row_ok = local_row < static_cast<size_t>(p.M);     // rows past M belong to the next problem
       const size_t row = local_row + static_cast<size_t>(e) * p.c_batch_rows;
       if (p.mask_mode != 0 && !pair_tile_computed(p, e, tm2, num_kb)) {
+        if (ACT != ACT_NONE) continue;                         // nothing reads it (see axb_gemm_swiglu)
         // a tile without data: zeros (nothing to add when accumulating), no accumulator buffer involved
         if (row_ok && !p.accumulate) {
           float z[32];
@@ -1384,10 +1465,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const int buf = t & 1;
       const uint32_t acc_phase = (t >> 1) & 1;
       ++t;
+      uint32_t z[32];
+      if (ACT == ACT_DSWIGLU) load_gate_up(p, row, row_ok, tn * BN, z);
       if (!mbar_wait(&tmem_full[buf], acc_phase, abort_flag, timeout)) { ok = false; break; }
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
-      if (walk.cols == BN) epilogue_row<BN>(p, taddr, row, row_ok, tn * BN);
+      if (ACT != ACT_NONE) epilogue_act<BN, ACT>(p, taddr, row, row_ok, tn * BN, z);     // whole tiles only
+      else if (walk.cols == BN) epilogue_row<BN>(p, taddr, row, row_ok, tn * BN);
       else if (tn * BN + walk.col < p.N) epilogue_row<BN / 2>(p, taddr, row, row_ok, tn * BN + walk.col);
       tcgen05_fence_before();
       __syncwarp();
@@ -1758,12 +1842,12 @@ static int pair_whole_tiles(long long total, int pairs) {
 }
 
 // tmBh: B with boxes of half as many rows, for the halves of tiles (any map for an MN-major B); null: whole tiles only
-template <int A_MN, int B_MN>
+template <int A_MN, int B_MN, int ACT = ACT_NONE>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap* tmBh, GemmParams& p, int device,
                        cudaStream_t stream) {
   using S = PairSmem;
   static bool configured[64] = {false};
-  auto kern = gemm_pair_kernel<A_MN, B_MN>;
+  auto kern = gemm_pair_kernel<A_MN, B_MN, ACT>;
   if (!configured[device & 63]) {
     AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
     configured[device & 63] = true;
@@ -2020,10 +2104,9 @@ extern "C" double axb_comm_stall_ms(int device, int reset) {
 // seg_counts (device, int32 [nb, nseg]; nullptr = no mask): the M rows (layouts 0 and 1) or the K rows (layout 2)
 // of every problem are nseg segments of seg_rows rows, of which only the first seg_counts[e][s] hold data and the
 // others are zero.  Tiles (K blocks in layout 2) without a data row are skipped; a skipped tile is stored as zeros.
-extern "C" int axb_gemm_batched(int layout, const void* A, const void* B, void* C, int nb, int M, int N, int K,
-                                int a_batch_rows, int b_batch_rows, int c_batch_rows, int in_dtype, int out_dtype,
-                                int accumulate, const int* seg_counts, int seg_rows, int nseg, int device,
-                                void* stream) {
+static int gemm_batched(int layout, const void* A, const void* B, void* C, void* aux, int act, int nb, int M, int N, int K,
+                        int a_batch_rows, int b_batch_rows, int c_batch_rows, int in_dtype, int out_dtype, int accumulate,
+                        const int* seg_counts, int seg_rows, int nseg, int device, void* stream) {
   using namespace axb;
   if (nb <= 0 || M <= 0 || N <= 0 || K <= 0) { set_error("axb_gemm_batched: empty problem"); return -1; }
   if (layout < 0 || layout > 2) { set_error("axb_gemm_batched: bad layout %d", layout); return -1; }
@@ -2047,7 +2130,7 @@ extern "C" int axb_gemm_batched(int layout, const void* A, const void* B, void* 
   if (b_mn == 0) { if (make_tmap_2d_16bit(&tmB, B, b_total, K, PAIR_BN / 2, in_dtype)) return -1; }
   else           { if (make_tmap_2d_16bit(&tmB, B, b_total, N, BK, in_dtype)) return -1; }
   GemmParams p;
-  p.C = C; p.bias = nullptr; p.aux = nullptr; p.M = M; p.N = N; p.K = K;
+  p.C = C; p.bias = nullptr; p.aux = aux; p.M = M; p.N = N; p.K = K;
   p.out_dtype = out_dtype; p.in_dtype = in_dtype; p.epilogue = 0; p.accumulate = accumulate;
   p.status = status_dev; p.timeout_ns = wait_timeout_ns();
   p.ar.n = 1; p.ag.n = 1; p.tn_offset = 0; p.kb_offset = 0; p.flag_batch = 1; p.debug = 0; p.pair = 1;
@@ -2062,9 +2145,38 @@ extern "C" int axb_gemm_batched(int layout, const void* A, const void* B, void* 
     p.seg_counts = seg_counts; p.seg_rows = seg_rows; p.nseg = nseg; p.mask_mode = (layout == 2) ? 2 : 1;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (act == ACT_SWIGLU) return launch_pair<0, 0, ACT_SWIGLU>(tmA, tmB, nullptr, p, device, s);
+  if (act == ACT_DSWIGLU) return launch_pair<0, 1, ACT_DSWIGLU>(tmA, tmB, nullptr, p, device, s);
   if (layout == 0) return launch_pair<0, 0>(tmA, tmB, nullptr, p, device, s);
   if (layout == 1) return launch_pair<0, 1>(tmA, tmB, nullptr, p, device, s);
   return launch_pair<1, 1>(tmA, tmB, nullptr, p, device, s);
+}
+
+extern "C" int axb_gemm_batched(int layout, const void* A, const void* B, void* C, int nb, int M, int N, int K,
+                                int a_batch_rows, int b_batch_rows, int c_batch_rows, int in_dtype, int out_dtype,
+                                int accumulate, const int* seg_counts, int seg_rows, int nseg, int device,
+                                void* stream) {
+  return gemm_batched(layout, A, B, C, nullptr, axb::ACT_NONE, nb, M, N, K, a_batch_rows, b_batch_rows, c_batch_rows, in_dtype,
+                      out_dtype, accumulate, seg_counts, seg_rows, nseg, device, stream);
+}
+
+// The products of a gated feed-forward layer with its activation in the epilogue, bf16, gate and up columns alternating in
+// blocks of 8 (operands, batches and mask as in axb_gemm_batched; a tile without a data row is left unwritten):
+//   backward 0:  P = A [M, K] B [N, K]^T,  out [M, N / 2] = silu(gate) * up,  saved [M, N] = P unless null;  N % 16 == 0
+//   backward 1:  P = A [M, K] B [K, N] = d(out),  out [M, 2N] = d(saved) from saved [M, 2N]
+// Bound by the tensor cores like the plain products; the passes over memory that go away were at the bandwidth.  One B200,
+// 8 experts, 16384 of 20480 rows in use, hidden 2048, ffn 8192: the two forward products and SwiGLU 1344 -> 1206 us, the
+// gradient product and the adjoint of SwiGLU 690 -> 512; layer forward and backward 4944 -> 4633 us.
+extern "C" int axb_gemm_swiglu(int backward, const void* A, const void* B, void* out, void* saved, int nb, int M, int N, int K,
+                               const int* seg_counts, int seg_rows, int nseg, int device, void* stream) {
+  using namespace axb;
+  if ((!backward && N % 16) || (backward && !saved)) { set_error("axb_gemm_swiglu: bad arguments"); return -1; }
+  if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(saved)) & 31) {
+    set_error("axb_gemm_swiglu: outputs must be 32-byte aligned");
+    return -1;
+  }
+  return gemm_batched(backward ? 1 : 0, A, B, out, saved, backward ? ACT_DSWIGLU : ACT_SWIGLU, nb, M, N, K, M, backward ? K : N, M,
+                      0, 0, 0, seg_counts, seg_rows, nseg, device, stream);
 }
 
 extern "C" int axb_gemm(int layout, const void* A, const void* B, void* C, const void* bias, void* aux, int M, int N,

@@ -38,6 +38,7 @@ class KernelError(RuntimeError):
 # (some fifteen of them for a GEMM).
 _SIGNATURES = {
     "axb_gemm": "ippppp" "iiiiiiii" "p",
+    "axb_gemm_swiglu": "i" "pppp" "iiii" "p" "iii" "p",
     "axb_norm_fwd": "ppppp" "iii" "f" "iiii" "p",
     "axb_norm_bwd": "pppppppppp" "iiiiiiii" "p",
     "axb_add_norm_fwd": "ppppppp" "iii" "f" "iiii" "p",

@@ -3,6 +3,8 @@ that are not tensor parallel (router, expert MLPs)."""
 
 import torch
 
+from . import _lib
+from .activation import swiglu
 from .gemm import bmm_nn, bmm_nt, bmm_tn, matmul_nn, matmul_nt, matmul_tn
 
 
@@ -58,3 +60,59 @@ def linear_batched(x, w, seg=None, seg_rows=0):
     then skip the tiles without data - the output rows of skipped tiles are zeros, which is what the full product
     would give when the layer has no bias."""
     return _BatchedLinearFn.apply(x, w, seg, seg_rows)
+
+
+def _swiglu_gemm(backward, a, b, out, saved, seg, seg_rows):
+    """``axb_gemm_swiglu`` over the problems of ``a[E, M, K]`` (forward ``b[E, N, K]``, backward ``b[E, K, N]``)."""
+    E, M, K = a.shape
+    N = b.shape[2] if backward else b.shape[1]
+    if seg is not None:
+        assert seg.dtype == torch.int32 and seg.is_cuda and seg.is_contiguous() and seg.shape[0] == E
+    _lib.check(_lib.lib().axb_gemm_swiglu(1 if backward else 0, _lib.addr(a), _lib.addr(b), _lib.addr(out), _lib.addr(saved), E, M,
+                                          N, K, _lib.addr(seg), seg_rows, 0 if seg is None else seg.shape[1], a.device.index,
+                                          _lib.stream()), "axb_gemm_swiglu")
+    return out
+
+
+class _SwiGLUExpertsFn(torch.autograd.Function):
+    """``swiglu(x @ w1.T) @ w2.T`` per expert with the activation and its adjoint in the epilogues of the GEMMs around them:
+    the gated product is written once and read once, the activation's gradient is never stored."""
+
+    @staticmethod
+    def forward(ctx, x, w1, w2, seg, seg_rows, keep):
+        E, rows, _ = x.shape
+        gu = torch.empty((E, rows, w1.shape[1]), dtype=x.dtype, device=x.device) if keep else None
+        h = _swiglu_gemm(False, x, w1, torch.empty((E, rows, w2.shape[2]), dtype=x.dtype, device=x.device), gu, seg, seg_rows)
+        ctx.save_for_backward(x, w1, w2, gu, h)
+        ctx.seg, ctx.seg_rows = seg, seg_rows
+        return bmm_nt(h, w2, seg=seg, seg_rows=seg_rows)
+
+    @staticmethod
+    def backward(ctx, g):
+        x, w1, w2, gu, h = ctx.saved_tensors
+        seg = dict(seg=ctx.seg, seg_rows=ctx.seg_rows)
+        g = g.contiguous()
+        g = g if g.data_ptr() % 16 == 0 else g.clone()
+        gx = gw1 = gw2 = None
+        if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
+            dgu = _swiglu_gemm(True, g, w2, torch.empty_like(gu), gu, **seg)
+            gx = bmm_nn(dgu, w1, **seg) if ctx.needs_input_grad[0] else None
+            gw1 = bmm_tn(dgu, x, out_dtype=w1.dtype, **seg) if ctx.needs_input_grad[1] else None
+        if ctx.needs_input_grad[2]:
+            gw2 = bmm_tn(g, h, out_dtype=w2.dtype, **seg)
+        return gx, gw1, gw2, None, None, None
+
+
+def swiglu_experts(x, w1, w2, seg=None, seg_rows=0):
+    """``swiglu(x[E, rows, hidden] @ w1[E, 2 * ffn, hidden].T) @ w2[E, hidden, ffn].T``; ``seg`` / ``seg_rows`` as in
+    ``linear_batched``."""
+    E, rows, hidden = x.shape
+    ffn = w2.shape[2]
+    ts = (x, w1, w2)
+    # the GEMMs of the backward reduce over rows, hidden and 2 * ffn in blocks of 64 that must not reach the next problem
+    if (all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in ts)
+            and x.numel() > 0 and rows % 64 == 0 and hidden % 64 == 0 and ffn % 32 == 0
+            and w1.shape == (E, 2 * ffn, hidden) and w2.shape == (E, hidden, ffn)):
+        keep = torch.is_grad_enabled() and any(t.requires_grad for t in ts)
+        return _SwiGLUExpertsFn.apply(x, w1, w2, seg, seg_rows, keep)
+    return linear_batched(swiglu(linear_batched(x, w1, seg, seg_rows)), w2, seg, seg_rows)

@@ -254,8 +254,7 @@ class ExpertParallelMoE(nn.Module):
         (capacity buffers make the shapes uniform).  ``seg`` (int32 [n_local, rows / seg_rows]): how many rows of
         each ``seg_rows``-row capacity segment hold tokens - the others are zero, and the GEMMs skip the tiles
         (weight gradient: the K blocks) that contain none."""
-        h = ops.swiglu(ops.linear_batched(x, self.w1, seg, seg_rows))
-        return ops.linear_batched(h, self.w2, seg, seg_rows)
+        return ops.swiglu_experts(x, self.w1, self.w2, seg, seg_rows)
 
     def _forward_local(self, x2, logits, C):
         """The layer when every expert is on this GPU: same routing, capacity and statistics as the general path; the

@@ -65,3 +65,43 @@ def test_gemm_halved_tiles(layout, M, N, K, dtype):
         out = ops.matmul_nt(x, y, bias=bias, epilogue=ops.EPI_BIAS_GELU, aux=aux)
         assert _rel(aux, z + bias.double()) < tol
         assert _rel(out, torch.nn.functional.gelu(z + bias.double(), approximate="tanh")) < tol
+
+
+@pytest.mark.parametrize("E,rows,hidden,ffn,counts", [(1, 64, 64, 32, None), (3, 192, 128, 96, [[0], [64], [191]]), (2, 640, 192, 160, [[1], [500]]),
+                                                      (2, 512, 256, 288, [[70, 0], [256, 3]]), (8, 2560, 512, 1024, None)])
+def test_swiglu_experts(E, rows, hidden, ffn, counts):
+    """Gated feed-forward layers with the activation in the GEMMs: tiles with and without data rows, N that ends inside a
+    chunk, one segment and two, against the layer in 64 bits.  Memory that no kernel writes holds NaN, so that reading a
+    row without data would show.  Tolerance: the stored product, the activation and its gradient are rounded to bf16 (three
+    roundings of 2^-9 forward, five backward)."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib
+
+    torch.manual_seed(rows)
+    x = torch.randn(E, rows, hidden, device=DEV).bfloat16()
+    w1 = (torch.randn(E, 2 * ffn, hidden, device=DEV) * hidden ** -0.5).bfloat16().requires_grad_(True)
+    w2 = (torch.randn(E, hidden, ffn, device=DEV) * ffn ** -0.5).bfloat16().requires_grad_(True)
+    dy = torch.randn(E, rows, hidden, device=DEV).bfloat16()
+    seg, seg_rows = None, 0
+    if counts is not None:
+        seg, seg_rows = torch.tensor(counts, dtype=torch.int32, device=DEV), rows // len(counts[0])
+        live = (torch.arange(seg_rows, device=DEV)[None, None] < seg[:, :, None]).view(E, rows, 1)
+        x, dy = x * live, dy * live
+    x.requires_grad_(True)
+    poison = [torch.full((n * E * rows,), float("nan"), device=DEV, dtype=BF16) for n in (ffn, 2 * ffn, ffn, 2 * ffn, hidden)]
+    del poison
+    y = ops.swiglu_experts(x, w1, w2, seg, seg_rows)
+    poison = [torch.full((n * E * rows,), float("nan"), device=DEV, dtype=BF16) for n in (ffn, 2 * ffn, ffn, 2 * ffn, hidden)]
+    del poison
+    got = torch.autograd.grad(y, [x, w1, w2], dy)
+    with torch.no_grad():
+        assert torch.equal(ops.swiglu_experts(x, w1, w2, seg, seg_rows), y)
+    assert _lib.device_status() == 0
+    x64, a64, b64 = (t.detach().double().requires_grad_(True) for t in (x, w1, w2))
+    v = (x64 @ a64.transpose(1, 2)).reshape(E, rows, ffn // 8, 2, 8)
+    y64 = (torch.nn.functional.silu(v[..., 0, :]) * v[..., 1, :]).reshape(E, rows, ffn) @ b64.transpose(1, 2)
+    want = torch.autograd.grad(y64, [x64, a64, b64], dy.double())
+    for e in range(E):
+        assert _rel(y[e], y64[e]) < 3 * 2.0 ** -9
+        for g, w in zip(got, want):
+            assert bool(torch.isfinite(g[e]).all()) and _rel(g[e], w[e]) < 5 * 2.0 ** -9
