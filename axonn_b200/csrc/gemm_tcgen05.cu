@@ -345,6 +345,7 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t taddr
 enum PairAct {
   ACT_NONE = 0,
   ACT_SWIGLU = 1,     // C [rows, N / 2] = silu(gate) * up of the product; aux [rows, N] receives the product, unless null
+  ACT_CE = 3,         // C [rows, N] the product (logits); aux float2 [N tiles][rows]: maximum and sum of exponentials of its row
   ACT_DSWIGLU = 2,    // the product is the gradient of that result; aux [rows, 2N] the saved product, C [rows, 2N] its gradient
 };
 
@@ -362,6 +363,55 @@ __device__ __forceinline__ void load_gate_up(const GemmParams& p, size_t row, bo
 }
 
 __device__ __forceinline__ float2 bf16x2_f32(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
+
+// Logits with the statistics of their softmax: every thread has a row of the tile and keeps a running maximum and sum over its
+// columns, of the rounded logits that are stored.  A row of -inf has the sum zero, a NaN reaches the sum.
+template <int BN>
+__device__ __forceinline__ void epilogue_ce(const GemmParams& p, uint32_t taddr, size_t row, bool row_ok, int col0) {
+  float m = -INFINITY, s = 0.f;
+#pragma unroll 1
+  for (int c = 0; c < BN / 32; ++c) {
+    const int col = col0 + c * 32;
+    if (col >= p.N) break;  // uniform across the warp
+    uint32_t r[32];
+    tmem_ld_32x32(taddr + c * 32, r);
+    tmem_ld_wait(r);
+    uint32_t w[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) w[i] = pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]), 0);
+    if (col + 32 > p.N) {                                // N is a multiple of 8
+#pragma unroll
+      for (int i = 0; i < 16; ++i) if (col + 2 * i >= p.N) w[i] = 0xff80ff80u;
+    }
+    if (row_ok) {
+      uint16_t* dst = reinterpret_cast<uint16_t*>(p.C) + row * p.N + col;
+      if (col + 32 <= p.N && ((reinterpret_cast<uintptr_t>(p.C) | static_cast<uintptr_t>(p.N) * 2) & 31) == 0) {
+        st_global_32b(dst, *reinterpret_cast<uint32_t (*)[8]>(w));
+        st_global_32b(dst + 16, *reinterpret_cast<uint32_t (*)[8]>(w + 8));
+      } else {
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+          if (col + g * 8 < p.N) *reinterpret_cast<uint4*>(dst + g * 8) = make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
+      }
+    }
+    __nv_bfloat162 m2 = *reinterpret_cast<const __nv_bfloat162*>(&w[0]);
+#pragma unroll
+    for (int i = 1; i < 16; ++i) m2 = __hmax2(m2, *reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+    const float2 mf = __bfloat1622float2(m2);
+    const float mx = fmaxf(m, fmaxf(mf.x, mf.y));
+    const float ref = mx == -INFINITY ? 0.f : mx;
+    s *= __expf((m == -INFINITY ? ref : m) - ref);
+    m = mx;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float2 d = __fadd2_rn(bf16x2_f32(w[i]), make_float2(-ref, -ref));
+      acc = __fadd2_rn(acc, make_float2(__expf(d.x), __expf(d.y)));
+    }
+    s += acc.x + acc.y;
+  }
+  if (row_ok) reinterpret_cast<float2*>(p.aux)[static_cast<size_t>(col0 / BN) * p.M + row] = make_float2(m, s);
+}
 
 // One row of the tile like epilogue_row.  The activations are computed from the rounded product that is stored (SwiGLU), and
 // from the fp32 gradient (its adjoint).  Saved values are requested a chunk ahead; those of the first chunk (`z`) before
@@ -1470,7 +1520,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!mbar_wait(&tmem_full[buf], acc_phase, abort_flag, timeout)) { ok = false; break; }
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
-      if (ACT != ACT_NONE) epilogue_act<BN, ACT>(p, taddr, row, row_ok, tn * BN, z);     // whole tiles only
+      if (ACT == ACT_CE) epilogue_ce<BN>(p, taddr, row, row_ok, tn * BN);
+      else if (ACT != ACT_NONE) epilogue_act<BN, ACT>(p, taddr, row, row_ok, tn * BN, z);     // whole tiles only
       else if (walk.cols == BN) epilogue_row<BN>(p, taddr, row, row_ok, tn * BN);
       else if (tn * BN + walk.col < p.N) epilogue_row<BN / 2>(p, taddr, row, row_ok, tn * BN + walk.col);
       tcgen05_fence_before();
@@ -1952,6 +2003,21 @@ static bool pair_mode_enabled() {
   return v == 1;
 }
 
+// Plain GEMMs run on CTA pairs whenever those need less time than single CTAs with 128x128 tiles.  A pair's 256x256
+// tile is twice the work per SM, but single CTAs reach only 0.6 of its rate (their operands exceed the shared-memory
+// bandwidth), so the pairs win as long as they need at most 5 waves where single CTAs need 6 of half the size - in
+// particular with one wave of pairs against two, which the demand for a full wave of pairs used to rule out.  One B200,
+// bf16 (M x N x K): 2048 x 2048 x 16384 119 -> 96 us, 777 x 4096 x 4096 29.7 -> 26.2, 640 x 4096 x 1024 13.3 -> 11.9.  Over the
+// 40 shapes of M 129 .. 8192, N 512 .. 16384 that only this clause sends to pairs, their time is 0.80 - 0.94 of the
+// single CTAs' at K 4096, 0.89 - 1.01 at K 1024 and 0.88 - 1.03 (N 3072 and 5120) at K 128 .. 768.
+static bool plain_on_pairs(int M, int N, int device) {
+  const long long tiles_m = (M + BM - 1) / BM, sms = usable_sms(device), all_sms = sm_count(device);
+  const long long wide_tiles = tiles_m * ((N + 255) / 256), pair_tiles = (tiles_m + 1) / 2 * ((N + 255) / 256);
+  const long long single_tiles = tiles_m * ((N + 127) / 128);
+  const long long pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2), single_waves = (single_tiles + sms - 1) / sms;
+  return pair_mode_enabled() && ((wide_tiles >= all_sms && pair_tiles >= all_sms / 2) || 6 * pair_waves <= 5 * single_waves);
+}
+
 }  // namespace axb
 
 static int gemm_common(int layout, const void* A, const void* B, void* C, const void* bias, void* aux, int M, int N,
@@ -1984,18 +2050,7 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
   // K-major operand [R, K]: box 64(K) x tile rows.  MN-major operand [K, R]: box 64(R) x 64(K).
   if (a_mn == 0) { if (make_tmap_2d_16bit(&tmA, A, M, K, BM, in_dtype)) return -1; }
   else           { if (make_tmap_2d_16bit(&tmA, A, K, M, BK, in_dtype)) return -1; }
-  // Plain GEMMs run on CTA pairs whenever those need less time than single CTAs with 128x128 tiles.  A pair's 256x256
-  // tile is twice the work per SM, but single CTAs reach only 0.6 of its rate (their operands exceed the shared-memory
-  // bandwidth), so the pairs win as long as they need at most 5 waves where single CTAs need 6 of half the size - in
-  // particular with one wave of pairs against two, which the demand for a full wave of pairs used to rule out.  One B200,
-  // bf16 (M x N x K): 2048 x 2048 x 16384 119 -> 96 us, 777 x 4096 x 4096 29.7 -> 26.2, 640 x 4096 x 1024 13.3 -> 11.9.  Over the
-  // 40 shapes of M 129 .. 8192, N 512 .. 16384 that only this clause sends to pairs, their time is 0.80 - 0.94 of the
-  // single CTAs' at K 4096, 0.89 - 1.01 at K 1024 and 0.88 - 1.03 (N 3072 and 5120) at K 128 .. 768.
-  const long long pair_tiles = static_cast<long long>((tiles_m + 1) / 2) * ((N + 255) / 256);
-  const long long single_tiles = static_cast<long long>(tiles_m) * ((N + 127) / 128);
-  const int sms = usable_sms(device);
-  const long long pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2), single_waves = (single_tiles + sms - 1) / sms;
-  const bool pair = !comm && pair_mode_enabled() && ((BN == 256 && enough_pairs) || 6 * pair_waves <= 5 * single_waves);
+  const bool pair = !comm && plain_on_pairs(M, N, device);
   if (pair) BN = 256;
   const int splitk = (comm || pair || BN != 128) ? 1 : splitk_ctas(M, N, K, usable_sms(device), device);
   if (b_mn == 0) { if (make_tmap_2d_16bit(&tmB, B, N, K, (pair || comm_pair) ? BN / 2 : BN, in_dtype)) return -1; }
@@ -2056,7 +2111,8 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
   }
   if (pair) {
     CUtensorMap tmBh = tmB;
-    if (b_mn == 0 && pair_whole_tiles(pair_tiles, sms / 2) != pair_tiles && make_tmap_2d_16bit(&tmBh, B, N, K, BN / 4, in_dtype)) return -1;
+    const long long pair_tiles = static_cast<long long>((tiles_m + 1) / 2) * ((N + 255) / 256);
+    if (b_mn == 0 && pair_whole_tiles(pair_tiles, usable_sms(device) / 2) != pair_tiles && make_tmap_2d_16bit(&tmBh, B, N, K, BN / 4, in_dtype)) return -1;
     if (layout == 0) return launch_pair<0, 0>(tmA, tmB, &tmBh, p, device, s);
     if (layout == 1) return launch_pair<0, 1>(tmA, tmB, &tmBh, p, device, s);
     return launch_pair<1, 1>(tmA, tmB, &tmBh, p, device, s);
@@ -2145,6 +2201,7 @@ static int gemm_batched(int layout, const void* A, const void* B, void* C, void*
     p.seg_counts = seg_counts; p.seg_rows = seg_rows; p.nseg = nseg; p.mask_mode = (layout == 2) ? 2 : 1;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (act == ACT_CE) return launch_pair<0, 0, ACT_CE>(tmA, tmB, nullptr, p, device, s);
   if (act == ACT_SWIGLU) return launch_pair<0, 0, ACT_SWIGLU>(tmA, tmB, nullptr, p, device, s);
   if (act == ACT_DSWIGLU) return launch_pair<0, 1, ACT_DSWIGLU>(tmA, tmB, nullptr, p, device, s);
   if (layout == 0) return launch_pair<0, 0>(tmA, tmB, nullptr, p, device, s);
@@ -2177,6 +2234,20 @@ extern "C" int axb_gemm_swiglu(int backward, const void* A, const void* B, void*
   }
   return gemm_batched(backward ? 1 : 0, A, B, out, saved, backward ? ACT_DSWIGLU : ACT_SWIGLU, nb, M, N, K, M, backward ? K : N, M,
                       0, 0, 0, seg_counts, seg_rows, nseg, device, stream);
+}
+
+// logits [M, N] = A [M, K] B [N, K]^T (bf16) with, for every row and 256 columns, (maximum, sum of exp(logit - maximum)) in
+// part, float2 [ceil(N / 256)][M] (axb_ce_fwd_parts puts them together).  axb_gemm_on_pairs: is the product one of those
+// that run on CTA pairs, which have this epilogue?  One B200, 4096 x 50304, hidden 2048: the product takes no longer than
+// without, and the pass over the logits (84 us) becomes one over the parts (11 us); loss with its gradients 2295 -> 2238 us.
+extern "C" int axb_gemm_on_pairs(int M, int N, int device) { return M > 0 && N > 0 && axb::plain_on_pairs(M, N, device); }
+extern "C" int axb_gemm_ce(const void* A, const void* B, void* logits, void* part, int M, int N, int K, int device, void* stream) {
+  using namespace axb;
+  if ((reinterpret_cast<uintptr_t>(logits) & 15) || (reinterpret_cast<uintptr_t>(part) & 7)) {
+    set_error("axb_gemm_ce: outputs must be aligned to 16 and 8 bytes");
+    return -1;
+  }
+  return gemm_batched(0, A, B, logits, part, ACT_CE, 1, M, N, K, M, N, M, 0, 0, 0, nullptr, 0, 0, device, stream);
 }
 
 extern "C" int axb_gemm(int layout, const void* A, const void* B, void* C, const void* bias, void* aux, int M, int N,

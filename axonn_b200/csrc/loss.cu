@@ -110,6 +110,36 @@ ce_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const long long* __restr
   }
 }
 
+// The same statistics from those of 256 columns each that the GEMM left (axb_gemm_ce): part float2 [parts][rows].  A block has
+// 32 rows, a warp every eighth part of them.
+__global__ void __launch_bounds__(256)
+ce_parts_kernel(const float2* __restrict__ part, int parts, const __nv_bfloat16* __restrict__ logits,
+                const long long* __restrict__ targets, float* __restrict__ stats, float* __restrict__ lse, int rows, int V) {
+  __shared__ float2 red[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + lane;
+  auto join = [](float2& a, const float2 b) {
+    const float m = fmaxf(a.x, b.x), ref = m == -INFINITY ? 0.f : m;
+    a = make_float2(m, a.y * __expf((a.x == -INFINITY ? ref : a.x) - ref) + b.y * __expf((b.x == -INFINITY ? ref : b.x) - ref));
+  };
+  float2 a = make_float2(-INFINITY, 0.f);
+  if (row < rows) {
+#pragma unroll 8
+    for (int i = w; i < parts; i += 8) join(a, __ldg(part + static_cast<size_t>(i) * rows + row));
+  }
+  red[w][lane] = a;
+  __syncthreads();
+  if (w != 0 || row >= rows) return;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) join(a, red[i][lane]);
+  const long long t = targets[row];
+  stats[3 * static_cast<size_t>(row)] = a.x;
+  stats[3 * static_cast<size_t>(row) + 1] = a.y;
+  stats[3 * static_cast<size_t>(row) + 2] = (t >= 0 && t < V) ? __bfloat162float(logits[static_cast<size_t>(row) * V + t]) : 0.f;
+  // a row of -inf only: NaN, as its softmax is
+  lse[row] = a.x == -INFINITY && a.y == 0.f ? __int_as_float(0x7fffffff) : a.x + logf(a.y);
+}
+
 // mean = mean over the rows whose target is not ignore_index of lse - target logit, kept = max(number of them, 1).
 // One block: the rows' losses are a few hundred KB at most, and the fixed order keeps the result reproducible.
 __global__ void __launch_bounds__(1024)
@@ -187,6 +217,16 @@ extern "C" int axb_ce_fwd(const void* logits, const long long* targets, float* s
 extern "C" int axb_ce_fwd_mean(const void* logits, const long long* targets, float* stats, float* lse, float* mean,
                                float* kept, int rows, int V, long long ignore_index, void* stream) {
   return ce_fwd(logits, targets, stats, lse, mean, kept, rows, V, 0, ignore_index, stream);
+}
+// axb_ce_fwd_mean with the statistics of every 256 columns at hand
+extern "C" int axb_ce_fwd_parts(const void* part, const void* logits, const long long* targets, float* stats, float* lse,
+                                float* mean, float* kept, int rows, int V, long long ignore_index, void* stream) {
+  ce_parts_kernel<<<(rows + 31) / 32, 256, 0, (cudaStream_t)stream>>>((const float2*)part, (V + 255) / 256, (const __nv_bfloat16*)logits,
+                                                                    targets, stats, lse, rows, V);
+  AXB_CUDA(cudaGetLastError());
+  ce_mean_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(stats, lse, targets, mean, kept, rows, ignore_index);
+  AXB_CUDA(cudaGetLastError());
+  return 0;
 }
 extern "C" int axb_ce_bwd(void* logits, const long long* targets, const float* lse, const float* scale, int rows, int V,
                           int vocab_start, long long ignore_index, void* stream) {

@@ -18,6 +18,7 @@ import math
 import torch
 import torch.distributed as dist
 import torch.nn as nn
+from torch.autograd import forward_ad
 
 from .. import axonn as ax
 from .. import ops
@@ -37,6 +38,25 @@ def _tag_sharded(param, shard_group):
     param.needs_depth_parallel_gradient_sync = True
     param.process_group_for_norm_reduction = shard_group
     return param
+
+
+def _is_plain_product(layer, x):
+    """Is calling ``layer`` on ``x`` nothing but ``x @ W.T``, so that a fused operation may take its place?  An ordinary
+    ``Linear`` without bias, collectives, hooks or autocast, and nothing that traces or transforms the call."""
+    return (type(layer) is Linear and layer.bias is None and _is_plain_call(layer, x))
+
+
+def _is_plain_call(layer, x):
+    hooks = nn.modules.module
+    return (layer.inner_group_size * layer.outer_group_size * layer.depth_group_size == 1
+            and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks
+                     or hooks._global_forward_hooks or hooks._global_forward_pre_hooks or hooks._global_backward_hooks
+                     or hooks._global_backward_pre_hooks)
+            and layer.forward.__func__ is Linear.forward
+            and type(x) in (torch.Tensor, nn.Parameter) and type(layer.weight) is nn.Parameter
+            and not torch.is_autocast_enabled("cuda") and not torch.compiler.is_compiling()
+            and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active()
+            and forward_ad._current_level < 0)
 
 
 class TPNorm(nn.Module):
@@ -224,6 +244,10 @@ class ParallelLMHead(nn.Module):
     def forward(self, x, targets=None):
         if self.gather_group is not None:
             x = Gather.apply(x, self.gather_group, -1)
+        if targets is not None and _is_plain_product(self.proj, x):
+            loss = ops.projected_cross_entropy(x, self.proj.weight, targets, self.proj.local_weight_shape)
+            if loss is not None:
+                return loss
         logits = self.proj(x)
         if targets is None:
             return logits

@@ -39,6 +39,9 @@ class KernelError(RuntimeError):
 _SIGNATURES = {
     "axb_gemm": "ippppp" "iiiiiiii" "p",
     "axb_gemm_swiglu": "i" "pppp" "iiii" "p" "iii" "p",
+    "axb_gemm_on_pairs": "iii",
+    "axb_gemm_ce": "pppp" "iiii" "p",
+    "axb_ce_fwd_parts": "ppppppp" "ii" "l" "p",
     "axb_norm_fwd": "ppppp" "iii" "f" "iiii" "p",
     "axb_norm_bwd": "pppppppppp" "iiiiiiii" "p",
     "axb_add_norm_fwd": "ppppppp" "iii" "f" "iiii" "p",

@@ -11,6 +11,7 @@ import torch
 import torch.distributed as dist
 
 from . import _lib
+from .gemm import matmul_nn, matmul_tn
 
 
 class _CrossEntropyFn(torch.autograd.Function):
@@ -87,3 +88,54 @@ def cross_entropy(logits, targets, group=None, ignore_index=-100):
     is this rank's contiguous slice of the vocabulary (rank order = slice order).
     On GPU the logits buffer is consumed: backward overwrites it with the gradient."""
     return _CrossEntropyFn.apply(logits, targets, group, ignore_index)
+
+
+class _ProjectedCrossEntropyFn(torch.autograd.Function):
+    """``cross_entropy(x @ w.T, targets)`` whose softmax statistics come from the epilogue of the projection: the logits are
+    written once, read and overwritten by their gradient once, and read by the two GEMMs of the backward."""
+
+    @staticmethod
+    def forward(ctx, x, weight, targets, shape, ignore_index):
+        V, H = shape
+        x2 = x.reshape(-1, H)
+        t = targets.reshape(-1).contiguous()
+        rows = x2.shape[0]
+        dev = x.device
+        z = torch.empty((rows, V), dtype=x.dtype, device=dev)
+        part = torch.empty(((V + 255) // 256, rows, 2), dtype=torch.float32, device=dev)
+        L = _lib.lib()
+        _lib.check(L.axb_gemm_ce(_lib.addr(x2), _lib.addr(weight), _lib.addr(z), _lib.addr(part), rows, V, H, dev.index,
+                                 _lib.stream()), "axb_gemm_ce")
+        stats = torch.empty((rows, 3), dtype=torch.float32, device=dev)
+        lse = torch.empty(rows, dtype=torch.float32, device=dev)
+        # two tensors: the loss is returned, and a view made in here could not be modified in place later
+        mean, kept = (torch.empty((), dtype=torch.float32, device=dev) for _ in range(2))
+        _lib.check(L.axb_ce_fwd_parts(_lib.addr(part), _lib.addr(z), _lib.addr(t), _lib.addr(stats), _lib.addr(lse),
+                                      _lib.addr(mean), _lib.addr(kept), rows, V, ignore_index, _lib.stream()), "axb_ce_fwd_parts")
+        _lib.add_launches(1)
+        ctx.save_for_backward(x, weight, z, t, lse, kept)
+        ctx.shape, ctx.ignore_index = shape, ignore_index
+        return mean
+
+    @staticmethod
+    def backward(ctx, g):
+        x, weight, z, t, lse, kept = ctx.saved_tensors
+        V, H = ctx.shape
+        scale = (g.float() / kept).reshape(1).contiguous()
+        _lib.check(_lib.lib().axb_ce_bwd(_lib.addr(z), _lib.addr(t), _lib.addr(lse), _lib.addr(scale), z.shape[0], V, 0,
+                                         ctx.ignore_index, _lib.stream()), "axb_ce_bwd")
+        gx = matmul_nn(z, weight.view(V, H)).view(x.shape) if ctx.needs_input_grad[0] else None
+        gw = matmul_tn(z, x.reshape(-1, H)).view(weight.shape) if ctx.needs_input_grad[1] else None
+        return gx, gw, None, None, None
+
+
+def projected_cross_entropy(x, weight, targets, shape, ignore_index=-100):
+    """Mean cross-entropy of the logits ``x[..., H] @ weight.T`` with ``weight`` holding ``shape = (V, H)``; ``None`` when the
+    projection is not one of those whose kernel has the statistics in its epilogue (few rows, other types)."""
+    V, H = shape
+    if (x.is_cuda and weight.is_cuda and targets.is_cuda and x.dtype == weight.dtype == torch.bfloat16 and V % 8 == 0 and H % 8 == 0
+            and x.dim() > 0 and x.shape[-1] == H and weight.numel() == V * H and x.numel() > 0 and targets.dtype == torch.int64
+            and targets.numel() * H == x.numel() and x.is_contiguous() and weight.is_contiguous() and x.data_ptr() % 16 == 0
+            and weight.data_ptr() % 16 == 0 and _lib.lib().axb_gemm_on_pairs(x.numel() // H, V, x.device.index)):
+        return _ProjectedCrossEntropyFn.apply(x, weight, targets, shape, ignore_index)
+    return None

@@ -105,3 +105,81 @@ def test_swiglu_experts(E, rows, hidden, ffn, counts):
         assert _rel(y[e], y64[e]) < 3 * 2.0 ** -9
         for g, w in zip(got, want):
             assert bool(torch.isfinite(g[e]).all()) and _rel(g[e], w[e]) < 5 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("T,H,V", [(2048, 256, 4104), (1031, 264, 12808), (300, 64, 40000), (4096, 128, 50304)])
+def test_projected_cross_entropy(T, H, V):
+    """Projection and loss in one: a vocabulary that ends inside a chunk of 32 and inside a tile, rows that are no multiple of
+    anything, ignored and out-of-range targets, a row of -inf logits' neighbours.  The logits are bf16, so the loss is
+    compared with the unfused operations on the same product (fp32 sums: 1e-5) and the gradients with 64 bits (2^-8)."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib
+
+    assert _lib.lib().axb_gemm_on_pairs(T, V, 0)
+    torch.manual_seed(T)
+    x = torch.randn(1, T, H, device=DEV).bfloat16().requires_grad_(True)
+    w = (torch.randn(V * H, device=DEV) * 0.2).bfloat16().requires_grad_(True)
+    t = torch.randint(0, V, (1, T), device=DEV)
+    t[0, ::7] = -100
+    t[0, 1], t[0, 2] = V - 1, 0
+    loss = ops.projected_cross_entropy(x, w, t, (V, H))
+    ref = ops.cross_entropy(ops.matmul_nt(x.detach()[0], w.detach().view(V, H)), t)
+    assert abs(float(loss.detach()) - float(ref)) <= 1e-5 * abs(float(ref))
+    got = torch.autograd.grad(loss, [x, w], torch.full((), 3.0, device=DEV))
+    x64, w64 = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
+    z = x64[0] @ w64.view(V, H).t()
+    z = z + (z.detach().float().bfloat16().double() - z.detach())
+    want = torch.autograd.grad(3 * torch.nn.functional.cross_entropy(z, t[0]), [x64, w64])
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and _rel(a, b) < 2.0 ** -8
+    assert _lib.device_status() == 0
+
+
+def test_projected_cross_entropy_odd_rows():
+    """All logits of a row -inf: a NaN loss, as without fusion; a NaN input reaches the loss; -inf in single columns."""
+    from axonn_b200 import ops
+
+    T, H, V = 512, 64, 12800
+    for kind in ("inf", "nan", "columns"):
+        x, w = torch.ones(1, T, H, device=DEV).bfloat16(), torch.zeros(V, H, device=DEV).bfloat16()
+        w[:, 0] = torch.linspace(-3, 3, V, device=DEV).bfloat16()
+        if kind == "inf":
+            x[0, 5, 0] = float("inf")
+            w[:, 0] = -1.0
+        elif kind == "nan":
+            x[0, 5, 0] = float("nan")
+        else:
+            w[100:900, 0] = float("-inf")
+        t = torch.full((1, T), V - 1, device=DEV)
+        a = ops.projected_cross_entropy(x, w.view(-1), t, (V, H))
+        b = ops.cross_entropy(ops.matmul_nt(x[0], w), t)
+        assert bool(a.isnan()) == bool(b.isnan()) and (kind == "columns") != bool(a.isnan())
+        if kind == "columns":
+            assert abs(float(a) - float(b)) <= 1e-5 * abs(float(b))
+
+
+def test_lm_head_with_hooks():
+    """The head takes the fused path only when calling the projection is nothing but the product."""
+    import torch.distributed as dist
+
+    from axonn_b200 import axonn as ax
+    from axonn_b200.models import blocks
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    if not ax.is_initialized:
+        ax.init(G_inter=1, G_data=1, G_intra_r=1, G_intra_c=1, G_intra_d=1)
+    torch.manual_seed(0)
+    head = blocks.ParallelLMHead(128, 12800, dtype=BF16)
+    x, t = torch.randn(2, 200, 128, device=DEV, dtype=BF16, requires_grad=True), torch.randint(0, 12800, (2, 200), device=DEV)
+    assert blocks._is_plain_product(head.proj, x)
+    fused = head(x, t)
+    assert type(fused.grad_fn).__name__.startswith("_ProjectedCrossEntropy")
+    gf = torch.autograd.grad(fused, [x, head.proj.weight])
+    seen = []
+    handle = head.proj.register_forward_hook(lambda m, i, o: seen.append(o.shape))
+    plain = head(x, t)
+    handle.remove()
+    assert seen == [torch.Size([2, 200, 12800])] and abs(float(plain.detach()) - float(fused.detach())) < 1e-5 * float(plain.detach())
+    for a, b in zip(gf, torch.autograd.grad(plain, [x, head.proj.weight])):
+        assert a.shape == b.shape and _rel(a, b) < 2.0 ** -8
