@@ -75,6 +75,7 @@ struct GemmParams {
   // (mode 2) without a data row are not computed; a skipped tile is stored as zeros.
   const int* seg_counts;
   int seg_rows, nseg, mask_mode;
+  float* colsum;     // ACT_DGELU
   int whole_tiles;   // plain CTA-pair kernel: tiles from this one on are computed as two halves of their columns (PairWalk)
   int debug;      // ablation builds only (-DAXB_ABLATION, then read once from AXB_AR_DEBUG; otherwise 0 and every branch on it is compiled out): 1 no flagger fence, 2 no peer stores, 4 no reducer fence, 8 no reduction, 16 no partial stores, 128 register-path reducer instead of the shared-memory ring
 };
@@ -344,7 +345,10 @@ __device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t taddr
 // ---- epilogues of a gated feed-forward layer (bf16, CTA-pair kernel only); gate and up columns alternate in blocks of 8
 enum PairAct {
   ACT_NONE = 0,
+  ACT_GELU = 5,       // the plain epilogue (bias and GELU, saved pre-activation) on eight warps
   ACT_SWIGLU = 1,     // C [rows, N / 2] = silu(gate) * up of the product; aux [rows, N] receives the product, unless null
+  ACT_DGELU = 4,      // the product is the gradient of a GELU (tanh form); aux [rows, N] its input, C [rows, N] that one's gradient;
+                      // colsum fp32 [ceil(rows / 32)][N] the column sums of every 32 rows of C
   ACT_CE = 3,         // C [rows, N] the product (logits); aux float2 [N tiles][rows]: maximum and sum of exponentials of its row
   ACT_DSWIGLU = 2,    // the product is the gradient of that result; aux [rows, 2N] the saved product, C [rows, 2N] its gradient
 };
@@ -363,6 +367,60 @@ __device__ __forceinline__ void load_gate_up(const GemmParams& p, size_t row, bo
 }
 
 __device__ __forceinline__ float2 bf16x2_f32(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w)); }
+
+// v[i] of the lanes (one row each) summed over the warp; lane l gets column l.  31 exchanges instead of 5 for every column.
+__device__ __forceinline__ float column_sums32(float (&v)[32], int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float give = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  return v[0];
+}
+
+// Gradient of a GELU's input from the fp32 gradient of its output, with the column sums for the bias of the layer before it.
+template <int BN>
+__device__ __forceinline__ void epilogue_dgelu(const GemmParams& p, uint32_t taddr, size_t row, bool row_ok, int col0, uint32_t (&z)[32]) {
+  const int lane = threadIdx.x & 31;
+  const uint16_t* src = reinterpret_cast<const uint16_t*>(p.aux) + row * p.N;
+#pragma unroll 1
+  for (int c = 0; c < BN / 32; ++c) {
+    const int col = col0 + c * 32;
+    if (col >= p.N) break;  // uniform across the warp
+    uint32_t r[32], zc[16];
+    tmem_ld_32x32(taddr + c * 32, r);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) zc[i] = z[i];
+    if (c + 1 < BN / 32 && row_ok) {
+      if (col + 32 < p.N) ld_global_32b(src + col + 32, z);            // N is a multiple of 16
+      if (col + 48 < p.N) ld_global_32b(src + col + 48, z + 8);
+    }
+    tmem_ld_wait(r);
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float2 a = bf16x2_f32(zc[i]);
+      const bool live = row_ok && col + 2 * i < p.N;
+      v[2 * i] = live ? __uint_as_float(r[2 * i]) * gelu_tanh_grad(a.x) : 0.f;
+      v[2 * i + 1] = live ? __uint_as_float(r[2 * i + 1]) * gelu_tanh_grad(a.y) : 0.f;
+    }
+    if (row_ok) {
+      uint16_t* dst = reinterpret_cast<uint16_t*>(p.C) + row * p.N + col;
+      uint32_t o[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) o[i] = pack2(v[2 * i], v[2 * i + 1], 0);
+      st_global_32b(dst, *reinterpret_cast<uint32_t (*)[8]>(o));
+      if (col + 16 < p.N) st_global_32b(dst + 16, *reinterpret_cast<uint32_t (*)[8]>(o + 8));
+    }
+    const float sum = column_sums32(v, lane);
+    const size_t group = (row - lane) >> 5;                            // row - lane: the warp's first row, a multiple of 32
+    if (row - lane < static_cast<size_t>(p.M) && col + lane < p.N) p.colsum[group * p.N + col + lane] = sum;
+  }
+}
 
 // Logits with the statistics of their softmax: every thread has a row of the tile and keeps a running maximum and sum over its
 // columns, of the rounded logits that are stored.  A row of -inf has the sum zero, a NaN reaches the sum.
@@ -1307,7 +1365,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // traffic per SM and flop drops by a third against the single-CTA 128x256 tile, which is what bounds that
 // kernel's tensor-pipe utilisation.  TMA loads carry no multicast; the only cluster-wide signals are the
 // tcgen05.commit arrivals and plain remote mbarrier arrivals.
-constexpr int PAIR_THREADS = 192;   // TMA warp, MMA warp, 4 epilogue warps
 constexpr int PAIR_BN = 256;
 struct PairSmem {
   static constexpr int A_BYTES = BM * BK * 2;
@@ -1356,8 +1413,17 @@ struct PairWalk {
   }
 };
 
+// Epilogue warps per CTA.  Four store a tile's 128 rows in far less time than its MMAs take, but the arithmetic of an
+// activation is 16 to 20 instructions for each of the 256 columns of a thread, and one warp alone issues one in three cycles:
+// with eight warps, each with half of the columns, it stays below the MMAs' time.
+// One B200, bf16, back to back, four / eight warps: gradient of a GELU with its bias sums 16384 x 8192 x 2048 647 / 511 us (plain
+// product 435 / 409), adjoint of SwiGLU 593 / 548, bias, GELU and the saved pre-activation 16384 x 4096 x 1024 157 / 144,
+// SwiGLU at that size 273 / 269.
+template <int ACT>
+__host__ __device__ constexpr int pair_epi_warps() { return ACT == ACT_NONE || ACT == ACT_CE ? 4 : 8; }
+
 template <int A_MN, int B_MN, int ACT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epi_warps<ACT>(), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmBh, const GemmParams p) {
   using S = PairSmem;
@@ -1382,7 +1448,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 8); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 2 * pair_epi_warps<ACT>()); }
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -1489,7 +1555,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
   } else {
     // ------------------------------------------------------------------ epilogue (both CTAs, own 128 rows)
+    constexpr int PARTS = pair_epi_warps<ACT>() / 4, PN = BN / PARTS;   // warps that share 32 rows, columns of each
     const int q = warp & 3;
+    const int part = PARTS == 1 ? 0 : (warp - 2) >> 2;
     bool ok = true;
     int t = 0;
     PairWalk walk;
@@ -1507,7 +1575,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           float z[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) z[i] = 0.f;
-          for (int c = 0; c < BN / 32 && tn * BN + c * 32 < p.N; ++c)
+          for (int c = part * (PN / 32); c < (part + 1) * (PN / 32) && tn * BN + c * 32 < p.N; ++c)
             store_row32(p.C, p.out_dtype, row, p.N, tn * BN + c * 32, p.N, z, false);
         }
         continue;
@@ -1516,17 +1584,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t acc_phase = (t >> 1) & 1;
       ++t;
       uint32_t z[32];
-      if (ACT == ACT_DSWIGLU) load_gate_up(p, row, row_ok, tn * BN, z);
+      const int col0 = tn * BN + part * PN;
+      if (ACT == ACT_DSWIGLU) load_gate_up(p, row, row_ok, col0, z);
+      if (ACT == ACT_DGELU && row_ok && col0 < p.N) {
+        const uint16_t* src = reinterpret_cast<const uint16_t*>(p.aux) + row * p.N + col0;
+        ld_global_32b(src, z);
+        if (col0 + 16 < p.N) ld_global_32b(src + 16, z + 8);
+      }
       if (!mbar_wait(&tmem_full[buf], acc_phase, abort_flag, timeout)) { ok = false; break; }
       tcgen05_fence_after();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
-      if (ACT == ACT_CE) epilogue_ce<BN>(p, taddr, row, row_ok, tn * BN);
-      else if (ACT != ACT_NONE) epilogue_act<BN, ACT>(p, taddr, row, row_ok, tn * BN, z);     // whole tiles only
-      else if (walk.cols == BN) epilogue_row<BN>(p, taddr, row, row_ok, tn * BN);
-      else if (tn * BN + walk.col < p.N) epilogue_row<BN / 2>(p, taddr, row, row_ok, tn * BN + walk.col);
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN + part * PN;
+      if (ACT == ACT_CE) epilogue_ce<BN>(p, taddr, row, row_ok, col0);                   // these have whole tiles only
+      else if (ACT == ACT_DGELU) epilogue_dgelu<PN>(p, taddr, row, row_ok, col0, z);
+      else if (ACT == ACT_SWIGLU || ACT == ACT_DSWIGLU) epilogue_act<PN, ACT>(p, taddr, row, row_ok, col0, z);
+      else if (walk.cols == BN) { if (col0 < p.N) epilogue_row<PN>(p, taddr, row, row_ok, col0); }
+      else if (part == 0 && tn * BN + walk.col < p.N) epilogue_row<BN / 2>(p, taddr, row, row_ok, tn * BN + walk.col);
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_leader(&tmem_empty[buf]);   // 8 arrivals (4 warps x 2 CTAs) free the buffer
+      if (lane == 0) mbar_arrive_leader(&tmem_empty[buf]);   // the epilogue warps of both CTAs free the buffer
     }
     if (!ok && lane == 0) report_status(p.status, 0x144u);
   }
@@ -1911,7 +1986,7 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   const int items = p.whole_tiles + 2 * (total - p.whole_tiles);
   const int grid = 2 * (items < pairs ? items : pairs);
   p.gemm_ctas = grid;
-  kern<<<grid, PAIR_THREADS, S::TOTAL, stream>>>(tmA, tmB, tmBh ? *tmBh : tmB, p);
+  kern<<<grid, 64 + 32 * pair_epi_warps<ACT>(), S::TOTAL, stream>>>(tmA, tmB, tmBh ? *tmBh : tmB, p);
   AXB_CUDA(cudaGetLastError());
   return 0;
 }
@@ -2113,6 +2188,7 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
     CUtensorMap tmBh = tmB;
     const long long pair_tiles = static_cast<long long>((tiles_m + 1) / 2) * ((N + 255) / 256);
     if (b_mn == 0 && pair_whole_tiles(pair_tiles, usable_sms(device) / 2) != pair_tiles && make_tmap_2d_16bit(&tmBh, B, N, K, BN / 4, in_dtype)) return -1;
+    if (layout == 0 && epilogue >= 2) return launch_pair<0, 0, ACT_GELU>(tmA, tmB, &tmBh, p, device, s);
     if (layout == 0) return launch_pair<0, 0>(tmA, tmB, &tmBh, p, device, s);
     if (layout == 1) return launch_pair<0, 1>(tmA, tmB, &tmBh, p, device, s);
     return launch_pair<1, 1>(tmA, tmB, &tmBh, p, device, s);
@@ -2162,7 +2238,7 @@ extern "C" double axb_comm_stall_ms(int device, int reset) {
 // others are zero.  Tiles (K blocks in layout 2) without a data row are skipped; a skipped tile is stored as zeros.
 static int gemm_batched(int layout, const void* A, const void* B, void* C, void* aux, int act, int nb, int M, int N, int K,
                         int a_batch_rows, int b_batch_rows, int c_batch_rows, int in_dtype, int out_dtype, int accumulate,
-                        const int* seg_counts, int seg_rows, int nseg, int device, void* stream) {
+                        const int* seg_counts, int seg_rows, int nseg, int device, void* stream, float* colsum = nullptr) {
   using namespace axb;
   if (nb <= 0 || M <= 0 || N <= 0 || K <= 0) { set_error("axb_gemm_batched: empty problem"); return -1; }
   if (layout < 0 || layout > 2) { set_error("axb_gemm_batched: bad layout %d", layout); return -1; }
@@ -2186,7 +2262,7 @@ static int gemm_batched(int layout, const void* A, const void* B, void* C, void*
   if (b_mn == 0) { if (make_tmap_2d_16bit(&tmB, B, b_total, K, PAIR_BN / 2, in_dtype)) return -1; }
   else           { if (make_tmap_2d_16bit(&tmB, B, b_total, N, BK, in_dtype)) return -1; }
   GemmParams p;
-  p.C = C; p.bias = nullptr; p.aux = aux; p.M = M; p.N = N; p.K = K;
+  p.C = C; p.bias = nullptr; p.aux = aux; p.colsum = colsum; p.M = M; p.N = N; p.K = K;
   p.out_dtype = out_dtype; p.in_dtype = in_dtype; p.epilogue = 0; p.accumulate = accumulate;
   p.status = status_dev; p.timeout_ns = wait_timeout_ns();
   p.ar.n = 1; p.ag.n = 1; p.tn_offset = 0; p.kb_offset = 0; p.flag_batch = 1; p.debug = 0; p.pair = 1;
@@ -2201,6 +2277,7 @@ static int gemm_batched(int layout, const void* A, const void* B, void* C, void*
     p.seg_counts = seg_counts; p.seg_rows = seg_rows; p.nseg = nseg; p.mask_mode = (layout == 2) ? 2 : 1;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (act == ACT_DGELU) return launch_pair<0, 1, ACT_DGELU>(tmA, tmB, nullptr, p, device, s);
   if (act == ACT_CE) return launch_pair<0, 0, ACT_CE>(tmA, tmB, nullptr, p, device, s);
   if (act == ACT_SWIGLU) return launch_pair<0, 0, ACT_SWIGLU>(tmA, tmB, nullptr, p, device, s);
   if (act == ACT_DSWIGLU) return launch_pair<0, 1, ACT_DSWIGLU>(tmA, tmB, nullptr, p, device, s);
@@ -2234,6 +2311,21 @@ extern "C" int axb_gemm_swiglu(int backward, const void* A, const void* B, void*
   }
   return gemm_batched(backward ? 1 : 0, A, B, out, saved, backward ? ACT_DSWIGLU : ACT_SWIGLU, nb, M, N, K, M, backward ? K : N, M,
                       0, 0, 0, seg_counts, seg_rows, nseg, device, stream);
+}
+
+// dz [M, N] = (A [M, K] B [K, N]) * gelu'(z [M, N]), bf16, and the column sums of every 32 rows of dz in part, fp32
+// [ceil(M / 32)][N].  N % 16 == 0, K % 64 == 0.
+// One B200, back to back: 16384 x 8192 x 2048 511 us, the plain product and the pass over its result (gelu_bwd_colsum) 409 +
+// 154; 4096 rows 135 against 107 + 43; 2048 x 14336 x 4096 203 against 187 + 41.  At K = 1024 196 against 109 + 78.
+extern "C" int axb_gemm_dgelu(const void* A, const void* B, void* dz, const void* z, float* part, int M, int N, int K, int device,
+                              void* stream) {
+  using namespace axb;
+  if (N % 16) { set_error("axb_gemm_dgelu: N must be a multiple of 16"); return -1; }
+  if ((reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(z)) & 31) {
+    set_error("axb_gemm_dgelu: tensors must be 32-byte aligned");
+    return -1;
+  }
+  return gemm_batched(1, A, B, dz, const_cast<void*>(z), ACT_DGELU, 1, M, N, K, M, K, M, 0, 0, 0, nullptr, 0, 0, device, stream, part);
 }
 
 // logits [M, N] = A [M, K] B [N, K]^T (bf16) with, for every row and 256 columns, (maximum, sum of exp(logit - maximum)) in

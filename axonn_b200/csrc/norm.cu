@@ -1217,6 +1217,14 @@ extern "C" int axb_colsum(const void* x, float* part, void* out, int rows, int N
   return 0;
 }
 
+// out[c] = sum over the rows of part [rows, N] fp32, in a fixed order
+extern "C" int axb_fold_columns(const float* part, void* out, int rows, int N, int out_dtype, void* stream) {
+  using namespace axb;
+  fold_partials_kernel<<<(N + 31) / 32, dim3(32, 32), 0, static_cast<cudaStream_t>(stream)>>>(part, nullptr, out, nullptr, rows, N, out_dtype);
+  AXB_CUDA(cudaGetLastError());
+  return 0;
+}
+
 // dx = dy * gelu'(x) (tanh form) and colsum[c] = sum_r dx[r, c] in one pass.  part: [axb_colsum_splits, N] fp32.
 extern "C" int axb_gelu_bwd_colsum(const void* dy, const void* x, void* dx, float* part, void* colsum, int rows,
                                    int N, int dtype, int out_dtype, int device, void* stream) {

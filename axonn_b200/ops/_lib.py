@@ -40,6 +40,8 @@ _SIGNATURES = {
     "axb_gemm": "ippppp" "iiiiiiii" "p",
     "axb_gemm_swiglu": "i" "pppp" "iiii" "p" "iii" "p",
     "axb_gemm_on_pairs": "iii",
+    "axb_gemm_dgelu": "ppppp" "iiii" "p",
+    "axb_fold_columns": "pp" "iii" "p",
     "axb_gemm_ce": "pppp" "iiii" "p",
     "axb_ce_fwd_parts": "ppppppp" "ii" "l" "p",
     "axb_norm_fwd": "ppppp" "iii" "f" "iiii" "p",

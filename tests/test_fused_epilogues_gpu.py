@@ -183,3 +183,75 @@ def test_lm_head_with_hooks():
     assert seen == [torch.Size([2, 200, 12800])] and abs(float(plain.detach()) - float(fused.detach())) < 1e-5 * float(plain.detach())
     for a, b in zip(gf, torch.autograd.grad(plain, [x, head.proj.weight])):
         assert a.shape == b.shape and _rel(a, b) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("act,bias", [("gelu", True), ("gelu", False), ("swiglu", False)])
+@pytest.mark.parametrize("rows,hidden,ffn", [(2500, 2048, 4112), (1031, 2112, 8208), (300, 2048, 20000)])
+def test_mlp_function(act, bias, rows, hidden, ffn):
+    """The feed-forward block as one function: rows that end inside a group of 32, columns inside a chunk, with and without
+    bias, each gradient by itself, against 64 bits (roundings of 2^-9: three forward, five backward; bias sums are fp32)."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib
+
+    torch.manual_seed(rows)
+    wide = 2 * ffn if act == "swiglu" else ffn
+    x = torch.randn(1, rows, hidden, device=DEV).bfloat16().requires_grad_(True)
+    w1 = (torch.randn(wide * hidden, device=DEV) * hidden ** -0.5).bfloat16().requires_grad_(True)
+    w2 = (torch.randn(ffn * hidden, device=DEV) * ffn ** -0.5).bfloat16().requires_grad_(True)
+    b1 = torch.randn(wide, device=DEV).bfloat16().requires_grad_(True) if bias else None
+    b2 = torch.randn(hidden, device=DEV).bfloat16().requires_grad_(True) if bias else None
+    y = ops.mlp(x, w1, b1, w2, b2, hidden, ffn, act)
+    assert y is not None and y.shape == x.shape
+    leaves = [t for t in (x, w1, b1, w2, b2) if t is not None]
+    dy = torch.randn_like(y)
+    got = torch.autograd.grad(y, leaves, dy, retain_graph=True)
+    for t, g in zip(leaves, got):                    # one at a time gives the same bits
+        assert torch.equal(torch.autograd.grad(y, t, dy, retain_graph=True)[0], g)
+    assert _lib.device_status() == 0
+    l64 = [t.detach().double().requires_grad_(True) for t in leaves]
+    it = iter(l64)
+    x64, a64 = next(it), next(it)
+    c64 = next(it) if bias else 0
+    d64 = next(it)
+    e64 = next(it) if bias else 0
+    z = x64 @ a64.view(wide, hidden).t() + c64
+    if act == "swiglu":
+        v = z.reshape(1, rows, ffn // 8, 2, 8)
+        h = (torch.nn.functional.silu(v[..., 0, :]) * v[..., 1, :]).reshape(1, rows, ffn)
+    else:
+        h = torch.nn.functional.gelu(z, approximate="tanh")
+    y64 = h @ d64.view(hidden, ffn).t() + e64
+    assert _rel(y, y64) < 3 * 2.0 ** -9
+    for g, w in zip(got, torch.autograd.grad(y64, l64, dy.double())):
+        assert g.shape == w.shape and _rel(g, w) < 5 * 2.0 ** -9
+
+
+def test_mlp_module_routes():
+    """The module takes the function in training and its two layers everywhere else, with the same values."""
+    import torch.distributed as dist
+
+    from axonn_b200 import axonn as ax
+    from axonn_b200 import ops
+    from axonn_b200.models.blocks import ParallelMLP
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    if not ax.is_initialized:
+        ax.init(G_inter=1, G_data=1, G_intra_r=1, G_intra_c=1, G_intra_d=1)
+    torch.manual_seed(0)
+    x = torch.randn(2, 1000, 2048, device=DEV, dtype=BF16, requires_grad=True)
+    for act in ("gelu", "swiglu"):
+        m = ParallelMLP(2048, 2048, act, bias=act == "gelu", dtype=BF16)
+        y = m(x)
+        assert "MLP" in type(y.grad_fn).__name__
+        grads = torch.autograd.grad(y, [x, *m.parameters()], torch.ones_like(y))
+        seen = []
+        handle = m.fc2.register_forward_pre_hook(lambda mod, i: seen.append(i[0].shape))
+        z = m(x)
+        handle.remove()
+        assert seen == [torch.Size([2, 1000, 2048])] and _rel(y, z) < 2.0 ** -8
+        for a, b in zip(grads, torch.autograd.grad(z, [x, *m.parameters()], torch.ones_like(z))):
+            assert a.shape == b.shape and _rel(a, b) < 2.0 ** -7
+        with torch.no_grad():
+            assert _rel(m(x), y) < 2.0 ** -8
+        assert ops.mlp(x[:, :1], m.fc1.weight, m.fc1.bias, m.fc2.weight, m.fc2.bias, 2048, 2048, act) is None
