@@ -177,7 +177,8 @@ class ParallelMLP(nn.Module):
                           init_method=lambda w: nn.init.normal_(w, std=out_init_std or init_std))
 
     def forward(self, x):
-        if all(type(f) is Linear and f.expert_mode and not f.skip_bias_add and _is_plain_call(f, x) for f in (self.fc1, self.fc2)):
+        if torch.is_grad_enabled() and all(type(f) is Linear and f.expert_mode and not f.skip_bias_add and _is_plain_call(f, x)
+                                           for f in (self.fc1, self.fc2)):
             y = ops.mlp(x, self.fc1.weight, self.fc1.bias, self.fc2.weight, self.fc2.bias, self.fc2.out_features,
                         self.fc2.in_features, self.activation)
             if y is not None:

@@ -70,10 +70,9 @@ class GPT(nn.Module):
 
     def forward(self, tokens, targets=None):
         B, S = tokens.shape
-        pos = torch.arange(S, device=tokens.device)
-        if self.sequence_group is not None:
-            pos = pos + dist.get_rank(self.sequence_group) * S      # this rank's slice of the positions
-        x = self.tok_emb(tokens) + self.pos_emb(pos)[None]
+        first = 0 if self.sequence_group is None else dist.get_rank(self.sequence_group) * S
+        pos = self.pos_emb.rows(first, S, tokens.device)            # this rank's slice of the positions
+        x = self.tok_emb(tokens) + pos[None]
         delta = None   # MLP output of the previous block, added to x inside the next norm kernel
         for blk in self.blocks:
             if self.cfg.activation_checkpointing and self.training:
@@ -147,8 +146,7 @@ class DistributedGPT(nn.Module):
     def forward(self, x):
         if self.first:
             tokens = x.long()
-            pos = torch.arange(tokens.shape[1], device=tokens.device)
-            x = self.tok_emb(tokens) + self.pos_emb(pos)[None]
+            x = self.tok_emb(tokens) + self.pos_emb.rows(0, tokens.shape[1], tokens.device)[None]
         n = len(self.blocks)
         for lo in range(0, n, self.ckp_coeff):
             hi = min(n, lo + self.ckp_coeff)

@@ -131,3 +131,21 @@ def test_rope_counts_as_in_place():
         z.sum().backward()
     with torch.inference_mode():
         ops.apply_rope(torch.randn(1, 8, 2, 64, device=DEV, dtype=BF16), table)
+
+
+def test_embedding_rows():
+    """Rows of consecutive positions: a slice of the table without gradients, the layer itself with them, with a hook, and
+    past the end of the table (where the layer refuses)."""
+    from axonn_b200.intra_layer import Embedding
+
+    e = Embedding(40, 64, expert_mode=True, transpose=True, dtype=BF16)
+    dev = torch.device("cuda", 0)
+    ref = e(torch.arange(3, 20, device=dev))
+    assert ref.requires_grad and e.rows(3, 17, dev).requires_grad
+    with torch.no_grad():
+        got = e.rows(3, 17, dev)
+        assert torch.equal(got, ref) and got.data_ptr() == e.weight.data_ptr() + 3 * 64 * 2 and e.rows(0, 0, dev).shape == (0, 64)
+        seen = []
+        handle = e.register_forward_hook(lambda m, i, o: seen.append(o.shape))
+        assert torch.equal(e.rows(3, 17, dev), ref) and seen == [torch.Size([17, 64])]
+        handle.remove()
