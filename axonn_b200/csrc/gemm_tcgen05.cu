@@ -1967,9 +1967,10 @@ static int pair_whole_tiles(long long total, int pairs) {
   return static_cast<int>(rest != 0 && 2 * rest <= pairs ? total - rest : total);
 }
 
-// tmBh: B with boxes of half as many rows, for the halves of tiles (any map for an MN-major B); null: whole tiles only
+// tmBh: B with boxes of half as many rows, for the halves of tiles (any map for an MN-major B); null: whole tiles only.
+// sms: what the caller read from usable_sms, on which its choice of tmBh depends (another thread may change it meanwhile).
 template <int A_MN, int B_MN, int ACT = ACT_NONE>
-static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap* tmBh, GemmParams& p, int device,
+static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap* tmBh, GemmParams& p, int sms, int device,
                        cudaStream_t stream) {
   using S = PairSmem;
   static bool configured[64] = {false};
@@ -1981,7 +1982,7 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   p.tiles_m = (p.M + BM - 1) / BM;
   p.tiles_n = (p.N + PAIR_BN - 1) / PAIR_BN;
   const int total = ((p.tiles_m + 1) / 2) * p.tiles_n * p.nb;
-  const int pairs = usable_sms(device) / 2;
+  const int pairs = sms / 2;
   p.whole_tiles = tmBh ? pair_whole_tiles(total, pairs) : total;
   const int items = p.whole_tiles + 2 * (total - p.whole_tiles);
   const int grid = 2 * (items < pairs ? items : pairs);
@@ -2185,13 +2186,14 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
     return launch_comm_pair<1, 1>(tmA, tmB, p, device, s);
   }
   if (pair) {
+    const int sms = usable_sms(device);
     CUtensorMap tmBh = tmB;
     const long long pair_tiles = static_cast<long long>((tiles_m + 1) / 2) * ((N + 255) / 256);
-    if (b_mn == 0 && pair_whole_tiles(pair_tiles, usable_sms(device) / 2) != pair_tiles && make_tmap_2d_16bit(&tmBh, B, N, K, BN / 4, in_dtype)) return -1;
-    if (layout == 0 && epilogue >= 2) return launch_pair<0, 0, ACT_GELU>(tmA, tmB, &tmBh, p, device, s);
-    if (layout == 0) return launch_pair<0, 0>(tmA, tmB, &tmBh, p, device, s);
-    if (layout == 1) return launch_pair<0, 1>(tmA, tmB, &tmBh, p, device, s);
-    return launch_pair<1, 1>(tmA, tmB, &tmBh, p, device, s);
+    if (b_mn == 0 && pair_whole_tiles(pair_tiles, sms / 2) != pair_tiles && make_tmap_2d_16bit(&tmBh, B, N, K, BN / 4, in_dtype)) return -1;
+    if (layout == 0 && epilogue >= 2) return launch_pair<0, 0, ACT_GELU>(tmA, tmB, &tmBh, p, sms, device, s);
+    if (layout == 0) return launch_pair<0, 0>(tmA, tmB, &tmBh, p, sms, device, s);
+    if (layout == 1) return launch_pair<0, 1>(tmA, tmB, &tmBh, p, sms, device, s);
+    return launch_pair<1, 1>(tmA, tmB, &tmBh, p, sms, device, s);
   }
   if (splitk > 1) {
     if (layout == 0) return launch_splitk<0, 0>(tmA, tmB, p, splitk, device, s);
@@ -2277,13 +2279,14 @@ static int gemm_batched(int layout, const void* A, const void* B, void* C, void*
     p.seg_counts = seg_counts; p.seg_rows = seg_rows; p.nseg = nseg; p.mask_mode = (layout == 2) ? 2 : 1;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (act == ACT_DGELU) return launch_pair<0, 1, ACT_DGELU>(tmA, tmB, nullptr, p, device, s);
-  if (act == ACT_CE) return launch_pair<0, 0, ACT_CE>(tmA, tmB, nullptr, p, device, s);
-  if (act == ACT_SWIGLU) return launch_pair<0, 0, ACT_SWIGLU>(tmA, tmB, nullptr, p, device, s);
-  if (act == ACT_DSWIGLU) return launch_pair<0, 1, ACT_DSWIGLU>(tmA, tmB, nullptr, p, device, s);
-  if (layout == 0) return launch_pair<0, 0>(tmA, tmB, nullptr, p, device, s);
-  if (layout == 1) return launch_pair<0, 1>(tmA, tmB, nullptr, p, device, s);
-  return launch_pair<1, 1>(tmA, tmB, nullptr, p, device, s);
+  const int sms = usable_sms(device);
+  if (act == ACT_DGELU) return launch_pair<0, 1, ACT_DGELU>(tmA, tmB, nullptr, p, sms, device, s);
+  if (act == ACT_CE) return launch_pair<0, 0, ACT_CE>(tmA, tmB, nullptr, p, sms, device, s);
+  if (act == ACT_SWIGLU) return launch_pair<0, 0, ACT_SWIGLU>(tmA, tmB, nullptr, p, sms, device, s);
+  if (act == ACT_DSWIGLU) return launch_pair<0, 1, ACT_DSWIGLU>(tmA, tmB, nullptr, p, sms, device, s);
+  if (layout == 0) return launch_pair<0, 0>(tmA, tmB, nullptr, p, sms, device, s);
+  if (layout == 1) return launch_pair<0, 1>(tmA, tmB, nullptr, p, sms, device, s);
+  return launch_pair<1, 1>(tmA, tmB, nullptr, p, sms, device, s);
 }
 
 extern "C" int axb_gemm_batched(int layout, const void* A, const void* B, void* C, int nb, int M, int N, int K,

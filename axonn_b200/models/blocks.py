@@ -52,7 +52,7 @@ def _is_plain_call(layer, x):
             and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks
                      or hooks._global_forward_hooks or hooks._global_forward_pre_hooks or hooks._global_backward_hooks
                      or hooks._global_backward_pre_hooks)
-            and layer.forward.__func__ is Linear.forward
+            and getattr(layer.forward, "__func__", None) is Linear.forward      # not replaced on the instance
             and type(x) in (torch.Tensor, nn.Parameter) and type(layer.weight) is nn.Parameter
             and not torch.is_autocast_enabled("cuda") and not torch.compiler.is_compiling()
             and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active()

@@ -183,6 +183,9 @@ def test_lm_head_with_hooks():
     assert seen == [torch.Size([2, 200, 12800])] and abs(float(plain.detach()) - float(fused.detach())) < 1e-5 * float(plain.detach())
     for a, b in zip(gf, torch.autograd.grad(plain, [x, head.proj.weight])):
         assert a.shape == b.shape and _rel(a, b) < 2.0 ** -8
+    own = head.proj.forward
+    head.proj.forward = lambda *a, **k: own(*a, **k)                   # replaced on the instance
+    assert not blocks._is_plain_product(head.proj, x) and float(head(x, t).detach()) == float(plain.detach())
 
 
 @pytest.mark.parametrize("act,bias", [("gelu", True), ("gelu", False), ("swiglu", False)])
