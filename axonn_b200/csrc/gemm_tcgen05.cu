@@ -1584,7 +1584,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t acc_phase = (t >> 1) & 1;
       ++t;
       uint32_t z[32];
-      const int col0 = tn * BN + part * PN;
+      const bool whole = walk.cols == BN;
+      const int off = whole ? part * PN : part * (PN / 2);            // this warp's columns inside the item
+      const int col0 = tn * BN + walk.col + off;
       if (ACT == ACT_DSWIGLU) load_gate_up(p, row, row_ok, col0, z);
       if (ACT == ACT_DGELU && row_ok && col0 < p.N) {
         const uint16_t* src = reinterpret_cast<const uint16_t*>(p.aux) + row * p.N + col0;
@@ -1593,12 +1595,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       if (!mbar_wait(&tmem_full[buf], acc_phase, abort_flag, timeout)) { ok = false; break; }
       tcgen05_fence_after();
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN + part * PN;
-      if (ACT == ACT_CE) epilogue_ce<BN>(p, taddr, row, row_ok, col0);                   // these have whole tiles only
-      else if (ACT == ACT_DGELU) epilogue_dgelu<PN>(p, taddr, row, row_ok, col0, z);
-      else if (ACT == ACT_SWIGLU || ACT == ACT_DSWIGLU) epilogue_act<PN, ACT>(p, taddr, row, row_ok, col0, z);
-      else if (walk.cols == BN) { if (col0 < p.N) epilogue_row<PN>(p, taddr, row, row_ok, col0); }
-      else if (part == 0 && tn * BN + walk.col < p.N) epilogue_row<BN / 2>(p, taddr, row, row_ok, tn * BN + walk.col);
+      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN + off;
+      if (ACT == ACT_CE) {
+        epilogue_ce<BN>(p, taddr, row, row_ok, col0);                  // whole tiles only: statistics of 256 columns
+      } else if (ACT == ACT_DGELU) {
+        if (whole) epilogue_dgelu<PN>(p, taddr, row, row_ok, col0, z);
+        else epilogue_dgelu<PN / 2>(p, taddr, row, row_ok, col0, z);
+      } else if (ACT == ACT_SWIGLU || ACT == ACT_DSWIGLU) {
+        if (whole) epilogue_act<PN, ACT>(p, taddr, row, row_ok, col0, z);
+        else epilogue_act<PN / 2, ACT>(p, taddr, row, row_ok, col0, z);
+      } else if (col0 < p.N) {
+        if (whole) epilogue_row<PN>(p, taddr, row, row_ok, col0);
+        else epilogue_row<PN / 2>(p, taddr, row, row_ok, col0);
+      }
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_leader(&tmem_empty[buf]);   // the epilogue warps of both CTAs free the buffer
@@ -2280,10 +2289,17 @@ static int gemm_batched(int layout, const void* A, const void* B, void* C, void*
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int sms = usable_sms(device);
-  if (act == ACT_DGELU) return launch_pair<0, 1, ACT_DGELU>(tmA, tmB, nullptr, p, sms, device, s);
+  // a single problem without a mask may have the tiles of its last wave in halves
+  const CUtensorMap* halves = nullptr;
+  CUtensorMap tmBh = tmB;
+  if (nb == 1 && p.mask_mode == 0 && (act == ACT_SWIGLU || act == ACT_DSWIGLU || act == ACT_DGELU)) {
+    if (b_mn == 0 && make_tmap_2d_16bit(&tmBh, B, b_total, K, PAIR_BN / 4, in_dtype)) return -1;
+    halves = &tmBh;
+  }
+  if (act == ACT_DGELU) return launch_pair<0, 1, ACT_DGELU>(tmA, tmB, halves, p, sms, device, s);
   if (act == ACT_CE) return launch_pair<0, 0, ACT_CE>(tmA, tmB, nullptr, p, sms, device, s);
-  if (act == ACT_SWIGLU) return launch_pair<0, 0, ACT_SWIGLU>(tmA, tmB, nullptr, p, sms, device, s);
-  if (act == ACT_DSWIGLU) return launch_pair<0, 1, ACT_DSWIGLU>(tmA, tmB, nullptr, p, sms, device, s);
+  if (act == ACT_SWIGLU) return launch_pair<0, 0, ACT_SWIGLU>(tmA, tmB, halves, p, sms, device, s);
+  if (act == ACT_DSWIGLU) return launch_pair<0, 1, ACT_DSWIGLU>(tmA, tmB, halves, p, sms, device, s);
   if (layout == 0) return launch_pair<0, 0>(tmA, tmB, nullptr, p, sms, device, s);
   if (layout == 1) return launch_pair<0, 1>(tmA, tmB, nullptr, p, sms, device, s);
   return launch_pair<1, 1>(tmA, tmB, nullptr, p, sms, device, s);

@@ -8,6 +8,7 @@ PyTorch composition used on CPU (and as the numerical oracle in the tests).
 from .activation import gelu_backward_colsum, gelu, gelu_backward, swiglu  # noqa: F401
 from .attention import flash_attention, flash_attention_packed  # noqa: F401
 from .gemm import (  # noqa: F401
+    gemm_on_pairs,
     EPI_BIAS,
     EPI_BIAS_GELU,
     EPI_GELU,
@@ -18,7 +19,7 @@ from .gemm import (  # noqa: F401
 )
 from .linear import linear, linear_batched, swiglu_experts  # noqa: F401
 from .loss import cross_entropy, projected_cross_entropy  # noqa: F401
-from .mlp import mlp  # noqa: F401
+from .mlp import mlp, swiglu_projection  # noqa: F401
 from .multi_tensor import (  # noqa: F401
     all_reduce_bucketed_,
     multi_tensor_clip_factor,

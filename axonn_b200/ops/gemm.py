@@ -40,6 +40,11 @@ def _rowmajor(t):
     return t if t.is_contiguous() else t.contiguous()
 
 
+def gemm_on_pairs(M, N, device) -> bool:
+    """Does the ``M x N`` product run on the CTA-pair kernel, which has the epilogues with an activation?"""
+    return bool(_lib.lib().axb_gemm_on_pairs(M, N, device))
+
+
 def _launch(layout, a, b, M, N, K, out, bias=None, epilogue=EPI_NONE, accumulate=False, aux=None):
     if K % 8 or N % 8 or (layout == 2 and M % 8):
         raise ValueError(f"gemm dims must be multiples of 8 for 16-byte TMA strides, got M={M} N={N} K={K}")

@@ -149,3 +149,26 @@ def test_embedding_rows():
         handle = e.register_forward_hook(lambda m, i, o: seen.append(o.shape))
         assert torch.equal(e.rows(3, 17, dev), ref) and seen == [torch.Size([17, 64])]
         handle.remove()
+
+
+@pytest.mark.parametrize("rows,hidden,ffn", [(129, 64, 40000), (1000, 256, 2056), (2048, 136, 4104), (777, 512, 8),
+                                             (800, 64, 3080), (200, 64, 4096), (1100, 64, 2456)])
+def test_swiglu_block(rows, hidden, ffn):
+    """The gated block without gradients, rows and columns that end inside tiles and chunks, on the fused product and (few
+    columns, few rows) without it: the bits of the layers with their activation between them."""
+    from axonn_b200 import ops
+    from axonn_b200.models.blocks import ParallelMLP
+
+    torch.manual_seed(rows)
+    m = ParallelMLP(hidden, ffn, "swiglu", bias=False, dtype=BF16)
+    for x in (torch.randn(rows, hidden, device=DEV, dtype=BF16), torch.randn(1, rows, 2 * hidden, device=DEV, dtype=BF16)[..., :hidden],
+              torch.randn(2, 3, hidden, device=DEV, dtype=BF16)):
+        with torch.no_grad():
+            want = m.fc2(ops.swiglu(m.fc1(x)))
+            got = m(x)
+        assert got.shape == want.shape and torch.equal(got, want)
+    from axonn_b200.ops import _lib
+
+    with torch.no_grad():
+        h = ops.swiglu_projection(torch.randn(rows, hidden, device=DEV, dtype=BF16), m.fc1.weight, hidden)
+        assert (h is not None) == bool(_lib.lib().axb_gemm_on_pairs(rows, 2 * ffn, 0))

@@ -189,7 +189,7 @@ def test_lm_head_with_hooks():
 
 
 @pytest.mark.parametrize("act,bias", [("gelu", True), ("gelu", False), ("swiglu", False)])
-@pytest.mark.parametrize("rows,hidden,ffn", [(2500, 2048, 4112), (1031, 2112, 8208), (300, 2048, 20000)])
+@pytest.mark.parametrize("rows,hidden,ffn", [(2500, 2048, 4112), (1031, 2112, 8208), (300, 2048, 20000), (2300, 2048, 2192), (800, 2048, 6416)])
 def test_mlp_function(act, bias, rows, hidden, ffn):
     """The feed-forward block as one function: rows that end inside a group of 32, columns inside a chunk, with and without
     bias, each gradient by itself, against 64 bits (roundings of 2^-9: three forward, five backward; bias sums are fp32)."""
