@@ -19,8 +19,8 @@
 //               (described at reducer_warps / watcher_thread below).
 //
 // gemm_pair_kernel: clusters of two CTAs (tcgen05.mma.cta_group::2) compute
-// 256x256 tiles for plain GEMMs; warps 0-5 as above in each CTA, MMAs issued
-// by the even CTA for both.
+// 256x256 tiles for plain GEMMs; warps 0-5 as above in each CTA (0-9 where the
+// epilogue computes an activation), MMAs issued by the even CTA for both.
 //
 // Operand layouts: each of A and B is either K-major (row = M/N index, K
 // contiguous) or MN-major (row = K index, M/N contiguous); both are expressed
