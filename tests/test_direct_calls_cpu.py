@@ -1,0 +1,60 @@
+"""When a layer may launch its kernel by itself: the decision, asked on CPU ranks with the launch replaced by a record."""
+
+import torch
+
+from _dist import run_distributed
+
+
+def _without_gradients(rank, world, grid, transpose, bias, expert):
+    """Tensors of these ranks count as CUDA tensors and the GEMM is a stub that writes zeros."""
+    import torch.distributed as dist
+
+    from axonn_b200 import axonn as ax
+    from axonn_b200.intra_layer import Linear
+    from axonn_b200.intra_layer import fully_connected as fc
+    from axonn_b200.intra_layer.communication import _drop
+
+    ax.init(G_inter=1, G_data=1, G_intra_r=grid[0], G_intra_c=grid[1], G_intra_d=1)
+    launches = []
+
+    class Lib:
+        def axb_gemm(self, *args):
+            launches.append(args)
+            return 0
+
+    fc.no_graph = lambda *ts: not (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in ts))
+    fc._lib.lib, fc._lib.stream = lambda: Lib(), lambda: None
+    torch.manual_seed(1)
+    seq = torch.nn.Linear(64, 128, bias=bias).bfloat16()
+    layer = Linear(64, 128, bias=bias, transpose=transpose, expert_mode=expert, dtype=torch.bfloat16)
+    layer.load_state_dict(seq.state_dict())
+    X = torch.randn(8, 64).bfloat16()
+    x = _drop(X, 1, layer.inner_group) if expert else _drop(X, 0, dist.group.WORLD)
+    with_grad = layer(x)
+    assert not launches
+    with torch.no_grad():
+        y = layer(x)
+    assert y.shape == with_grad.shape
+    if not launches:
+        assert torch.equal(y, with_grad)
+        if not expert:
+            want = _drop(seq(X), 0, dist.group.WORLD)
+            assert (y.float() - want.float()).norm() <= 2 ** -7 * want.float().norm()
+    return len(launches)
+
+
+def _cases(rank, world, cases):
+    return [_without_gradients(rank, world, *case) for case in cases]
+
+
+def test_easy_mode_on_a_grid_is_not_one_launch():
+    """Easy mode trades batch for channels whichever group is larger than one: the output is this rank's rows of the whole
+    product, without gradients too."""
+    cases = [(grid, transpose, bias, False) for grid in ((2, 1), (1, 2)) for transpose in (False, True) for bias in (False, True)]
+    assert run_distributed(_cases, 2, cases) == [[0] * 8] * 2
+
+
+def test_expert_mode_on_a_grid():
+    """Expert mode keeps the shard of the outer group, so only the inner group's sum rules the launch out."""
+    cases = [((2, 1), False, False, True), ((2, 1), True, False, True), ((1, 2), True, False, True), ((1, 2), False, False, True)]
+    assert run_distributed(_cases, 2, cases) == [[1, 0, 1, 0]] * 2
