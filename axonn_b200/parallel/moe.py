@@ -263,7 +263,8 @@ class ExpertParallelMoE(nn.Module):
         needs of its reduction dimension."""
         T, E, k = x2.shape[0], self.n_experts, self.top_k
         rows = (C + 63) // 64 * 64
-        if E <= _ROUTE_MAX_EXPERTS:
+        # the kernel reads bf16; under autocast a router whose product is torch's (8 does not divide E) gives autocast's type
+        if E <= _ROUTE_MAX_EXPERTS and logits.dtype == torch.bfloat16:
             gate, self.last_aux_loss, dest, inverse, counts, stats = _LocalRoute.apply(logits, k, C, rows)
             self.last_assignments_per_expert, self.last_dropped_per_expert = stats[:E], stats[E:2 * E]
             self.last_drop_fraction = stats[2 * E]

@@ -64,3 +64,37 @@ def test_route_nan_and_infinities():
     assert experts == [[0, 1], [0, 1], [1, 2], [0, 1]]
     assert bool(gate[:2].isnan().all()) and bool(torch.isfinite(gate[2:]).all())
     assert stats[:4].tolist() == [3.0, 4.0, 1.0, 0.0]
+
+
+@pytest.fixture
+def _grid():
+    import torch.distributed as dist
+
+    from axonn_b200 import axonn as ax
+
+    if not dist.is_initialized():
+        dist.init_process_group("nccl", store=dist.HashStore(), rank=0, world_size=1)
+    if not ax.is_initialized:
+        ax.init(G_inter=1, G_data=1, G_intra_r=1, G_intra_c=1, G_intra_d=1)
+
+
+@pytest.mark.parametrize("E", [4, 8])
+@pytest.mark.parametrize("cast", [torch.float16, torch.float32])
+def test_router_under_autocast(_grid, E, cast):
+    """With 4 experts the router's product has autocast's type and the routing takes it as it is; with 8 it is bf16.  The
+    same experts as softmax and top-k of those logits, and the router's gradient of the balance loss by them (2^-7)."""
+    from axonn_b200 import ops
+    from axonn_b200.parallel.moe import ExpertParallelMoE, route_top_k
+
+    torch.manual_seed(E)
+    layer = ExpertParallelMoE(64, 64, n_experts=E, top_k=2, dtype=torch.bfloat16, init_std=0.3)
+    x = torch.randn(300, 64, device=DEV, dtype=torch.bfloat16)
+    with torch.autocast("cuda", dtype=cast):
+        logits = ops.linear(x, layer.router)
+        idx, aux = (route_top_k(logits, 2, 10 ** 6)[i] for i in (0, 4))
+        layer(x)
+    assert logits.dtype == (cast if E == 4 else torch.bfloat16)
+    assert torch.equal(layer.last_assignments_per_expert, torch.bincount(idx.reshape(-1), minlength=E).float())
+    assert abs(float(layer.last_aux_loss.detach()) - float(aux.detach())) <= 1e-5 * float(aux.detach())
+    (got,), (want,) = (torch.autograd.grad(v, layer.router) for v in (layer.last_aux_loss, aux))
+    assert float((got - want).float().norm()) <= 2.0 ** -7 * float(want.float().norm())
