@@ -147,7 +147,8 @@ int axb_moe_slots(const long long* idx, long long n, int E, int C, int Cp, int* 
                   float* assigned, void* stream);
 #define AXB_MOE_MAX_EXPERTS 32
 int axb_moe_route(const void* logits, int T, int E, int k, int C, int Cp, int* idx, float* gate, int* dest, int* inverse,
-                  int* counts, float* assigned, float* dropped, float* aux, float* drop_fraction, float* scratch, void* stream);
+                  int* counts, float* assigned, float* assigned_too, float* dropped, float* aux, float* drop_fraction,
+                  float* scratch, void* stream);
 int axb_moe_route_bwd(const void* logits, int T, int E, int k, const int* idx, const float* gate, const float* dgate,
                       const float* daux, const float* assigned, void* dlogits, void* stream);
 int axb_moe_rows(const void* x, const int* inverse, void* out, const float* gate, const void* other, float* dgate,

@@ -25,6 +25,7 @@ struct RouteStats {
   float inv_tokens, inv_assignments;
   unsigned int* blocks_done;     // zero on entry
   float* prob_sum;               // [E] scratch
+  float* assigned;               // [E] a second copy of the assignments
   float* dropped;                // [E]
   float* aux;                    // E * sum_e (share of the assignments) * (mean probability)
   float* drop_fraction;
@@ -78,6 +79,7 @@ moe_slots_kernel(const Index* __restrict__ idx, int n, int C, int Cp, int* __res
   for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
   if (lane != 0) return;
   st.prob_sum[e] = p;
+  st.assigned[e] = static_cast<float>(base);
   st.dropped[e] = static_cast<float>(max(base - C, 0));
   __threadfence();
   if (atomicAdd(st.blocks_done, 1u) != gridDim.x - 1) return;
@@ -304,11 +306,11 @@ extern "C" int axb_moe_slots(const long long* idx, long long n, int E, int C, in
 }
 
 // Router and slots of T tokens over E <= AXB_MOE_MAX_EXPERTS experts, two launches.  logits [T, E] bf16; idx [T, k] int32 chosen
-// experts; gate [T, k] their renormalised probabilities; dest, inverse, counts, assigned as in axb_moe_slots; dropped [E];
-// aux and drop_fraction scalars.  scratch: (ceil(T / 128) + 1) * E + 1 words.
+// experts; gate [T, k] their renormalised probabilities; dest, inverse, counts, assigned as in axb_moe_slots; assigned_too [E] the
+// same as assigned (for a caller who keeps one and hands on the other); dropped [E]; aux and drop_fraction scalars.  scratch: (ceil(T / 128) + 1) * E + 1 words.
 extern "C" int axb_moe_route(const void* logits, int T, int E, int k, int C, int Cp, int* idx, float* gate, int* dest,
-                             int* inverse, int* counts, float* assigned, float* dropped, float* aux, float* drop_fraction,
-                             float* scratch, void* stream) {
+                             int* inverse, int* counts, float* assigned, float* assigned_too, float* dropped, float* aux,
+                             float* drop_fraction, float* scratch, void* stream) {
   const long long n = static_cast<long long>(T) * k;
   if (T <= 0 || k <= 0 || k > E || E > AXB_MOE_MAX_EXPERTS || n > 0x7ffffff0ll || C <= 0 || Cp < C ||
       static_cast<long long>(E) * Cp > 0x7fffffffll) {
@@ -321,7 +323,7 @@ extern "C" int axb_moe_route(const void* logits, int T, int E, int k, int C, int
   auto kern = E <= 8 ? moe_route_kernel<8> : (E <= 16 ? moe_route_kernel<16> : moe_route_kernel<AXB_MOE_MAX_EXPERTS>);
   kern<<<grid, MR_THREADS, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)logits, T, E, k, idx, gate, scratch, done);
   AXB_CUDA(cudaGetLastError());
-  const RouteStats st{scratch, grid, 1.f / T, 1.f / static_cast<float>(n), done, prob_sum, dropped, aux, drop_fraction};
+  const RouteStats st{scratch, grid, 1.f / T, 1.f / static_cast<float>(n), done, prob_sum, assigned_too, dropped, aux, drop_fraction};
   moe_slots_kernel<int><<<E, MS_THREADS, 0, (cudaStream_t)stream>>>(idx, static_cast<int>(n), C, Cp, dest, inverse, counts, assigned, st);
   AXB_CUDA(cudaGetLastError());
   return 0;

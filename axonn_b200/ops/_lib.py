@@ -66,7 +66,7 @@ _SIGNATURES = {
     "axb_multi_clip_factor": "p" "il" "f" "pp",
     "axb_multi_scale": "p" "il" "pp",
     "axb_multi_adamw": "p" "il" "fffffff" "ppp",
-    "axb_moe_route": "piiiii" "pppppppppp" "p",
+    "axb_moe_route": "piiiii" "ppppppppppp" "p",
     "axb_moe_route_bwd": "piii" "pppppp" "p",
     "axb_prune_topk": "p" "lil" "p" "i" "p",
 }

@@ -70,14 +70,14 @@ class _LocalRoute(torch.autograd.Function):
         T, E = logits.shape
         dev = logits.device
         idx, dest, inverse, counts = (torch.empty(n, dtype=torch.int32, device=dev) for n in (T * k, T * k, E * rows, E))
-        gate, aux, stats, scratch = (torch.empty(n, dtype=torch.float32, device=dev)
-                                     for n in ((T, k), (), 2 * E + 1, ((T + 127) // 128 + 1) * E + 1))
+        gate, aux, stats, assigned, scratch = (torch.empty(n, dtype=torch.float32, device=dev)
+                                               for n in ((T, k), (), 2 * E + 1, E, ((T + 127) // 128 + 1) * E + 1))
         word = stats.data_ptr()
         _lib.check(_lib.lib().axb_moe_route(_lib.addr(logits), T, E, k, C, rows, _lib.addr(idx), _lib.addr(gate),
-                                            _lib.addr(dest), _lib.addr(inverse), _lib.addr(counts), word, word + 4 * E,
-                                            _lib.addr(aux), word + 8 * E, _lib.addr(scratch), _lib.stream()), "axb_moe_route")
+                                            _lib.addr(dest), _lib.addr(inverse), _lib.addr(counts), _lib.addr(assigned), word,
+                                            word + 4 * E, _lib.addr(aux), word + 8 * E, _lib.addr(scratch), _lib.stream()), "axb_moe_route")
         _lib.add_launches(1)
-        ctx.save_for_backward(logits, idx, gate, stats)
+        ctx.save_for_backward(logits, idx, gate, assigned)      # the statistics are the caller's, who may sum them in place
         ctx.mark_non_differentiable(dest, inverse, counts, stats)
         ctx.set_materialize_grads(False)
         ctx.k = k
@@ -86,7 +86,7 @@ class _LocalRoute(torch.autograd.Function):
     @staticmethod
     @once_differentiable
     def backward(ctx, dgate, daux, *_):
-        logits, idx, gate, stats = ctx.saved_tensors
+        logits, idx, gate, assigned = ctx.saved_tensors
         if dgate is None and daux is None:
             return None, None, None, None
         T, E = logits.shape
@@ -94,7 +94,7 @@ class _LocalRoute(torch.autograd.Function):
         daux = None if daux is None else daux.float()
         dlogits = torch.empty_like(logits)
         _lib.check(_lib.lib().axb_moe_route_bwd(_lib.addr(logits), T, E, ctx.k, _lib.addr(idx), _lib.addr(gate), _lib.addr(dgate),
-                                                _lib.addr(daux), _lib.addr(stats), _lib.addr(dlogits), _lib.stream()),
+                                                _lib.addr(daux), _lib.addr(assigned), _lib.addr(dlogits), _lib.stream()),
                    "axb_moe_route_bwd")
         return dlogits, None, None, None
 

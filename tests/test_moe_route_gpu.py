@@ -98,3 +98,19 @@ def test_router_under_autocast(_grid, E, cast):
     assert abs(float(layer.last_aux_loss.detach()) - float(aux.detach())) <= 1e-5 * float(aux.detach())
     (got,), (want,) = (torch.autograd.grad(v, layer.router) for v in (layer.last_aux_loss, aux))
     assert float((got - want).float().norm()) <= 2.0 ** -7 * float(want.float().norm())
+
+
+def test_statistics_belong_to_the_caller(_grid):
+    """Sums over ranks or steps are made in place, before the backward too, and do not reach the gradient."""
+    from axonn_b200.parallel.moe import ExpertParallelMoE
+
+    torch.manual_seed(0)
+    layer = ExpertParallelMoE(64, 64, n_experts=8, top_k=2, dtype=torch.bfloat16, init_std=0.3)
+    x = torch.randn(300, 64, device=DEV, dtype=torch.bfloat16)
+    grads = []
+    for add in (0, 1000):
+        loss = layer(x).float().square().sum() + layer.last_aux_loss
+        for t in (layer.last_assignments_per_expert, layer.last_dropped_per_expert, layer.last_drop_fraction):
+            t += add
+        grads.append(torch.autograd.grad(loss, layer.router)[0])
+    assert torch.equal(*grads)
