@@ -186,7 +186,7 @@ class ParallelMLP(nn.Module):
         if self.activation == "swiglu":
             f = self.fc1
             # the cheap questions first: blocks of few rows are bound by host time (200 x 2048 x 4096 46 -> 53 us without them)
-            if (not torch.is_grad_enabled() and x.is_cuda and x.numel() >= 512 * f.in_features
+            if (type(f) is Linear and not torch.is_grad_enabled() and x.is_cuda and x.numel() >= 512 * f.in_features
                     and ops.gemm_on_pairs(x.numel() // f.in_features, f.out_features, x.device.index) and _is_plain_product(f, x)):
                 h = ops.swiglu_projection(x, f.weight, f.in_features)
                 if h is not None:

@@ -172,3 +172,17 @@ def test_swiglu_block(rows, hidden, ffn):
     with torch.no_grad():
         h = ops.swiglu_projection(torch.randn(rows, hidden, device=DEV, dtype=BF16), m.fc1.weight, hidden)
         assert (h is not None) == bool(_lib.lib().axb_gemm_on_pairs(rows, 2 * ffn, 0))
+
+
+def test_replaced_first_layer():
+    """A gated block whose first layer was replaced by a module of any kind runs that module, with gradients and without."""
+    from axonn_b200.models.blocks import ParallelMLP
+
+    torch.manual_seed(0)
+    m = ParallelMLP(64, 4096, "swiglu", bias=False, dtype=BF16)
+    x = torch.randn(2000, 64, device=DEV, dtype=BF16)
+    want = m(x)
+    m.fc1 = torch.nn.Sequential(m.fc1, torch.nn.Identity())
+    assert torch.equal(m(x), want)
+    with torch.no_grad():
+        assert torch.equal(m(x), want)
