@@ -18,6 +18,13 @@ from ..intra_layer import Embedding
 from .blocks import ParallelLMHead, TPNorm, TransformerBlock, count_parameters
 
 
+def _positions(embedding, first, count, device):
+    """Embeddings of ``count`` consecutive positions, from whatever module stands for the position embedding."""
+    if isinstance(embedding, Embedding):
+        return embedding.rows(first, count, device)
+    return embedding(torch.arange(first, first + count, device=device))
+
+
 @dataclass
 class GPTConfig:
     """Shape of a GPT-style model; ``gpt_1p3b()`` is the benchmark configuration, ``tiny()`` the test one."""
@@ -71,7 +78,7 @@ class GPT(nn.Module):
     def forward(self, tokens, targets=None):
         B, S = tokens.shape
         first = 0 if self.sequence_group is None else dist.get_rank(self.sequence_group) * S
-        pos = self.pos_emb.rows(first, S, tokens.device)            # this rank's slice of the positions
+        pos = _positions(self.pos_emb, first, S, tokens.device)     # this rank's slice of the positions
         x = self.tok_emb(tokens) + pos[None]
         delta = None   # MLP output of the previous block, added to x inside the next norm kernel
         for blk in self.blocks:
@@ -146,7 +153,7 @@ class DistributedGPT(nn.Module):
     def forward(self, x):
         if self.first:
             tokens = x.long()
-            x = self.tok_emb(tokens) + self.pos_emb.rows(0, tokens.shape[1], tokens.device)[None]
+            x = self.tok_emb(tokens) + _positions(self.pos_emb, 0, tokens.shape[1], tokens.device)[None]
         n = len(self.blocks)
         for lo in range(0, n, self.ckp_coeff):
             hi = min(n, lo + self.ckp_coeff)

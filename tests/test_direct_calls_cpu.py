@@ -58,3 +58,27 @@ def test_expert_mode_on_a_grid():
     """Expert mode keeps the shard of the outer group, so only the inner group's sum rules the launch out."""
     cases = [((2, 1), False, False, True), ((2, 1), True, False, True), ((1, 2), True, False, True), ((1, 2), False, False, True)]
     assert run_distributed(_cases, 2, cases) == [[1, 0, 1, 0]] * 2
+
+
+def _other_position_embedding(rank, world):
+    from axonn_b200 import axonn as ax
+    from axonn_b200.models import GPT, GPTConfig
+    from axonn_b200.models.gpt import DistributedGPT
+
+    ax.init(G_inter=1, G_data=1, G_intra_r=1, G_intra_c=1, G_intra_d=1)
+    cfg = GPTConfig.tiny()
+    for model in (GPT(cfg, dtype=torch.float32), DistributedGPT(cfg, dtype=torch.float32)):
+        tokens = torch.randint(0, cfg.vocab, (2, 8))
+        want = model(tokens)
+        own = model.pos_emb
+        table = own.weight.detach().view(cfg.seq_len, cfg.hidden)
+        model.pos_emb = torch.nn.Embedding.from_pretrained(table)
+        assert torch.equal(model(tokens), want)
+        with torch.no_grad():
+            assert torch.equal(model(tokens), want)
+    return True
+
+
+def test_replaced_position_embedding():
+    """A GPT runs with any module in the place of its position embedding."""
+    assert run_distributed(_other_position_embedding, 1) == [True]
