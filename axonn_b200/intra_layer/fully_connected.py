@@ -32,7 +32,7 @@ from torch.autograd import Function
 from .. import axonn as ax
 from .. import ops
 from ..ops import _lib
-from ..ops.direct import no_graph
+from ..ops.direct import no_graph, own_forward
 from ..parallel import fused
 from ..utils import divide
 from . import overlap_communication as oc
@@ -291,6 +291,7 @@ class AsyncLinear(Function):
         return grad_input, grad_weight, grad_bias, None, None, None, None, None, None
 
 
+@own_forward
 class Linear(torch.nn.Module):
     """Drop-in ``nn.Linear`` whose weight is sharded over the 3-D grid.
 

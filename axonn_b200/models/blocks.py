@@ -18,12 +18,12 @@ import math
 import torch
 import torch.distributed as dist
 import torch.nn as nn
-from torch.autograd import forward_ad
 
 from .. import axonn as ax
 from .. import ops
 from ..intra_layer import Gather, Linear
 from ..intra_layer.communication import _drop, _gather
+from ..ops.direct import plain_layer, plain_tensors
 from ..utils import divide
 
 
@@ -41,22 +41,16 @@ def _tag_sharded(param, shard_group):
 
 
 def _is_plain_product(layer, x):
-    """Is calling ``layer`` on ``x`` nothing but ``x @ W.T``, so that a fused operation may take its place?  An ordinary
-    ``Linear`` without bias, collectives, hooks or autocast, and nothing that traces or transforms the call."""
-    return (type(layer) is Linear and layer.bias is None and _is_plain_call(layer, x))
+    """Is calling ``layer`` on ``x`` nothing but ``x @ W.T``, so that a fused operation may take its place?"""
+    return type(layer) is Linear and layer.bias is None and _is_plain_call(layer, x)
 
 
 def _is_plain_call(layer, x):
-    hooks = nn.modules.module
-    return (layer.inner_group_size * layer.outer_group_size * layer.depth_group_size == 1
-            and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks
-                     or hooks._global_forward_hooks or hooks._global_forward_pre_hooks or hooks._global_backward_hooks
-                     or hooks._global_backward_pre_hooks)
-            and getattr(layer.forward, "__func__", None) is Linear.forward      # not replaced on the instance
-            and type(x) in (torch.Tensor, nn.Parameter) and type(layer.weight) is nn.Parameter
-            and not torch.is_autocast_enabled("cuda") and not torch.compiler.is_compiling()
-            and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active()
-            and forward_ad._current_level < 0)
+    """Is calling the ``Linear`` ``layer`` on ``x`` nothing but its product and bias?  No collectives, hooks, replaced forward or
+    autocast, and nothing that traces or transforms the call."""
+    return (layer.inner_group_size * layer.outer_group_size * layer.depth_group_size == 1 and plain_layer(layer)
+            and type(layer.weight) is nn.Parameter and plain_tensors(x, layer.weight, layer.bias)
+            and not torch.is_autocast_enabled("cuda"))
 
 
 class TPNorm(nn.Module):

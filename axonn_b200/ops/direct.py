@@ -1,21 +1,48 @@
-"""When an operation may launch its kernel without an autograd function around it.
+"""When a kernel may stand in for a call: for an autograd function (``no_graph``), for the call of a layer (``plain_layer``).
 
-The function costs more host time than the launch (4 us against 5 us, and as much again in reshapes and saved tensors), and
-evaluating a model without gradients is bound by host time for short prompts."""
+An autograd function costs more host time than the launch (4 us against 5 us, and as much again in reshapes and saved tensors),
+and evaluating a model without gradients is bound by host time for short prompts."""
 
 import torch
 from torch.autograd import forward_ad
 
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
+_module = torch.nn.modules.module
+_CALL = torch.nn.Module.__call__
+_own_forward = {}
 
 
 def no_graph(*tensors) -> bool:
     """No gradient can be asked of an operation on ``tensors`` (``None`` entries are skipped) and nothing looks at it from
-    outside: grad mode is off or none of them requires a gradient, they are ordinary CUDA tensors, and no tracer, compiler,
-    function transform or forward-mode level is active."""
-    grad = torch.is_grad_enabled()
+    outside: grad mode is off or none of them requires a gradient, and they are ``plain_tensors``."""
+    if torch.is_grad_enabled():
+        for t in tensors:
+            if t is not None and t.requires_grad:
+                return False
+    return plain_tensors(*tensors)
+
+
+def plain_tensors(*tensors) -> bool:
+    """Ordinary CUDA tensors (``None`` entries are skipped) while no tracer, compiler, function transform or forward-mode level
+    is active."""
     for t in tensors:
-        if t is not None and (type(t) not in _PLAIN or not t.is_cuda or (grad and t.requires_grad)):
+        if t is not None and (type(t) not in _PLAIN or not t.is_cuda):
             return False
     return (not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None
             and forward_ad._current_level < 0 and not torch.compiler.is_compiling())
+
+
+def own_forward(cls):
+    """Class decorator: calls of such layers may be replaced (see ``plain_layer``) while ``cls.forward`` is what it is now."""
+    _own_forward[cls] = cls.forward
+    return cls
+
+
+def plain_layer(layer) -> bool:
+    """Is calling ``layer`` nothing but the forward that its class was defined with?  Of a class marked with ``own_forward`` and no
+    other, its forward replaced neither on the instance nor on the class, neither hooks nor a compiled call in its way."""
+    cls = type(layer)
+    return (cls in _own_forward and cls.forward is _own_forward[cls] and cls.__call__ is _CALL and "forward" not in layer.__dict__
+            and layer._compiled_call_impl is None
+            and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks
+                     or _module._has_any_global_hook()))

@@ -186,3 +186,40 @@ def test_replaced_first_layer():
     assert torch.equal(m(x), want)
     with torch.no_grad():
         assert torch.equal(m(x), want)
+
+
+def test_replaced_forwards(monkeypatch):
+    """A forward replaced on the instance or on the class is called, whatever could stand in for the original."""
+    from axonn_b200.intra_layer import Embedding, Linear
+    from axonn_b200.models import blocks
+    from axonn_b200.ops.direct import plain_layer
+
+    dev = torch.device("cuda", 0)
+    e, head = Embedding(40, 64, expert_mode=True, dtype=BF16), blocks.ParallelLMHead(64, 12800, dtype=BF16)
+    m = blocks.ParallelMLP(64, 4096, "swiglu", bias=False, dtype=BF16)
+    x, t = torch.randn(2000, 64, device=DEV, dtype=BF16), torch.randint(0, 12800, (2000,), device=DEV)
+
+    def calls():
+        with torch.no_grad():
+            e.rows(3, 4, dev), m(x), head(x, t)
+        m(x), head(x, t)
+
+    seen = []
+    calls()
+    for layer in (e, m.fc1, m.fc2, head.proj):
+        assert plain_layer(layer)
+        own = layer.forward
+        layer.forward = lambda *a, own=own, **k: (seen.append(own), own(*a, **k))[1]
+        assert not plain_layer(layer)
+    calls()
+    assert len(seen) == 1 + 2 * 3
+    for layer in (e, m.fc1, m.fc2, head.proj):
+        del layer.forward
+    seen.clear()
+    for cls in (Embedding, Linear):
+        own = cls.forward
+        monkeypatch.setattr(cls, "forward", lambda self, *a, own=own, **k: (seen.append(own), own(self, *a, **k))[1])
+    calls()
+    assert len(seen) == 1 + 2 * 3
+    monkeypatch.undo()
+    assert all(plain_layer(layer) for layer in (e, m.fc1, m.fc2, head.proj))
