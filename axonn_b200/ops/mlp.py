@@ -40,11 +40,12 @@ class _MLPFn(torch.autograd.Function):
             _swiglu_gemm(False, x2[None], v1[None], h, z, None, 0)
         else:
             h = matmul_nt(x2, v1, bias=b1, epilogue=EPI_GELU if b1 is None else EPI_BIAS_GELU, aux=z)
-        y = matmul_nt(h, v2, bias=b2, epilogue=EPI_NONE if b2 is None else EPI_BIAS)
+        # a view made in here could not be modified in place later: the result has its shape from the beginning
+        y = torch.empty((*x.shape[:-1], hidden), dtype=x.dtype, device=x.device)
+        matmul_nt(h, v2, bias=b2, epilogue=EPI_NONE if b2 is None else EPI_BIAS, out=y.view(-1, hidden))
         ctx.save_for_backward(x, w1, w2, z, h)
         ctx.hidden, ctx.act, ctx.b1, ctx.b2 = hidden, act, None if b1 is None else b1.dtype, None if b2 is None else b2.dtype
-        target = (*x.shape[:-1], hidden)
-        return y if y.shape == target else y.reshape(target)
+        return y
 
     @staticmethod
     def backward(ctx, g):

@@ -82,3 +82,18 @@ def _other_position_embedding(rank, world):
 def test_replaced_position_embedding():
     """A GPT runs with any module in the place of its position embedding."""
     assert run_distributed(_other_position_embedding, 1) == [True]
+
+
+def test_feed_forward_result_in_place():
+    """What the fused feed-forward block returns may be modified in place (a residual added to it), in any number of
+    dimensions."""
+    from axonn_b200.ops.mlp import _MLPFn
+
+    torch.manual_seed(0)
+    w1, w2 = (torch.randn(128 * 64, requires_grad=True) for _ in range(2))
+    for shape in ((6, 64), (2, 3, 64)):
+        x = torch.randn(shape, requires_grad=True)
+        y = _MLPFn.apply(x, w1, None, w2, None, 64, "gelu")
+        z = _MLPFn.apply(x, w1, None, w2, None, 64, "gelu") + x
+        y += x
+        assert torch.equal(y, z) and y.shape == shape and y.grad_fn is not None
