@@ -40,6 +40,13 @@ def _rowmajor(t):
     return t if t.is_contiguous() else t.contiguous()
 
 
+def as_written(t):
+    """``t`` dense and on a 32-byte boundary, for kernels that are given its address: itself or a copy.  A tensor saved for a
+    backward comes back from hooks (offloading, compression) in whatever layout they give it."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 32 == 0 else t.clone()
+
+
 def gemm_on_pairs(M, N, device) -> bool:
     """Does the ``M x N`` product run on the CTA-pair kernel, which has the epilogues with an activation?"""
     return bool(_lib.lib().axb_gemm_on_pairs(M, N, device))

@@ -5,7 +5,7 @@ import torch
 
 from . import _lib
 from .activation import swiglu
-from .gemm import bmm_nn, bmm_nt, bmm_tn, matmul_nn, matmul_nt, matmul_tn
+from .gemm import as_written, bmm_nn, bmm_nt, bmm_tn, matmul_nn, matmul_nt, matmul_tn
 
 
 class _LinearFn(torch.autograd.Function):
@@ -91,11 +91,11 @@ class _SwiGLUExpertsFn(torch.autograd.Function):
     def backward(ctx, g):
         x, w1, w2, gu, h = ctx.saved_tensors
         seg = dict(seg=ctx.seg, seg_rows=ctx.seg_rows)
-        g = g.contiguous()
-        g = g if g.data_ptr() % 16 == 0 else g.clone()
+        g = as_written(g)
         gx = gw1 = gw2 = None
         if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
-            dgu = _swiglu_gemm(True, g, w2, torch.empty_like(gu), gu, **seg)
+            gu = as_written(gu)
+            dgu = _swiglu_gemm(True, g, as_written(w2), torch.empty_like(gu), gu, **seg)
             gx = bmm_nn(dgu, w1, **seg) if ctx.needs_input_grad[0] else None
             gw1 = bmm_tn(dgu, x, out_dtype=w1.dtype, **seg) if ctx.needs_input_grad[1] else None
         if ctx.needs_input_grad[2]:

@@ -11,7 +11,7 @@ import torch
 import torch.distributed as dist
 
 from . import _lib
-from .gemm import matmul_nn, matmul_tn
+from .gemm import as_written, matmul_nn, matmul_tn
 
 
 class _CrossEntropyFn(torch.autograd.Function):
@@ -120,11 +120,12 @@ class _ProjectedCrossEntropyFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         x, weight, z, t, lse, kept = ctx.saved_tensors
+        z, t, lse = as_written(z), t.contiguous(), lse.contiguous()
         V, H = ctx.shape
         scale = (g.float() / kept).reshape(1).contiguous()
         _lib.check(_lib.lib().axb_ce_bwd(_lib.addr(z), _lib.addr(t), _lib.addr(lse), _lib.addr(scale), z.shape[0], V, 0,
                                          ctx.ignore_index, _lib.stream()), "axb_ce_bwd")
-        gx = matmul_nn(z, weight.view(V, H)).view(x.shape) if ctx.needs_input_grad[0] else None
+        gx = matmul_nn(z, weight.reshape(V, H)).view(x.shape) if ctx.needs_input_grad[0] else None
         gw = matmul_tn(z, x.reshape(-1, H)).view(weight.shape) if ctx.needs_input_grad[1] else None
         return gx, gw, None, None, None
 

@@ -4,7 +4,7 @@ import torch
 
 from . import _lib
 from .direct import no_graph
-from .gemm import EPI_BIAS, EPI_BIAS_GELU, EPI_GELU, EPI_NONE, matmul_nn, matmul_nt, matmul_tn
+from .gemm import EPI_BIAS, EPI_BIAS_GELU, EPI_GELU, EPI_NONE, as_written, matmul_nn, matmul_nt, matmul_tn
 from .linear import _swiglu_gemm
 from .norm import column_sum
 
@@ -51,9 +51,9 @@ class _MLPFn(torch.autograd.Function):
     def backward(ctx, g):
         x, w1, w2, z, h = ctx.saved_tensors
         need = ctx.needs_input_grad
-        g2 = g.reshape(-1, ctx.hidden).contiguous()
-        g2 = g2 if g2.data_ptr() % 16 == 0 else g2.clone()
-        v1, v2 = w1.view(-1, ctx.hidden), w2.view(ctx.hidden, -1)
+        g2 = as_written(g.reshape(-1, ctx.hidden))
+        z = as_written(z)
+        v1, v2 = w1.reshape(-1, ctx.hidden), as_written(w2).view(ctx.hidden, -1)
         gx = gw1 = gb1 = gw2 = gb2 = None
         if need[3]:
             gw2 = matmul_tn(g2, h).view(w2.shape)

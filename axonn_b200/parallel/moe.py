@@ -86,7 +86,7 @@ class _LocalRoute(torch.autograd.Function):
     @staticmethod
     @once_differentiable
     def backward(ctx, dgate, daux, *_):
-        logits, idx, gate, assigned = ctx.saved_tensors
+        logits, idx, gate, assigned = (t.contiguous() for t in ctx.saved_tensors)
         if dgate is None and daux is None:
             return None, None, None, None
         T, E = logits.shape

@@ -258,3 +258,45 @@ def test_mlp_module_routes():
         with torch.no_grad():
             assert _rel(m(x), y) < 2.0 ** -8
         assert ops.mlp(x[:, :1], m.fc1.weight, m.fc1.bias, m.fc2.weight, m.fc2.bias, 2048, 2048, act) is None
+
+
+@pytest.mark.parametrize("layout", ["gaps", "shifted"])
+@pytest.mark.parametrize("op", ["gelu", "swiglu", "experts", "loss", "route"])
+def test_saved_tensors_in_other_layouts(op, layout):
+    """Hooks on saved tensors give them back with gaps between the elements, or dense but 16 bytes off: the same gradients."""
+    from axonn_b200 import ops
+    from axonn_b200.parallel import moe
+
+    torch.manual_seed(0)
+
+    def leaf(*shape):
+        return (torch.randn(shape, device=DEV) * 0.05).bfloat16().requires_grad_(True)
+
+    if op in ("gelu", "swiglu"):
+        leaves = [leaf(4, 1024, 2048), leaf((2 if op == "swiglu" else 1) * 4096 * 2048), leaf(2048 * 4096)]
+        call = lambda: ops.mlp(leaves[0], leaves[1], None, leaves[2], None, 2048, 4096, op)  # noqa: E731
+    elif op == "experts":
+        leaves = [leaf(2, 4096, 64), leaf(2, 4096, 64), leaf(2, 64, 2048)]
+        call = lambda: ops.swiglu_experts(*leaves)  # noqa: E731
+    elif op == "loss":
+        leaves = [leaf(1, 4096, 64), leaf(4096 * 64)]
+        t = torch.randint(0, 4096, (1, 4096), device=DEV)
+        call = lambda: ops.projected_cross_entropy(*leaves, t, (4096, 64))  # noqa: E731
+    else:
+        leaves = [leaf(300, 8)]
+        call = lambda: (lambda g, a: (g * torch.arange(600, device=DEV).view(300, 2)).sum() + a)(  # noqa: E731
+            *moe._LocalRoute.apply(leaves[0], 2, 40, 64)[:2])
+
+    def unpack(t):
+        if layout == "gaps":
+            return torch.stack([t, t], -1)[..., 0]
+        buf = torch.empty(t.numel() + 16 // t.element_size(), dtype=t.dtype, device=t.device)
+        return buf[16 // t.element_size():].view(t.shape).copy_(t)
+
+    y = call()
+    dy = torch.randn_like(y)
+    want = torch.autograd.grad(y, leaves, dy)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach().clone(), unpack):
+        y = call()
+    for a, b in zip(torch.autograd.grad(y, leaves, dy), want):
+        assert torch.equal(a, b)
