@@ -73,6 +73,7 @@ class _CrossEntropyFn(torch.autograd.Function):
             _lib.check(_lib.lib().axb_ce_bwd(_lib.addr(z), _lib.addr(t), _lib.addr(lse), _lib.addr(scale),
                                              z.shape[0], V, ctx.start,
                                              ctx.ignore_index, _lib.stream()), "axb_ce_bwd")
+            torch.autograd.graph.increment_version(z)      # written through its address: a second backward has to notice
             return z.reshape(ctx.shape), None, None, None
         p = (z.float() - lse[:, None]).exp()
         loc = t - ctx.start
@@ -86,7 +87,7 @@ class _CrossEntropyFn(torch.autograd.Function):
 def cross_entropy(logits, targets, group=None, ignore_index=-100):
     """Mean token cross-entropy.  With ``group`` the last dimension of ``logits``
     is this rank's contiguous slice of the vocabulary (rank order = slice order).
-    On GPU the logits buffer is consumed: backward overwrites it with the gradient."""
+    On GPU the logits buffer is consumed: backward overwrites it with the gradient, and a second backward raises an error."""
     return _CrossEntropyFn.apply(logits, targets, group, ignore_index)
 
 
@@ -132,7 +133,8 @@ class _ProjectedCrossEntropyFn(torch.autograd.Function):
 
 def projected_cross_entropy(x, weight, targets, shape, ignore_index=-100):
     """Mean cross-entropy of the logits ``x[..., H] @ weight.T`` with ``weight`` holding ``shape = (V, H)``; ``None`` when the
-    projection is not one of those whose kernel has the statistics in its epilogue (few rows, other types)."""
+    projection is not one of those whose kernel has the statistics in its epilogue (few rows, other types).  As in
+    ``cross_entropy``, the backward overwrites the logits with their gradient, and a second one raises an error."""
     V, H = shape
     if (x.is_cuda and weight.is_cuda and targets.is_cuda and x.dtype == weight.dtype == torch.bfloat16 and V % 8 == 0 and H % 8 == 0
             and x.dim() > 0 and x.shape[-1] == H and weight.numel() == V * H and x.numel() > 0 and targets.dtype == torch.int64

@@ -300,3 +300,27 @@ def test_saved_tensors_in_other_layouts(op, layout):
         y = call()
     for a, b in zip(torch.autograd.grad(y, leaves, dy), want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("fused", [True, False])
+def test_logits_are_consumed(fused):
+    """The backward of the loss overwrites the logits, so that a second one is refused instead of taking gradients for
+    logits - unless hooks keep a copy of them."""
+    from axonn_b200 import ops
+
+    torch.manual_seed(0)
+    x, w = (torch.randn(4096, 64, device=DEV).bfloat16().requires_grad_(True) for _ in range(2))
+    t = torch.randint(0, 4096, (4096,), device=DEV)
+
+    def call():
+        return ops.projected_cross_entropy(x, w, t, (4096, 64)) if fused else ops.cross_entropy(ops.linear(x, w), t)
+
+    loss = call()
+    want = torch.autograd.grad(loss, [x, w], retain_graph=True)
+    with pytest.raises(RuntimeError, match="modified by an inplace"):
+        torch.autograd.grad(loss, [x, w])
+    with torch.autograd.graph.saved_tensors_hooks(lambda s: s.detach().clone(), lambda s: s.clone()):
+        loss = call()
+    for _ in range(2):
+        for a, b in zip(torch.autograd.grad(loss, [x, w], retain_graph=True), want):
+            assert torch.equal(a, b)
