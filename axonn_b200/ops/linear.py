@@ -2,6 +2,7 @@
 that are not tensor parallel (router, expert MLPs)."""
 
 import torch
+from torch.autograd.function import once_differentiable
 
 from . import _lib
 from .activation import swiglu
@@ -88,6 +89,7 @@ class _SwiGLUExpertsFn(torch.autograd.Function):
         return bmm_nt(h, w2, seg=seg, seg_rows=seg_rows)
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
         x, w1, w2, gu, h = ctx.saved_tensors
         seg = dict(seg=ctx.seg, seg_rows=ctx.seg_rows)

@@ -9,6 +9,7 @@ import ctypes
 
 import torch
 import torch.distributed as dist
+from torch.autograd.function import once_differentiable
 
 from . import _lib
 from .gemm import as_written, matmul_nn, matmul_tn
@@ -119,6 +120,7 @@ class _ProjectedCrossEntropyFn(torch.autograd.Function):
         return mean
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
         x, weight, z, t, lse, kept = ctx.saved_tensors
         z, t, lse = as_written(z), t.contiguous(), lse.contiguous()

@@ -1,6 +1,7 @@
 """Two-layer feed-forward block on one GPU as one autograd function, with the activation's adjoint in the GEMM before it."""
 
 import torch
+from torch.autograd.function import once_differentiable
 
 from . import _lib
 from .direct import no_graph
@@ -48,6 +49,7 @@ class _MLPFn(torch.autograd.Function):
         return y
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, g):
         x, w1, w2, z, h = ctx.saved_tensors
         need = ctx.needs_input_grad

@@ -324,3 +324,25 @@ def test_logits_are_consumed(fused):
     for _ in range(2):
         for a, b in zip(torch.autograd.grad(loss, [x, w], retain_graph=True), want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("op", ["gelu", "experts", "loss"])
+def test_second_derivatives_are_refused(op):
+    """... not left out: the fused backwards are kernels that no graph sees."""
+    from axonn_b200 import ops
+
+    def leaf(*shape):
+        return (torch.randn(shape, device=DEV) * 0.05).bfloat16().requires_grad_(True)
+
+    if op == "gelu":
+        leaves = [leaf(4096, 2048), leaf(4096 * 2048), leaf(2048 * 4096)]
+        y = ops.mlp(leaves[0], leaves[1], None, leaves[2], None, 2048, 4096, op)
+    elif op == "experts":
+        leaves = [leaf(2, 512, 64), leaf(2, 256, 64), leaf(2, 64, 128)]
+        y = ops.swiglu_experts(*leaves)
+    else:
+        leaves = [leaf(4096, 64), leaf(4096 * 64)]
+        y = ops.projected_cross_entropy(*leaves, torch.randint(0, 4096, (4096,), device=DEV), (4096, 64))
+    (g,) = torch.autograd.grad((y * y).sum(), leaves[-1], create_graph=True)
+    with pytest.raises(RuntimeError, match="once_differentiable"):
+        torch.autograd.grad(g.float().sum(), leaves[0])
