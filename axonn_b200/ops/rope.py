@@ -72,8 +72,11 @@ class _RopeFn(torch.autograd.Function):
 def apply_rope(x, table):
     """Rotate ``x`` (``[B, S, heads, D]`` or ``[B, S, groups, heads, D]``).  On GPU ``x``
     must be a non-leaf tensor (it is updated in place)."""
-    if no_graph(x, table):
-        if not x.is_inference():
+    inference = x.is_inference()
+    # outside inference mode an inference tensor may not be modified: the autograd function refuses it
+    if no_graph(x, table) and (not inference or torch.is_inference_mode_enabled()):
+        if not inference:
             torch.autograd.graph.increment_version(x)  # as any in-place operation does: x may be saved in a graph elsewhere
-        return _rope_apply(x, table, False)
+        out = _rope_apply(x, table, False)
+        return out.detach() if out.requires_grad else out      # the rotation is not in x's graph
     return _RopeFn.apply(x, table)

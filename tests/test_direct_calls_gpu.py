@@ -130,7 +130,13 @@ def test_rope_counts_as_in_place():
     with pytest.raises(RuntimeError, match="modified by an inplace"):
         z.sum().backward()
     with torch.inference_mode():
-        ops.apply_rope(torch.randn(1, 8, 2, 64, device=DEV, dtype=BF16), table)
+        kept = ops.apply_rope(torch.randn(1, 8, 2, 64, device=DEV, dtype=BF16), table)
+    with torch.no_grad(), pytest.raises(RuntimeError, match="inference"):
+        ops.apply_rope(kept, table)
+    y = x * 1
+    with torch.no_grad():
+        out = ops.apply_rope(y, table)               # rotated outside the graph, so it is not part of it
+    assert out.data_ptr() == y.data_ptr() and not out.requires_grad and out.grad_fn is None
 
 
 def test_embedding_rows():
