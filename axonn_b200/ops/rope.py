@@ -72,10 +72,9 @@ class _RopeFn(torch.autograd.Function):
 def apply_rope(x, table):
     """Rotate ``x`` (``[B, S, heads, D]`` or ``[B, S, groups, heads, D]``).  On GPU ``x``
     must be a non-leaf tensor (it is updated in place)."""
-    inference = x.is_inference()
     # outside inference mode an inference tensor may not be modified: the autograd function refuses it
-    if no_graph(x, table) and (not inference or torch.is_inference_mode_enabled()):
-        if not inference:
+    if no_graph(x, table) and (torch.is_inference_mode_enabled() or not x.is_inference()):
+        if not x.is_inference():
             torch.autograd.graph.increment_version(x)  # as any in-place operation does: x may be saved in a graph elsewhere
         out = _rope_apply(x, table, False)
         return out.detach() if out.requires_grad else out      # the rotation is not in x's graph
