@@ -61,8 +61,7 @@ def clip_grad_norm_(parameters, max_norm, norm_type=2.0, error_if_nonfinite=Fals
         else:
             plain.append(p.grad)
     all_grads = plain + [g for gs in by_group.values() for g in gs]
-    # a limit that is a tensor stays on its device: as a kernel argument it would have to be read by the host
-    if norm_type == 2.0 and not error_if_nonfinite and not torch.is_tensor(max_norm) and _one_table(all_grads) and all(
+    if norm_type == 2.0 and not error_if_nonfinite and _one_table(all_grads) and all(
             replicas == 1 and dist.get_world_size(group) == 1 for group, replicas in by_group):
         # nothing to reduce over ranks: norm and factor come from one kernel over all gradients
         total_norm, clip = ops.multi_tensor_clip_factor(all_grads, max_norm)
