@@ -128,6 +128,7 @@ class _ProjectedCrossEntropyFn(torch.autograd.Function):
         scale = (g.float() / kept).reshape(1).contiguous()
         _lib.check(_lib.lib().axb_ce_bwd(_lib.addr(z), _lib.addr(t), _lib.addr(lse), _lib.addr(scale), z.shape[0], V, 0,
                                          ctx.ignore_index, _lib.stream()), "axb_ce_bwd")
+        torch.autograd.graph.increment_version(z)
         gx = matmul_nn(z, weight.reshape(V, H)).view(x.shape) if ctx.needs_input_grad[0] else None
         gw = matmul_tn(z, x.reshape(-1, H)).view(weight.shape) if ctx.needs_input_grad[1] else None
         return gx, gw, None, None, None
