@@ -351,8 +351,12 @@ class Linear(torch.nn.Module):
         """``activation="gelu"`` fuses bias + GELU (tanh form) into the layer; only
         meaningful when the bias is added inside the layer (expert mode, no
         ``skip_bias_add``)."""
-        if self._takes_one_launch(x, activation):
-            return self._forward_direct(x, activation)
+        # a training step is asked nothing else (one B200, host-bound, forward of a 64 x 256 x 256 layer: 38 us if it is, 34 so)
+        w = self.weight
+        if not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)):
+            b = self.bias
+            if self._takes_one_launch(x, w, b, activation):
+                return self._forward_direct(x, w, b, activation)
         lead_shape = x.shape[:-1]
         x = x.reshape(-1, x.shape[-1])
         switch_layout = self._switches_layout
@@ -385,10 +389,9 @@ class Linear(torch.nn.Module):
         """Easy mode on a tensor-parallel grid: batch and channels change places between the ranks around the product."""
         return not self.expert_mode and self.inner_group_size * self.outer_group_size > 1
 
-    def _takes_one_launch(self, x, activation):
+    def _takes_one_launch(self, x, w, b, activation):
         """Is the layer one GEMM on ``x``, with no gradient and no collective around it?  Outside expert mode the outer group
         counts too: the general path gathers the batch over it and trades the feature shards for rows of the whole output."""
-        w, b = self.weight, self.bias
         if self._switches_layout or self.inner_group_size * self.depth_group_size != 1 or activation not in (None, "gelu"):
             return False
         if b is not None and (not self.expert_mode or self.skip_bias_add or b.dtype != w.dtype):
@@ -398,10 +401,9 @@ class Linear(torch.nn.Module):
                     or x.shape[-1] != k or w.shape != (n * k,) or x.numel() == 0 or not no_graph(x, w, b)
                     or not x.is_contiguous() or not w.is_contiguous() or torch.is_autocast_enabled("cuda"))
 
-    def _forward_direct(self, x, activation):
+    def _forward_direct(self, x, w, b, activation):
         """The layer as one GEMM launch.  One B200 (host-bound): 24 tokens through 2048 -> 8192 -> 2048 78 -> 31 us; the saved
         pre-activation of a GELU layer is not written either."""
-        w, b = self.weight, self.bias
         n, k = self.local_out_features, self.local_in_features
         out = x.new_empty(x.shape[:-1] + (n,))
         epilogue = (ops.EPI_NONE if b is None else ops.EPI_BIAS) if activation is None else (

@@ -171,22 +171,26 @@ class ParallelMLP(nn.Module):
                           init_method=lambda w: nn.init.normal_(w, std=out_init_std or init_std))
 
     def forward(self, x):
-        if torch.is_grad_enabled() and all(type(f) is Linear and f.expert_mode and not f.skip_bias_add and _is_plain_call(f, x)
-                                           for f in (self.fc1, self.fc2)):
-            y = ops.mlp(x, self.fc1.weight, self.fc1.bias, self.fc2.weight, self.fc2.bias, self.fc2.out_features,
-                        self.fc2.in_features, self.activation)
-            if y is not None:
-                return y
-        if self.activation == "swiglu":
-            f = self.fc1
-            # the cheap questions first: blocks of few rows are bound by host time (200 x 2048 x 4096 46 -> 53 us without them)
-            if (type(f) is Linear and not torch.is_grad_enabled() and x.is_cuda and x.numel() >= 512 * f.in_features
-                    and ops.gemm_on_pairs(x.numel() // f.in_features, f.out_features, x.device.index) and _is_plain_product(f, x)):
-                h = ops.swiglu_projection(x, f.weight, f.in_features)
+        fc1, fc2 = self.fc1, self.fc2
+        # the cheap questions first - what stands here, and whether a fused operation takes the sizes: blocks of few rows are
+        # bound by host time (one B200, forward of a training step, 64 x 256 x 1024: 103 us with all questions, 80 so)
+        if (torch.is_grad_enabled() or self.activation == "swiglu") and x.is_cuda and type(fc1) is Linear:
+            rows = x.numel() // max(fc1.in_features, 1)
+            if torch.is_grad_enabled():
+                if (type(fc2) is Linear and ops.mlp_takes(rows, fc2.out_features, fc2.in_features, self.activation, x.device.index)
+                        and all(f.expert_mode and not f.skip_bias_add and _is_plain_call(f, x) for f in (fc1, fc2))):
+                    y = ops.mlp(x, fc1.weight, fc1.bias, fc2.weight, fc2.bias, fc2.out_features, fc2.in_features, self.activation)
+                    if y is not None:
+                        return y
+            # from 512 rows (one B200, host-bound, hidden 1024, ffn 4096: 34 us against 43 from there on; below, the questions alone
+            # cost what the launch saves, 200 x 2048 x 4096 46 -> 53 us)
+            elif rows >= 512 and ops.gemm_on_pairs(rows, fc1.out_features, x.device.index) and _is_plain_product(fc1, x):
+                h = ops.swiglu_projection(x, fc1.weight, fc1.in_features)
                 if h is not None:
-                    return self.fc2(h)
-            return self.fc2(ops.swiglu(self.fc1(x)))
-        return self.fc2(self.fc1(x, activation="gelu"))
+                    return fc2(h)
+        if self.activation == "swiglu":
+            return fc2(ops.swiglu(fc1(x)))
+        return fc2(fc1(x, activation="gelu"))
 
 
 class TransformerBlock(nn.Module):
@@ -251,8 +255,11 @@ class ParallelLMHead(nn.Module):
     def forward(self, x, targets=None):
         if self.gather_group is not None:
             x = Gather.apply(x, self.gather_group, -1)
-        if targets is not None and _is_plain_product(self.proj, x):
-            loss = ops.projected_cross_entropy(x, self.proj.weight, targets, self.proj.local_weight_shape)
+        proj = self.proj
+        if (targets is not None and x.is_cuda and type(proj) is Linear
+                and ops.gemm_on_pairs(x.numel() // max(proj.in_features, 1), proj.out_features, x.device.index)
+                and _is_plain_product(proj, x)):
+            loss = ops.projected_cross_entropy(x, proj.weight, targets, proj.local_weight_shape)
             if loss is not None:
                 return loss
         logits = self.proj(x)

@@ -19,7 +19,7 @@ from .gemm import (  # noqa: F401
 )
 from .linear import linear, linear_batched, swiglu_experts  # noqa: F401
 from .loss import cross_entropy, projected_cross_entropy  # noqa: F401
-from .mlp import mlp, swiglu_projection  # noqa: F401
+from .mlp import mlp, mlp_takes, swiglu_projection  # noqa: F401
 from .multi_tensor import (  # noqa: F401
     all_reduce_bucketed_,
     multi_tensor_clip_factor,

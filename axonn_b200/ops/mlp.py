@@ -5,7 +5,7 @@ from torch.autograd.function import once_differentiable
 
 from . import _lib
 from .direct import no_graph
-from .gemm import EPI_BIAS, EPI_BIAS_GELU, EPI_GELU, EPI_NONE, as_written, matmul_nn, matmul_nt, matmul_tn
+from .gemm import EPI_BIAS, EPI_BIAS_GELU, EPI_GELU, EPI_NONE, as_written, gemm_on_pairs, matmul_nn, matmul_nt, matmul_tn
 from .linear import _swiglu_gemm
 from .norm import column_sum
 
@@ -73,6 +73,15 @@ class _MLPFn(torch.autograd.Function):
         return gx, gw1, gb1, gw2, gb2, None, None
 
 
+def mlp_takes(rows, hidden, ffn, act, device):
+    """Are the sizes ones for which ``mlp`` has its kernels?"""
+    # GELU: below this the gradient GEMM's main loop is shorter than the epilogue's arithmetic (16384 rows, ffn 4 * hidden:
+    # 1024 196 us against 187 for the GEMM and the pass after it, 2048 511 against 570)
+    if act == "gelu" and hidden < 2048:
+        return False
+    return gemm_on_pairs(rows, ffn, device) and (act == "gelu" or gemm_on_pairs(rows, 2 * ffn, device))
+
+
 def mlp(x, w1, b1, w2, b2, hidden, ffn, act):
     """The block for a training step (``w1`` holds ``[ffn, hidden]``, ``[2 * ffn, hidden]`` with SwiGLU; ``w2`` ``[hidden, ffn]``;
     flat tensors are fine), or ``None`` where its kernels do not apply: other types, few rows, no gradient needed."""
@@ -84,12 +93,7 @@ def mlp(x, w1, b1, w2, b2, hidden, ffn, act):
             or x.dim() == 0 or x.shape[-1] != hidden or x.numel() == 0 or hidden % 64 or ffn % 16
             or w1.numel() != wide * hidden or w2.numel() != ffn * hidden):
         return None
-    # GELU: below this the gradient GEMM's main loop is shorter than the epilogue's arithmetic (16384 rows, ffn 4 * hidden:
-    # 1024 196 us against 187 for the GEMM and the pass after it, 2048 511 against 570)
-    if act == "gelu" and hidden < 2048:
-        return None
-    L, rows, dev = _lib.lib(), x.numel() // hidden, x.device.index
-    if not L.axb_gemm_on_pairs(rows, ffn, dev) or (act == "swiglu" and not L.axb_gemm_on_pairs(rows, wide, dev)):
+    if not mlp_takes(x.numel() // hidden, hidden, ffn, act, x.device.index):
         return None
     return _MLPFn.apply(x, w1, b1, w2, b2, hidden, act)
 
@@ -104,7 +108,7 @@ def swiglu_projection(x, w1, hidden):
             and x.data_ptr() % 16 == 0 and w1.data_ptr() % 16 == 0):
         return None
     rows, wide = x.numel() // hidden, w1.numel() // hidden
-    if not _lib.lib().axb_gemm_on_pairs(rows, wide, x.device.index):
+    if not gemm_on_pairs(rows, wide, x.device.index):
         return None
     h = x.new_empty(x.shape[:-1] + (wide // 2,))
     return _swiglu_gemm(False, x.view(1, rows, hidden), w1.view(1, wide, hidden), h, None, None, 0)

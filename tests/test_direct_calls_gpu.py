@@ -229,3 +229,21 @@ def test_replaced_forwards(monkeypatch):
     assert len(seen) == 1 + 2 * 3
     monkeypatch.undo()
     assert all(plain_layer(layer) for layer in (e, m.fc1, m.fc2, head.proj))
+
+
+def test_small_training_steps_are_not_asked(monkeypatch):
+    """Blocks of few rows are bound by host time: in a training step they do not go through the questions of the fused
+    operations, which could not take them."""
+    from axonn_b200.intra_layer import fully_connected
+    from axonn_b200.models import blocks
+
+    def asked(*_):
+        raise AssertionError("asked")
+
+    monkeypatch.setattr(blocks, "plain_layer", asked)
+    monkeypatch.setattr(blocks, "plain_tensors", asked)
+    monkeypatch.setattr(fully_connected, "no_graph", asked)
+    x, t = torch.randn(1, 64, 256, device=DEV, dtype=BF16, requires_grad=True), torch.randint(0, 512, (1, 64), device=DEV)
+    for act in ("gelu", "swiglu"):
+        blocks.ParallelMLP(256, 1024, act, bias=act == "gelu", dtype=BF16)(x)
+    blocks.ParallelLMHead(256, 512, dtype=BF16)(x, t)
