@@ -40,6 +40,7 @@ int axb_gemm_swiglu(int backward, const void* A, const void* B, void* out, void*
 int axb_gemm_on_pairs(int M, int N, int device);
 int axb_gemm_dgelu(const void* A, const void* B, void* dz, const void* z, float* part, int M, int N, int K, int device, void* stream);
 int axb_fold_columns(const float* part, void* out, int rows, int N, int out_dtype, void* stream);
+int axb_gemm_ce_pays(int M, int N, int K, int device);
 int axb_gemm_ce(const void* A, const void* B, void* logits, void* part, int M, int N, int K, int device, void* stream);
 int axb_ce_fwd_parts(const void* part, const void* logits, const long long* targets, float* stats, float* lse, float* mean,
                      float* kept, int rows, int V, long long ignore_index, void* stream);

@@ -2352,6 +2352,23 @@ extern "C" int axb_gemm_dgelu(const void* A, const void* B, void* dz, const void
 // that run on CTA pairs, which have this epilogue?  One B200, 4096 x 50304, hidden 2048: the product takes no longer than
 // without, and the pass over the logits (84 us) becomes one over the parts (11 us); loss with its gradients 2295 -> 2238 us.
 extern "C" int axb_gemm_on_pairs(int M, int N, int device) { return M > 0 && N > 0 && axb::plain_on_pairs(M, N, device); }
+// Do the statistics in the epilogue (with a kernel over the parts) take less time than the plain product and a pass over the
+// logits (axb_gemm, axb_ce_fwd_mean)?  They keep tiles whole where the plain product halves those of a small last wave, the kernel
+// over the parts has a block for 32 rows and walks V / 2048 parts in each warp, and four epilogue warps take longer than the main
+// loop of a small K.  One B200, loss with its mean, epilogue / pass, over K 64 .. 4096:
+//   2048 rows and more 0.45 - 1.02 (4096 x 50304 x 2048 572 / 664 us), but 2048 x 2560 x 4096 (1.1 waves, the last in halves) 51.1 / 48.0;
+//   1024 .. 2047 rows, K >= 512, last wave not in halves or 4 waves and more 0.86 - 1.01 (1024 x 32000 x 1024 57.8 / 63.7), with fewer
+//     waves 0.98 - 1.15 (1024 x 4864 x 4096 52.2 / 45.5), K < 512 0.84 - 1.06 (1100 x 50304 x 64 64.9 / 61.1);
+//   768 .. 1023 rows, 7 waves and more 0.88 - 0.98 (768 x 50304 x 1024 67.8 / 77.1), fewer 0.96 - 1.07 (768 x 14000 x 2048 47.1 / 45.3);
+//   fewer rows 0.95 - 1.22 (300 x 32000 x 128 25.6 / 21.7).
+extern "C" int axb_gemm_ce_pays(int M, int N, int K, int device) {
+  const int pairs = axb::usable_sms(device) / 2;
+  const long long tiles = (static_cast<long long>(M) + 255) / 256 * ((static_cast<long long>(N) + 255) / 256);
+  const bool halved = axb::pair_whole_tiles(tiles, pairs) != tiles;
+  if (M >= 2048) return !(halved && tiles < 2ll * pairs && K > 2048);
+  if (M < 768 || K < 512) return 0;
+  return tiles >= 7ll * pairs || (M >= 1024 && (!halved || tiles >= 4ll * pairs));
+}
 extern "C" int axb_gemm_ce(const void* A, const void* B, void* logits, void* part, int M, int N, int K, int device, void* stream) {
   using namespace axb;
   if ((reinterpret_cast<uintptr_t>(logits) & 15) || (reinterpret_cast<uintptr_t>(part) & 7)) {

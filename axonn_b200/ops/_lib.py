@@ -42,6 +42,7 @@ _SIGNATURES = {
     "axb_gemm_on_pairs": "iii",
     "axb_gemm_dgelu": "ppppp" "iiii" "p",
     "axb_fold_columns": "pp" "iii" "p",
+    "axb_gemm_ce_pays": "iiii",
     "axb_gemm_ce": "pppp" "iiii" "p",
     "axb_ce_fwd_parts": "ppppppp" "ii" "l" "p",
     "axb_norm_fwd": "ppppp" "iii" "f" "iiii" "p",

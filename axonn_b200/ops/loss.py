@@ -12,7 +12,7 @@ import torch.distributed as dist
 from torch.autograd.function import once_differentiable
 
 from . import _lib
-from .gemm import as_written, matmul_nn, matmul_tn
+from .gemm import as_written, matmul_nn, matmul_nt, matmul_tn
 
 
 class _CrossEntropyFn(torch.autograd.Function):
@@ -92,9 +92,13 @@ def cross_entropy(logits, targets, group=None, ignore_index=-100):
     return _CrossEntropyFn.apply(logits, targets, group, ignore_index)
 
 
+def _statistics_in_epilogue(rows, V, H, device):
+    return bool(_lib.lib().axb_gemm_ce_pays(rows, V, H, device))
+
+
 class _ProjectedCrossEntropyFn(torch.autograd.Function):
-    """``cross_entropy(x @ w.T, targets)`` whose softmax statistics come from the epilogue of the projection: the logits are
-    written once, read and overwritten by their gradient once, and read by the two GEMMs of the backward."""
+    """``cross_entropy(x @ w.T, targets)``; the softmax statistics come from the epilogue of the projection where that is faster,
+    so that the logits are written once, read and overwritten by their gradient once, and read by the two GEMMs of the backward."""
 
     @staticmethod
     def forward(ctx, x, weight, targets, shape, ignore_index):
@@ -103,17 +107,23 @@ class _ProjectedCrossEntropyFn(torch.autograd.Function):
         t = targets.reshape(-1).contiguous()
         rows = x2.shape[0]
         dev = x.device
-        z = torch.empty((rows, V), dtype=x.dtype, device=dev)
-        part = torch.empty(((V + 255) // 256, rows, 2), dtype=torch.float32, device=dev)
         L = _lib.lib()
-        _lib.check(L.axb_gemm_ce(_lib.addr(x2), _lib.addr(weight), _lib.addr(z), _lib.addr(part), rows, V, H, dev.index,
-                                 _lib.stream()), "axb_gemm_ce")
         stats = torch.empty((rows, 3), dtype=torch.float32, device=dev)
         lse = torch.empty(rows, dtype=torch.float32, device=dev)
         # two tensors: the loss is returned, and a view made in here could not be modified in place later
         mean, kept = (torch.empty((), dtype=torch.float32, device=dev) for _ in range(2))
-        _lib.check(L.axb_ce_fwd_parts(_lib.addr(part), _lib.addr(z), _lib.addr(t), _lib.addr(stats), _lib.addr(lse),
-                                      _lib.addr(mean), _lib.addr(kept), rows, V, ignore_index, _lib.stream()), "axb_ce_fwd_parts")
+        if _statistics_in_epilogue(rows, V, H, dev.index):
+            z = torch.empty((rows, V), dtype=x.dtype, device=dev)
+            part = torch.empty(((V + 255) // 256, rows, 2), dtype=torch.float32, device=dev)
+            _lib.check(L.axb_gemm_ce(_lib.addr(x2), _lib.addr(weight), _lib.addr(z), _lib.addr(part), rows, V, H, dev.index,
+                                     _lib.stream()), "axb_gemm_ce")
+            _lib.check(L.axb_ce_fwd_parts(_lib.addr(part), _lib.addr(z), _lib.addr(t), _lib.addr(stats), _lib.addr(lse),
+                                          _lib.addr(mean), _lib.addr(kept), rows, V, ignore_index, _lib.stream()),
+                       "axb_ce_fwd_parts")
+        else:
+            z = matmul_nt(x2, weight.view(V, H))
+            _lib.check(L.axb_ce_fwd_mean(_lib.addr(z), _lib.addr(t), _lib.addr(stats), _lib.addr(lse), _lib.addr(mean),
+                                         _lib.addr(kept), rows, V, ignore_index, _lib.stream()), "axb_ce_fwd_mean")
         _lib.add_launches(1)
         ctx.save_for_backward(x, weight, z, t, lse, kept)
         ctx.shape, ctx.ignore_index = shape, ignore_index

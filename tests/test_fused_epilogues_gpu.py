@@ -111,21 +111,23 @@ def test_swiglu_experts(E, rows, hidden, ffn, counts, in_gemm, monkeypatch):
             assert bool(torch.isfinite(g[e]).all()) and _rel(g[e], w[e]) < 5 * 2.0 ** -9
 
 
+@pytest.mark.parametrize("in_gemm", [True, False])
 @pytest.mark.parametrize("T,H,V", [(2048, 256, 4104), (1031, 264, 12808), (300, 64, 40000), (4096, 128, 50304)])
-def test_projected_cross_entropy(T, H, V):
-    """Projection and loss in one: a vocabulary that ends inside a chunk of 32 and inside a tile, rows that are no multiple of
+def test_projected_cross_entropy(T, H, V, in_gemm, monkeypatch):
+    """Projection and loss in one, statistics in the epilogue or in a pass of their own: a vocabulary that ends inside a chunk of 32 and inside a tile, rows that are no multiple of
     anything, ignored and out-of-range targets, a row of -inf logits' neighbours.  The logits are bf16, so the loss is
     compared with the unfused operations on the same product (fp32 sums: 1e-5) and the gradients with 64 bits (2^-8)."""
     from axonn_b200 import ops
     from axonn_b200.ops import _lib
 
     assert _lib.lib().axb_gemm_on_pairs(T, V, 0)
+    monkeypatch.setattr(sys.modules["axonn_b200.ops.loss"], "_statistics_in_epilogue", lambda *_: in_gemm)
     torch.manual_seed(T)
     x = torch.randn(1, T, H, device=DEV).bfloat16().requires_grad_(True)
     w = (torch.randn(V * H, device=DEV) * 0.2).bfloat16().requires_grad_(True)
     t = torch.randint(0, V, (1, T), device=DEV)
     t[0, ::7] = -100
-    t[0, 1], t[0, 2] = V - 1, 0
+    t[0, 1], t[0, 2], t[0, 3], t[0, 4], t[0, 5] = V - 1, 0, V, V + 5, -1
     loss = ops.projected_cross_entropy(x, w, t, (V, H))
     ref = ops.cross_entropy(ops.matmul_nt(x.detach()[0], w.detach().view(V, H)), t)
     assert abs(float(loss.detach()) - float(ref)) <= 1e-5 * abs(float(ref))
@@ -133,16 +135,20 @@ def test_projected_cross_entropy(T, H, V):
     x64, w64 = x.detach().double().requires_grad_(True), w.detach().double().requires_grad_(True)
     z = x64[0] @ w64.view(V, H).t()
     z = z + (z.detach().float().bfloat16().double() - z.detach())
-    want = torch.autograd.grad(3 * torch.nn.functional.cross_entropy(z, t[0]), [x64, w64])
+    # a target outside the vocabulary has the loss of a target whose logit is zero, and counts
+    kept, inside = t[0] != -100, (t[0] >= 0) & (t[0] < V)
+    own = z.gather(1, torch.where(inside, t[0], 0)[:, None])[:, 0] * inside
+    want = torch.autograd.grad(3 * ((z.logsumexp(1) - own) * kept).sum() / kept.sum(), [x64, w64])
     for a, b in zip(got, want):
         assert a.shape == b.shape and _rel(a, b) < 2.0 ** -8
     assert _lib.device_status() == 0
 
 
-def test_projected_cross_entropy_odd_rows():
+def test_projected_cross_entropy_odd_rows(monkeypatch):
     """All logits of a row -inf: a NaN loss, as without fusion; a NaN input reaches the loss; -inf in single columns."""
     from axonn_b200 import ops
 
+    monkeypatch.setattr(sys.modules["axonn_b200.ops.loss"], "_statistics_in_epilogue", lambda *_: True)
     T, H, V = 512, 64, 12800
     for kind in ("inf", "nan", "columns"):
         x, w = torch.ones(1, T, H, device=DEV).bfloat16(), torch.zeros(V, H, device=DEV).bfloat16()
