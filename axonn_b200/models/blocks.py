@@ -256,13 +256,14 @@ class ParallelLMHead(nn.Module):
         if self.gather_group is not None:
             x = Gather.apply(x, self.gather_group, -1)
         proj = self.proj
-        if (targets is not None and x.is_cuda and type(proj) is Linear
-                and ops.gemm_on_pairs(x.numel() // max(proj.in_features, 1), proj.out_features, x.device.index)
-                and _is_plain_product(proj, x)):
-            loss = ops.projected_cross_entropy(x, proj.weight, targets, proj.local_weight_shape)
+        if targets is not None and x.is_cuda and type(proj) is Linear:
+            rows = x.numel() // max(proj.in_features, 1)
+            fused = (rows * proj.out_features >= 1 << 20 and ops.gemm_on_pairs(rows, proj.out_features, x.device.index)
+                     and _is_plain_product(proj, x))
+            loss = ops.projected_cross_entropy(x, proj.weight, targets, proj.local_weight_shape) if fused else None
             if loss is not None:
                 return loss
-        logits = self.proj(x)
+        logits = proj(x)
         if targets is None:
             return logits
         return ops.cross_entropy(logits, targets, group=self.group)

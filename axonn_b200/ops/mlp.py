@@ -90,13 +90,13 @@ class _MLPFn(torch.autograd.Function):
 
 
 def mlp_takes(rows, hidden, ffn, act, device):
-    """Are the sizes ones for which ``mlp`` has its kernels?"""
+    """Are the sizes ones for which ``mlp`` has its kernels?  (Few elements are turned away without asking the library.)"""
     # GELU: below this the gradient GEMM's main loop is shorter than the epilogue's arithmetic.  One B200, ffn 4 * hidden, with the
     # adjoint in the GEMM / after it, 4096 and 16384 rows: hidden 1024 53.3 / 46.1 and 175 / 162 us, 1280 68.3 / 61.8 and 227 / 226,
     # 1536 82.9 / 81.6 and 290 / 300, 1792 100 / 103 and 365 / 385, 2048 117 / 126 and 445 / 488
     if act == "gelu" and hidden < 2048:
         return False
-    return gemm_on_pairs(rows, ffn, device) and (act == "gelu" or gemm_on_pairs(rows, 2 * ffn, device))
+    return rows * ffn >= 1 << 20 and gemm_on_pairs(rows, ffn, device) and (act == "gelu" or gemm_on_pairs(rows, 2 * ffn, device))
 
 
 def mlp(x, w1, b1, w2, b2, hidden, ffn, act):
