@@ -2359,14 +2359,15 @@ extern "C" int axb_gemm_on_pairs(int M, int N, int device) { return M > 0 && N >
 //   2048 rows and more 0.45 - 1.02 (4096 x 50304 x 2048 572 / 664 us), but 2048 x 2560 x 4096 (1.1 waves, the last in halves) 51.1 / 48.0;
 //   1024 .. 2047 rows, K >= 512, last wave not in halves or 4 waves and more 0.86 - 1.01 (1024 x 32000 x 1024 57.8 / 63.7), with fewer
 //     waves 0.98 - 1.15 (1024 x 4864 x 4096 52.2 / 45.5), K < 512 0.84 - 1.06 (1100 x 50304 x 64 64.9 / 61.1);
-//   768 .. 1023 rows, 7 waves and more 0.88 - 0.98 (768 x 50304 x 1024 67.8 / 77.1), fewer 0.96 - 1.07 (768 x 14000 x 2048 47.1 / 45.3);
+//   513 .. 1023 rows, 7 waves and more 0.88 - 0.98 (768 x 50304 x 1024 67.8 / 77.1), fewer 0.96 - 1.07 (768 x 14000 x 2048 47.1 / 45.3);
 //   fewer rows 0.95 - 1.22 (300 x 32000 x 128 25.6 / 21.7).
+// The head called as a layer, forward and backward, is bound by the host below some 200 us and 1 % apart there.
 extern "C" int axb_gemm_ce_pays(int M, int N, int K, int device) {
   const int pairs = axb::usable_sms(device) / 2;
   const long long tiles = (static_cast<long long>(M) + 255) / 256 * ((static_cast<long long>(N) + 255) / 256);
   const bool halved = axb::pair_whole_tiles(tiles, pairs) != tiles;
   if (M >= 2048) return !(halved && tiles < 2ll * pairs && K > 2048);
-  if (M < 768 || K < 512) return 0;
+  if (M <= 512 || K < 512) return 0;
   return tiles >= 7ll * pairs || (M >= 1024 && (!halved || tiles >= 4ll * pairs));
 }
 extern "C" int axb_gemm_ce(const void* A, const void* B, void* logits, void* part, int M, int N, int K, int device, void* stream) {

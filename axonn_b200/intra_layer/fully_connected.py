@@ -353,11 +353,13 @@ class Linear(torch.nn.Module):
         ``skip_bias_add``)."""
         # a training step is asked nothing else (one B200, host-bound, forward of a 64 x 256 x 256 layer: 38 us if it is, 34 so)
         w, bias = self.weight, self.bias
-        if not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)) and self._takes_one_launch(x, w, bias, activation):
-            return self._forward_direct(x, w, bias, activation)
+        if not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad)):
+            y = self._forward_direct(x, w, bias, activation)
+            if y is not None:
+                return y
         lead_shape = x.shape[:-1]
         x = x.reshape(-1, x.shape[-1])
-        switch_layout = self._switches_layout
+        switch_layout = (not self.expert_mode) and self.inner_group_size * self.outer_group_size > 1
         if switch_layout:
             inner_sizes = gather_batch_sizes(x.shape[0], self.inner_group, device=x.device)
             x = GatherBatchScatterChannels.apply(x, inner_sizes, self.inner_group)
@@ -381,27 +383,21 @@ class Linear(torch.nn.Module):
             return x, bias
         return x + bias.to(x.dtype)
 
-    @property
-    def _switches_layout(self):
-        """Easy mode on a tensor-parallel grid: batch and channels change places between the ranks around the product."""
-        return not self.expert_mode and self.inner_group_size * self.outer_group_size > 1
-
-    def _takes_one_launch(self, x, w, b, activation):
-        """Is the layer one GEMM on ``x``, with no gradient and no collective around it?  Outside expert mode the outer group
-        counts too: the general path gathers the batch over it and trades the feature shards for rows of the whole output."""
-        if self._switches_layout or self.inner_group_size * self.depth_group_size != 1 or activation not in (None, "gelu"):
-            return False
-        if b is not None and (not self.expert_mode or self.skip_bias_add or b.dtype != w.dtype):
-            return False
-        n, k = self.local_out_features, self.local_in_features
-        return not (n % 8 or k % 8 or x.dtype != w.dtype or w.dtype not in (torch.bfloat16, torch.float16) or x.dim() == 0
-                    or x.shape[-1] != k or w.shape != (n * k,) or x.numel() == 0 or not no_graph(x, w, b)
-                    or not x.is_contiguous() or not w.is_contiguous() or torch.is_autocast_enabled("cuda"))
-
     def _forward_direct(self, x, w, b, activation):
-        """The layer as one GEMM launch.  One B200 (host-bound): 24 tokens through 2048 -> 8192 -> 2048 78 -> 31 us; the saved
+        """The layer as one GEMM launch, when it needs no gradient and no collective; ``None`` when the general path has to
+        run.  Outside expert mode the outer group counts too: the general path gathers the batch over it and trades the feature
+        shards for rows of the whole output.  One B200 (host-bound): 24 tokens through 2048 -> 8192 -> 2048 78 -> 31 us; the saved
         pre-activation of a GELU layer is not written either."""
+        if (self.inner_group_size * self.depth_group_size != 1 or (self.outer_group_size != 1 and not self.expert_mode)
+                or (activation is not None and activation != "gelu")):
+            return None
+        if b is not None and (not self.expert_mode or self.skip_bias_add or b.dtype != w.dtype):
+            return None
         n, k = self.local_out_features, self.local_in_features
+        if (n % 8 or k % 8 or x.dtype != w.dtype or w.dtype not in (torch.bfloat16, torch.float16) or x.dim() == 0
+                or x.shape[-1] != k or w.shape != (n * k,) or x.numel() == 0 or not no_graph(x, w, b)
+                or not x.is_contiguous() or not w.is_contiguous() or torch.is_autocast_enabled("cuda")):
+            return None
         out = x.new_empty(x.shape[:-1] + (n,))
         epilogue = (ops.EPI_NONE if b is None else ops.EPI_BIAS) if activation is None else (
             ops.EPI_GELU if b is None else ops.EPI_BIAS_GELU)

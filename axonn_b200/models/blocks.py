@@ -258,8 +258,7 @@ class ParallelLMHead(nn.Module):
         proj = self.proj
         if targets is not None and x.is_cuda and type(proj) is Linear:
             rows = x.numel() // max(proj.in_features, 1)
-            fused = (rows * proj.out_features >= 1 << 20 and ops.gemm_on_pairs(rows, proj.out_features, x.device.index)
-                     and _is_plain_product(proj, x))
+            fused = ops.gemm_on_pairs(rows, proj.out_features, x.device.index) and _is_plain_product(proj, x)
             loss = ops.projected_cross_entropy(x, proj.weight, targets, proj.local_weight_shape) if fused else None
             if loss is not None:
                 return loss

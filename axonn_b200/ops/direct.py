@@ -14,12 +14,14 @@ _own_forward = {}
 
 def no_graph(*tensors) -> bool:
     """No gradient can be asked of an operation on ``tensors`` (``None`` entries are skipped) and nothing looks at it from
-    outside: grad mode is off or none of them requires a gradient, and they are ``plain_tensors``."""
-    if torch.is_grad_enabled():
-        for t in tensors:
-            if t is not None and t.requires_grad:
-                return False
-    return plain_tensors(*tensors)
+    outside: grad mode is off or none of them requires a gradient, and they are ``plain_tensors`` (written out here: a call
+    costs 0.4 us, in each of the twenty operations of a small model)."""
+    grad = torch.is_grad_enabled()
+    for t in tensors:
+        if t is not None and (type(t) not in _PLAIN or not t.is_cuda or (grad and t.requires_grad)):
+            return False
+    return (not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None
+            and forward_ad._current_level < 0 and not torch.compiler.is_compiling())
 
 
 def plain_tensors(*tensors) -> bool:
