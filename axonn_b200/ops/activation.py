@@ -96,29 +96,24 @@ class _SwiGLUFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         (gu,) = ctx.saved_tensors
-        return swiglu_backward(dout, gu)
-
-
-def swiglu_backward(dout, gu):
-    """Gradient of ``swiglu(gu)`` by ``gu``."""
-    F2 = gu.shape[-1]
-    Fh = F2 // 2
-    if gu.is_cuda:
-        g2 = gu.reshape(-1, F2).contiguous()
-        d2 = dout.reshape(-1, Fh).contiguous()
-        dgu = torch.empty_like(g2)
-        _lib.check(_lib.lib().axb_swiglu_bwd(_lib.addr(d2), _lib.addr(g2), _lib.addr(dgu),
-                                             g2.shape[0], Fh,
-                                             _lib.stream()), "axb_swiglu_bwd")
-        return dgu.reshape(gu.shape)
-    g, u = (t.float() for t in _split_gu(gu))
-    s = torch.sigmoid(g)
-    silu = g * s
-    d = dout.float()
-    dg, du = d * u * (s + silu * (1 - s)), d * silu
-    lead = gu.shape[:-1]
-    out = torch.stack([dg.reshape(*lead, Fh // 8, 8), du.reshape(*lead, Fh // 8, 8)], -2)
-    return out.reshape(gu.shape).to(gu.dtype)
+        F2 = gu.shape[-1]
+        Fh = F2 // 2
+        if gu.is_cuda:
+            g2 = gu.reshape(-1, F2).contiguous()
+            d2 = dout.reshape(-1, Fh).contiguous()
+            dgu = torch.empty_like(g2)
+            _lib.check(_lib.lib().axb_swiglu_bwd(_lib.addr(d2), _lib.addr(g2), _lib.addr(dgu),
+                                                 g2.shape[0], Fh,
+                                                 _lib.stream()), "axb_swiglu_bwd")
+            return dgu.reshape(gu.shape)
+        g, u = (t.float() for t in _split_gu(gu))
+        s = torch.sigmoid(g)
+        silu = g * s
+        d = dout.float()
+        dg, du = d * u * (s + silu * (1 - s)), d * silu
+        lead = gu.shape[:-1]
+        out = torch.stack([dg.reshape(*lead, Fh // 8, 8), du.reshape(*lead, Fh // 8, 8)], -2)
+        return out.reshape(gu.shape).to(gu.dtype)
 
 
 def _split_gu(gu):

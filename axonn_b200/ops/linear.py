@@ -5,7 +5,7 @@ import torch
 from torch.autograd.function import once_differentiable
 
 from . import _lib
-from .activation import swiglu, swiglu_backward
+from .activation import swiglu
 from .gemm import as_written, bmm_nn, bmm_nt, bmm_tn, matmul_nn, matmul_nt, matmul_tn
 
 
@@ -75,16 +75,6 @@ def _swiglu_gemm(backward, a, b, out, saved, seg, seg_rows):
     return out
 
 
-def swiglu_adjoint_in_gemm(rows, hidden, ffn, single):
-    """Is the gradient GEMM with SwiGLU's adjoint in its epilogue faster than the product and the pass after it (``rows`` of all
-    problems)?  The epilogue costs a tile of 256 columns however few of them there are, and that of the last tiles is not hidden
-    behind a main loop.  One B200, fused / separate, from 16 M elements on 0.69 - 0.98 (8 experts of 2560 rows, hidden 2048, ffn 8192
-    483 / 696 us).  Below, hidden 2048 and more 0.83 - 1.04; one block whose ffn fills its tiles 0.86 - 0.99 (8192 x 1024, hidden 256
-    20.8 / 22.5); others up to 1.16 (16384 x 320, hidden 384 20.6 / 17.7) and as experts 1.25 (8 of 128 rows, hidden 64, ffn 256
-    11.4 / 9.1; of 320 rows, hidden 512, ffn 2048 22.0 / 19.8)."""
-    return hidden >= 2048 or rows * ffn >= 1 << 24 or (single and ffn % 256 == 0)
-
-
 class _SwiGLUExpertsFn(torch.autograd.Function):
     """``swiglu(x @ w1.T) @ w2.T`` per expert with the activation and its adjoint in the epilogues of the GEMMs around them:
     the gated product is written once and read once, the activation's gradient is never stored."""
@@ -107,12 +97,7 @@ class _SwiGLUExpertsFn(torch.autograd.Function):
         gx = gw1 = gw2 = None
         if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
             gu = as_written(gu)
-            E, rows, hidden = g.shape
-            if swiglu_adjoint_in_gemm(E * rows, hidden, w2.shape[2], False):
-                dgu = _swiglu_gemm(True, g, as_written(w2), torch.empty_like(gu), gu, **seg)
-            else:
-                # rows of tiles without data are unwritten in gu, and here as well: nothing below reads them
-                dgu = swiglu_backward(bmm_nn(g, w2, **seg), gu)
+            dgu = _swiglu_gemm(True, g, as_written(w2), torch.empty_like(gu), gu, **seg)
             gx = bmm_nn(dgu, w1, **seg) if ctx.needs_input_grad[0] else None
             gw1 = bmm_tn(dgu, x, out_dtype=w1.dtype, **seg) if ctx.needs_input_grad[1] else None
         if ctx.needs_input_grad[2]:

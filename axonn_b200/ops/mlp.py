@@ -4,10 +4,10 @@ import torch
 from torch.autograd.function import once_differentiable
 
 from . import _lib
-from .activation import gelu_backward, gelu_backward_colsum, swiglu_backward
+from .activation import gelu_backward, gelu_backward_colsum
 from .direct import no_graph
 from .gemm import EPI_BIAS, EPI_BIAS_GELU, EPI_GELU, EPI_NONE, as_written, gemm_on_pairs, matmul_nn, matmul_nt, matmul_tn
-from .linear import _swiglu_gemm, swiglu_adjoint_in_gemm
+from .linear import _swiglu_gemm
 from .norm import column_sum
 
 _OUT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
@@ -72,9 +72,7 @@ class _MLPFn(torch.autograd.Function):
         if ctx.b2 is not None and need[4]:
             gb2 = column_sum(g2, out_dtype=ctx.b2)
         if need[0] or need[1] or need[2]:
-            if ctx.act == "swiglu" and not swiglu_adjoint_in_gemm(g2.shape[0], ctx.hidden, v2.shape[1], True):
-                dz = swiglu_backward(matmul_nn(g2, v2), z)
-            elif ctx.act == "swiglu":
+            if ctx.act == "swiglu":
                 dz = _swiglu_gemm(True, g2[None], v2[None], torch.empty_like(z), z, None, 0)
             elif _gelu_adjoint_in_gemm(z.shape[0], ctx.hidden, z.shape[1]):
                 dz, gb1 = _dgelu_gemm(g2, v2, z, ctx.b1 if ctx.b1 is not None and need[2] else None)

@@ -69,18 +69,16 @@ def test_gemm_halved_tiles(layout, M, N, K, dtype):
         assert _rel(out, torch.nn.functional.gelu(z + bias.double(), approximate="tanh")) < tol
 
 
-@pytest.mark.parametrize("in_gemm", [True, False])
 @pytest.mark.parametrize("E,rows,hidden,ffn,counts", [(1, 64, 64, 32, None), (3, 192, 128, 96, [[0], [64], [191]]), (2, 640, 192, 160, [[1], [500]]),
                                                       (2, 512, 256, 288, [[70, 0], [256, 3]]), (8, 2560, 512, 1024, None)])
-def test_swiglu_experts(E, rows, hidden, ffn, counts, in_gemm, monkeypatch):
-    """Gated feed-forward layers with the activation in the GEMMs, its adjoint too or after them: tiles with and without data rows, N that ends inside a
+def test_swiglu_experts(E, rows, hidden, ffn, counts):
+    """Gated feed-forward layers with the activation in the GEMMs: tiles with and without data rows, N that ends inside a
     chunk, one segment and two, against the layer in 64 bits.  Memory that no kernel writes holds NaN, so that reading a
     row without data would show.  Tolerance: the stored product, the activation and its gradient are rounded to bf16 (three
     roundings of 2^-9 forward, five backward)."""
     from axonn_b200 import ops
     from axonn_b200.ops import _lib
 
-    monkeypatch.setattr(sys.modules["axonn_b200.ops.linear"], "swiglu_adjoint_in_gemm", lambda *_: in_gemm)
     torch.manual_seed(rows)
     x = torch.randn(E, rows, hidden, device=DEV).bfloat16()
     w1 = (torch.randn(E, 2 * ffn, hidden, device=DEV) * hidden ** -0.5).bfloat16().requires_grad_(True)
@@ -208,7 +206,6 @@ def test_mlp_function(act, bias, rows, hidden, ffn, in_gemm, monkeypatch):
     from axonn_b200.ops import _lib
 
     monkeypatch.setattr(sys.modules["axonn_b200.ops.mlp"], "_gelu_adjoint_in_gemm", lambda *_: in_gemm)
-    monkeypatch.setattr(sys.modules["axonn_b200.ops.mlp"], "swiglu_adjoint_in_gemm", lambda *_: in_gemm)
     torch.manual_seed(rows)
     wide = 2 * ffn if act == "swiglu" else ffn
     x = torch.randn(1, rows, hidden, device=DEV).bfloat16().requires_grad_(True)
