@@ -4,7 +4,6 @@ import torch
 from torch.autograd.function import once_differentiable
 
 from . import _lib
-from .activation import gelu_backward, gelu_backward_colsum
 from .direct import no_graph
 from .gemm import EPI_BIAS, EPI_BIAS_GELU, EPI_GELU, EPI_NONE, as_written, gemm_on_pairs, matmul_nn, matmul_nt, matmul_tn
 from .linear import _swiglu_gemm
@@ -14,7 +13,10 @@ _OUT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
 def _dgelu_gemm(g, w2, z, bias_dtype):
-    """``(g @ w2) * gelu'(z)`` and its column sums."""
+    """``(g @ w2) * gelu'(z)`` and its column sums.  One B200, against the product and the pass after it: 16384 x 8192 x 2048 445 / 488
+    us, 4096 rows 117 / 126, hidden 4096 and ffn 16384 378 / 414.  Few tiles leave the epilogue in sight (2048 x 2048 x 2048 46.5 / 42.3,
+    1300 x 8192 x 2048 53.4 / 52.1); such blocks, forward and backward, are bound by the host's launches, of which it saves one:
+    246 / 257 and 303 / 303."""
     rows, ffn = z.shape
     L = _lib.lib()
     dz = torch.empty_like(z)
@@ -27,15 +29,6 @@ def _dgelu_gemm(g, w2, z, bias_dtype):
     _lib.check(L.axb_fold_columns(_lib.addr(part), _lib.addr(db), part.shape[0], ffn, _OUT[bias_dtype], _lib.stream()),
                "axb_fold_columns")
     return dz, db
-
-
-def _gelu_adjoint_in_gemm(rows, hidden, ffn):
-    """Is the gradient GEMM with GELU's adjoint in its epilogue faster than the product and the pass after it?  The pass costs by
-    the element, the epilogue of the last tiles is not hidden behind a main loop (of ``hidden`` steps) whatever the size.  One B200,
-    fused / separate: hidden 2048 from 16 M elements 0.91 - 0.99 (2048 x 8192 69.0 / 70.8 us, 8192 x 2048 63.7 / 65.2), 8 - 16 M
-    0.97 - 1.02 (1300 x 8192 53.4 / 52.1), fewer 1.04 - 1.10 (2048 x 2048 46.5 / 42.3); hidden 2560 - 8192 from 8 M 0.80 - 0.99,
-    fewer 0.95 - 1.06."""
-    return rows * ffn >= (1 << 24 if hidden < 2560 else 1 << 23)
 
 
 class _MLPFn(torch.autograd.Function):
@@ -74,12 +67,8 @@ class _MLPFn(torch.autograd.Function):
         if need[0] or need[1] or need[2]:
             if ctx.act == "swiglu":
                 dz = _swiglu_gemm(True, g2[None], v2[None], torch.empty_like(z), z, None, 0)
-            elif _gelu_adjoint_in_gemm(z.shape[0], ctx.hidden, z.shape[1]):
-                dz, gb1 = _dgelu_gemm(g2, v2, z, ctx.b1 if ctx.b1 is not None and need[2] else None)
-            elif ctx.b1 is not None and need[2]:
-                dz, gb1 = gelu_backward_colsum(matmul_nn(g2, v2), z, out_dtype=ctx.b1)
             else:
-                dz = gelu_backward(matmul_nn(g2, v2), z)
+                dz, gb1 = _dgelu_gemm(g2, v2, z, ctx.b1 if ctx.b1 is not None and need[2] else None)
             if need[1]:
                 gw1 = matmul_tn(dz, x.reshape(-1, ctx.hidden)).view(w1.shape)
             if need[0]:
