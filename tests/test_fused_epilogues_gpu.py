@@ -1,5 +1,7 @@
 """GEMM epilogues at the edges of their rules: alignment of the output, remainders of tiles, masked rows."""
 
+import sys
+
 import pytest
 import torch
 
