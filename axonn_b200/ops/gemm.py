@@ -40,11 +40,12 @@ def _rowmajor(t):
     return t if t.is_contiguous() else t.contiguous()
 
 
-def as_written(t):
-    """``t`` dense and on a 32-byte boundary, for kernels that are given its address: itself or a copy.  A tensor saved for a
-    backward comes back from hooks (offloading, compression) in whatever layout they give it."""
+def as_written(t, alignment=16):
+    """``t`` dense and on a boundary of ``alignment`` bytes (16: what a TMA operand needs, 32: an epilogue's input), for kernels
+    that are given its address: itself or a copy.  A tensor saved for a backward comes back from hooks (offloading, compression)
+    in whatever layout they give it."""
     t = t.contiguous()
-    return t if t.data_ptr() % 32 == 0 else t.clone()
+    return t if t.data_ptr() % alignment == 0 else t.clone()
 
 
 def gemm_on_pairs(M, N, device) -> bool:

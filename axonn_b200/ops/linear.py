@@ -101,7 +101,7 @@ class _SwiGLUExpertsFn(torch.autograd.Function):
         g = as_written(g)
         gx = gw1 = gw2 = None
         if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
-            gu = as_written(gu)
+            gu = as_written(gu, 32)
             dgu = _swiglu_gemm(True, g, as_written(w2), torch.empty_like(gu), gu, **seg)
             gx = bmm_nn(dgu, w1, **seg) if ctx.needs_input_grad[0] else None
             gw1 = bmm_tn(dgu, x, out_dtype=w1.dtype, **seg) if ctx.needs_input_grad[1] else None

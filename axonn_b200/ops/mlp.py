@@ -57,7 +57,7 @@ class _MLPFn(torch.autograd.Function):
         x, w1, w2, z, h = ctx.saved_tensors
         need = ctx.needs_input_grad
         g2 = as_written(g.reshape(-1, ctx.hidden))
-        z = as_written(z)
+        z = as_written(z, 32)
         v1, v2 = w1.reshape(-1, ctx.hidden), as_written(w2).view(ctx.hidden, -1)
         gx = gw1 = gb1 = gw2 = gb2 = None
         if need[3]:

@@ -97,3 +97,16 @@ def test_feed_forward_result_in_place():
         z = _MLPFn.apply(x, w1, None, w2, None, 64, "gelu") + x
         y += x
         assert torch.equal(y, z) and y.shape == shape and y.grad_fn is not None
+
+
+def test_operands_are_copied_only_where_a_kernel_needs_it():
+    """Weights inside a flat buffer lie on 16 bytes, which is enough for an operand."""
+    from axonn_b200.ops.gemm import as_written
+
+    flat = torch.arange(128, dtype=torch.float32)
+    flat = flat[(-flat.data_ptr() // 4) % 8:]                          # starts on 32 bytes
+    t = flat[4:68].view(8, 8)
+    assert t.data_ptr() % 32 == 16 and as_written(t) is t
+    for got in (as_written(t, 32), as_written(t.t().contiguous().t()), as_written(flat[1:65].view(8, 8))):
+        assert got.is_contiguous() and got.data_ptr() % 16 == 0 and got.data_ptr() not in (t.data_ptr(), flat[1:].data_ptr())
+    assert torch.equal(as_written(t, 32), t) and torch.equal(as_written(t.t()), t.t())
