@@ -59,17 +59,17 @@ __device__ __forceinline__ void store_from_f32(void* p, long long i, int dtype, 
   else reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
 }
 
-// Clipping by the norm of one table: with `blocks_done` (zero on entry) the block that arrives last has the whole sum and
+// Clipping by the norm of one table (CLIP): with `blocks_done` zero on entry, the block that arrives last has the whole sum and
 // writes the norm and the factor min(1, max_norm / (norm + 1e-6)) itself.  As tensor operations after the kernel (square
 // root, sum, reciprocal, ...) that was seven launches of 2 us each: clipping and AdamW of 50 M parameters 305 -> 277 us.
 struct ClipOut {
-  unsigned int* blocks_done;     // null: squared norm only
+  unsigned int* blocks_done;
   float* norm;
   float* factor;
   float max_norm;
 };
 
-template <int PARTS>      // units per chunk
+template <int PARTS, bool CLIP>      // units per chunk
 __global__ void __launch_bounds__(MT_THREADS)
 multi_l2norm_sq_kernel(const long long* __restrict__ table, int n, long long total_chunks, float* __restrict__ out,
                        const ClipOut clip) {
@@ -126,7 +126,7 @@ multi_l2norm_sq_kernel(const long long* __restrict__ table, int n, long long tot
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (threadIdx.x == 0) {
       atomicAdd(out, acc);
-      if (clip.blocks_done) {
+      if (CLIP) {
         __threadfence();
         if (atomicAdd(clip.blocks_done, 1u) == gridDim.x - 1) {
           __threadfence();
@@ -357,24 +357,25 @@ static inline bool mt_long_tensors(int n, long long total_chunks) { return total
 
 using namespace axb;
 
+template <bool CLIP>
 static int l2norm_sq(const long long* table, int n, long long total_chunks, float* out, const ClipOut& clip, void* stream) {
   // Every block ends with an atomic: few blocks.  Whole chunks, unless there are so few of them that the last wave counts
   // and the tensors are long and found in one round of the search.  From DRAM, whole / quarters: 12 tensors of 64 chunks
   // 30.8 / 28.7 us, 8 of 10 12.3 / 10.2; 33 of 16 22.6 / 22.6, 300 of 16 121 / 127, 1500 of one half 31 / 45.
   if (n <= 32 && mt_long_tensors(n, total_chunks) && total_chunks < 16ll * sm_count_current())
-    multi_l2norm_sq_kernel<MT_PARTS><<<mt_grid(total_chunks * MT_PARTS, 4), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, out, clip);
+    multi_l2norm_sq_kernel<MT_PARTS, CLIP><<<mt_grid(total_chunks * MT_PARTS, 4), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, out, clip);
   else
-    multi_l2norm_sq_kernel<1><<<mt_grid(total_chunks, 8), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, out, clip);
+    multi_l2norm_sq_kernel<1, CLIP><<<mt_grid(total_chunks, 8), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, out, clip);
   AXB_CUDA(cudaGetLastError());
   return 0;
 }
 extern "C" int axb_multi_l2norm_sq(const long long* table, int n, long long total_chunks, float* out, void* stream) {
-  return l2norm_sq(table, n, total_chunks, out, ClipOut{nullptr, nullptr, nullptr, 0.f}, stream);
+  return l2norm_sq<false>(table, n, total_chunks, out, ClipOut{}, stream);
 }
 // words: four 32-bit words, the first two zero on entry: squared norm, block counter, norm, min(1, max_norm / (norm + 1e-6)).
 extern "C" int axb_multi_clip_factor(const long long* table, int n, long long total_chunks, float max_norm, float* words,
                                      void* stream) {
-  return l2norm_sq(table, n, total_chunks, words,
+  return l2norm_sq<true>(table, n, total_chunks, words,
                    ClipOut{reinterpret_cast<unsigned int*>(words + 1), words + 2, words + 3, max_norm}, stream);
 }
 extern "C" int axb_multi_scale(const long long* table, int n, long long total_chunks, const float* scale, void* stream) {
