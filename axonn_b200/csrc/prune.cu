@@ -122,7 +122,9 @@ __device__ __forceinline__ bool prune_last_block(unsigned int* counter) {
 // The pass is not bound by its atomics alone: the writes of whatever filled the tensor still go to memory meanwhile, and
 // counters without atomics or without bank conflicts took as long.  One B200, with the refill of the tensor: 117 M bf16 221 ->
 // 215 us, 67 M 133 -> 127, 67 M fp32 294 -> 280, 25 M fp32 128 -> 120.
-constexpr long long PR_LONG_BYTES = 64ll << 20;
+// The three passes of fp32 gain from 64 MB to some 400 MB only: 100 M 423 -> 421, but 117 M 483 -> 487, 400 M 1531 -> 1543; 16-bit
+// tensors at any length (800 M 1394 -> 1372).
+constexpr long long PR_LONG_BYTES = 64ll << 20, PR_LONG_F32_BYTES = 400ll << 20;
 template <bool LONG>
 __global__ void __launch_bounds__(PR_THREADS)
 prune_hist1_kernel(const void* __restrict__ g, long long n, int dtype, long long k, unsigned int* __restrict__ hist,
@@ -260,7 +262,8 @@ int prune_topk_launch(void* g, long long n, int dtype, long long k, unsigned int
     configured[device & 63] = true;
   }
   const int sms = sm_count(device);
-  const bool is_long = n * (dtype == PR_F32 ? 4 : 2) >= PR_LONG_BYTES;
+  const long long bytes = n * (dtype == PR_F32 ? 4 : 2);
+  const bool is_long = bytes >= PR_LONG_BYTES && (dtype != PR_F32 || bytes <= PR_LONG_F32_BYTES);
   auto hist = is_long ? prune_hist1_kernel<true> : prune_hist1_kernel<false>;
   hist<<<sms, PR_THREADS, PR_BINS1 * 4, s>>>(g, n, dtype, k, hist1, meta);
   AXB_CUDA(cudaGetLastError());

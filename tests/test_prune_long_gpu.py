@@ -55,3 +55,10 @@ def test_prune_lengths_and_offsets(n, at):
     buf = torch.empty(n + 16, device=DEV, dtype=torch.bfloat16)
     g = buf[at:at + n].copy_(torch.randn(n, device=DEV))
     _check(g, 0.2)
+
+
+@pytest.mark.parametrize("n", [100 << 20, (100 << 20) + 4])
+def test_prune_fp32_around_the_upper_length(n):
+    """fp32 tensors go through the passes from either end up to a length, and from the beginning past it."""
+    torch.manual_seed(1)
+    _check(torch.randn(n, device=DEV), 0.1)
