@@ -77,6 +77,7 @@ struct GemmParams {
   int seg_rows, nseg, mask_mode;
   float* colsum;     // ACT_DGELU
   int whole_tiles;   // plain CTA-pair kernel: tiles from this one on are computed as two halves of their columns (PairWalk)
+  int group;         // ... tile rows walked together
   int debug;      // ablation builds only (-DAXB_ABLATION, then read once from AXB_AR_DEBUG; otherwise 0 and every branch on it is compiled out): 1 no flagger fence, 2 no peer stores, 4 no reducer fence, 8 no reduction, 16 no partial stores, 128 register-path reducer instead of the shared-memory ring
 };
 
@@ -1383,6 +1384,48 @@ __device__ __forceinline__ bool pair_tile_computed(const GemmParams& p, int e, i
   return true;
 }
 
+// One segment per problem (all tokens of an expert come from this rank): the tile rows with data are the first ones of each
+// problem, and the pairs deal out just those.  The dealt list holding all tile rows gave the rows of a group to the pairs by
+// their parity, so that the pairs of the skipped rows had up to a tenth less to do, and a ninth row of tiles was walked by
+// itself, every column of the weights read again for it.  One B200, layer of 8 experts forward and backward, 16384 of 20480
+// rows in use, hidden 2048, ffn 8192: 4580 -> 4270 us.
+constexpr int PAIR_MAX_LIVE = 128;                   // problems; more of them skip the tiles without data one by one
+__device__ __forceinline__ void list_live_rows(const GemmParams& p, int tiles_m2, int* live_start) {
+  const int lane = threadIdx.x & 31;
+  int sum = 0;
+  if (lane == 0) live_start[0] = 0;
+  for (int e0 = 0; e0 < p.nb; e0 += 32) {
+    const int e = e0 + lane;
+    int n = e < p.nb ? min(tiles_m2, (min(max(__ldg(p.seg_counts + e), 0), p.M) + 2 * BM - 1) / (2 * BM)) : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int below = __shfl_up_sync(0xffffffffu, n, o);
+      if (lane >= o) n += below;
+    }
+    if (e < p.nb) live_start[e + 1] = sum + n;
+    sum += __shfl_sync(0xffffffffu, n, 31);
+  }
+}
+
+// Rows of the tiles that are not listed: 32 rows x 256 columns per warp and step.
+__device__ __forceinline__ void zero_dead_rows(const GemmParams& p, const int* live_start, int tiles_m2, int rank, int q) {
+  float z[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) z[i] = 0.f;
+  int t = blockIdx.x >> 1;                           // index among the tiles of the rows without data
+  for (int e = 0; e < p.nb; ++e) {
+    const int first = live_start[e + 1] - live_start[e], tiles = (tiles_m2 - first) * p.tiles_n;
+    for (; t < tiles; t += gridDim.x >> 1) {
+      const size_t local_row = static_cast<size_t>(2 * (first + t / p.tiles_n) + rank) * BM + q * 32 + (threadIdx.x & 31);
+      if (local_row >= static_cast<size_t>(p.M)) continue;
+      const int n0 = t % p.tiles_n * PAIR_BN;
+      for (int c = n0; c < min(n0 + PAIR_BN, p.N); c += 32)
+        store_row32(p.C, p.out_dtype, local_row + static_cast<size_t>(e) * p.c_batch_rows, p.N, c, p.N, z, false);
+    }
+    t -= tiles;
+  }
+}
+
 // K blocks of problem e that the kernel walks.  With one segment per problem (all tokens of an expert come from this
 // rank) the blocks with data are the first ones, and the producer and the MMA issuer loop over just those instead of
 // asking for every block: the question was a dependent global load in front of every MMA.
@@ -1391,25 +1434,55 @@ __device__ __forceinline__ int pair_kb_count(const GemmParams& p, int e, int num
   return min(num_kb, (__ldg(p.seg_counts + e) + BK - 1) / BK);
 }
 
+// Tile rows that are walked together, column by column: groups of about eight, of equal size.
+__host__ __device__ inline int pair_group(int tiles_m2) {
+  const int groups = tiles_m2 < 12 ? 1 : (tiles_m2 + 4) >> 3;
+  return (tiles_m2 + groups - 1) / groups;
+}
+
+// Tiles of a plain GEMM on `pairs` CTA pairs that are computed whole: all, unless the last wave is at most half full.
+__host__ __device__ inline int pair_whole_tiles(long long total, int pairs) {
+  const long long rest = total % pairs;
+  return static_cast<int>(rest != 0 && 2 * rest <= pairs ? total - rest : total);
+}
+
 // Work of a CTA pair: tiles, dealt in turn.  When the last wave would leave half of the pairs or more without a tile, its tiles
 // are cut into two halves of 128 columns, one for each of two pairs: the same MMAs with N = 128, half the time.
 // One B200, bf16, whole tiles / with halves: 777 x 6144 x 4096 (96 tiles on 74 pairs) 46.7 / 38.8 us, 1024 x 6144 x 2048 26.9 /
 // 22.3, 1024 x 6144 x 512 14.8 / 10.5, 8192 x 2048 x 4096 111 / 103; no difference within the noise of the power cap for the
 // weight gradients 8192 x 2048 x 16384.  More than half of the pairs busy: halves would need a second round, nothing gained.
 // (Sharing the K blocks of the last wave between all pairs, partial sums through global memory, was 20 - 30 us slower.)
+template <bool LIVE>
 struct PairWalk {
-  int it;
+  const int* live;                       // LIVE: the listed tile rows (list_live_rows)
+  int it, total, whole;                  // item index, tiles, tiles computed whole
   int tile, col, cols;                   // the current item: tile, first column inside it, columns
-  __device__ __forceinline__ PairWalk() : it(blockIdx.x >> 1) {}
-  __device__ __forceinline__ bool next(const GemmParams& p, int total) {
-    const int h = it - p.whole_tiles;
+  int e, tm2, tn;                        // its problem, tile row and column (locate)
+  __device__ __forceinline__ PairWalk(const GemmParams& p, const int* live_start, int tiles_m2)
+      : live(live_start), it(blockIdx.x >> 1), e(0) {
+    total = (LIVE ? live[p.nb] : tiles_m2 * p.nb) * p.tiles_n;
+    whole = LIVE ? pair_whole_tiles(total, gridDim.x >> 1) : p.whole_tiles;
+  }
+  __device__ __forceinline__ bool next() {
+    const int h = it - whole;
     if (h < 0) {
       tile = it; col = 0; cols = PAIR_BN;
     } else {
-      tile = p.whole_tiles + (h >> 1); col = (h & 1) * (PAIR_BN / 2); cols = PAIR_BN / 2;
+      tile = whole + (h >> 1); col = (h & 1) * (PAIR_BN / 2); cols = PAIR_BN / 2;
     }
     it += gridDim.x >> 1;
     return tile < total;
+  }
+  __device__ __forceinline__ void locate(const GemmParams& p, int tiles_m2) {
+    if (LIVE) {
+      while (tile >= live[e + 1] * p.tiles_n) ++e;
+      const int rows = live[e + 1] - live[e];
+      tile_coords(tile - live[e] * p.tiles_n, rows, p.tiles_n, pair_group(rows), tm2, tn);
+    } else {
+      const int per_batch = tiles_m2 * p.tiles_n;
+      e = tile / per_batch;
+      tile_coords(tile - e * per_batch, tiles_m2, p.tiles_n, p.group, tm2, tn);
+    }
   }
 };
 
@@ -1422,7 +1495,7 @@ struct PairWalk {
 template <int ACT>
 __host__ __device__ constexpr int pair_epi_warps() { return ACT == ACT_NONE || ACT == ACT_CE ? 4 : 8; }
 
-template <int A_MN, int B_MN, int ACT>
+template <int A_MN, int B_MN, int ACT, bool LIVE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epi_warps<ACT>(), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmBh, const GemmParams p) {
@@ -1442,10 +1515,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t rank = cluster_cta_rank();         // 0: leader (issues the MMAs), 1: peer
   const int num_kb = (p.K + BK - 1) / BK;
   const int tiles_m2 = (p.tiles_m + 1) >> 1;         // 256-row tile rows
-  const int per_batch = tiles_m2 * p.tiles_n;
-  const int total = per_batch * p.nb;
   const uint64_t timeout = p.timeout_ns;
+  __shared__ int live_start[LIVE ? PAIR_MAX_LIVE + 1 : 1];   // tile rows with data of the problems before each one
 
+  if (LIVE && warp == 2) list_live_rows(p, tiles_m2, live_start);
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 2 * pair_epi_warps<ACT>()); }
@@ -1466,17 +1539,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (elect_one()) {
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
-      PairWalk walk;
-      while (ok && walk.next(p, total)) {
-        const int e = walk.tile / per_batch;
-        int tm2, tn; tile_coords(walk.tile - e * per_batch, tiles_m2, p.tiles_n, 8, tm2, tn);
+      PairWalk<LIVE> walk(p, live_start, tiles_m2);
+      while (ok && walk.next()) {
+        walk.locate(p, tiles_m2);
+        const int e = walk.e, tm2 = walk.tm2, tn = walk.tn;
         const int m0 = (2 * tm2 + static_cast<int>(rank)) * BM;
         const bool whole = walk.cols == BN;
         const int n0 = tn * BN + walk.col + static_cast<int>(rank) * (walk.cols / 2);   // this CTA's half of the B tile
         const uint32_t stage_bytes = 2 * (S::A_BYTES + (whole ? S::B_BYTES : S::B_BYTES / 2));
         // row coordinate of problem e in the stacked operands (rows = M or N for a K-major operand, K otherwise)
         const int a_r = e * p.a_batch_rows, b_r = e * p.b_batch_rows;
-        if (p.mask_mode == 1 && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, tm2 * 2 * BM, 2 * BM)) continue;
+        if (p.mask_mode == 1 && !LIVE && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, tm2 * 2 * BM, 2 * BM)) continue;
         const int kb_end = pair_kb_count(p, e, num_kb);
         for (int kb = 0; kb < kb_end; ++kb) {
           if (p.mask_mode == 2 && p.nseg > 1 && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, kb * BK, BK)) continue;
@@ -1513,14 +1586,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       int t = 0;
-      PairWalk walk;
-      while (ok && walk.next(p, total)) {
-        const int e = walk.tile / per_batch;
+      PairWalk<LIVE> walk(p, live_start, tiles_m2);
+      while (ok && walk.next()) {
         const uint32_t idesc = walk.cols == BN ? idesc_whole : idesc_half;
-        if (p.mask_mode != 0) {
-          int tm2, tn; tile_coords(walk.tile - e * per_batch, tiles_m2, p.tiles_n, 8, tm2, tn);
-          if (!pair_tile_computed(p, e, tm2, num_kb)) continue;      // no accumulator buffer is used for it
+        if (!LIVE && p.mask_mode != 0) {
+          walk.locate(p, tiles_m2);
+          if (!pair_tile_computed(p, walk.e, walk.tm2, num_kb)) continue;      // no accumulator buffer is used for it
         }
+        const int e = walk.e;
         const int buf = t & 1;
         const uint32_t acc_phase = (t >> 1) & 1;
         ++t;
@@ -1560,15 +1633,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int part = PARTS == 1 ? 0 : (warp - 2) >> 2;
     bool ok = true;
     int t = 0;
-    PairWalk walk;
-    while (ok && walk.next(p, total)) {
-      const int e = walk.tile / per_batch;
-      int tm2, tn; tile_coords(walk.tile - e * per_batch, tiles_m2, p.tiles_n, 8, tm2, tn);
+    // tile rows without data are not listed: zeros (nothing to add when accumulating), while the first tile is multiplied
+    if (LIVE && ACT == ACT_NONE && !p.accumulate) zero_dead_rows(p, live_start, tiles_m2, rank, q);
+    PairWalk<LIVE> walk(p, live_start, tiles_m2);
+    while (ok && walk.next()) {
+      walk.locate(p, tiles_m2);
+      const int e = walk.e, tm2 = walk.tm2, tn = walk.tn;
       const int tm = 2 * tm2 + static_cast<int>(rank);
       const size_t local_row = static_cast<size_t>(tm) * BM + q * 32 + lane;
       const bool row_ok = local_row < static_cast<size_t>(p.M);     // rows past M belong to the next problem
       const size_t row = local_row + static_cast<size_t>(e) * p.c_batch_rows;
-      if (p.mask_mode != 0 && !pair_tile_computed(p, e, tm2, num_kb)) {
+      if (!LIVE && p.mask_mode != 0 && !pair_tile_computed(p, e, tm2, num_kb)) {
         if (ACT != ACT_NONE) continue;                         // nothing reads it (see axb_gemm_swiglu)
         // a tile without data: zeros (nothing to add when accumulating), no accumulator buffer involved
         if (row_ok && !p.accumulate) {
@@ -1970,20 +2045,14 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p,
   return 0;
 }
 
-// Tiles of a plain GEMM on `pairs` CTA pairs that are computed whole: all, unless the last wave is at most half full.
-static int pair_whole_tiles(long long total, int pairs) {
-  const long long rest = total % pairs;
-  return static_cast<int>(rest != 0 && 2 * rest <= pairs ? total - rest : total);
-}
-
 // tmBh: B with boxes of half as many rows, for the halves of tiles (any map for an MN-major B); null: whole tiles only.
 // sms: what the caller read from usable_sms, on which its choice of tmBh depends (another thread may change it meanwhile).
-template <int A_MN, int B_MN, int ACT = ACT_NONE>
+template <int A_MN, int B_MN, int ACT = ACT_NONE, bool LIVE = false>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap* tmBh, GemmParams& p, int sms, int device,
                        cudaStream_t stream) {
   using S = PairSmem;
   static bool configured[64] = {false};
-  auto kern = gemm_pair_kernel<A_MN, B_MN, ACT>;
+  auto kern = gemm_pair_kernel<A_MN, B_MN, ACT, LIVE>;
   if (!configured[device & 63]) {
     AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
     configured[device & 63] = true;
@@ -1992,8 +2061,9 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   p.tiles_n = (p.N + PAIR_BN - 1) / PAIR_BN;
   const int total = ((p.tiles_m + 1) / 2) * p.tiles_n * p.nb;
   const int pairs = sms / 2;
+  p.group = pair_group((p.tiles_m + 1) / 2);
   p.whole_tiles = tmBh ? pair_whole_tiles(total, pairs) : total;
-  const int items = p.whole_tiles + 2 * (total - p.whole_tiles);
+  const int items = LIVE ? total : p.whole_tiles + 2 * (total - p.whole_tiles);
   const int grid = 2 * (items < pairs ? items : pairs);
   p.gemm_ctas = grid;
   kern<<<grid, 64 + 32 * pair_epi_warps<ACT>(), S::TOTAL, stream>>>(tmA, tmB, tmBh ? *tmBh : tmB, p);
@@ -2279,6 +2349,7 @@ static int gemm_batched(int layout, const void* A, const void* B, void* C, void*
   p.ar.n = 1; p.ag.n = 1; p.tn_offset = 0; p.kb_offset = 0; p.flag_batch = 1; p.debug = 0; p.pair = 1;
   p.nb = nb; p.a_batch_rows = a_batch_rows; p.b_batch_rows = b_batch_rows; p.c_batch_rows = c_batch_rows;
   p.seg_counts = nullptr; p.seg_rows = 0; p.nseg = 0; p.mask_mode = 0;
+  bool live = false;                       // only the tile rows with data are dealt out
   if (seg_counts) {
     const long long masked = (layout == 2) ? K : M;
     if (seg_rows <= 0 || nseg <= 0 || static_cast<long long>(seg_rows) * nseg != masked) {
@@ -2286,15 +2357,22 @@ static int gemm_batched(int layout, const void* A, const void* B, void* C, void*
       return -1;
     }
     p.seg_counts = seg_counts; p.seg_rows = seg_rows; p.nseg = nseg; p.mask_mode = (layout == 2) ? 2 : 1;
+    live = p.mask_mode == 1 && nseg == 1 && nb <= PAIR_MAX_LIVE;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int sms = usable_sms(device);
-  // a single problem without a mask may have the tiles of its last wave in halves
+  // a single problem without a mask may have the tiles of its last wave in halves, and so may a list of tiles
   const CUtensorMap* halves = nullptr;
   CUtensorMap tmBh = tmB;
-  if (nb == 1 && p.mask_mode == 0 && (act == ACT_SWIGLU || act == ACT_DSWIGLU || act == ACT_DGELU)) {
+  if (live || (nb == 1 && p.mask_mode == 0 && (act == ACT_SWIGLU || act == ACT_DSWIGLU || act == ACT_DGELU))) {
     if (b_mn == 0 && make_tmap_2d_16bit(&tmBh, B, b_total, K, PAIR_BN / 4, in_dtype)) return -1;
     halves = &tmBh;
+  }
+  if (live) {
+    if (act == ACT_SWIGLU) return launch_pair<0, 0, ACT_SWIGLU, true>(tmA, tmB, halves, p, sms, device, s);
+    if (act == ACT_DSWIGLU) return launch_pair<0, 1, ACT_DSWIGLU, true>(tmA, tmB, halves, p, sms, device, s);
+    if (layout == 0) return launch_pair<0, 0, ACT_NONE, true>(tmA, tmB, halves, p, sms, device, s);
+    return launch_pair<0, 1, ACT_NONE, true>(tmA, tmB, halves, p, sms, device, s);
   }
   if (act == ACT_DGELU) return launch_pair<0, 1, ACT_DGELU>(tmA, tmB, halves, p, sms, device, s);
   if (act == ACT_CE) return launch_pair<0, 0, ACT_CE>(tmA, tmB, nullptr, p, sms, device, s);
