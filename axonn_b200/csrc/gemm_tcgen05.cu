@@ -20,7 +20,9 @@
 //
 // gemm_pair_kernel: clusters of two CTAs (tcgen05.mma.cta_group::2) compute
 // 256x256 tiles for plain GEMMs; warps 0-5 as above in each CTA (0-9 where the
-// epilogue computes an activation), MMAs issued by the even CTA for both.
+// epilogue computes an activation), MMAs issued by the even CTA for both.  Plain
+// products choose the tiles' width, and may exchange the operands' roles, so that a
+// ragged number of tokens fills its tiles and the last wave (pair_tiles).
 //
 // Operand layouts: each of A and B is either K-major (row = M/N index, K
 // contiguous) or MN-major (row = K index, M/N contiguous); both are expressed
@@ -76,6 +78,7 @@ struct GemmParams {
   const int* seg_counts;
   int seg_rows, nseg, mask_mode;
   float* colsum;     // ACT_DGELU
+  int bn;            // plain CTA-pair kernel: columns of a tile, a multiple of 16 up to 256
   int whole_tiles;   // plain CTA-pair kernel: tiles from this one on are computed as two halves of their columns (PairWalk)
   int group;         // ... tile rows walked together
   int debug;      // ablation builds only (-DAXB_ABLATION, then read once from AXB_AR_DEBUG; otherwise 0 and every branch on it is compiled out): 1 no flagger fence, 2 no peer stores, 4 no reducer fence, 8 no reduction, 16 no partial stores, 128 register-path reducer instead of the shared-memory ring
@@ -315,31 +318,85 @@ __device__ __forceinline__ void add_bias32(const uint4 (&b)[4], int dtype, float
 // registers are written as soon as it is issued, so the wait has them as operands).  Loading the accumulator a chunk ahead
 // as well costs registers and gains nothing: one B200, bf16, ahead / now: 24 x 1024 x 256 6.0 / 5.8 us, with bias 7.0 / 6.7;
 // 777 x 4096 x 4096 26.1 / 25.5, 27.8 / 27.7, with GELU and the saved pre-activation 30.7 / 30.4.
-template <int BN>
-__device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t taddr, size_t row, bool row_ok, int col0) {
+// `end`: first column that is not this thread's.
+__device__ __forceinline__ void epilogue_row(const GemmParams& p, uint32_t taddr, size_t row, bool row_ok, int col0, int end) {
   const bool biased = p.epilogue == 1 || p.epilogue == 2;
   uint4 bn[4] = {};
-  if (biased) load_bias32(p, col0, bn);
+  if (biased && col0 < end) load_bias32(p, col0, bn);
 #pragma unroll 1
-  for (int c = 0; c < BN / 32; ++c) {
-    const int col = col0 + c * 32;
-    if (col >= p.N) break;  // uniform across the warp
+  for (int col = col0; col < end; col += 32, taddr += 32) {     // uniform across the warp
     uint32_t r[32];
-    tmem_ld_32x32(taddr + c * 32, r);
+    tmem_ld_32x32(taddr, r);
     tmem_ld_wait(r);
     float v[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
     if (biased) {
       add_bias32(bn, p.in_dtype, v);
-      if (c + 1 < BN / 32 && col + 32 < p.N) load_bias32(p, col + 32, bn);
+      if (col + 32 < end) load_bias32(p, col + 32, bn);
     }
     if (p.epilogue >= 2) {
-      if (p.aux != nullptr && row_ok) store_row32(p.aux, p.out_dtype, row, p.N, col, p.N, v, false);
+      if (p.aux != nullptr && row_ok) store_row32(p.aux, p.out_dtype, row, p.N, col, end, v, false);
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
     }
-    if (row_ok) store_row32(p.C, p.out_dtype, row, p.N, col, p.N, v, p.accumulate != 0);
+    if (row_ok) store_row32(p.C, p.out_dtype, row, p.N, col, end, v, p.accumulate != 0);
+  }
+}
+
+// Epilogue of a product with its operands' roles exchanged: the tile's rows are output columns (features), its columns
+// output rows (tokens) of C [N, M]; 16-bit outputs, no accumulation.  A thread holds one feature of 32 tokens; they go through
+// shared memory (rows of 80 bytes: neither the 2-byte stores of a token nor the 16-byte loads of eight lanes meet in a bank)
+// and each lane stores 64 consecutive bytes of one token.
+constexpr int SWAP_PITCH = 80;
+__device__ __forceinline__ void store_swapped(const GemmParams& p, void* base, int feature0, int token0, int end, uint8_t* stage, const float (&v)[32]) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();                                      // the previous chunk has been read
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const uint32_t w = pack2(v[2 * i], v[2 * i + 1], p.out_dtype);
+    *reinterpret_cast<uint16_t*>(stage + (2 * i) * SWAP_PITCH + lane * 2) = static_cast<uint16_t>(w);
+    *reinterpret_cast<uint16_t*>(stage + (2 * i + 1) * SWAP_PITCH + lane * 2) = static_cast<uint16_t>(w >> 16);
+  }
+  __syncwarp();
+  const int token = token0 + lane;
+  if (token >= end) return;
+  uint16_t* dst = reinterpret_cast<uint16_t*>(base) + static_cast<size_t>(token) * p.M + feature0;
+  const uint4* src = reinterpret_cast<const uint4*>(stage + lane * SWAP_PITCH);
+  if (feature0 + 32 <= p.M && ((reinterpret_cast<uintptr_t>(base) | static_cast<uintptr_t>(p.M) * 2) & 31) == 0) {
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      const uint4 a = src[2 * g], b = src[2 * g + 1];
+      const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      st_global_32b(dst + g * 16, w);
+    }
+  } else {
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+      if (feature0 + g * 8 < p.M) *reinterpret_cast<uint4*>(dst + g * 8) = src[g];      // M is a multiple of 8
+  }
+}
+template <bool GELU>
+__device__ __forceinline__ void epilogue_swapped(const GemmParams& p, uint32_t taddr, int feature0, int token0, int end, uint8_t* stage) {
+  const int feature = feature0 + (threadIdx.x & 31);
+  float bias = -0.f;                                 // x + -0 is x, whatever its sign
+  if ((p.epilogue == 1 || p.epilogue == 2) && feature < p.M)
+    bias = p.in_dtype == 0 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.bias)[feature])
+                           : __half2float(reinterpret_cast<const __half*>(p.bias)[feature]);
+#pragma unroll 1
+  for (int token = token0; token < end; token += 32, taddr += 32) {   // uniform across the warp
+    uint32_t r[32];
+    tmem_ld_32x32(taddr, r);
+    tmem_ld_wait(r);
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) + bias;
+    if (GELU) {
+      if (p.aux != nullptr) store_swapped(p, p.aux, feature0, token, end, stage, v);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
+    }
+    store_swapped(p, p.C, feature0, token, end, stage, v);
   }
 }
 
@@ -1256,7 +1313,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const bool row_ok = row < static_cast<size_t>(p.M);
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN;
       if (p.ar.n <= 1) {
-        epilogue_row<BN>(p, taddr, row, row_ok, tn * BN);
+        epilogue_row(p, taddr, row, row_ok, tn * BN, min(tn * BN + BN, p.N));
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) { if (PAIR) mbar_arrive_leader(&tmem_empty[buf]); else mbar_arrive(&tmem_empty[buf]); }
@@ -1374,6 +1431,9 @@ struct PairSmem {
   static constexpr int STAGES = 6;
   static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 4) * 8 + 16 + 1024 /* alignment slack */;
+  static constexpr int SWAP_OFFSET = BAR_OFFSET + 256, SWAP_WARP_BYTES = 32 * SWAP_PITCH;    // store_swapped, eight warps
+  static constexpr int TOTAL_SWAP = SWAP_OFFSET + 8 * SWAP_WARP_BYTES + 1024;
+  static_assert((2 * STAGES + 4) * 8 + 16 <= 256 && TOTAL_SWAP <= 232448, "shared memory of a CTA");
 };
 
 // Masked batched mode: is the 256-row tile pair tm2 of problem e computed at all?  (mode 1: one of its rows holds
@@ -1455,20 +1515,20 @@ __host__ __device__ inline int pair_whole_tiles(long long total, int pairs) {
 template <bool LIVE>
 struct PairWalk {
   const int* live;                       // LIVE: the listed tile rows (list_live_rows)
-  int it, total, whole;                  // item index, tiles, tiles computed whole
+  int it, total, whole, bn;              // item index, tiles, tiles computed whole, columns of a tile
   int tile, col, cols;                   // the current item: tile, first column inside it, columns
   int e, tm2, tn;                        // its problem, tile row and column (locate)
   __device__ __forceinline__ PairWalk(const GemmParams& p, const int* live_start, int tiles_m2)
-      : live(live_start), it(blockIdx.x >> 1), e(0) {
+      : live(live_start), it(blockIdx.x >> 1), bn(p.bn), e(0) {
     total = (LIVE ? live[p.nb] : tiles_m2 * p.nb) * p.tiles_n;
     whole = LIVE ? pair_whole_tiles(total, gridDim.x >> 1) : p.whole_tiles;
   }
   __device__ __forceinline__ bool next() {
     const int h = it - whole;
     if (h < 0) {
-      tile = it; col = 0; cols = PAIR_BN;
+      tile = it; col = 0; cols = bn;
     } else {
-      tile = whole + (h >> 1); col = (h & 1) * (PAIR_BN / 2); cols = PAIR_BN / 2;
+      tile = whole + (h >> 1); col = (h & 1) * (bn / 2); cols = bn / 2;
     }
     it += gridDim.x >> 1;
     return tile < total;
@@ -1495,7 +1555,7 @@ struct PairWalk {
 template <int ACT>
 __host__ __device__ constexpr int pair_epi_warps() { return ACT == ACT_NONE || ACT == ACT_CE ? 4 : 8; }
 
-template <int A_MN, int B_MN, int ACT, bool LIVE>
+template <int A_MN, int B_MN, int ACT, bool LIVE, bool SWAP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epi_warps<ACT>(), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmBh, const GemmParams p) {
@@ -1544,9 +1604,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         walk.locate(p, tiles_m2);
         const int e = walk.e, tm2 = walk.tm2, tn = walk.tn;
         const int m0 = (2 * tm2 + static_cast<int>(rank)) * BM;
-        const bool whole = walk.cols == BN;
-        const int n0 = tn * BN + walk.col + static_cast<int>(rank) * (walk.cols / 2);   // this CTA's half of the B tile
-        const uint32_t stage_bytes = 2 * (S::A_BYTES + (whole ? S::B_BYTES : S::B_BYTES / 2));
+        const bool whole = walk.cols == p.bn;
+        const int half = walk.cols / 2;
+        const int n0 = tn * p.bn + walk.col + static_cast<int>(rank) * half;             // this CTA's half of the B tile
+        // a row of 64 K values per column, or blocks of 64 columns
+        const uint32_t stage_bytes = 2 * (S::A_BYTES + (B_MN == 0 ? half : (half + 63) / 64 * 64) * (BK * 2));
         // row coordinate of problem e in the stacked operands (rows = M or N for a K-major operand, K otherwise)
         const int a_r = e * p.a_batch_rows, b_r = e * p.b_batch_rows;
         if (p.mask_mode == 1 && !LIVE && !rows_hold_data(p.seg_counts, p.seg_rows, p.nseg, e, tm2 * 2 * BM, 2 * BM)) continue;
@@ -1569,7 +1631,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tma_load_2d_pair(sB, whole ? &tmB : &tmBh, &full_bar[stage], k0, n0 + b_r);
           } else {
 #pragma unroll
-            for (int j = 0; j < BN / 128; ++j) if (j == 0 || whole) tma_load_2d_pair(sB + j * (BK * 128), &tmB, &full_bar[stage], n0 + 64 * j, k0 + b_r);
+            for (int j = 0; j < BN / 128; ++j) if (64 * j < half) tma_load_2d_pair(sB + j * (BK * 128), &tmB, &full_bar[stage], n0 + 64 * j, k0 + b_r);
           }
           if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
         }
@@ -1579,8 +1641,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
     if (rank == 0 && elect_one()) {
-      const uint32_t idesc_whole = umma_idesc(p.in_dtype == 0 ? 1 : 0, A_MN, B_MN, 2 * BM, BN);
-      const uint32_t idesc_half = umma_idesc(p.in_dtype == 0 ? 1 : 0, A_MN, B_MN, 2 * BM, BN / 2);
+      const uint32_t idesc_whole = umma_idesc(p.in_dtype == 0 ? 1 : 0, A_MN, B_MN, 2 * BM, p.bn);
+      const uint32_t idesc_half = umma_idesc(p.in_dtype == 0 ? 1 : 0, A_MN, B_MN, 2 * BM, p.bn / 2);
       const uint32_t a_lbo = A_MN ? BK * 128 : 16, a_sbo = 1024, a_kstep = A_MN ? UMMA_K * 128 : UMMA_K * 2;
       const uint32_t b_lbo = B_MN ? BK * 128 : 16, b_sbo = 1024, b_kstep = B_MN ? UMMA_K * 128 : UMMA_K * 2;
       int stage = 0; uint32_t phase = 0;
@@ -1588,7 +1650,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int t = 0;
       PairWalk<LIVE> walk(p, live_start, tiles_m2);
       while (ok && walk.next()) {
-        const uint32_t idesc = walk.cols == BN ? idesc_whole : idesc_half;
+        const uint32_t idesc = walk.cols == p.bn ? idesc_whole : idesc_half;
         if (!LIVE && p.mask_mode != 0) {
           walk.locate(p, tiles_m2);
           if (!pair_tile_computed(p, walk.e, walk.tm2, num_kb)) continue;      // no accumulator buffer is used for it
@@ -1659,9 +1721,29 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint32_t acc_phase = (t >> 1) & 1;
       ++t;
       uint32_t z[32];
+      const int n0 = tn * p.bn + walk.col;
+      if (ACT == ACT_NONE || ACT == ACT_GELU) {
+        if (!mbar_wait(&tmem_full[buf], acc_phase, abort_flag, timeout)) { ok = false; break; }
+        tcgen05_fence_after();
+        // the item's chunks of 32 columns, shared between the warps
+        const int share = (walk.cols + 32 * PARTS - 1) / (32 * PARTS) * 32, c0 = part * share;
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * BN + c0;
+        const int end = min(n0 + min(c0 + share, walk.cols), p.N);
+        if (SWAP) {
+          uint8_t* stage = smem + S::SWAP_OFFSET + (warp - 2) * S::SWAP_WARP_BYTES;
+          epilogue_swapped<ACT == ACT_GELU>(p, taddr, tm * BM + q * 32, n0 + c0, end, stage);
+        } else {
+          epilogue_row(p, taddr, row, row_ok, n0 + c0, end);
+        }
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_leader(&tmem_empty[buf]);   // the epilogue warps of both CTAs free the buffer
+        continue;
+      }
+      // the other epilogues: tiles of 256 columns
       const bool whole = walk.cols == BN;
       const int off = whole ? part * PN : part * (PN / 2);            // this warp's columns inside the item
-      const int col0 = tn * BN + walk.col + off;
+      const int col0 = n0 + off;
       if (ACT == ACT_DSWIGLU) load_gate_up(p, row, row_ok, col0, z);
       if (ACT == ACT_DGELU && row_ok && col0 < p.N) {
         const uint16_t* src = reinterpret_cast<const uint16_t*>(p.aux) + row * p.N + col0;
@@ -1679,9 +1761,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       } else if (ACT == ACT_SWIGLU || ACT == ACT_DSWIGLU) {
         if (whole) epilogue_act<PN, ACT>(p, taddr, row, row_ok, col0, z);
         else epilogue_act<PN / 2, ACT>(p, taddr, row, row_ok, col0, z);
-      } else if (col0 < p.N) {
-        if (whole) epilogue_row<PN>(p, taddr, row, row_ok, col0);
-        else epilogue_row<PN / 2>(p, taddr, row, row_ok, col0);
       }
       tcgen05_fence_before();
       __syncwarp();
@@ -2047,18 +2126,18 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p,
 
 // tmBh: B with boxes of half as many rows, for the halves of tiles (any map for an MN-major B); null: whole tiles only.
 // sms: what the caller read from usable_sms, on which its choice of tmBh depends (another thread may change it meanwhile).
-template <int A_MN, int B_MN, int ACT = ACT_NONE, bool LIVE = false>
+template <int A_MN, int B_MN, int ACT = ACT_NONE, bool LIVE = false, bool SWAP = false>
 static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap* tmBh, GemmParams& p, int sms, int device,
                        cudaStream_t stream) {
-  using S = PairSmem;
+  constexpr int smem_bytes = SWAP ? PairSmem::TOTAL_SWAP : PairSmem::TOTAL;
   static bool configured[64] = {false};
-  auto kern = gemm_pair_kernel<A_MN, B_MN, ACT, LIVE>;
+  auto kern = gemm_pair_kernel<A_MN, B_MN, ACT, LIVE, SWAP>;
   if (!configured[device & 63]) {
-    AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
+    AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
     configured[device & 63] = true;
   }
   p.tiles_m = (p.M + BM - 1) / BM;
-  p.tiles_n = (p.N + PAIR_BN - 1) / PAIR_BN;
+  p.tiles_n = (p.N + p.bn - 1) / p.bn;
   const int total = ((p.tiles_m + 1) / 2) * p.tiles_n * p.nb;
   const int pairs = sms / 2;
   p.group = pair_group((p.tiles_m + 1) / 2);
@@ -2066,7 +2145,7 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   const int items = LIVE ? total : p.whole_tiles + 2 * (total - p.whole_tiles);
   const int grid = 2 * (items < pairs ? items : pairs);
   p.gemm_ctas = grid;
-  kern<<<grid, 64 + 32 * pair_epi_warps<ACT>(), S::TOTAL, stream>>>(tmA, tmB, tmBh ? *tmBh : tmB, p);
+  kern<<<grid, 64 + 32 * pair_epi_warps<ACT>(), smem_bytes, stream>>>(tmA, tmB, tmBh ? *tmBh : tmB, p);
   AXB_CUDA(cudaGetLastError());
   return 0;
 }
@@ -2173,6 +2252,57 @@ static bool plain_on_pairs(int M, int N, int device) {
   return pair_mode_enabled() && ((wide_tiles >= all_sms && pair_tiles >= all_sms / 2) || 6 * pair_waves <= 5 * single_waves);
 }
 
+// Tiles of a plain product on CTA pairs: their width, and whether the operands change roles (the rows of B become the 256
+// rows of a tile, the rows of A its columns, so that the width can follow a ragged number of tokens).  bn 0: not on pairs.
+struct PairTiles { int bn; bool swap; };
+
+// Time of a product on `pairs` CTA pairs in columns of work: waves of tiles, the last one in halves where it is small.  A tile
+// costs 80 columns beside its own (its 256 rows are loaded whatever its width, and loads from the L2 bound narrow tiles), and 2 %
+// more where half of its width is an odd multiple of 8.
+static float pair_cost(unsigned tile_rows, unsigned cols, unsigned bn, unsigned pairs) {
+  const unsigned total = tile_rows * ((cols + bn - 1) / bn), waves = total / pairs, rest = total - waves * pairs;
+  float cost = static_cast<float>(waves * (bn + 80));
+  if (rest != 0) cost += bn % 32 == 0 && 2 * rest <= pairs ? bn / 2 + 80 : bn + 80;
+  return bn % 32 == 0 ? cost : 1.02f * cost;
+}
+
+// Widths from 96 to 256 columns in either orientation; 256 with the roles as they are unless another one saves 2 % or more.
+// Exchanged roles take a little longer at the end of the launch (300 columns of one K block).  A B whose columns are
+// contiguous (layouts 1 and 2) is loaded in blocks of 64 that have to start on 128 bytes: other widths made it slower.
+// One B200, bf16, 256 / chosen (M x N x K): 777 x 6144 x 4096 41.9 / 35.4 us (144, exchanged), 777 x 4096 x 4096 26.8 / 23.9 (208,
+// exchanged), 777 x 3072 x 1024 10.9 / 6.5 (144, exchanged), 1300 x 50304 x 2048 215 / 184 (224, exchanged), 4096 x 2048 x 50304 in layout
+// 1 663 / 635 (240, exchanged).  Over 243 shapes of M 300 .. 4096, N 1024 .. 50304, K 1024 .. 50304, layouts 0 (plain, bias, GELU)
+// and 1 on average 0.916 of the time, at best 0.60, at worst 1.023 (4096 x 2048 x 2048, layout 1); the best widths of
+// each shape would give 0.910.
+static PairTiles pair_tiles(int M, int N, int K, int layout, bool can_swap, int pairs) {
+  PairTiles best = {PAIR_BN, false};
+  const unsigned rows_m = (M + 2 * BM - 1) / (2 * BM), rows_n = (N + 2 * BM - 1) / (2 * BM);
+  if (layout > 1 || static_cast<long long>(rows_m) * rows_n > (1 << 20)) return best;
+  float least = 0.98f * pair_cost(rows_m, N, PAIR_BN, pairs);
+  // no width can do better than full waves of the widest tiles without a padded row: the search costs 0.3 us of host time
+  if (static_cast<float>(M) * static_cast<float>(N) * (PAIR_BN + 80) >= least * (2.f * BM * PAIR_BN) * pairs) return best;
+  for (int swap = layout == 0 ? 0 : 1; swap <= (can_swap ? 1 : 0); ++swap) {
+    for (int bn = PAIR_BN; bn >= 96; bn -= 16) {
+      const float cost = swap ? pair_cost(rows_n, M, bn, pairs) + 300.f * BK / K : pair_cost(rows_m, N, bn, pairs);
+      if (cost < least) { least = cost; best = {bn, swap != 0}; }
+    }
+  }
+  return best;
+}
+
+// Products too small for plain_on_pairs that are not split along K either: narrow tiles on pairs where they need one wave.
+// Their kernel has six warps instead of the sixteen of the single CTAs' (which serves the fused collectives), and a
+// tile of half the width has its epilogue done sooner.  One B200, bf16, single CTAs / pairs: 308 x 768 x 256 5.5 / 4.6 us,
+// 308 x 1024 x 1024 7.6 / 6.8, 1000 x 1024 x 1024 7.8 / 7.2, layout 1 308 x 1024 x 256 5.3 / 4.7.  Over M 64 .. 1531, N 256 .. 6144, K 256 ..
+// 1024 0.82 - 1.0; with K 2048 and 4096 0.92 - 1.4.
+static PairTiles pair_tiles_small(int M, int N, int K, int layout, bool can_swap, int pairs) {
+  if (!pair_mode_enabled() || K > 1024 || layout > 1 || (layout == 1 && !can_swap)) return {0, false};
+  const int rows = layout == 1 ? N : M, cols = layout == 1 ? M : N;
+  for (int bn = 64; bn <= 128; bn += 64)
+    if (static_cast<long long>((rows + 2 * BM - 1) / (2 * BM)) * ((cols + bn - 1) / bn) <= pairs) return {bn, layout == 1};
+  return {0, false};
+}
+
 }  // namespace axb
 
 static int gemm_common(int layout, const void* A, const void* B, void* C, const void* bias, void* aux, int M, int N,
@@ -2203,13 +2333,24 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
 
   CUtensorMap tmA, tmB;
   // K-major operand [R, K]: box 64(K) x tile rows.  MN-major operand [K, R]: box 64(R) x 64(K).
-  if (a_mn == 0) { if (make_tmap_2d_16bit(&tmA, A, M, K, BM, in_dtype)) return -1; }
-  else           { if (make_tmap_2d_16bit(&tmA, A, K, M, BK, in_dtype)) return -1; }
-  const bool pair = !comm && plain_on_pairs(M, N, device);
-  if (pair) BN = 256;
-  const int splitk = (comm || pair || BN != 128) ? 1 : splitk_ctas(M, N, K, usable_sms(device), device);
-  if (b_mn == 0) { if (make_tmap_2d_16bit(&tmB, B, N, K, (pair || comm_pair) ? BN / 2 : BN, in_dtype)) return -1; }
-  else           { if (make_tmap_2d_16bit(&tmB, B, K, N, BK, in_dtype)) return -1; }
+  const bool wide_pair = !comm && plain_on_pairs(M, N, device);
+  if (wide_pair) BN = 256;
+  const int splitk = (comm || wide_pair || BN != 128) ? 1 : splitk_ctas(M, N, K, usable_sms(device), device);
+  const bool can_swap = out_dtype != 2 && !accumulate && (layout == 0 || (layout == 1 && epilogue < 2));
+  const int sms = usable_sms(device);
+  PairTiles tiles = {0, false};
+  if (wide_pair) tiles = pair_tiles(M, N, K, layout, can_swap, sms / 2);
+  else if (!comm && splitk == 1) tiles = pair_tiles_small(M, N, K, layout, can_swap, sms / 2);
+  const bool pair = tiles.bn != 0;
+  if (tiles.swap) {                                 // rows of B as the rows of the tiles, rows of A as their columns
+    if ((b_mn == 0 ? make_tmap_2d_16bit(&tmA, B, N, K, BM, in_dtype) : make_tmap_2d_16bit(&tmA, B, K, N, BK, in_dtype)) ||
+        make_tmap_2d_16bit(&tmB, A, M, K, tiles.bn / 2, in_dtype)) return -1;
+  } else {
+    if (a_mn == 0) { if (make_tmap_2d_16bit(&tmA, A, M, K, BM, in_dtype)) return -1; }
+    else           { if (make_tmap_2d_16bit(&tmA, A, K, M, BK, in_dtype)) return -1; }
+    if (b_mn == 0) { if (make_tmap_2d_16bit(&tmB, B, N, K, pair ? tiles.bn / 2 : (comm_pair ? BN / 2 : BN), in_dtype)) return -1; }
+    else           { if (make_tmap_2d_16bit(&tmB, B, K, N, BK, in_dtype)) return -1; }
+  }
 
   GemmParams p;
   p.C = C; p.bias = bias; p.aux = aux; p.M = M; p.N = N; p.K = K;
@@ -2265,14 +2406,21 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
     return launch_comm_pair<1, 1>(tmA, tmB, p, device, s);
   }
   if (pair) {
-    const int sms = usable_sms(device);
+    const bool swap = tiles.swap;
+    p.bn = tiles.bn;
+    if (swap) { p.M = N; p.N = M; }
+    const long long total = static_cast<long long>((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + p.bn - 1) / p.bn);
     CUtensorMap tmBh = tmB;
-    const long long pair_tiles = static_cast<long long>((tiles_m + 1) / 2) * ((N + 255) / 256);
-    if (b_mn == 0 && pair_whole_tiles(pair_tiles, sms / 2) != pair_tiles && make_tmap_2d_16bit(&tmBh, B, N, K, BN / 4, in_dtype)) return -1;
-    if (layout == 0 && epilogue >= 2) return launch_pair<0, 0, ACT_GELU>(tmA, tmB, &tmBh, p, sms, device, s);
-    if (layout == 0) return launch_pair<0, 0>(tmA, tmB, &tmBh, p, sms, device, s);
-    if (layout == 1) return launch_pair<0, 1>(tmA, tmB, &tmBh, p, sms, device, s);
-    return launch_pair<1, 1>(tmA, tmB, &tmBh, p, sms, device, s);
+    const CUtensorMap* halves = p.bn % 32 == 0 ? &tmBh : nullptr;
+    if ((b_mn == 0 || swap) && halves && pair_whole_tiles(total, sms / 2) != total &&
+        make_tmap_2d_16bit(&tmBh, swap ? A : B, p.N, K, p.bn / 4, in_dtype)) return -1;
+    if (swap && layout == 1) return launch_pair<1, 0, ACT_NONE, false, true>(tmA, tmB, halves, p, sms, device, s);
+    if (swap && epilogue >= 2) return launch_pair<0, 0, ACT_GELU, false, true>(tmA, tmB, halves, p, sms, device, s);
+    if (swap) return launch_pair<0, 0, ACT_NONE, false, true>(tmA, tmB, halves, p, sms, device, s);
+    if (layout == 0 && epilogue >= 2) return launch_pair<0, 0, ACT_GELU>(tmA, tmB, halves, p, sms, device, s);
+    if (layout == 0) return launch_pair<0, 0>(tmA, tmB, halves, p, sms, device, s);
+    if (layout == 1) return launch_pair<0, 1>(tmA, tmB, halves, p, sms, device, s);
+    return launch_pair<1, 1>(tmA, tmB, halves, p, sms, device, s);
   }
   if (splitk > 1) {
     if (layout == 0) return launch_splitk<0, 0>(tmA, tmB, p, splitk, device, s);
@@ -2347,6 +2495,7 @@ static int gemm_batched(int layout, const void* A, const void* B, void* C, void*
   p.out_dtype = out_dtype; p.in_dtype = in_dtype; p.epilogue = 0; p.accumulate = accumulate;
   p.status = status_dev; p.timeout_ns = wait_timeout_ns();
   p.ar.n = 1; p.ag.n = 1; p.tn_offset = 0; p.kb_offset = 0; p.flag_batch = 1; p.debug = 0; p.pair = 1;
+  p.bn = PAIR_BN;
   p.nb = nb; p.a_batch_rows = a_batch_rows; p.b_batch_rows = b_batch_rows; p.c_batch_rows = c_batch_rows;
   p.seg_counts = nullptr; p.seg_rows = 0; p.nseg = 0; p.mask_mode = 0;
   bool live = false;                       // only the tile rows with data are dealt out
