@@ -130,15 +130,53 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
       : "memory");
 }
 
-// 32 accumulator columns x `scale` -> 32 consecutive bf16 values
-__device__ __forceinline__ void fs_store32(__nv_bfloat16* dst, const uint32_t (&v)[32], float scale) {
+// 16 tensor-memory lanes x 32 columns: thread t gets, of columns 8 g + 2 (t % 4) and the next one, lanes t / 4 (r[4 g], r[4 g + 1])
+// and t / 4 + 8 (r[4 g + 2], r[4 g + 3]).  The store is its counterpart for pairs of columns packed into one of 32 bits.
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st_16x16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+      : : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+      : "memory");
+}
+
+// 4 x 4 transpose among the four lanes of a quad: lane j gives w[i] to lane i, which gets it as w[j].
+__device__ __forceinline__ void quad_transpose(uint32_t& w0, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
+  const bool odd = (threadIdx.x & 1) != 0, upper = (threadIdx.x & 2) != 0;
+  uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? w0 : w1, 1), b = __shfl_xor_sync(0xffffffffu, odd ? w2 : w3, 1);
+  if (odd) { w0 = a; w2 = b; } else { w1 = a; w3 = b; }
+  a = __shfl_xor_sync(0xffffffffu, upper ? w0 : w2, 2); b = __shfl_xor_sync(0xffffffffu, upper ? w1 : w3, 2);
+  if (upper) { w0 = a; w1 = b; } else { w2 = a; w3 = b; }
+}
+
+// 32 accumulator rows x 32 columns of a warp, times `scale`, as bf16: `dst` is where column 0 of row 0 goes, rows lie `pitch`
+// elements apart, the first `rows` of them exist.  A store instruction writes 64 consecutive bytes of eight rows: with a row per lane
+// it touched 32 lines with 16 bytes each, and the 64 KB of an item's dK and dV took 6900 cycles, now 3400.  One B200, with the delta
+// kernel, before / after: dK / dV of 8 x 2048, 16 heads, head_dim 128 331 / 297 us, head_dim 64 217 / 208, dQ 264 / 252.
+__device__ __forceinline__ void fs_store_block(__nv_bfloat16* dst, size_t pitch, int rows, uint32_t taddr, float scale) {
+  const int lane = threadIdx.x & 31;
+  dst += static_cast<size_t>(lane >> 2) * pitch + (lane & 3) * 8;
+  uint32_t v[32];
+  tmem_ld_16x32(taddr, v);
+  tmem_ld_16x32(taddr + (16u << 16), v + 16);
+  tmem_ld_wait(v);
 #pragma unroll
-  for (int t = 0; t < 4; ++t) {
-    uint32_t wv[4];
+  for (int e = 0; e < 4; ++e) {                       // rows lane / 4 + 8 e
+    uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      wv[i] = fs_pack(make_float2(__uint_as_float(v[t * 8 + 2 * i]) * scale, __uint_as_float(v[t * 8 + 2 * i + 1]) * scale));
-    *reinterpret_cast<uint4*>(dst + t * 8) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+    for (int g = 0; g < 4; ++g) {
+      const int i = (e >> 1) * 16 + g * 4 + (e & 1) * 2;
+      w[g] = fs_pack(make_float2(__uint_as_float(v[i]) * scale, __uint_as_float(v[i + 1]) * scale));
+    }
+    quad_transpose(w[0], w[1], w[2], w[3]);
+    if ((lane >> 2) + 8 * e < rows) *reinterpret_cast<uint4*>(dst + 8 * e * pitch) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -387,13 +425,10 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
       // dQ row r, 32 columns per quarter -> packed gradient tensor, query slot of this head
       const int g = w.head / p.qpk, jq = w.head % p.qpk;
       if (quarter < HD / 32) {
-        uint32_t v[32];
-        tmem_ld_32x32(tm_dq + lane_base + quarter * 32, v);
-        tmem_ld_wait();
-        if (srow < p.S) {
-          const size_t pos = static_cast<size_t>(w.b) * p.S + srow;
-          fs_store32(p.dqkv + ((pos * p.G + g) * (p.qpk + 2) + jq) * HD + quarter * 32, v, p.scale);
-        }
+        const int row0 = w.i * 128 + q4 * 32;           // the warp's first query
+        const size_t pos = static_cast<size_t>(w.b) * p.S + row0;
+        fs_store_block(p.dqkv + ((pos * p.G + g) * (p.qpk + 2) + jq) * HD + quarter * 32, static_cast<size_t>(p.G) * (p.qpk + 2) * HD,
+                       p.S - row0, tm_dq + lane_base + quarter * 32, p.scale);
       }
       // the next item's first dQ MMA overwrites these columns; it waits for ds_full, which this thread arrives on
       // after these reads
@@ -617,20 +652,23 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
     }
    }
   } else {
-    // ------------------------------------------------------------------ P^T, dS^T: thread = (key row, 32 of the step's 64 queries)
+    // ------------------------------------------------------------------ P^T, dS^T: warp = 32 keys x 32 of the step's 64 queries
     // Warps 4-11 take the steps of score buffer 0 (first 64 queries of every tile), warps 12-19 those of buffer 1.
     // P^T is handed on before dP^T is waited for: the first MMA warp then issues dV and the next scores while the threads
     // still work on dS^T, and each warp's chain (scores -> P -> dV, dP -> dS -> dK) is its own.  One B200, this kernel with the
     // delta kernel, both handed on together / one by one: 1 x 4096, 32 heads over 8, head_dim 128 258 / 229 us, 1 x 777 62.3 /
     // 55, 8 x 2048, 16 heads, head_dim 64 252 / 244.  The dQ kernel gains nothing from the same split (22.0 / 21.9, 176 / 176).
+    // A thread has 4 keys x 8 queries of the block (tmem_ld_16x32) and reads 8 + 8 values of -lse and -delta: with a key and all 32
+    // queries per thread it read 64, and their broadcasts took 1000 of the 3600 cycles of shared-memory bandwidth that a tile
+    // needs, which is what bounds this kernel.  8 x 2048, 16 heads, head_dim 128 350 / 335 us, head_dim 64 247 / 217.
     asm volatile(FS_REGS_SOFTMAX);
     const int q4 = warp & 3;
     const int hq = (warp - 4) >> 3;
     const int half = ((warp - 4) >> 2) & 1;
-    const int r = q4 * 32 + lane;                     // key row inside the tile
     const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
     const uint32_t t_s = tmem_base + lane_base + hq * 64 + half * 32, t_dp = t_s + 128;
-    const int qc0 = hq * 64 + half * 32;              // first query column of this thread inside the tile
+    // first key row and query column of this thread's scores inside the tile (tmem_ld_16x32)
+    const int r0 = q4 * 32 + (lane >> 2), qc = hq * 64 + half * 32 + (lane & 3) * 2;
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     bool ok = true;
     uint32_t tq = 0;                                  // query tiles so far: this buffer's steps, ring stage and phases
@@ -646,31 +684,31 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
             !mbar_wait(&t_full[hq], tq & 1, abort_flag, timeout)) { ok = false; break; }
         tcgen05_fence_after();
         uint32_t sv[32];
-        tmem_ld_32x32(t_s, sv);
+        tmem_ld_16x32(t_s, sv);
+        tmem_ld_16x32(t_s + (16u << 16), sv + 16);
         tmem_ld_wait(sv);
-        const float4* lv = reinterpret_cast<const float4*>(lse_s + st * 256 + qc0);
-        const float4* dvv = reinterpret_cast<const float4*>(lse_s + st * 256 + 128 + qc0);
         if (diag) {                                   // the key lies after the query: probability 0
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (r > qc0 + i) sv[i] = 0xff800000u;
+            if (r0 + (i >> 4) * 16 + ((i >> 1) & 1) * 8 > qc + ((i >> 2) & 3) * 8 + (i & 1)) sv[i] = 0xff800000u;
         }
+        const float* lv = lse_s + st * 256 + qc;
         float2 pr[16];
         uint32_t pk[16];
 #pragma unroll
-        for (int v4 = 0; v4 < 8; ++v4) {
-          const float4 l4 = lv[v4];
+        for (int g = 0; g < 4; ++g) {
+          const float2 nl2 = *reinterpret_cast<const float2*>(lv + g * 8);
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int i = v4 * 2 + e;
-            const float2 nl2 = e ? make_float2(l4.z, l4.w) : make_float2(l4.x, l4.y);
+          for (int e = 0; e < 4; ++e) {               // 16 lanes each e >> 1, 8 lanes each e & 1
+            const int i = (e >> 1) * 8 + g * 2 + (e & 1);
             const float2 x = __ffma2_rn(make_float2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), sc2, nl2);
             pr[i] = make_float2(exp2f(x.x), exp2f(x.y));
             pk[i] = fs_pack(pr[i]);
           }
         }
-        // into this thread's own score columns: the other half's thread of the row may not have read its scores yet
-        tmem_st_32x16(t_s, pk);
+        // into this warp's own score columns: the other half's warp may not have read its scores yet
+        tmem_st_16x16(t_s, pk);
+        tmem_st_16x16(t_s + (16u << 16), pk + 8);
         tmem_st_wait();
         tcgen05_fence_before();
         __syncwarp();
@@ -678,20 +716,21 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
         if (!mbar_wait(&t_full[2 + hq], tq & 1, abort_flag, timeout)) { ok = false; break; }
         tcgen05_fence_after();
         uint32_t dv[32];
-        tmem_ld_32x32(t_dp, dv);
+        tmem_ld_16x32(t_dp, dv);
+        tmem_ld_16x32(t_dp + (16u << 16), dv + 16);
         tmem_ld_wait(dv);
 #pragma unroll
-        for (int v4 = 0; v4 < 8; ++v4) {
-          const float4 d4 = dvv[v4];
+        for (int g = 0; g < 4; ++g) {
+          const float2 nd2 = *reinterpret_cast<const float2*>(lv + 128 + g * 8);
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int i = v4 * 2 + e;
-            const float2 nd2 = e ? make_float2(d4.z, d4.w) : make_float2(d4.x, d4.y);
+          for (int e = 0; e < 4; ++e) {
+            const int i = (e >> 1) * 8 + g * 2 + (e & 1);
             const float2 t2 = __fadd2_rn(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), nd2);
             pk[i] = fs_pack(__fmul2_rn(pr[i], t2));   // the softmax scale is applied to the finished dK
           }
         }
-        tmem_st_32x16(t_dp, pk);
+        tmem_st_16x16(t_dp, pk);
+        tmem_st_16x16(t_dp + (16u << 16), pk + 8);
         tmem_st_wait();
         tcgen05_fence_before();
         __syncwarp();
@@ -702,19 +741,15 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
       }
       if (!ok || !mbar_wait(acc_done, it & 1, abort_flag, timeout)) { ok = false; break; }
       tcgen05_fence_after();
-      // half 0 stores dK row r, half 1 stores dV row r into the key / value slots of the packed gradient tensor; the
+      // half 0 stores dK, half 1 stores dV, each warp 32 rows, into the key / value slots of the packed gradient tensor; the
       // warps of buffer 0 take the even, those of buffer 1 the odd 32-column blocks
-      const int krow = w.jt * 128 + r;
-      const size_t kvpos = static_cast<size_t>(w.b) * p.S + krow;
+      const int row0 = w.jt * 128 + q4 * 32;            // the warp's first key
+      const size_t kvpos = static_cast<size_t>(w.b) * p.S + row0;
       __nv_bfloat16* dst = p.dqkv + ((kvpos * p.G + w.g) * (p.qpk + 2) + p.qpk + half) * HD;
       const uint32_t src = tmem_base + lane_base + (half ? 384 : 256);
 #pragma unroll
-      for (int cc = hq; cc < HD / 32; cc += 2) {
-        uint32_t v[32];
-        tmem_ld_32x32(src + cc * 32, v);
-        tmem_ld_wait();
-        if (krow < p.S) fs_store32(dst + cc * 32, v, half ? 1.f : p.scale);
-      }
+      for (int cc = hq; cc < HD / 32; cc += 2)
+        fs_store_block(dst + cc * 32, static_cast<size_t>(p.G) * (p.qpk + 2) * HD, p.S - row0, src + cc * 32, half ? 1.f : p.scale);
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_free);
