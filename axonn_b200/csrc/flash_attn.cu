@@ -435,26 +435,14 @@ fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams
       tcgen05_fence_after();
       const float inv_l = 1.f / (RAGGED ? lr : l);
       const size_t heads = static_cast<size_t>(p.G) * p.qpk;
-      const int qpos = (2 * w.u + x) * FA_BQ + r;
-      const size_t qrow = static_cast<size_t>(w.b) * p.S + qpos;
-      __nv_bfloat16* dst = p.out + (qrow * heads + w.head) * HD;
+      const int row0 = (2 * w.u + x) * FA_BQ + q4 * 32, qpos = row0 + lane;
+      float inv[4];                                    // of the rows that this thread stores
 #pragma unroll
-      for (int c = 0; c < HD / 32; ++c) {
-        uint32_t v[32];
-        tmem_ld_32x32(o_addr + c * 32, v);
-        tmem_ld_wait();
+      for (int e = 0; e < 4; ++e) inv[e] = __shfl_sync(0xffffffffu, inv_l, (lane >> 2) + 8 * e);
+      __nv_bfloat16* dst = p.out + ((static_cast<size_t>(w.b) * p.S + row0) * heads + w.head) * HD;
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          uint32_t wv[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int e = t * 8 + i * 2;
-            const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[e]) * inv_l, __uint_as_float(v[e + 1]) * inv_l);
-            wv[i] = *reinterpret_cast<const uint32_t*>(&h);
-          }
-          if (!RAGGED || qpos < p.S) *reinterpret_cast<uint4*>(dst + c * 32 + t * 8) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-        }
-      }
+      for (int c = 0; c < HD / 32; ++c)
+        store_rows_bf16(dst + c * 32, heads * HD, RAGGED ? p.S - row0 : 32, o_addr + c * 32, inv);
       if (!RAGGED || qpos < p.S)
         p.lse[(static_cast<size_t>(w.b) * heads + w.head) * p.S + qpos] = (m + log2f(l)) * 0.6931471805599453f;
       // the next item's first PV MMA overwrites O: it waits for this thread's next arrival on p_full, which follows

@@ -130,54 +130,12 @@ __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r
       : "memory");
 }
 
-// 16 tensor-memory lanes x 32 columns: thread t gets, of columns 8 g + 2 (t % 4) and the next one, lanes t / 4 (r[4 g], r[4 g + 1])
-// and t / 4 + 8 (r[4 g + 2], r[4 g + 3]).  The store is its counterpart for pairs of columns packed into one of 32 bits.
-__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
+// Counterpart of tmem_ld_16x32 for pairs of columns packed into one of 32 bits.
 __device__ __forceinline__ void tmem_st_16x16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
       : : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
       : "memory");
-}
-
-// 4 x 4 transpose among the four lanes of a quad: lane j gives w[i] to lane i, which gets it as w[j].
-__device__ __forceinline__ void quad_transpose(uint32_t& w0, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
-  const bool odd = (threadIdx.x & 1) != 0, upper = (threadIdx.x & 2) != 0;
-  uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? w0 : w1, 1), b = __shfl_xor_sync(0xffffffffu, odd ? w2 : w3, 1);
-  if (odd) { w0 = a; w2 = b; } else { w1 = a; w3 = b; }
-  a = __shfl_xor_sync(0xffffffffu, upper ? w0 : w2, 2); b = __shfl_xor_sync(0xffffffffu, upper ? w1 : w3, 2);
-  if (upper) { w0 = a; w1 = b; } else { w2 = a; w3 = b; }
-}
-
-// 32 accumulator rows x 32 columns of a warp, times `scale`, as bf16: `dst` is where column 0 of row 0 goes, rows lie `pitch`
-// elements apart, the first `rows` of them exist.  A store instruction writes 64 consecutive bytes of eight rows: with a row per lane
-// it touched 32 lines with 16 bytes each, and the 64 KB of an item's dK and dV took 6900 cycles, now 3400.  One B200, with the delta
-// kernel, before / after: dK / dV of 8 x 2048, 16 heads, head_dim 128 331 / 297 us, head_dim 64 217 / 208, dQ 264 / 252.
-__device__ __forceinline__ void fs_store_block(__nv_bfloat16* dst, size_t pitch, int rows, uint32_t taddr, float scale) {
-  const int lane = threadIdx.x & 31;
-  dst += static_cast<size_t>(lane >> 2) * pitch + (lane & 3) * 8;
-  uint32_t v[32];
-  tmem_ld_16x32(taddr, v);
-  tmem_ld_16x32(taddr + (16u << 16), v + 16);
-  tmem_ld_wait(v);
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {                       // rows lane / 4 + 8 e
-    uint32_t w[4];
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      const int i = (e >> 1) * 16 + g * 4 + (e & 1) * 2;
-      w[g] = fs_pack(make_float2(__uint_as_float(v[i]) * scale, __uint_as_float(v[i + 1]) * scale));
-    }
-    quad_transpose(w[0], w[1], w[2], w[3]);
-    if ((lane >> 2) + 8 * e < rows) *reinterpret_cast<uint4*>(dst + 8 * e * pitch) = make_uint4(w[0], w[1], w[2], w[3]);
-  }
 }
 
 // Work item k of this CTA: query tiles sorted by decreasing length (tile i walks i + 1 key tiles), dealt to the
@@ -427,8 +385,9 @@ fa_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constan
       if (quarter < HD / 32) {
         const int row0 = w.i * 128 + q4 * 32;           // the warp's first query
         const size_t pos = static_cast<size_t>(w.b) * p.S + row0;
-        fs_store_block(p.dqkv + ((pos * p.G + g) * (p.qpk + 2) + jq) * HD + quarter * 32, static_cast<size_t>(p.G) * (p.qpk + 2) * HD,
-                       p.S - row0, tm_dq + lane_base + quarter * 32, p.scale);
+        const float scale[4] = {p.scale, p.scale, p.scale, p.scale};
+        store_rows_bf16(p.dqkv + ((pos * p.G + g) * (p.qpk + 2) + jq) * HD + quarter * 32, static_cast<size_t>(p.G) * (p.qpk + 2) * HD,
+                        p.S - row0, tm_dq + lane_base + quarter * 32, scale);
       }
       // the next item's first dQ MMA overwrites these columns; it waits for ds_full, which this thread arrives on
       // after these reads
@@ -747,9 +706,10 @@ fa_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_consta
       const size_t kvpos = static_cast<size_t>(w.b) * p.S + row0;
       __nv_bfloat16* dst = p.dqkv + ((kvpos * p.G + w.g) * (p.qpk + 2) + p.qpk + half) * HD;
       const uint32_t src = tmem_base + lane_base + (half ? 384 : 256);
+      const float sc = half ? 1.f : p.scale, scale[4] = {sc, sc, sc, sc};
 #pragma unroll
       for (int cc = hq; cc < HD / 32; cc += 2)
-        fs_store_block(dst + cc * 32, static_cast<size_t>(p.G) * (p.qpk + 2) * HD, p.S - row0, src + cc * 32, half ? 1.f : p.scale);
+        store_rows_bf16(dst + cc * 32, static_cast<size_t>(p.G) * (p.qpk + 2) * HD, p.S - row0, src + cc * 32, scale);
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_free);
