@@ -32,7 +32,7 @@ from torch.autograd import Function
 from .. import axonn as ax
 from .. import ops
 from ..ops import _lib
-from ..ops.direct import no_graph, own_forward
+from ..ops.direct import host_paths, no_graph, own_forward
 from ..parallel import fused
 from ..utils import divide
 from . import overlap_communication as oc
@@ -394,6 +394,9 @@ class Linear(torch.nn.Module):
         if b is not None and (not self.expert_mode or self.skip_bias_add or b.dtype != w.dtype):
             return None
         n, k = self.local_out_features, self.local_in_features
+        host = host_paths() if x.is_cuda else None
+        if host is not None:
+            return host.linear(x, w, b, n, k, activation is not None)
         if (n % 8 or k % 8 or x.dtype != w.dtype or w.dtype not in (torch.bfloat16, torch.float16) or x.dim() == 0
                 or x.shape[-1] != k or w.shape != (n * k,) or x.numel() == 0 or not no_graph(x, w, b)
                 or not x.is_contiguous() or not w.is_contiguous() or torch.is_autocast_enabled("cuda")):

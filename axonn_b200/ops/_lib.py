@@ -3,7 +3,8 @@
 The kernels are plain ``extern "C"`` launchers compiled by nvcc for sm_100a
 (see ``axonn_b200/utils/build.py``); they are called through ctypes with raw
 device pointers and the current CUDA stream, so the library has no dependency
-on the PyTorch C++ ABI.  On a machine with a GPU a missing library is an error,
+on the PyTorch C++ ABI; the host paths of calls that are bound by host time are
+a module of their own, which has (``host``).  On a machine with a GPU a missing library is an error,
 never a silent fallback.
 """
 
@@ -25,8 +26,18 @@ LIB_PATH = os.environ.get("AXONN_LIB_PATH") or (
     _DEBUG_LIB if os.environ.get("AXONN_DEBUG_BOUNDS", "0") not in ("", "0") and os.path.exists(_DEBUG_LIB)
     else os.path.join(LIB_DIR, "libaxonn_b200.so"))
 
-# number of kernels launched through this library since the last reset
-launch_count = 0
+# Kernels launched through this library since the last reset are ``launch_count`` (see ``__getattr__``): those counted here and
+# those of the native host paths.
+_launches = 0
+_HOST = _UNSET = object()
+_HOST_LAUNCHERS = ("axb_norm_fwd", "axb_norm_bwd", "axb_add_norm_fwd", "axb_add_norm_bwd", "axb_norm_grid", "axb_gemm",
+                   "axb_flash_attn_fwd", "axb_last_error")
+
+
+def __getattr__(name):
+    if name == "launch_count":
+        return _launches + (_HOST.launches() if _HOST is not _UNSET and _HOST is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 class KernelError(RuntimeError):
@@ -112,6 +123,37 @@ def lib():
     return _LIB
 
 
+def host():
+    """The native host paths (``csrc/host_ops.cpp``), bound to the loaded library; ``None`` where they have not been built for this
+    PyTorch (or ``AXONN_HOST_OPS=0``): the Python code beside every use of them launches the same kernels."""
+    return _HOST if _HOST is not _UNSET else _load_host()
+
+
+def _load_host():
+    global _HOST
+    L = lib()
+    with _LOCK:
+        if _HOST is _UNSET:
+            import importlib.util
+
+            from ..utils.build import host_path
+
+            path, module = host_path(), None
+            if os.environ.get("AXONN_HOST_OPS", "1") != "0" and os.path.exists(path):
+                spec = importlib.util.spec_from_file_location("axonn_host", path)
+                try:
+                    module = importlib.util.module_from_spec(spec)
+                    spec.loader.exec_module(module)
+                except ImportError as e:
+                    warnings.warn(f"the native host paths do not load ({e}); rebuild them (axonn_b200/utils/build.py)", stacklevel=2)
+                    module = None
+                else:
+                    module.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in _HOST_LAUNCHERS}, KernelError,
+                                torch.nn.Parameter)
+            _HOST = module
+    return _HOST
+
+
 def set_wait_timeout_ms(ms: int):
     """Deadline of every device-side wait (mbarrier, peer flag).  A kernel whose wait runs out returns and
     reports through the status word (``check_status``).  Default 120000 ms; ``AXONN_COMM_TIMEOUT_MS`` sets it
@@ -144,21 +186,21 @@ def ptr(t) -> ctypes.c_void_p:
 
 
 def check(status: int, what: str):
-    global launch_count
+    global _launches
     if status != 0:
         msg = lib().axb_last_error()
         raise KernelError(f"{what} failed (status {status}): {msg.decode() if msg else ''}")
-    launch_count += 1
+    _launches += 1
 
 
 def add_launches(n: int):
-    global launch_count
-    launch_count += n
+    global _launches
+    _launches += n
 
 
 def reset_launch_count():
-    global launch_count
-    launch_count = 0
+    global _launches
+    _launches = -_HOST.launches() if _HOST is not _UNSET and _HOST is not None else 0
 
 
 _STATUS_NAMES = {

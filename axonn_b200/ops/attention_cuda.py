@@ -11,7 +11,7 @@ import torch
 from torch.autograd.function import once_differentiable
 
 from . import _lib
-from .direct import no_graph
+from .direct import host_paths, no_graph
 
 _BWD_DEFAULT = "split"
 
@@ -116,6 +116,11 @@ class _FlashPacked(torch.autograd.Function):
 
 def flash_attention_packed_cuda(qkv, causal, scale):
     assert causal
+    host = host_paths()
+    if host is not None:
+        out = host.attention(qkv, scale)
+        if out is not None:
+            return out
     if no_graph(qkv):
         return flash_fwd_packed(qkv, scale)[0]
     return _FlashPacked.apply(qkv, scale)

@@ -6,6 +6,8 @@ and evaluating a model without gradients is bound by host time for short prompts
 import torch
 from torch.autograd import forward_ad
 
+from . import _lib
+
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
 _module = torch.nn.modules.module
 _CALL = torch.nn.Module.__call__
@@ -32,6 +34,12 @@ def plain_tensors(*tensors) -> bool:
             return False
     return (not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None
             and forward_ad._current_level < 0 and not torch.compiler.is_compiling())
+
+
+def host_paths():
+    """The native host paths (``_lib.host``) while neither a compiler nor a forward-mode level is active - they ask everything else
+    themselves -, otherwise ``None``."""
+    return None if forward_ad._current_level >= 0 or torch.compiler.is_compiling() else _lib.host()
 
 
 def own_forward(cls):

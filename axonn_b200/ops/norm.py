@@ -12,7 +12,7 @@ import torch
 import torch.distributed as dist
 
 from . import _lib
-from .direct import no_graph
+from .direct import host_paths, no_graph
 
 _DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
@@ -261,28 +261,40 @@ def _norm_direct(x, delta, gamma, beta, eps, rms, group):
     return h, y
 
 
+def _norm(x, delta, gamma, beta, eps, rms, group):
+    """``norm(x)``, or ``(h, norm(h))`` of ``h = x + delta``.  On one rank the questions, the launches and the autograd node are native
+    (one B200, host-bound, forward and backward of 16 rows: RMSNorm 111 -> 74 us, LayerNorm with the residual 131 -> 91)."""
+    host = host_paths() if x.is_cuda and _group_size(group) == 1 else None
+    if host is not None:
+        out = host.norm(x, delta, gamma, beta, eps, rms)
+        if out is not None:
+            return out
+    direct = _norm_direct(x, delta, gamma, beta, eps, rms, group)
+    if delta is not None:
+        return direct or _AddNormFn.apply(x, delta, gamma, beta, eps, rms, group)
+    return _NormFn.apply(x, gamma, beta, eps, rms, group) if direct is None else direct[1]
+
+
 def add_layer_norm(x, delta, gamma, beta, eps=1e-5, group=None):
     """``h = x + delta; y = LayerNorm(h)`` in one kernel; returns ``(h, y)``."""
-    return _norm_direct(x, delta, gamma, beta, eps, False, group) or _AddNormFn.apply(x, delta, gamma, beta, eps, False, group)
+    return _norm(x, delta, gamma, beta, eps, False, group)
 
 
 def add_rms_norm(x, delta, gamma, eps=1e-6, group=None):
     """``h = x + delta; y = RMSNorm(h)`` in one kernel; returns ``(h, y)``."""
-    return _norm_direct(x, delta, gamma, None, eps, True, group) or _AddNormFn.apply(x, delta, gamma, None, eps, True, group)
+    return _norm(x, delta, gamma, None, eps, True, group)
 
 
 def layer_norm(x, gamma, beta, eps=1e-5, group=None):
     """LayerNorm over the last dimension; with ``group`` the last dimension is one
     shard of a hidden dimension split over that process group."""
-    direct = _norm_direct(x, None, gamma, beta, eps, False, group)
-    return _NormFn.apply(x, gamma, beta, eps, False, group) if direct is None else direct[1]
+    return _norm(x, None, gamma, beta, eps, False, group)
 
 
 def rms_norm(x, gamma, eps=1e-6, group=None):
     """RMSNorm over the last dimension; with ``group`` the last dimension is one shard of a hidden dimension
     split over that process group."""
-    direct = _norm_direct(x, None, gamma, None, eps, True, group)
-    return _NormFn.apply(x, gamma, None, eps, True, group) if direct is None else direct[1]
+    return _norm(x, None, gamma, None, eps, True, group)
 
 
 def column_sum(x, out_dtype=torch.float32):

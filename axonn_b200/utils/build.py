@@ -19,6 +19,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 OBJ_DIR = os.path.join(LIB_DIR, "obj")
 LIB_PATH = os.path.join(LIB_DIR, "libaxonn_b200.so")
+HOST_SRC = os.path.join(CSRC, "host_ops.cpp")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -44,6 +45,39 @@ def _newest_input():
 
 def up_to_date():
     return os.path.exists(LIB_PATH) and os.path.getmtime(LIB_PATH) >= _newest_input()
+
+
+def host_path():
+    """Where the native host paths are for this PyTorch and this Python, whose C++ interfaces they use."""
+    import torch
+
+    return os.path.join(LIB_DIR, f"axonn_host-{torch.__version__}-{sys.implementation.cache_tag}.so")
+
+
+def build_host(force=False):
+    """The native host paths (``csrc/host_ops.cpp``): a Python module against PyTorch's C++ API, without device code."""
+    out = host_path()
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= os.path.getmtime(HOST_SRC):
+        return out
+    import sysconfig
+
+    import torch
+
+    gxx = shutil.which("g++")
+    if gxx is None:
+        raise RuntimeError("g++ not found: cannot build axonn_b200's native host paths")
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    dirs = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+            sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = [gxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += ["-I" + d for d in dirs] + [HOST_SRC, "-o", out + ".tmp", "-L" + os.path.join(root, "lib")]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    os.replace(out + ".tmp", out)
+    return out
 
 
 def _compile(src, verbose):
@@ -80,10 +114,13 @@ def build_variant(out_path, extra_flags, obj_dir):
 
 def build_library(force=False, verbose=True):
     if not force and up_to_date():
+        build_host()
         return LIB_PATH
     os.makedirs(OBJ_DIR, exist_ok=True)
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as ex:
+        host = ex.submit(build_host, force)
         results = list(ex.map(lambda s: _compile(s, verbose), sources()))
+        host.result()
     objs = [o for o, _ in results]
     log = "\n".join(l for _, l in results if l)
     with open(os.path.join(LIB_DIR, "ptxas.log"), "a") as f:
