@@ -151,9 +151,20 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* t
       : : "r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
+// Fetches a tile into the L2.  The L2 is where every writer's data is, so a tile may be fetched before its writer has finished.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* tmap, int32_t c0, int32_t c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1) : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }
+
+// --- programmatic dependent launch.  A kernel launched with the attribute may start before its predecessor in the stream has
+// ended, once all of that one's CTAs have called pdl_launch_next or ended (at its end, if it never calls it); pdl_wait returns when
+// the predecessor has ended and its writes are visible.  Every thread that reads or writes global memory calls pdl_wait first, and a
+// CTA calls pdl_launch_next after its tensor memory is allocated: a CTA of the next kernel may be given what is left.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // --- tcgen05 / TMEM
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {

@@ -215,6 +215,25 @@ __device__ __forceinline__ void store_vec8(void* base, int out_dtype, size_t off
   }
 }
 
+// The same for 4 elements (offset a multiple of 4).
+__device__ __forceinline__ void store_vec4(void* base, int out_dtype, size_t off, const float (&v)[4], bool accumulate) {
+  float f[4] = {v[0], v[1], v[2], v[3]};
+  if (out_dtype == 2) {
+    float4* p = reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + off);
+    if (accumulate) { const float4 o = *p; f[0] += o.x; f[1] += o.y; f[2] += o.z; f[3] += o.w; }
+    *p = make_float4(f[0], f[1], f[2], f[3]);
+  } else {
+    uint2* p = reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(base) + off);
+    if (accumulate) {
+      const uint2 o = *p;
+      float a, b;
+      unpack2(o.x, out_dtype, a, b); f[0] += a; f[1] += b;
+      unpack2(o.y, out_dtype, a, b); f[2] += a; f[3] += b;
+    }
+    *p = make_uint2(pack2(f[0], f[1], out_dtype), pack2(f[2], f[3], out_dtype));
+  }
+}
+
 // One 32-byte sector per thread.  A thread of the epilogue owns a row of the tile, so the lanes of a store lie a row pitch
 // apart and nothing merges them before the L2: with 16-byte stores it received every sector as two partial writes, beside
 // the operand tiles that it serves all the time.  One B200, bf16, back to back, 16 -> 32 bytes: 16384 x 8192 x 2048 with GELU
@@ -1780,21 +1799,21 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 // Plain GEMM for problems with too few 128x128 tiles to occupy the GPU (a short prompt through a wide layer, weight
 // gradients of narrow layers): a cluster of Z CTAs shares one output tile, CTA z multiplies its part of the K blocks
 // into its own TMEM accumulator, and the fp32 partials are summed through distributed shared memory - every CTA leaves
-// its partial in its (drained) operand ring and finishes 128 / Z columns of the tile from all Z of them, in rank order.
-// No workspace, no atomics, one launch.  Such a problem is bound by reading the weights once; with one CTA per tile
-// the loads of tiles < SMs / 2 CTAs in flight do not fill the memory system.
-// Measured on a B200 (graph replay, bias epilogue): 24 x 8192 x 2048 22.0 -> 12.4 us, 24 x 2048 x 8192 31.7 -> 10.7 us (33.5 MB
-// of weights each).  splitk_ctas says when it is taken.
+// its partial in its (drained) operand ring and finishes 1 / Z of the tile's rows from all Z of them, in rank order.
+// No workspace, no atomics, one launch.  Such a problem is bound by reading the weights once and by what stands around that
+// (launch, first loads, exchange): the ring holds the rows that A has instead of 128 and with them up to nine stages of
+// weights, and the kernel is launched while its predecessor still runs (pdl_wait).  Two products in turn, 24 tokens, 2048 -> 8192 ->
+// 2048, weights from DRAM: 26.5 -> 19.5 us on one B200 (their 67 MB take 10.2).  splitk_ctas says when it is taken.
 constexpr int SK_THREADS = 192;   // TMA warp, MMA warp, 4 epilogue warps
 struct SplitKSmem {
   static constexpr int BN = 128;
-  static constexpr int A_BYTES = BM * BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2;
-  static constexpr int STAGES = 6;
+  static constexpr int B_BYTES = BN * BK * 2;
+  static constexpr int MAX_STAGES = 9;
   static constexpr int PART_LD = BN + 4;           // floats per partial row: 16-byte words of 8 rows hit all banks
-  static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
-  static constexpr int TOTAL = BAR_OFFSET + (2 * STAGES + 1) * 8 + 16 + 1024 /* alignment slack */;
-  static_assert(BM * PART_LD * 4 <= BAR_OFFSET, "the partial tile lies in the operand ring");
+  static constexpr int BAR_BYTES = (2 * MAX_STAGES + 1) * 8 + 16;
+  // one CTA per SM, or two
+  __host__ __device__ static constexpr int ring(bool small) { return small ? 100 * 1024 : 192 * 1024; }
+  __host__ __device__ static constexpr int total(bool small) { return ring(small) + BAR_BYTES + 1024 /* alignment slack */; }
 };
 
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_smem_addr, uint32_t cta) {
@@ -1805,17 +1824,70 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_smem_addr, uint32
   return v;
 }
 
+// CTA z of Z finishes its share of the tile's rows: the partials of all CTAs summed in rank order, bias, GELU, store.  A warp reads
+// whole rows of a partial (four columns per lane) and a thread has eight loads under way; with 1 / Z of the columns of every row the
+// reads were 64 bytes each, one after the other.  One B200, cold weights, 24 x 8192 x 2048 and 24 x 2048 x 8192 in turn: 22.7 ->
+// 19.8 us, 100 x 4096 x 1024 and 100 x 1024 x 4096 (z 4 and 8) 32.3 -> 15.
+template <int Z>
+__device__ __forceinline__ void splitk_finish(const GemmParams& p, uint32_t base, int z, int tm, int tn) {
+  using S = SplitKSmem;
+  constexpr int R = 8 / Z, GROUPS = S::BN / 4;                // rows at a time, column groups of a row
+  const int rows = min(BM, p.M - tm * BM), share = (rows + Z - 1) / Z, row0 = z * share, mine = min(share, rows - row0);
+  const bool biased = p.epilogue == 1 || p.epilogue == 2;
+  for (int u = threadIdx.x; u < (mine + R - 1) / R * GROUPS; u += SK_THREADS) {
+    const int row = row0 + u / GROUPS * R, c = u % GROUPS * 4, col = tn * S::BN + c;
+    if (col >= p.N) continue;                                 // N is a multiple of 8
+    uint32_t bias[2] = {};
+    if (biased) {
+      const uint16_t* src = reinterpret_cast<const uint16_t*>(p.bias) + col;
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        bias[i] = static_cast<uint32_t>(__ldg(src + 2 * i)) | (static_cast<uint32_t>(__ldg(src + 2 * i + 1)) << 16);
+    }
+    float4 a[R][Z];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int j = 0; j < Z; ++j)
+        if (row + r < row0 + mine) a[r][j] = ld_cluster_f4(base + ((row + r) * S::PART_LD + c) * 4, j);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (row + r >= row0 + mine) break;
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < Z; ++j) { v[0] += a[r][j].x; v[1] += a[r][j].y; v[2] += a[r][j].z; v[3] += a[r][j].w; }
+      if (biased) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float x, y;
+          unpack2(bias[i], p.in_dtype, x, y);
+          v[2 * i] += x; v[2 * i + 1] += y;
+        }
+      }
+      const size_t off = static_cast<size_t>(tm * BM + row + r) * p.N + col;
+      if (p.epilogue >= 2) {
+        if (p.aux != nullptr) store_vec4(p.aux, p.out_dtype, off, v, false);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = gelu_tanh(v[i]);
+      }
+      store_vec4(p.C, p.out_dtype, off, v, p.accumulate != 0);
+    }
+  }
+}
+
 template <int A_MN, int B_MN>
-__global__ void __launch_bounds__(SK_THREADS, 1)
+__global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p,
-                   int z_ctas) {
+                   int z_ctas, int rows_a, bool small_rings) {
+  const int arows = A_MN ? BM : rows_a;               // a K-major A only: otherwise all is known to the compiler
+  const bool small = !A_MN && small_rings;
   using S = SplitKSmem;
   constexpr int BN = S::BN;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::BAR_OFFSET);
-  uint64_t* empty_bar = full_bar + S::STAGES;
-  uint64_t* acc_full = empty_bar + S::STAGES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::ring(small));
+  uint64_t* empty_bar = full_bar + S::MAX_STAGES;
+  uint64_t* acc_full = empty_bar + S::MAX_STAGES;
   uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
 
@@ -1827,9 +1899,11 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const int kb0 = static_cast<int>(static_cast<long long>(num_kb) * z / z_ctas);
   const int kb1 = static_cast<int>(static_cast<long long>(num_kb) * (z + 1) / z_ctas);
   const uint64_t timeout = p.timeout_ns;
+  // rows of A past arows are whatever lies in the ring behind them: they make rows of the accumulator that nothing reads
+  const int a_bytes = arows * BK * 2, stage_bytes = a_bytes + S::B_BYTES, stages = min(S::MAX_STAGES, S::ring(small) / stage_bytes);
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < S::STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
+    for (int i = 0; i < S::MAX_STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     fence_mbar_init();
@@ -1840,17 +1914,23 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_launch_next();
 
   if (warp == 0) {
     if (elect_one()) {
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       const int m0 = tm * BM, n0 = tn * BN;
+      if (B_MN == 0) {
+        // the first weights into the L2 while the predecessor is still at work (all of them: slower, they pass twice)
+        for (int kb = kb0; kb < min(kb1, kb0 + 2); ++kb) tma_prefetch_2d(&tmB, kb * BK, n0);
+      }
+      pdl_wait();
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, timeout)) { ok = false; break; }
-        uint8_t* sA = smem + stage * S::STAGE_BYTES;
-        uint8_t* sB = sA + S::A_BYTES;
-        mbar_expect_tx(&full_bar[stage], S::STAGE_BYTES);
+        uint8_t* sA = smem + stage * stage_bytes;
+        uint8_t* sB = sA + a_bytes;
+        mbar_expect_tx(&full_bar[stage], stage_bytes);
         const int k0 = kb * BK;
         if (A_MN == 0) {
           tma_load_2d(sA, &tmA, &full_bar[stage], k0, m0);
@@ -1864,7 +1944,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 #pragma unroll
           for (int j = 0; j < BN / 64; ++j) tma_load_2d(sB + j * (BK * 128), &tmB, &full_bar[stage], n0 + 64 * j, k0);
         }
-        if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
+        if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();     // give in-flight copies time to land before the CTA exits
@@ -1882,13 +1962,13 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(&full_bar[stage], phase, abort_flag, timeout)) { ok = false; break; }
         tcgen05_fence_after();
-        const uint32_t a_addr = smem_u32(smem + stage * S::STAGE_BYTES), b_addr = a_addr + S::A_BYTES;
+        const uint32_t a_addr = smem_u32(smem + stage * stage_bytes), b_addr = a_addr + a_bytes;
 #pragma unroll
         for (int k = 0; k < BK / UMMA_K; ++k)
           umma_f16(tmem_base, umma_smem_desc(a_addr + k * a_kstep, a_lbo, 1024), umma_smem_desc(b_addr + k * b_kstep, b_lbo, 1024),
                    idesc, (kb == kb0 && k == 0) ? 0u : 1u);
         umma_commit(&empty_bar[stage]);
-        if (++stage == S::STAGES) { stage = 0; phase ^= 1; }
+        if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if (ok) umma_commit(acc_full);
       else {
@@ -1924,34 +2004,11 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   if (warp == 1) { __syncwarp(); tcgen05_fence_after(); tmem_dealloc(tmem_base, BN); }
   __syncwarp();
   cluster_sync_all();                 // all partials of the tile are in shared memory
+  pdl_wait();
   if (*abort_flag == 0) {
-    const int groups = BN / 8 / z_ctas;                       // 8-column groups finished by this CTA
-    const int rows = min(BM, p.M - tm * BM);
-    const uint32_t base = smem_u32(smem);
-    for (int u = threadIdx.x; u < rows * groups; u += SK_THREADS) {
-      const int row = u / groups, cg = z * groups + u % groups;
-      const int col = tn * BN + cg * 8;
-      if (col >= p.N) continue;                               // N is a multiple of 8
-      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int j = 0; j < z_ctas; ++j) {
-        const uint32_t addr = base + (row * S::PART_LD + cg * 8) * 4;
-        const float4 a = ld_cluster_f4(addr, j), b = ld_cluster_f4(addr + 16, j);
-        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w; v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
-      }
-      if (p.epilogue == 1 || p.epilogue == 2) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          v[i] += (p.in_dtype == 0) ? __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(p.bias) + col + i))
-                                    : __half2float(__ldg(reinterpret_cast<const __half*>(p.bias) + col + i));
-      }
-      const size_t off = static_cast<size_t>(tm * BM + row) * p.N + col;
-      if (p.epilogue >= 2) {
-        if (p.aux != nullptr) store_vec8(p.aux, p.out_dtype, off, v, false);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = gelu_tanh(v[i]);
-      }
-      store_vec8(p.C, p.out_dtype, off, v, p.accumulate != 0);
-    }
+    if (z_ctas == 2) splitk_finish<2>(p, smem_u32(smem), z, tm, tn);
+    else if (z_ctas == 4) splitk_finish<4>(p, smem_u32(smem), z, tm, tn);
+    else splitk_finish<8>(p, smem_u32(smem), z, tm, tn);
   }
   __syncwarp();
   cluster_sync_all();                 // a CTA's partial stays valid until its peers have read it
@@ -2152,70 +2209,74 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
 
 // Clusters of z split-K CTAs that the device holds at once (one CTA per SM; a cluster does not cross a GPC, so this is
 // less than SMs / z), cached per device.
-static int splitk_max_clusters(int z, int device) {
-  static std::atomic<int> cached[64][4];
+static int splitk_max_clusters(int z, bool small, int device) {
+  static std::atomic<int> cached[64][2][4];
   const int i = z == 8 ? 3 : (z == 4 ? 2 : 1);
-  int n = cached[device & 63][i].load(std::memory_order_relaxed);
+  int n = cached[device & 63][small][i].load(std::memory_order_relaxed);
   if (n == 0) {
     auto kern = gemm_splitk_kernel<0, 0>;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(z); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = SplitKSmem::TOTAL;
+    cfg.gridDim = dim3(z); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = SplitKSmem::total(small);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = z; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitKSmem::TOTAL) != cudaSuccess ||
+    // the attribute is the kernel's, not this launch's: the larger of the two rings
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitKSmem::total(false)) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = -1;                                           // not available: never split
     }
-    cached[device & 63][i].store(n, std::memory_order_relaxed);
+    cached[device & 63][small][i].store(n, std::memory_order_relaxed);
   }
   return n;
 }
 
-// CTAs per output tile of the split-K kernel, 1 = do not split.  All tiles have to be in flight at once and every CTA needs
-// 4 K blocks to work on; among 2, 4 and 8 CTAs the one that saves most wins, if any saves at all: a K block that a CTA does
-// not walk saves 0.16 us, and the exchange of the partial tiles costs as much as a number of K blocks that grows with
-// the rows in the tile.  Measured on a B200 for z = 1, 2, 4, 8 over M 1 .. 512, N 128 .. 8192, K 512 .. 16384, warm and cold
-// weights (us, one CTA / split): 24 x 1024 x 1024 7.6 / 6.1 (z 4), 128 x 1024 x 1024 8.0 / 9.0 (z 2, not taken), 128 x 1024 x
-// 4096 15.7 / 10.9 (z 4), 1000 x 1024 x 4096 16.5 / 14.3 (z 2).  Nothing in that range is slower than one CTA by more
-// than 2 %; splitting whenever every CTA had its 4 K blocks was, by up to 37 % (512 x 2048 x 512).
-static int splitk_ctas(int M, int N, int K, int sms, int device) {
-  static constexpr struct { int z; float per_row; } kCost[3] = {{2, 0.14f}, {4, 0.18f}, {8, 0.29f}};
+// Rows of A in a stage of the split-K kernel.
+static int splitk_rows(int M) { return M <= 96 ? (M + 31) / 32 * 32 : BM; }
+
+// CTAs per output tile of the split-K kernel (z 1: do not split) and whether their rings are the small ones.  All clusters have to
+// be in flight at once, every CTA needs 2 K blocks to work on, and the blocks that it does not walk have to outweigh the exchange of
+// its partial rows (25 rows cost as much as one block).  One CTA per SM with the large ring is as fast as or faster than two
+// with small ones at the same or half the split; only where one per SM leaves nothing to split, tiles of few rows are halved.
+// One B200, bf16 with bias, graph replay, weights from DRAM / from the L2, before (at most 6 stages, exchange by columns, no
+// programmatic launch) / now: 24 x 1024 x 512 6.7 / 3.8 us, 24 x 2048 x 2048 7.7 / 5.8 and 7.4 / 5.0, 24 x 8192 x 2048 13.4 / 9.4 and 12.3 /
+// 6.9, 24 x 2048 x 8192 13.6 / 10.5 and 10.5 / 8.7, 64 x 1024 x 8192 12.4 / 9.0, 128 x 1024 x 2048 11.7 / 7.3, 24 x 16384 x 2048 22.5 / 14.5.
+struct SplitK { int z; bool small; };
+static SplitK splitk_ctas(int layout, int M, int N, int K, int sms, int device) {
+  const int rows = M < BM ? M : BM, num_kb = (K + BK - 1) / BK;
   const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + SplitKSmem::BN - 1) / SplitKSmem::BN);
-  const int num_kb = (K + BK - 1) / BK, rows = M < BM ? M : BM;
-  int best = 1;
-  float best_gain = 0.f;
-  for (const auto& c : kCost) {
-    const float gain = static_cast<float>(num_kb) * (c.z - 1) / c.z - (1.f + c.per_row * rows);
-    if (num_kb >= 4 * c.z && tiles * c.z <= sms && gain > best_gain && tiles <= splitk_max_clusters(c.z, device)) {
-      best = c.z;
-      best_gain = gain;
-    }
-  }
-  return best;
+  for (int z = 8; z >= 2; z /= 2)
+    if (num_kb >= 2 * z && 25 * (num_kb - num_kb / z) > rows && tiles * z <= sms && tiles <= splitk_max_clusters(z, false, device))
+      return {z, false};
+  if (layout != 2 && M <= 32 && num_kb >= 4 && tiles <= sms && tiles <= splitk_max_clusters(2, true, device)) return {2, true};
+  return {1, false};
 }
 
 template <int A_MN, int B_MN>
-static int launch_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int z, int device, cudaStream_t stream) {
+static int launch_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int z, int arows, bool small, int device, cudaStream_t stream) {
   using S = SplitKSmem;
   static bool configured[64] = {false};
   auto kern = gemm_splitk_kernel<A_MN, B_MN>;
   if (!configured[device & 63]) {
-    AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
+    AXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::total(false)));
     configured[device & 63] = true;
   }
   p.tiles_m = (p.M + BM - 1) / BM;
   p.tiles_n = (p.N + S::BN - 1) / S::BN;
   p.gemm_ctas = p.tiles_m * p.tiles_n * z;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.gemm_ctas); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = S::TOTAL; cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(p.gemm_ctas); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = S::total(small); cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = z; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  AXB_CUDA(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, z));
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  // Not where a CTA streams for long: the early CTAs of the next launch leave the others on SMs that are next to one another, and
+  // the operands arrive more slowly (one B200, with / without: layout 2, 24 x 8192 x 8192 38.5 / 35.8 us, 200 x 4096 x 8192 27.7 / 24.2).
+  const int blocks = (p.K + BK - 1) / BK / z;
+  cfg.attrs = attr; cfg.numAttrs = blocks <= (A_MN ? 16 : 32) ? 2 : 1;
+  AXB_CUDA(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, z, arows, small));
   return 0;
 }
 
@@ -2297,9 +2358,11 @@ static PairTiles pair_tiles(int M, int N, int K, int layout, bool can_swap, int 
 // 1024 0.82 - 1.0; with K 2048 and 4096 0.92 - 1.4.
 static PairTiles pair_tiles_small(int M, int N, int K, int layout, bool can_swap, int pairs) {
   if (!pair_mode_enabled() || K > 1024 || layout > 1 || (layout == 1 && !can_swap)) return {0, false};
-  const int rows = layout == 1 ? N : M, cols = layout == 1 ? M : N;
+  // up to 128 rows the features go on the rows of the tiles: the second CTA of a pair would have none of A's
+  const bool swap = layout == 1 || (M <= BM && can_swap);
+  const int rows = swap ? N : M, cols = swap ? M : N;
   for (int bn = 64; bn <= 128; bn += 64)
-    if (static_cast<long long>((rows + 2 * BM - 1) / (2 * BM)) * ((cols + bn - 1) / bn) <= pairs) return {bn, layout == 1};
+    if (static_cast<long long>((rows + 2 * BM - 1) / (2 * BM)) * ((cols + bn - 1) / bn) <= pairs) return {bn, swap};
   return {0, false};
 }
 
@@ -2335,18 +2398,20 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
   // K-major operand [R, K]: box 64(K) x tile rows.  MN-major operand [K, R]: box 64(R) x 64(K).
   const bool wide_pair = !comm && plain_on_pairs(M, N, device);
   if (wide_pair) BN = 256;
-  const int splitk = (comm || wide_pair || BN != 128) ? 1 : splitk_ctas(M, N, K, usable_sms(device), device);
+  const SplitK split = comm || wide_pair || BN != 128 ? SplitK{1, false} : splitk_ctas(layout, M, N, K, usable_sms(device), device);
   const bool can_swap = out_dtype != 2 && !accumulate && (layout == 0 || (layout == 1 && epilogue < 2));
   const int sms = usable_sms(device);
   PairTiles tiles = {0, false};
   if (wide_pair) tiles = pair_tiles(M, N, K, layout, can_swap, sms / 2);
-  else if (!comm && splitk == 1) tiles = pair_tiles_small(M, N, K, layout, can_swap, sms / 2);
+  else if (!comm && split.z == 1) tiles = pair_tiles_small(M, N, K, layout, can_swap, sms / 2);
   const bool pair = tiles.bn != 0;
+  // rows of A that a split-K stage holds
+  const int arows = split.z > 1 && a_mn == 0 ? splitk_rows(M) : BM;
   if (tiles.swap) {                                 // rows of B as the rows of the tiles, rows of A as their columns
     if ((b_mn == 0 ? make_tmap_2d_16bit(&tmA, B, N, K, BM, in_dtype) : make_tmap_2d_16bit(&tmA, B, K, N, BK, in_dtype)) ||
         make_tmap_2d_16bit(&tmB, A, M, K, tiles.bn / 2, in_dtype)) return -1;
   } else {
-    if (a_mn == 0) { if (make_tmap_2d_16bit(&tmA, A, M, K, BM, in_dtype)) return -1; }
+    if (a_mn == 0) { if (make_tmap_2d_16bit(&tmA, A, M, K, arows, in_dtype)) return -1; }
     else           { if (make_tmap_2d_16bit(&tmA, A, K, M, BK, in_dtype)) return -1; }
     if (b_mn == 0) { if (make_tmap_2d_16bit(&tmB, B, N, K, pair ? tiles.bn / 2 : (comm_pair ? BN / 2 : BN), in_dtype)) return -1; }
     else           { if (make_tmap_2d_16bit(&tmB, B, K, N, BK, in_dtype)) return -1; }
@@ -2422,10 +2487,10 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
     if (layout == 1) return launch_pair<0, 1>(tmA, tmB, halves, p, sms, device, s);
     return launch_pair<1, 1>(tmA, tmB, halves, p, sms, device, s);
   }
-  if (splitk > 1) {
-    if (layout == 0) return launch_splitk<0, 0>(tmA, tmB, p, splitk, device, s);
-    if (layout == 1) return launch_splitk<0, 1>(tmA, tmB, p, splitk, device, s);
-    return launch_splitk<1, 1>(tmA, tmB, p, splitk, device, s);
+  if (split.z > 1) {
+    if (layout == 0) return launch_splitk<0, 0>(tmA, tmB, p, split.z, arows, split.small, device, s);
+    if (layout == 1) return launch_splitk<0, 1>(tmA, tmB, p, split.z, arows, split.small, device, s);
+    return launch_splitk<1, 1>(tmA, tmB, p, split.z, arows, split.small, device, s);
   }
 #define AXB_DISPATCH(BN_, A_, B_) return launch<BN_, A_, B_>(tmA, tmB, p, device, s)
   if (BN == 256) {
