@@ -78,6 +78,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
                             int D, int pos_div, size_t row_stride, float sign) {
   const int half = D / 2, per_head = half / 8;
   const size_t total = rows * nh * per_head;
+  pdl_launch_next();
+  pdl_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int c = (int)(i % per_head) * 8;
     const size_t t = i / per_head;
@@ -141,8 +143,7 @@ extern "C" int axb_rope(void* x, const float* cs, long long rows, int S, int nh,
   if (D % 16) { set_error("rope: head_dim must be a multiple of 16"); return -1; }
   if (row_stride % 8) { set_error("rope: row stride must be a multiple of 8 elements"); return -1; }
   const size_t work = (size_t)rows * nh * (D / 16);
-  rope_kernel<<<ew_grid(work, 256), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)x, cs, (size_t)rows, S, nh, D, pos_div,
-                                                                   (size_t)row_stride, inverse ? -1.f : 1.f);
-  AXB_CUDA(cudaGetLastError());
+  AXB_CUDA(pdl_launch(rope_kernel, dim3(ew_grid(work, 256)), dim3(256), 0, (cudaStream_t)stream, (__nv_bfloat16*)x, cs, (size_t)rows, S, nh,
+                      D, pos_div, (size_t)row_stride, inverse ? -1.f : 1.f));
   return 0;
 }

@@ -157,6 +157,8 @@ fa_fwd_pingpong_kernel(const __grid_constant__ CUtensorMap tmQKV, const FaParams
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_launch_next();
+  pdl_wait();
   // columns: score buffers of A [0,64) [64,128), of B [128,192) [192,256) (P = the first 32 columns of a
   // buffer), O_A [256,256+HD), O_B [384,384+HD)
   // the register budget of a role must be set inside its branch: after a join the compiler assumes the smaller one
@@ -473,8 +475,7 @@ static int fa_launch_pingpong(const CUtensorMap& tm, const FaParams& p, int devi
   }
   const long long items = static_cast<long long>(p.B) * p.G * p.qpk * ((p.S + 2 * FA_BQ - 1) / (2 * FA_BQ));
   const int sms = sm_count(device);
-  kern<<<static_cast<int>(items < sms ? items : sms), FA2_THREADS, S_::TOTAL, s>>>(tm, p);   // persistent CTAs
-  AXB_CUDA(cudaGetLastError());
+  AXB_CUDA(pdl_launch(kern, dim3(static_cast<unsigned>(items < sms ? items : sms)), dim3(FA2_THREADS), S_::TOTAL, s, tm, p));   // persistent CTAs
   return 0;
 }
 

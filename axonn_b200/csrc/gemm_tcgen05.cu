@@ -1597,7 +1597,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint64_t timeout = p.timeout_ns;
   __shared__ int live_start[LIVE ? PAIR_MAX_LIVE + 1 : 1];   // tile rows with data of the problems before each one
 
-  if (LIVE && warp == 2) list_live_rows(p, tiles_m2, live_start);
+  if (LIVE) {
+    pdl_wait();
+    if (warp == 2) list_live_rows(p, tiles_m2, live_start);
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < S::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 2 * pair_epi_warps<ACT>()); }
@@ -1612,6 +1615,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_sync_all();     // both CTAs' barriers are initialised before any remote arrival or TMA signal
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  pdl_launch_next();
+  if (!LIVE) pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -2202,8 +2207,7 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   const int items = LIVE ? total : p.whole_tiles + 2 * (total - p.whole_tiles);
   const int grid = 2 * (items < pairs ? items : pairs);
   p.gemm_ctas = grid;
-  kern<<<grid, 64 + 32 * pair_epi_warps<ACT>(), smem_bytes, stream>>>(tmA, tmB, tmBh ? *tmBh : tmB, p);
-  AXB_CUDA(cudaGetLastError());
+  AXB_CUDA(pdl_launch(kern, dim3(grid), dim3(64 + 32 * pair_epi_warps<ACT>()), smem_bytes, stream, tmA, tmB, tmBh ? *tmBh : tmB, p));
   return 0;
 }
 
