@@ -163,6 +163,8 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
 // ended, once all of that one's CTAs have called pdl_launch_next or ended (at its end, if it never calls it); pdl_wait returns when
 // the predecessor has ended and its writes are visible.  Every thread that reads or writes global memory calls pdl_wait first, and a
 // CTA calls pdl_launch_next after its tensor memory is allocated: a CTA of the next kernel may be given what is left.
+// One B200: attention layer of 777 tokens (four launches) 96 -> 90 us, residual LayerNorm forward and backward 104.6 -> 102.7, loss
+// head of 4096 tokens 2057 -> 2016.  The attention backward's kernels are launched without: 1 % slower with (803 / 795 us).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... Params, typename... Args>

@@ -329,6 +329,8 @@ __global__ void __launch_bounds__(256)
 norm_fwd_warp_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta,
                      T* __restrict__ y, float* __restrict__ stats, int rows, int H, float eps,
                      const T* __restrict__ delta, T* __restrict__ hout) {
+  pdl_launch_next();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long nwarps = static_cast<long long>(gridDim.x) * 8;
   for (long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5); row < rows; row += nwarps) {
@@ -487,6 +489,8 @@ template <typename T, bool RMS, int NT, int TPR, int CH, int R>
 __global__ void __launch_bounds__(NT, (NormFwdRing<T, NT, CH, R>::MINB))
 norm_fwd_ring_kernel(const T* __restrict__ x, const T* __restrict__ gamma, const T* __restrict__ beta, T* __restrict__ y,
                      float* __restrict__ stats, int rows, int H, float eps, const T* __restrict__ delta, T* __restrict__ hout) {
+  pdl_launch_next();
+  pdl_wait();
   using Ring = NormFwdRing<T, NT, CH, R>;
   constexpr int ST = Ring::STAGES, GR = NT / TPR, WPG = TPR / 32, NV = RMS ? R : 2 * R;
   extern __shared__ __align__(16) uint8_t ring[];
@@ -632,8 +636,7 @@ static int norm_fwd_ring(const T* x, const T* gamma, const T* beta, T* y, float*
   }
   const int per_block = NT / TPR * R;
   const int want = (rows + per_block - 1) / per_block, cap = sm_count_current() * Ring::MINB;
-  kern<<<want < cap ? want : cap, NT, Ring::bytes(delta != nullptr), s>>>(x, gamma, beta, y, stats, rows, H, eps, delta, hout);
-  AXB_CUDA(cudaGetLastError());
+  AXB_CUDA(pdl_launch(kern, dim3(want < cap ? want : cap), dim3(NT), Ring::bytes(delta != nullptr), s, x, gamma, beta, y, stats, rows, H, eps, delta, hout));
   return 0;
 }
 
@@ -661,6 +664,8 @@ __global__ void __launch_bounds__(NT, (NormBwdRing<T, NT, CH, R>::MINB))
 norm_bwd_ring_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ gamma,
                      const float* __restrict__ stats, T* __restrict__ dx, float* __restrict__ dgamma_part,
                      float* __restrict__ dbeta_part, int rows, int H, const T* __restrict__ dres) {
+  pdl_launch_next();
+  pdl_wait();
   using Ring = NormBwdRing<T, NT, CH, R>;
   constexpr int ST = Ring::STAGES, GR = NT / TPR, WPG = TPR / 32, NV = RMS ? R : 2 * R;
   extern __shared__ __align__(16) uint8_t ring[];
@@ -850,8 +855,7 @@ static int norm_bwd_ring(const T* dy, const T* x, const T* gamma, const float* s
   const int per_block = NT / TPR * R;
   const int want = (rows + per_block - 1) / per_block, cap = min(max_blocks, sm_count_current() * Ring::MINB);
   *blocks_launched = want < cap ? want : cap;
-  kern<<<*blocks_launched, NT, Ring::bytes(dres != nullptr), s>>>(dy, x, gamma, stats, dx, dgp, dbp, rows, H, dres);
-  AXB_CUDA(cudaGetLastError());
+  AXB_CUDA(pdl_launch(kern, dim3(*blocks_launched), dim3(NT), Ring::bytes(dres != nullptr), s, dy, x, gamma, stats, dx, dgp, dbp, rows, H, dres));
   return 0;
 }
 
@@ -866,6 +870,8 @@ __device__ __forceinline__ void fold_store(void* o, int out_dtype, int c, float 
 }
 __global__ void fold_partials_kernel(const float* __restrict__ pa, const float* __restrict__ pb, void* __restrict__ oa,
                                      void* __restrict__ ob, int nblocks, int H, int out_dtype) {
+  pdl_launch_next();
+  pdl_wait();
   __shared__ float sa[32][33], sb[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
@@ -899,6 +905,8 @@ __global__ void fold_partials_kernel(const float* __restrict__ pa, const float* 
 template <typename T>
 __global__ void __launch_bounds__(256)
 colsum_partial_kernel(const T* __restrict__ x, float* __restrict__ part, int rows, int N) {
+  pdl_launch_next();
+  pdl_wait();
   __shared__ float red[8][32][9];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = (blockIdx.x * 32 + lane) * 8;
@@ -1033,8 +1041,8 @@ static int norm_fwd_t(const void* x, const void* gamma, const void* beta, void* 
   if (path == NormPath::WARP) {
     const int wgrid = min((rows + 7) / 8, grid * 2);
 #define AXB_NORM_FWD_WARP(RMS_, VPL_)                                                                           \
-  norm_fwd_warp_kernel<T, RMS_, VPL_><<<wgrid, 256, 0, s>>>((const T*)x, (const T*)gamma, (const T*)beta, (T*)y, \
-                                                           stats, rows, H, eps, (const T*)delta, (T*)hout)
+  AXB_CUDA(pdl_launch(norm_fwd_warp_kernel<T, RMS_, VPL_>, dim3(wgrid), dim3(256), 0, s, (const T*)x, (const T*)gamma, (const T*)beta,  \
+                      (T*)y, stats, rows, H, eps, (const T*)delta, (T*)hout))
     if (H == 1024) { if (rms) AXB_NORM_FWD_WARP(true, 4); else AXB_NORM_FWD_WARP(false, 4); }
     else if (H == 2048) { if (rms) AXB_NORM_FWD_WARP(true, 8); else AXB_NORM_FWD_WARP(false, 8); }
     else if constexpr (sizeof(T) == 4) { if (rms) AXB_NORM_FWD_WARP(true, 16); else AXB_NORM_FWD_WARP(false, 16); }
@@ -1185,8 +1193,8 @@ extern "C" int axb_add_norm_bwd(const void* dy, const void* dres, const void* x,
   else rc = norm_bwd_t<float>(dy, x, gamma, stats, dx, sums, dgamma_part, dbeta_part, rows, H, H_total, rms, mode, grid, s, &nblocks, dres);
   if (rc) return rc;
   if (mode != 1 && dgamma_part && dgamma) {
-    fold_partials_kernel<<<(H + 31) / 32, dim3(32, 32), 0, s>>>(dgamma_part, rms ? nullptr : dbeta_part, dgamma,
-                                                              rms ? nullptr : dbeta, nblocks, H, param_dtype);
+    AXB_CUDA(pdl_launch(fold_partials_kernel, dim3((H + 31) / 32), dim3(32, 32), 0, s, dgamma_part, rms ? nullptr : dbeta_part, dgamma,
+                        rms ? nullptr : dbeta, nblocks, H, param_dtype));
     AXB_CUDA(cudaGetLastError());
   }
   return 0;
@@ -1208,12 +1216,11 @@ extern "C" int axb_colsum(const void* x, float* part, void* out, int rows, int N
   const int splits = axb_colsum_splits(device, rows, N);
   dim3 grid((N / 8 + 31) / 32, splits);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (dtype == 0) colsum_partial_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, part, rows, N);
-  else if (dtype == 1) colsum_partial_kernel<__half><<<grid, 256, 0, s>>>((const __half*)x, part, rows, N);
-  else colsum_partial_kernel<float><<<grid, 256, 0, s>>>((const float*)x, part, rows, N);
+  if (dtype == 0) AXB_CUDA(pdl_launch(colsum_partial_kernel<__nv_bfloat16>, grid, dim3(256), 0, s, (const __nv_bfloat16*)x, part, rows, N));
+  else if (dtype == 1) AXB_CUDA(pdl_launch(colsum_partial_kernel<__half>, grid, dim3(256), 0, s, (const __half*)x, part, rows, N));
+  else AXB_CUDA(pdl_launch(colsum_partial_kernel<float>, grid, dim3(256), 0, s, (const float*)x, part, rows, N));
   AXB_CUDA(cudaGetLastError());
-  fold_partials_kernel<<<(N + 31) / 32, dim3(32, 32), 0, s>>>(part, nullptr, out, nullptr, splits, N, out_dtype);
-  AXB_CUDA(cudaGetLastError());
+  AXB_CUDA(pdl_launch(fold_partials_kernel, dim3((N + 31) / 32), dim3(32, 32), 0, s, part, nullptr, out, nullptr, splits, N, out_dtype));
   return 0;
 }
 
@@ -1240,7 +1247,6 @@ extern "C" int axb_gelu_bwd_colsum(const void* dy, const void* x, void* dx, floa
   else
     gelu_bwd_colsum_kernel<__half><<<grid, 256, 0, s>>>((const __half*)dy, (const __half*)x, (__half*)dx, part, rows, N);
   AXB_CUDA(cudaGetLastError());
-  fold_partials_kernel<<<(N + 31) / 32, dim3(32, 32), 0, s>>>(part, nullptr, colsum, nullptr, splits, N, out_dtype);
-  AXB_CUDA(cudaGetLastError());
+  AXB_CUDA(pdl_launch(fold_partials_kernel, dim3((N + 31) / 32), dim3(32, 32), 0, s, part, nullptr, colsum, nullptr, splits, N, out_dtype));
   return 0;
 }
