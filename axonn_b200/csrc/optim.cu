@@ -3,9 +3,9 @@
 // A launch covers a whole list of tensors through a device table; work is cut
 // into fixed-size chunks (the table holds their prefix sums), and a grid-stride
 // loop maps units of work -> (tensor, offset), so one launch replaces hundreds
-// of per-parameter launches.  A unit is a quarter of a chunk for the
-// optimizers, whose 28 bytes per element make a whole chunk too long a last
-// unit; squared norm and scale take whole chunks for tables of small tensors,
+// of per-parameter launches.  A unit is a quarter to a sixteenth of a chunk for
+// the optimizers, whose 28 bytes per element make a whole chunk too long a last
+// unit (the table's c: quarters); squared norm and scale take whole chunks for tables of small tensors,
 // where three of four quarters would be empty.  One B200, us, inputs warm in
 // the L2 where they fit; a: whole chunks found by binary search, b: quarters
 // found by a linear search, c: now
@@ -25,10 +25,10 @@ namespace axb {
 
 constexpr int MT_CHUNK = 1 << 16;
 constexpr int MT_PARTS = 4;                      // units per chunk of the optimizer kernels (and of the scale of long tensors)
-constexpr int MT_UNIT = MT_CHUNK / MT_PARTS;
 constexpr int MT_THREADS = 512;
 constexpr int ADAM_THREADS = 256;
 constexpr int ADAM_UNROLL = 2;
+
 
 // table row for norm/scale: {ptr, numel, dtype (0 fp32, 1 bf16, 2 fp16), chunk_prefix}
 // table row for adamw:      {master fp32, model bf16 or 0, grad, exp_avg, exp_avg_sq, numel, grad dtype, chunk_prefix}
@@ -73,6 +73,8 @@ template <int PARTS, bool CLIP>      // units per chunk
 __global__ void __launch_bounds__(MT_THREADS)
 multi_l2norm_sq_kernel(const long long* __restrict__ table, int n, long long total_chunks, float* __restrict__ out,
                        const ClipOut clip) {
+  pdl_launch_next();
+  pdl_wait();
   __shared__ float red[32];
   float acc = 0.f;
   constexpr int UNIT = MT_CHUNK / PARTS;
@@ -159,6 +161,8 @@ constexpr int SCALE_UNROLL = 4;
 template <int PARTS>      // units per chunk
 __global__ void __launch_bounds__(MT_THREADS)
 multi_scale_kernel(const long long* __restrict__ table, int n, long long total_chunks, const float* __restrict__ scale_ptr) {
+  pdl_launch_next();
+  pdl_wait();
   const float s = *scale_ptr;
   if (s == 1.f) return;
   constexpr int UNIT = MT_CHUNK / PARTS;
@@ -241,16 +245,20 @@ struct AdamArgs {
                                  // incomplete) => skip the whole step (may be null)
 };
 
+template <int PARTS>      // units per chunk
 __global__ void __launch_bounds__(ADAM_THREADS, 4)
 multi_adamw_kernel(const long long* __restrict__ table, int n, long long total_chunks, AdamArgs a) {
+  pdl_launch_next();
+  pdl_wait();
   if (a.found_inf && *a.found_inf != 0.f) return;
   if (a.status && *reinterpret_cast<const volatile unsigned int*>(a.status) != 0u) return;
   const float gs = a.grad_scale ? *a.grad_scale : 1.f;
   const float decay = 1.f - a.lr * a.weight_decay;
   const float step = a.lr / a.bias_c1;
   const float inv_sqrt_c2 = rsqrtf(a.bias_c2);
-  for (long long unit = blockIdx.x; unit < total_chunks * MT_PARTS; unit += gridDim.x) {
-    const long long chunk = unit / MT_PARTS;
+  constexpr int UNIT = MT_CHUNK / PARTS;
+  for (long long unit = blockIdx.x; unit < total_chunks * PARTS; unit += gridDim.x) {
+    const long long chunk = unit / PARTS;
     const int t = find_tensor(table, 8, 7, n, chunk);
     const long long* row = table + (size_t)t * 8;
     float* master = reinterpret_cast<float*>(row[0]);
@@ -260,8 +268,8 @@ multi_adamw_kernel(const long long* __restrict__ table, int n, long long total_c
     float* v = reinterpret_cast<float*>(row[4]);
     const long long numel = row[5];
     const int gdtype = (int)row[6];
-    const long long begin = (chunk - row[7]) * MT_CHUNK + (unit % MT_PARTS) * MT_UNIT;
-    const long long end = begin + MT_UNIT < numel ? begin + MT_UNIT : numel;
+    const long long begin = (chunk - row[7]) * MT_CHUNK + (unit % PARTS) * UNIT;
+    const long long end = begin + UNIT < numel ? begin + UNIT : numel;
     if (begin >= numel) continue;
     const bool aligned = ((reinterpret_cast<uintptr_t>(master) | reinterpret_cast<uintptr_t>(m) |
                            reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(grad) |
@@ -341,6 +349,8 @@ multi_adamw_kernel(const long long* __restrict__ table, int n, long long total_c
 // costs a PCIe round trip per warp, which serialises to milliseconds when every warp of a large grid does it.
 // One thread copies it into device memory first and the optimizer's blocks read that copy.
 __global__ void status_gate_kernel(const unsigned int* __restrict__ status, unsigned int* __restrict__ gate) {
+  pdl_launch_next();
+  pdl_wait();
   *gate = *reinterpret_cast<const volatile unsigned int*>(status);
 }
 
@@ -363,10 +373,9 @@ static int l2norm_sq(const long long* table, int n, long long total_chunks, floa
   // and the tensors are long and found in one round of the search.  From DRAM, whole / quarters: 12 tensors of 64 chunks
   // 30.8 / 28.7 us, 8 of 10 12.3 / 10.2; 33 of 16 22.6 / 22.6, 300 of 16 121 / 127, 1500 of one half 31 / 45.
   if (n <= 32 && mt_long_tensors(n, total_chunks) && total_chunks < 16ll * sm_count_current())
-    multi_l2norm_sq_kernel<MT_PARTS, CLIP><<<mt_grid(total_chunks * MT_PARTS, 4), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, out, clip);
+    AXB_CUDA(pdl_launch(multi_l2norm_sq_kernel<MT_PARTS, CLIP>, dim3(mt_grid(total_chunks * MT_PARTS, 4)), dim3(MT_THREADS), 0, (cudaStream_t)stream, table, n, total_chunks, out, clip));
   else
-    multi_l2norm_sq_kernel<1, CLIP><<<mt_grid(total_chunks, 8), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, out, clip);
-  AXB_CUDA(cudaGetLastError());
+    AXB_CUDA(pdl_launch(multi_l2norm_sq_kernel<1, CLIP>, dim3(mt_grid(total_chunks, 8)), dim3(MT_THREADS), 0, (cudaStream_t)stream, table, n, total_chunks, out, clip));
   return 0;
 }
 extern "C" int axb_multi_l2norm_sq(const long long* table, int n, long long total_chunks, float* out, void* stream) {
@@ -382,10 +391,9 @@ extern "C" int axb_multi_scale(const long long* table, int n, long long total_ch
   // quarters of a chunk where tensors are long: 29 against 30 us for 12 tensors of 64 chunks, 188 against 194 for 300 of 16,
   // but 104 against 96 for 1500 of 2
   if (mt_long_tensors(n, total_chunks))
-    multi_scale_kernel<MT_PARTS><<<mt_grid(total_chunks * MT_PARTS), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, scale);
+    AXB_CUDA(pdl_launch(multi_scale_kernel<MT_PARTS>, dim3(mt_grid(total_chunks * MT_PARTS)), dim3(MT_THREADS), 0, (cudaStream_t)stream, table, n, total_chunks, scale));
   else
-    multi_scale_kernel<1><<<mt_grid(total_chunks), MT_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, scale);
-  AXB_CUDA(cudaGetLastError());
+    AXB_CUDA(pdl_launch(multi_scale_kernel<1>, dim3(mt_grid(total_chunks)), dim3(MT_THREADS), 0, (cudaStream_t)stream, table, n, total_chunks, scale));
   return 0;
 }
 // Device-memory copy of the status word of the current device, refreshed on `stream` (see status_gate_kernel);
@@ -404,7 +412,7 @@ static unsigned int* refreshed_status_gate(cudaStream_t stream) {
     }
     gate = status ? gates[dev] : nullptr;
   }
-  if (gate) status_gate_kernel<<<1, 1, 0, stream>>>(status, gate);
+  if (gate) pdl_launch(status_gate_kernel, dim3(1), dim3(1), 0, stream, status, gate);
   return gate;
 }
 
@@ -427,7 +435,11 @@ extern "C" int axb_multi_adamw(const long long* table, int n, long long total_ch
   unsigned int* gate = refreshed_status_gate((cudaStream_t)stream);
   AXB_CUDA(cudaGetLastError());
   AdamArgs a{lr, beta1, beta2, eps, weight_decay, bias_c1, bias_c2, grad_scale, found_inf, gate};
-  multi_adamw_kernel<<<mt_grid(total_chunks * MT_PARTS), ADAM_THREADS, 0, (cudaStream_t)stream>>>(table, n, total_chunks, a);
-  AXB_CUDA(cudaGetLastError());
+  // Many small units: the blocks of the last wave are soon done.  One B200, quarters / eighths / sixteenths of a chunk: 12 tensors of 64
+  // chunks 239.0 / 225.5 / 224.5 us, 33 of 16 167 / 161 / 159, 10 of half a chunk 16.4 / 11.6 / 9.3; 300 of 16 1389 / 1372 / 1381.
+  // Quarters for many tensors of one chunk: most of the others would be empty, 3000 of 4096 elements 78 / 98, 300 of 2048 8 / 16.
+  const int parts = total_chunks < 2ll * n && n > 32 ? MT_PARTS : (total_chunks < 1024 ? 16 : 8);
+  const auto kern = parts == MT_PARTS ? multi_adamw_kernel<MT_PARTS> : parts == 8 ? multi_adamw_kernel<8> : multi_adamw_kernel<16>;
+  AXB_CUDA(pdl_launch(kern, dim3(mt_grid(total_chunks * parts)), dim3(ADAM_THREADS), 0, (cudaStream_t)stream, table, n, total_chunks, a));
   return 0;
 }
