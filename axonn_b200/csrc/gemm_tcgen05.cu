@@ -2211,27 +2211,26 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
   return 0;
 }
 
-// Clusters of z split-K CTAs that the device holds at once (one CTA per SM; a cluster does not cross a GPC, so this is
-// less than SMs / z), cached per device.
-static int splitk_max_clusters(int z, bool small, int device) {
-  static std::atomic<int> cached[64][2][4];
+// Clusters of z split-K CTAs with the large ring that the device holds at once (one CTA per SM; a cluster does not cross a GPC, so
+// this is less than SMs / z), cached per device; -1: none.
+static int splitk_max_clusters(int z, int device) {
+  static std::atomic<int> cached[64][4];
   const int i = z == 8 ? 3 : (z == 4 ? 2 : 1);
-  int n = cached[device & 63][small][i].load(std::memory_order_relaxed);
+  int n = cached[device & 63][i].load(std::memory_order_relaxed);
   if (n == 0) {
     auto kern = gemm_splitk_kernel<0, 0>;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(z); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = SplitKSmem::total(small);
+    cfg.gridDim = dim3(z); cfg.blockDim = dim3(SK_THREADS); cfg.dynamicSmemBytes = SplitKSmem::total(false);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = z; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    // the attribute is the kernel's, not this launch's: the larger of the two rings
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitKSmem::total(false)) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = -1;                                           // not available: never split
     }
-    cached[device & 63][small][i].store(n, std::memory_order_relaxed);
+    cached[device & 63][i].store(n, std::memory_order_relaxed);
   }
   return n;
 }
@@ -2251,9 +2250,9 @@ static SplitK splitk_ctas(int layout, int M, int N, int K, int sms, int device) 
   const int rows = M < BM ? M : BM, num_kb = (K + BK - 1) / BK;
   const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + SplitKSmem::BN - 1) / SplitKSmem::BN);
   for (int z = 8; z >= 2; z /= 2)
-    if (num_kb >= 2 * z && 25 * (num_kb - num_kb / z) > rows && tiles * z <= sms && tiles <= splitk_max_clusters(z, false, device))
+    if (num_kb >= 2 * z && 25 * (num_kb - num_kb / z) > rows && tiles * z <= sms && tiles <= splitk_max_clusters(z, device))
       return {z, false};
-  if (layout != 2 && M <= 32 && num_kb >= 4 && tiles <= sms && tiles <= splitk_max_clusters(2, true, device)) return {2, true};
+  if (layout != 2 && M <= 32 && num_kb >= 4 && tiles <= sms && splitk_max_clusters(2, device) > 0) return {2, true};
   return {1, false};
 }
 
