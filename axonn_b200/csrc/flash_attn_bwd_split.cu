@@ -46,7 +46,7 @@ struct FaSplitParams {
 // per scheduler with 32 scores per thread hide that latency, two warps with 64 do not.  Registers: 640 threads get 96
 // each at launch, 128 * 64 + 512 * 104 after the split are exactly those.
 // Measured on a B200, 8 x 2048, 16 heads, head_dim 128, back to back in one graph: dQ, dK / dV and delta kernel together 660 -
-// 700 us with two warps per scheduler, 584 - 599 us now (the library's backward 492 us).
+// 700 us with two warps per scheduler, 584 - 599 us with four, 502 - 516 us now (the library's backward 434 us in the same run).
 constexpr int FS_THREADS = 640;
 constexpr int FS_SOFTMAX_WARPS = 16;
 #define FS_REGS_CONTROL "setmaxnreg.dec.sync.aligned.u32 64;"
