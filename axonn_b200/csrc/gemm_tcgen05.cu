@@ -2657,10 +2657,18 @@ extern "C" int axb_gemm_on_pairs(int M, int N, int device) { return M > 0 && N >
 //   513 .. 1023 rows, 7 waves and more 0.88 - 0.98 (768 x 50304 x 1024 67.8 / 77.1), fewer 0.96 - 1.07 (768 x 14000 x 2048 47.1 / 45.3);
 //   fewer rows 0.95 - 1.22 (300 x 32000 x 128 25.6 / 21.7).
 // The head called as a layer, forward and backward, is bound by the host below some 200 us and 1 % apart there.
+// Since the plain product fits its tiles to ragged rows, epilogue / pass, K 2048, N 50304: 520 rows 108.7 / 95.7 us, 777 rows 143 / 136,
+// 1531 rows 211 / 232; K 4096, N 32000: 1100 rows 223 / 204, 1300 rows 272 / 250, 1531 rows 281 / 286.  Within 4 % of the better one over
+// 125 shapes of 520 .. 4096 rows, below 1024 rows 9 %.
 extern "C" int axb_gemm_ce_pays(int M, int N, int K, int device) {
   const int pairs = axb::usable_sms(device) / 2;
   const long long tiles = (static_cast<long long>(M) + 255) / 256 * ((static_cast<long long>(N) + 255) / 256);
   const bool halved = axb::pair_whole_tiles(tiles, pairs) != tiles;
+  // the plain product's tiles may fit a ragged M better (pair_tiles): 1.2 ns a column and K block against the pass over the logits
+  const axb::PairTiles best = axb::pair_tiles(M, N, K, 0, true, pairs);
+  const unsigned rows = ((best.swap ? N : M) + 255) / 256, cols = best.swap ? M : N;
+  const float saved = static_cast<float>((tiles + pairs - 1) / pairs) * (axb::PAIR_BN + 80) - axb::pair_cost(rows, cols, best.bn, pairs);
+  if (saved * (K / axb::BK) * 1.2e-3f > 0.4e-6f * M * N) return 0;
   if (M >= 2048) return !(halved && tiles < 2ll * pairs && K > 2048);
   if (M <= 512 || K < 512) return 0;
   return tiles >= 7ll * pairs || (M >= 1024 && (!halved || tiles >= 4ll * pairs));
