@@ -1951,14 +1951,11 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         }
         if (++stage == stages) { stage = 0; phase ^= 1; }
       }
-      if (!ok) {
-        const uint64_t t0 = globaltimer_ns();     // give in-flight copies time to land before the CTA exits
-        while (globaltimer_ns() - t0 < 200000ull) {}
-        report_status(p.status, 0x151u);
-      }
+      if (!ok) report_status(p.status, 0x151u);
     }
   } else if (warp == 1) {
     if (elect_one()) {
+      pdl_wait();                         // the deadline of a wait counts from here, not from somewhere in the predecessor's run
       const uint32_t idesc = umma_idesc(p.in_dtype == 0 ? 1 : 0, A_MN, B_MN, BM, BN);
       const uint32_t a_lbo = A_MN ? BK * 128 : 16, a_kstep = A_MN ? UMMA_K * 128 : UMMA_K * 2;
       const uint32_t b_lbo = B_MN ? BK * 128 : 16, b_kstep = B_MN ? UMMA_K * 128 : UMMA_K * 2;
@@ -1976,16 +1973,13 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if (ok) umma_commit(acc_full);
-      else {
-        const uint64_t t0 = globaltimer_ns();
-        while (globaltimer_ns() - t0 < 50000ull) {}   // let MMAs in flight finish before TMEM is released
-        report_status(p.status, 0x152u);
-      }
+      else report_status(p.status, 0x152u);
     }
   } else {
     // the accumulator is complete: every MMA has read its operands, the ring now holds this CTA's partial tile
     const int q = warp & 3;
     const int row = q * 32 + lane;
+    pdl_wait();
     if (!mbar_wait(acc_full, 0, abort_flag, timeout)) {
       if (lane == 0) report_status(p.status, 0x154u);
     } else {
@@ -2006,6 +2000,12 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   }
   tcgen05_fence_before();
   __syncthreads();
+  if (*abort_flag != 0) {
+    // Whoever gave up, the producer may have issued its last copies long before: they land, and the MMAs on them end, before
+    // the CTA gives its shared and tensor memory back.
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) {}
+  }
   if (warp == 1) { __syncwarp(); tcgen05_fence_after(); tmem_dealloc(tmem_base, BN); }
   __syncwarp();
   cluster_sync_all();                 // all partials of the tile are in shared memory

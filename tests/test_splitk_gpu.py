@@ -91,3 +91,31 @@ def test_overlapping_launches():
         got.zero_()
         g.replay()
         assert torch.equal(got, want)
+
+
+def test_deadline_starts_after_the_predecessor():
+    """A product that is launched while its predecessor still runs does not count that one's time against its own waits: 15 ms of
+    a product held to two SMs, before one with a deadline of 3 ms."""
+    from axonn_b200.ops import _lib, gemm
+
+    torch.manual_seed(1)
+    long_a, long_b = (torch.randn(4096, 8192, device=DEV).to(BF16) for _ in range(2))
+    a, b = torch.randn(24, 1024, device=DEV).to(BF16), torch.randn(1024, 1024, device=DEV).to(BF16)
+    want = gemm.matmul_nt(a, b)
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    L = _lib.lib()
+    torch.cuda.synchronize()
+    start.record()
+    try:
+        L.axb_gemm_set_max_ctas(2)
+        gemm.matmul_nt(long_a, long_b)
+        L.axb_gemm_set_max_ctas(0)
+        _lib.set_wait_timeout_ms(3)
+        got = gemm.matmul_nt(a, b)
+    finally:
+        L.axb_gemm_set_max_ctas(0)
+        _lib.set_wait_timeout_ms(120000)
+    end.record()
+    torch.cuda.synchronize()
+    assert start.elapsed_time(end) > 6
+    assert _lib.device_status() == 0 and torch.equal(got, want)
