@@ -18,6 +18,7 @@ void set_error(const char* fmt, ...) {
 
 int check_cuda(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return 0;
+  cudaGetLastError();      // the runtime keeps what a call returned (cudaLaunchKernelEx) and would report it after the next launch too
   set_error("%s: %s", what, cudaGetErrorString(e));
   return -1;
 }

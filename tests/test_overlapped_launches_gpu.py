@@ -1,5 +1,9 @@
 """Kernels that are launched while their predecessor still runs: the same bits as with a synchronisation after every layer."""
 
+import os
+import shutil
+import subprocess
+
 import pytest
 import torch
 import torch.distributed as dist
@@ -60,3 +64,24 @@ def test_blocks(batch, seq, hidden, llama, monkeypatch):
     for _ in range(10):
         for a, b in zip(run(), want):
             assert torch.equal(a, b)
+
+
+_REFUSED_LAUNCH = """
+#include "axonn_b200.h"
+#include "common.cuh"
+__global__ void kernel(int) {}
+static int launch() { AXB_CUDA(axb::pdl_launch(kernel, dim3(0), dim3(32), 0, nullptr, 1)); return 0; }
+int main() { return launch() == -1 && axb_last_error()[0] != 0 && cudaPeekAtLastError() == cudaSuccess ? 0 : 1; }
+"""
+
+
+@pytest.mark.skipif(not shutil.which("nvcc"), reason="needs nvcc")
+def test_a_refused_launch_is_reported_once(tmp_path):
+    """The runtime refuses an empty grid: the launcher returns that, and the runtime has nothing left for the next launch to find."""
+    import axonn_b200
+
+    csrc = os.path.join(os.path.dirname(axonn_b200.__file__), "csrc")
+    (tmp_path / "launch.cu").write_text(_REFUSED_LAUNCH)
+    subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-I", csrc, str(tmp_path / "launch.cu"),
+                    os.path.join(csrc, "common.cu"), "-o", str(tmp_path / "launch")], check=True)
+    subprocess.run([str(tmp_path / "launch")], check=True)
