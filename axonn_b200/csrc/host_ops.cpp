@@ -55,6 +55,13 @@ int dtype_code(const Tensor& t) {
 const void* addr(const optional<Tensor>& t) { return t ? t->data_ptr() : nullptr; }
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
+// Other Python threads run while this one allocates (the allocator may have to free blocks, which synchronises) and launches (a full
+// launch queue lets the caller wait).
+struct NoGil {
+  PyThreadState* const state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 // An ordinary CUDA tensor or parameter.
 bool plain(PyObject* o) {
   return (Py_TYPE(o) == reinterpret_cast<PyTypeObject*>(THPVariableClass) || Py_TYPE(o) == reinterpret_cast<PyTypeObject*>(parameter_type)) &&
@@ -145,12 +152,15 @@ PyObject* py_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || gamma.requires_grad() || (delta && delta->requires_grad()) ||
                                                    (beta && beta->requires_grad()));
   Tensor h, y, stats;
-  if (grad) {
-    const auto out = NormNode::apply(x, delta, gamma, beta, eps, rms);
-    h = out[0];
-    y = out[delta ? 1 : 0];
-  } else {
-    run_norm(x, delta, gamma, beta, eps, rms, h, y, stats);
+  {
+    NoGil no_gil;
+    if (grad) {
+      const auto out = NormNode::apply(x, delta, gamma, beta, eps, rms);
+      h = out[0];
+      y = out[delta ? 1 : 0];
+    } else {
+      run_norm(x, delta, gamma, beta, eps, rms, h, y, stats);
+    }
   }
   if (!delta) return THPVariable_Wrap(y);
   PyObject* pair = PyTuple_New(2);
@@ -182,10 +192,14 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (b && (b->scalar_type() != type || b->device() != x.device() || !b->is_contiguous() || b->numel() != rows_out || wants_grad(*b))) Py_RETURN_NONE;
   c10::SmallVector<int64_t, 5> shape(x.sizes().begin(), x.sizes().end());
   shape.back() = rows_out;
-  Tensor out = at::empty(shape, x.options());
   const int code = type == at::kBFloat16 ? 0 : 1, epilogue = gelu ? (b ? 2 : 3) : (b ? 1 : 0);
-  check(gemm(0, x.data_ptr(), w.data_ptr(), out.data_ptr(), addr(b), nullptr, static_cast<int>(x.numel() / k), static_cast<int>(rows_out),
-             static_cast<int>(k), code, code, epilogue, 0, x.get_device(), stream()), "axb_gemm");
+  Tensor out;
+  {
+    NoGil no_gil;
+    out = at::empty(shape, x.options());
+    check(gemm(0, x.data_ptr(), w.data_ptr(), out.data_ptr(), addr(b), nullptr, static_cast<int>(x.numel() / k), static_cast<int>(rows_out),
+               static_cast<int>(k), code, code, epilogue, 0, x.get_device(), stream()), "axb_gemm");
+  }
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }
@@ -203,9 +217,14 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   // 2^-100 < scale < 2^100, dense and on 16 bytes: see supported() in ops/attention_cuda.py
   if (qpk < 1 || (D != 64 && D != 128) || !(scale > 0x1p-100 && scale < 0x1p100) || reinterpret_cast<uintptr_t>(qkv.data_ptr()) % 16 ||
       std::max({B, S, G, qpk}) > INT32_MAX) Py_RETURN_NONE;
-  Tensor out = at::empty({B, S, G * qpk, D}, qkv.options()), lse = at::empty({B, G * qpk, S}, qkv.options().dtype(at::kFloat));
-  check(flash_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr<float>(), static_cast<int>(B), static_cast<int>(S), static_cast<int>(G),
-                  static_cast<int>(qpk), static_cast<int>(D), static_cast<float>(scale), qkv.get_device(), stream()), "axb_flash_attn_fwd");
+  Tensor out;
+  {
+    NoGil no_gil;
+    out = at::empty({B, S, G * qpk, D}, qkv.options());
+    const Tensor lse = at::empty({B, G * qpk, S}, qkv.options().dtype(at::kFloat));
+    check(flash_fwd(qkv.data_ptr(), out.data_ptr(), lse.data_ptr<float>(), static_cast<int>(B), static_cast<int>(S), static_cast<int>(G),
+                    static_cast<int>(qpk), static_cast<int>(D), static_cast<float>(scale), qkv.get_device(), stream()), "axb_flash_attn_fwd");
+  }
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
 }

@@ -2,6 +2,7 @@
 that either takes, refused where it was refused, seen by everything that looks at an operation."""
 
 import threading
+import time
 
 import pytest
 import torch
@@ -162,3 +163,35 @@ def test_launch_errors_keep_their_type():
     assert host.linear(x, w, None, 8, 8, False) is None and host.attention(x, 1.0) is None
     with pytest.raises(TypeError):
         host.norm(x, None, w, None, "eps", True)
+
+
+@pytest.mark.parametrize("path,grad", [("norm", False), ("norm", True), ("linear", False), ("attention", False)])
+def test_other_threads_run_while_a_launch_waits(path, grad):
+    """A launch that finds the queue full (more of them than it holds, behind half a second of work) holds up its own thread only."""
+    from axonn_b200.ops import _lib
+
+    host = _lib.host()
+    x, w = torch.randn(16, 64, device=DEV, dtype=BF16, requires_grad=grad), torch.ones(64, device=DEV, dtype=BF16)
+    weight, qkv = torch.randn(64 * 64, device=DEV, dtype=BF16), torch.randn(1, 8, 1, 3, 64, device=DEV, dtype=BF16)
+    call = {"norm": lambda: host.norm(x, None, w, None, 1e-5, True), "linear": lambda: host.linear(x, weight, None, 64, 64, False),
+            "attention": lambda: host.attention(qkv, 0.125)}[path]
+    assert call() is not None
+    torch.cuda.synchronize()
+    ticks, done = [time.perf_counter()], threading.Event()
+
+    def tick():
+        while not done.wait(1e-3):
+            ticks.append(time.perf_counter())
+    other = threading.Thread(target=tick)
+    other.start()
+    longest = 0.0
+    torch.cuda._sleep(10 ** 9)
+    for _ in range(3000):
+        t = time.perf_counter()
+        call()
+        longest = max(longest, time.perf_counter() - t)
+    done.set()
+    other.join()
+    torch.cuda.synchronize()
+    assert longest > 0.2                                               # the queue was full
+    assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.1
