@@ -4,7 +4,9 @@
 ``nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo`` (object files in
 parallel, then one link) into ``axonn_b200/lib/libaxonn_b200.so``.  nvcc
 cross-compiles without a GPU.  The library is rebuilt only when a source or
-header is newer than it.
+header is newer than it.  With it goes the module of native host paths, which
+wants PyTorch's headers and g++: where it cannot be built there is a warning, and
+the Python code launches the same kernels.
 """
 
 import glob
@@ -12,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -80,6 +83,14 @@ def build_host(force=False):
     return out
 
 
+def _build_host_if_possible(force):
+    """The native host paths are optional: the kernels neither need them nor PyTorch."""
+    try:
+        build_host(force)
+    except (ImportError, OSError, RuntimeError) as e:
+        warnings.warn(f"the native host paths are not built, the Python code launches the kernels instead: {e}", stacklevel=3)
+
+
 def _compile(src, verbose):
     obj = os.path.join(OBJ_DIR, os.path.basename(src)[:-3] + ".o")
     hdr_time = max([os.path.getmtime(f) for f in glob.glob(os.path.join(CSRC, "*.cuh")) +
@@ -114,13 +125,12 @@ def build_variant(out_path, extra_flags, obj_dir):
 
 def build_library(force=False, verbose=True):
     if not force and up_to_date():
-        build_host()
+        _build_host_if_possible(force)
         return LIB_PATH
     os.makedirs(OBJ_DIR, exist_ok=True)
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as ex:
-        host = ex.submit(build_host, force)
+        ex.submit(_build_host_if_possible, force)
         results = list(ex.map(lambda s: _compile(s, verbose), sources()))
-        host.result()
     objs = [o for o, _ in results]
     log = "\n".join(l for _, l in results if l)
     with open(os.path.join(LIB_DIR, "ptxas.log"), "a") as f:

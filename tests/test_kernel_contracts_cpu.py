@@ -4,6 +4,8 @@ import glob
 import os
 import re
 import shutil
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -61,3 +63,37 @@ def test_removed_switches_are_reported(name, monkeypatch):
     monkeypatch.setenv(name, "0")
     with pytest.warns(UserWarning, match=name):
         _lib.lib()
+
+
+@pytest.mark.parametrize("error", [ModuleNotFoundError("No module named 'torch'"), RuntimeError("g++ failed"), OSError("read-only")])
+@pytest.mark.parametrize("built", [False, True])
+def test_the_kernels_build_without_the_native_host_paths(error, built, monkeypatch, tmp_path):
+    """The module of native host paths is optional: whatever keeps it from being built, the kernel library is."""
+    from axonn_b200.utils import build
+
+    def no_host(force=False):
+        raise error
+
+    def tool(cmd, **_):                               # what nvcc would write
+        open(cmd[cmd.index("-o") + 1], "w").close()
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+    monkeypatch.setattr(build, "LIB_DIR", str(tmp_path))
+    monkeypatch.setattr(build, "OBJ_DIR", str(tmp_path / "obj"))
+    monkeypatch.setattr(build, "LIB_PATH", str(tmp_path / "lib.so"))
+    monkeypatch.setattr(build, "build_host", no_host)
+    monkeypatch.setattr(build, "_nvcc", lambda: "nvcc")
+    monkeypatch.setattr(build.subprocess, "run", tool)
+    if built:
+        open(build.LIB_PATH, "w").close()
+    with pytest.warns(UserWarning, match=str(error).split()[0]):
+        assert build.build_library(force=not built, verbose=False) == build.LIB_PATH
+    assert os.path.exists(build.LIB_PATH)
+
+
+def test_the_build_script_needs_no_torch():
+    """The script imports nothing outside the standard library (the compile job has only Python and the CUDA toolkit)."""
+    from axonn_b200.utils import build
+
+    code = "import sys, runpy; sys.modules['torch'] = None; g = runpy.run_path(sys.argv[1]); g['_build_host_if_possible'](False)"
+    r = subprocess.run([sys.executable, "-c", code, build.__file__], capture_output=True, text=True)
+    assert r.returncode == 0 and "native host paths are not built" in r.stderr
