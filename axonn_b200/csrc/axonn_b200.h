@@ -12,6 +12,8 @@ extern "C" {
 #endif
 
 const char* axb_last_error(void);
+/* Stands for this header (a checksum, see utils/build.py): callers that were compiled against it compare before they call. */
+unsigned int axb_interface(void);
 /* Status word set by kernels whose bounded waits expired (0 = clean); reading
  * clears it when `clear` is non-zero.  Host-mapped: no device sync needed. */
 unsigned int axb_device_status(int device, int clear);

@@ -59,6 +59,11 @@ extern "C" void axb_set_wait_timeout_ms(unsigned int ms) {
 
 extern "C" const char* axb_last_error(void) { return axb::g_err; }
 
+#ifndef AXB_INTERFACE
+#define AXB_INTERFACE 0u
+#endif
+extern "C" unsigned int axb_interface(void) { return AXB_INTERFACE; }
+
 extern "C" unsigned int axb_device_status(int device, int clear) {
   volatile unsigned int* w = axb::device_status_word(device, nullptr);
   if (!w) return 0xFFFFFFFFu;

@@ -19,20 +19,20 @@
 #include <atomic>
 #include <string>
 
+#include "axonn_b200.h"
+
 namespace {
 
 using at::Tensor;
 using std::optional;
 
-// launchers of the kernel library (csrc/axonn_b200.h)
-int (*norm_fwd)(const void*, const void*, const void*, void*, float*, int, int, int, float, int, int, int, int, void*);
-int (*norm_bwd)(const void*, const void*, const void*, const float*, void*, float*, float*, float*, void*, void*, int, int, int, int, int, int, int, int, void*);
-int (*add_norm_fwd)(const void*, const void*, void*, const void*, const void*, void*, float*, int, int, int, float, int, int, int, int, void*);
-int (*add_norm_bwd)(const void*, const void*, const void*, const void*, const float*, void*, float*, float*, float*, void*, void*, int, int, int, int, int, int, int, int, void*);
-int (*norm_grid)(int, int);
-int (*gemm)(int, const void*, const void*, void*, const void*, void*, int, int, int, int, int, int, int, int, void*);
-int (*flash_fwd)(const void*, void*, float*, int, int, int, int, int, float, int, void*);
-const char* (*last_error)();
+// Launchers of the kernel library, of the types that its header gives them; bind() fills them in.  The header's number comes from
+// the build, and a library of another one is not bound.
+#define AXB_LAUNCHERS(X) \
+  X(axb_norm_fwd, norm_fwd) X(axb_norm_bwd, norm_bwd) X(axb_add_norm_fwd, add_norm_fwd) X(axb_add_norm_bwd, add_norm_bwd) \
+  X(axb_norm_grid, norm_grid) X(axb_gemm, gemm) X(axb_flash_attn_fwd, flash_fwd) X(axb_last_error, last_error)
+#define AXB_DECLARE(symbol, name) decltype(&::symbol) name = nullptr;
+AXB_LAUNCHERS(AXB_DECLARE)
 PyObject *kernel_error = nullptr, *parameter_type = nullptr;
 std::atomic<long long> launches{0};
 
@@ -229,20 +229,24 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind({launcher name: address}, KernelError, Parameter)
+// bind({launcher name: address}, KernelError, Parameter, axb_interface() of the library they are from) -> False if it is another one
 PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  TORCH_CHECK(n == 3 && PyDict_Check(a[0]), "bind(launchers, error type, parameter type)");
-  const auto take = [&](const char* name, auto& fn) {
-    PyObject* v = PyDict_GetItemString(a[0], name);
-    TORCH_CHECK(v, "launcher ", name, " is missing");
+  TORCH_CHECK(n == 4 && PyDict_Check(a[0]), "bind(launchers, error type, parameter type, interface)");
+  if (PyLong_AsUnsignedLong(a[3]) != AXB_INTERFACE) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_FALSE;
+  }
+  const auto take = [&](const char* symbol, auto& fn) {
+    PyObject* v = PyDict_GetItemString(a[0], symbol);
+    TORCH_CHECK(v, "launcher ", symbol, " is missing");
     fn = reinterpret_cast<std::remove_reference_t<decltype(fn)>>(PyLong_AsVoidPtr(v));
   };
-  take("axb_norm_fwd", norm_fwd); take("axb_norm_bwd", norm_bwd); take("axb_add_norm_fwd", add_norm_fwd); take("axb_add_norm_bwd", add_norm_bwd);
-  take("axb_norm_grid", norm_grid); take("axb_gemm", gemm); take("axb_flash_attn_fwd", flash_fwd); take("axb_last_error", last_error);
+#define AXB_TAKE(symbol, name) take(#symbol, name);
+  AXB_LAUNCHERS(AXB_TAKE)
   Py_INCREF(a[1]); Py_INCREF(a[2]);
   kernel_error = a[1]; parameter_type = a[2];
-  Py_RETURN_NONE;
+  Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
 }
 

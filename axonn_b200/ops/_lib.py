@@ -141,15 +141,17 @@ def _load_host():
             path, module = host_path(), None
             if os.environ.get("AXONN_HOST_OPS", "1") != "0" and os.path.exists(path):
                 spec = importlib.util.spec_from_file_location("axonn_host", path)
+                launchers = {n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in _HOST_LAUNCHERS if hasattr(L, n)}
+                interface = L.axb_interface() & 0xFFFFFFFF if hasattr(L, "axb_interface") else 0
                 try:
                     module = importlib.util.module_from_spec(spec)
                     spec.loader.exec_module(module)
-                except ImportError as e:
-                    warnings.warn(f"the native host paths do not load ({e}); rebuild them (axonn_b200/utils/build.py)", stacklevel=2)
+                    why = "" if module.bind(launchers, KernelError, torch.nn.Parameter, interface) else "built for another kernel library"
+                except (ImportError, RuntimeError) as e:
+                    why = str(e)
+                if why:
+                    warnings.warn(f"the native host paths are not used ({why}); rebuild them (axonn_b200/utils/build.py)", stacklevel=2)
                     module = None
-                else:
-                    module.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in _HOST_LAUNCHERS}, KernelError,
-                                torch.nn.Parameter)
             _HOST = module
     return _HOST
 

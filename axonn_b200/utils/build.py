@@ -15,6 +15,7 @@ import shutil
 import subprocess
 import sys
 import warnings
+import zlib
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -23,6 +24,7 @@ LIB_DIR = os.path.join(PKG, "lib")
 OBJ_DIR = os.path.join(LIB_DIR, "obj")
 LIB_PATH = os.path.join(LIB_DIR, "libaxonn_b200.so")
 HOST_SRC = os.path.join(CSRC, "host_ops.cpp")
+HEADER = os.path.join(CSRC, "axonn_b200.h")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -50,6 +52,12 @@ def up_to_date():
     return os.path.exists(LIB_PATH) and os.path.getmtime(LIB_PATH) >= _newest_input()
 
 
+def _interface_flag():
+    """What the library and the module of native host paths are told of the header that both are compiled against."""
+    with open(HEADER, "rb") as f:
+        return f"-DAXB_INTERFACE={zlib.crc32(f.read())}u"
+
+
 def host_path():
     """Where the native host paths are for this PyTorch and this Python, whose C++ interfaces they use."""
     import torch
@@ -60,7 +68,7 @@ def host_path():
 def build_host(force=False):
     """The native host paths (``csrc/host_ops.cpp``): a Python module against PyTorch's C++ API, without device code."""
     out = host_path()
-    if not force and os.path.exists(out) and os.path.getmtime(out) >= os.path.getmtime(HOST_SRC):
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= max(map(os.path.getmtime, (HOST_SRC, HEADER))):
         return out
     import sysconfig
 
@@ -74,7 +82,7 @@ def build_host(force=False):
     dirs = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
             sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     cmd = [gxx, "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
-    cmd += ["-I" + d for d in dirs] + [HOST_SRC, "-o", out + ".tmp", "-L" + os.path.join(root, "lib")]
+    cmd += [_interface_flag()] + ["-I" + d for d in dirs + [CSRC]] + [HOST_SRC, "-o", out + ".tmp", "-L" + os.path.join(root, "lib")]
     cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
@@ -97,7 +105,7 @@ def _compile(src, verbose):
                     glob.glob(os.path.join(CSRC, "*.h"))] + [0])
     if os.path.exists(obj) and os.path.getmtime(obj) >= max(os.path.getmtime(src), hdr_time):
         return obj, ""
-    cmd = [_nvcc()] + NVCC_FLAGS + ["-I", CSRC, "-c", src, "-o", obj]
+    cmd = [_nvcc()] + NVCC_FLAGS + [_interface_flag(), "-I", CSRC, "-c", src, "-o", obj]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"nvcc failed for {src}:\n{r.stdout}\n{r.stderr}")
@@ -111,7 +119,7 @@ def build_variant(out_path, extra_flags, obj_dir):
     objs = []
     for src in sources():
         obj = os.path.join(obj_dir, os.path.basename(src)[:-3] + ".o")
-        r = subprocess.run([_nvcc()] + NVCC_FLAGS + list(extra_flags) + ["-I", CSRC, "-c", src, "-o", obj],
+        r = subprocess.run([_nvcc()] + NVCC_FLAGS + list(extra_flags) + [_interface_flag(), "-I", CSRC, "-c", src, "-o", obj],
                            capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed for {src}:\n{r.stdout}\n{r.stderr}")

@@ -97,3 +97,55 @@ def test_the_build_script_needs_no_torch():
     code = "import sys, runpy; sys.modules['torch'] = None; g = runpy.run_path(sys.argv[1]); g['_build_host_if_possible'](False)"
     r = subprocess.run([sys.executable, "-c", code, build.__file__], capture_output=True, text=True)
     assert r.returncode == 0 and "native host paths are not built" in r.stderr
+
+
+@native
+def test_native_host_paths_are_those_of_the_library(monkeypatch):
+    """The module calls the launchers by address: it is used with the library whose header it was compiled against, and no other."""
+    from axonn_b200.utils import build
+
+    L = _lib.lib()
+    if not os.path.exists(build.host_path()):
+        pytest.skip("native host paths not built")
+    assert f"-DAXB_INTERFACE={L.axb_interface() & 0xFFFFFFFF}u" == build._interface_flag()
+    monkeypatch.setattr(_lib, "_HOST", _lib._UNSET)
+    assert _lib.host() is not None
+
+    class Older:                                      # another header's number, or a library from before there was one
+        _name = "older.so"
+
+        def __init__(self, **more):
+            self.__dict__.update(more)
+
+        def __getattr__(self, name):
+            if name == "axb_interface":
+                raise AttributeError(name)
+            return getattr(L, name)
+    for other in (Older(), Older(axb_interface=lambda: 1)):
+        monkeypatch.setattr(_lib, "_HOST", _lib._UNSET)
+        monkeypatch.setattr(_lib, "_LIB", other)
+        with pytest.warns(UserWarning, match="another kernel library"):
+            assert _lib.host() is None
+
+
+def test_native_host_paths_are_rebuilt_with_the_header(monkeypatch, tmp_path):
+    from axonn_b200.utils import build
+
+    out, source, header = (str(tmp_path / n) for n in ("host.so", "host_ops.cpp", "axonn_b200.h"))
+    for i, f in enumerate((source, out, header)):     # the header is the newest
+        open(f, "w").close()
+        os.utime(f, (100 + i, 100 + i))
+    made = []
+
+    def tool(cmd, **_):
+        made.append(cmd)
+        open(cmd[cmd.index("-o") + 1], "w").close()
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+    monkeypatch.setattr(build, "HOST_SRC", source)
+    monkeypatch.setattr(build, "HEADER", header)
+    monkeypatch.setattr(build, "host_path", lambda: out)
+    monkeypatch.setattr(build, "_nvcc", lambda: "/usr/local/cuda/bin/nvcc")
+    monkeypatch.setattr(build.shutil, "which", lambda n: n)
+    monkeypatch.setattr(build.subprocess, "run", tool)
+    assert build.build_host() == out and len(made) == 1
+    assert build.build_host() == out and len(made) == 1
