@@ -50,12 +50,20 @@ volatile unsigned int* device_status_word(int device, unsigned int** dev_ptr) {
 static unsigned long long g_wait_timeout_ns = 120000000000ull;
 unsigned long long wait_timeout_ns() { return g_wait_timeout_ns; }
 
+// Upper bound on the CTAs of the next GEMM launches (0 = all SMs): lets two GEMMs that are launched on different
+// streams - a communication-bound fused kernel and a compute-bound one - share the GPU instead of queueing behind
+// each other (a persistent grid of one CTA per SM leaves no room for a second kernel).
+static int g_max_ctas = 0;
+int max_ctas() { return g_max_ctas; }
+
 }  // namespace axb
 
 // Deadline after which a device-side wait (mbarrier, peer flag) gives up and reports through the status word.
 extern "C" void axb_set_wait_timeout_ms(unsigned int ms) {
   axb::g_wait_timeout_ns = (ms < 1 ? 1ull : static_cast<unsigned long long>(ms)) * 1000000ull;
 }
+
+extern "C" void axb_gemm_set_max_ctas(int n) { axb::g_max_ctas = n; }
 
 extern "C" const char* axb_last_error(void) { return axb::g_err; }
 

@@ -16,6 +16,8 @@ namespace axb {
 // ----------------------------------------------------------------------------- host error state
 void set_error(const char* fmt, ...);
 int check_cuda(cudaError_t e, const char* what);
+// Cap on the CTAs of GEMM launches (axb_gemm_set_max_ctas), 0: none.
+int max_ctas();
 // Per-device word that kernels set when a bounded wait expires (0 = clean).
 // Lives in mapped pinned host memory so the host can read it without a sync.
 volatile unsigned int* device_status_word(int device, unsigned int** dev_ptr);
@@ -165,6 +167,8 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
 // CTA calls pdl_launch_next after its tensor memory is allocated: a CTA of the next kernel may be given what is left.
 // One B200: attention layer of 777 tokens (four launches) 96 -> 90 us, residual LayerNorm forward and backward 104.6 -> 102.7, loss
 // head of 4096 tokens 2057 -> 2016.  The attention backward's kernels are launched without: 1 % slower with (803 / 795 us).
+// While GEMMs are capped nothing is launched ahead: the SMs that the cap leaves are for another stream's kernel, not for blocks that
+// wait there for the end of the capped one.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... Params, typename... Args>
@@ -174,7 +178,7 @@ static inline cudaError_t pdl_launch(void (*kernel)(Params...), dim3 grid, dim3 
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  cfg.attrs = attr; cfg.numAttrs = max_ctas() == 0 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 

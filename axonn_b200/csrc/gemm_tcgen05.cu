@@ -2127,13 +2127,9 @@ int sm_count_current() {
 }
 
 // Communicating GEMM on CTA pairs: the kernel above with PAIR = true, launched as clusters of two.
-// Upper bound on the CTAs of the next GEMM launches (0 = all SMs): lets two GEMMs that are launched on different
-// streams - a communication-bound fused kernel and a compute-bound one - share the GPU instead of queueing behind
-// each other (a persistent grid of one CTA per SM leaves no room for a second kernel).
-static int g_max_ctas = 0;
 static inline int usable_sms(int device) {
-  const int sms = sm_count(device);
-  return (g_max_ctas >= 2 && g_max_ctas < sms) ? g_max_ctas : sms;
+  const int sms = sm_count(device), cap = max_ctas();
+  return (cap >= 2 && cap < sms) ? cap : sms;
 }
 
 template <int A_MN, int B_MN>
@@ -2278,7 +2274,7 @@ static int launch_splitk(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmPar
   // Not where a CTA streams for long: the early CTAs of the next launch leave the others on SMs that are next to one another, and
   // the operands arrive more slowly (one B200, with / without: layout 2, 24 x 8192 x 8192 38.5 / 35.8 us, 200 x 4096 x 8192 27.7 / 24.2).
   const int blocks = (p.K + BK - 1) / BK / z;
-  cfg.attrs = attr; cfg.numAttrs = blocks <= (A_MN ? 16 : 32) ? 2 : 1;
+  cfg.attrs = attr; cfg.numAttrs = blocks <= (A_MN ? 16 : 32) && max_ctas() == 0 ? 2 : 1;
   AXB_CUDA(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, z, arows, small));
   return 0;
 }
@@ -2511,7 +2507,6 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
 // Milliseconds the fused GEMM kernels spent stalled on peers since the last reset (sum over launches of the mean
 // over each launch's CTAs).  Synchronises the device; `device` must be current.  A diagnostic for reporting exposed
 // communication, not for use inside a timed region.
-extern "C" void axb_gemm_set_max_ctas(int n) { axb::g_max_ctas = n; }
 
 extern "C" double axb_comm_stall_ms(int device, int reset) {
   (void)device;

@@ -85,3 +85,33 @@ def test_a_refused_launch_is_reported_once(tmp_path):
     subprocess.run(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-I", csrc, str(tmp_path / "launch.cu"),
                     os.path.join(csrc, "common.cu"), "-o", str(tmp_path / "launch")], check=True)
     subprocess.run([str(tmp_path / "launch")], check=True)
+
+
+def test_a_cap_leaves_its_sms_to_the_other_stream():
+    """A column sum behind a product that is held to a few SMs does not wait on the others: what another stream launches has them."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib, gemm
+
+    a, b = (torch.randn(4096, 8192, device=DEV).to(BF16) for _ in range(2))
+    x, y = torch.randn(65536, 4096, device=DEV).to(BF16), torch.randn(1 << 24, device=DEV)
+    want = ops.column_sum(x)
+    y.mul_(1.0)
+    side, behind = torch.cuda.Stream(), torch.cuda.Event()
+    L = _lib.lib()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        try:
+            L.axb_gemm_set_max_ctas(2)
+            gemm.matmul_nt(a, b)                       # 15 ms
+            got = ops.column_sum(x)
+        finally:
+            L.axb_gemm_set_max_ctas(0)
+        behind.record()
+    done = torch.cuda.Event()
+    for _ in range(20):
+        y.mul_(1.0)
+    done.record()
+    done.synchronize()
+    assert not behind.query()                            # the product is still at work
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
