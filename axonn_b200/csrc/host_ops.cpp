@@ -6,6 +6,8 @@
 // refuses it.  Nothing is kept from one call to the next.  The kernels are those of the library that ops/_lib.py has loaded: bind()
 // is given the addresses of its launchers.
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/jit/frontend/tracer.h>
@@ -16,6 +18,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <algorithm>
 #include <atomic>
 #include <string>
 
@@ -105,7 +108,23 @@ struct NormNode : torch::autograd::Function<NormNode> {
     if (delta) return {h, y};
     return {y};
   }
+  // The kernels leave no graph: differentiating these gradients again is an error (first_derivative_only in ops/direct.py).
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    if (!at::GradMode::is_enabled()) return gradients(ctx, grads);
+    torch::autograd::variable_list out, inputs = ctx->get_saved_variables();
+    {
+      at::AutoGradMode no_grad(false);
+      out = gradients(ctx, grads);
+    }
+    inputs.insert(inputs.end(), grads.begin(), grads.end());
+    if (!std::any_of(inputs.begin(), inputs.end(), [](const Tensor& t) { return t.defined() && t.requires_grad(); })) return out;
+    const auto node = std::make_shared<torch::autograd::Error>("Norm: second derivatives are not implemented",
+                                                               torch::autograd::collect_next_edges(inputs));
+    for (Tensor& t : out)
+      if (t.defined()) torch::autograd::set_history(t = t.detach(), node);
+    return out;
+  }
+  static torch::autograd::variable_list gradients(torch::autograd::AutogradContext* ctx, const torch::autograd::variable_list& grads) {
     const auto saved = ctx->get_saved_variables();
     // what hooks (offloading, compression) give back may lie in another layout
     const Tensor h = saved[0].contiguous(), gamma = saved[1].contiguous(), stats = saved[2].contiguous();

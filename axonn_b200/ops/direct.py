@@ -3,6 +3,8 @@
 An autograd function costs more host time than the launch (4 us against 5 us, and as much again in reshapes and saved tensors),
 and evaluating a model without gradients is bound by host time for short prompts."""
 
+import functools
+
 import torch
 from torch.autograd import forward_ad
 
@@ -56,3 +58,32 @@ def plain_layer(layer) -> bool:
             and layer._compiled_call_impl is None
             and not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks
                      or _module._has_any_global_hook()))
+
+
+class _SecondDerivative(torch.autograd.Function):
+    """``outs`` as they are, as functions of ``inputs`` without a derivative."""
+
+    @staticmethod
+    def forward(ctx, what, n, *tensors):
+        ctx.what = what
+        return tuple(t if t is None else t.detach() for t in tensors[:n])
+
+    @staticmethod
+    def backward(ctx, *_):
+        raise RuntimeError(f"{ctx.what}: second derivatives are not implemented")
+
+
+def first_derivative_only(backward):
+    """Decorator of a ``Function.backward`` whose gradients come from kernels that leave no graph: differentiating them by what the
+    function was called with is an error, whatever they are added to.  (After ``once_differentiable`` they count as constants when the
+    incoming gradient needs none, which is how a loss that is a sum begins, and for ``torch.autograd.grad``, which walks only the part
+    of the graph that leads to the tensors it is given.)  The saved tensors stand for the inputs."""
+    @functools.wraps(backward)
+    def wrapper(ctx, *grads):
+        with torch.no_grad():
+            out = backward(ctx, *grads)
+        if not torch.is_grad_enabled():
+            return out
+        outs = out if isinstance(out, tuple) else (out,)
+        return _SecondDerivative.apply(type(ctx).__name__, len(outs), *outs, *grads, *ctx.saved_tensors)
+    return wrapper

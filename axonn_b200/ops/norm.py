@@ -12,7 +12,7 @@ import torch
 import torch.distributed as dist
 
 from . import _lib
-from .direct import host_paths, no_graph
+from .direct import first_derivative_only, host_paths, no_graph
 
 _DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
@@ -59,7 +59,7 @@ class _NormFn(torch.autograd.Function):
         if not x.is_cuda:
             x2 = x.reshape(-1, H).contiguous()
             y, mean, rstd = _torch_norm_fwd(x2, gamma, beta, eps, rms, group)
-            ctx.save_for_backward(x2, gamma, mean, rstd)
+            ctx.save_for_backward(x, gamma, mean, rstd)
             return y.reshape(shape)
         x2 = _dense_rows(x, H)
         rows = x2.numel() // H
@@ -83,17 +83,18 @@ class _NormFn(torch.autograd.Function):
             call(1)                              # partial (sum x, sum x^2) of my slice of the hidden dimension
             dist.all_reduce(stats, group=group)
             call(3)                              # finishes (mean, rstd) in place and applies them
-        ctx.save_for_backward(x2, g, stats)
+        ctx.save_for_backward(x2, g, stats, *(() if g is gamma else (gamma,)))
         return _shaped(y, shape)
 
     @staticmethod
+    @first_derivative_only
     def backward(ctx, dy):
         rms, group, n = ctx.rms, ctx.group, ctx.n
         H = ctx.shape[-1]
         if not dy.is_cuda:
             dy2 = dy.reshape(-1, H).contiguous()
-            x2, gamma, mean, rstd = ctx.saved_tensors
-            xh = (x2.float() - mean) * rstd
+            x, gamma, mean, rstd = ctx.saved_tensors
+            xh = (x.reshape(-1, H).float() - mean) * rstd
             gd = dy2.float() * gamma.float()
             s1 = torch.zeros_like(mean) if rms else gd.sum(-1, keepdim=True)
             s2 = (gd * xh).sum(-1, keepdim=True)
@@ -106,7 +107,7 @@ class _NormFn(torch.autograd.Function):
             dgamma = (dy2.float() * xh).sum(0).to(gamma.dtype)
             dbeta = dy2.float().sum(0).to(gamma.dtype) if ctx.has_beta else None
             return dx.to(dy.dtype).reshape(ctx.shape), dgamma, dbeta, None, None, None
-        x2, g, stats = ctx.saved_tensors
+        x2, g, stats = ctx.saved_tensors[:3]
         dy2 = _dense_rows(dy, H)
         rows = stats.shape[0]
         L = _lib.lib()
@@ -151,16 +152,15 @@ class _AddNormFn(torch.autograd.Function):
         if not x.is_cuda:
             x2 = x.reshape(-1, H).contiguous()
             d2 = delta.reshape(-1, H).contiguous()
-            h = x2 + d2
-            y, mean, rstd = _torch_norm_fwd(h, gamma, beta, eps, rms, group)
+            h = (x2 + d2).reshape(shape)
+            y, mean, rstd = _torch_norm_fwd(h.reshape(-1, H), gamma, beta, eps, rms, group)
             ctx.save_for_backward(h, gamma, mean, rstd)
-            return h.reshape(shape), y.reshape(shape)
+            return h, y.reshape(shape)
         x2, d2 = _dense_rows(x, H), _dense_rows(delta, H)
         rows = x2.numel() // H
         L = _lib.lib()
         dev = x2.device.index
-        h = torch.empty_like(x2)
-        y = torch.empty_like(x2)
+        h, y = (torch.empty(shape, dtype=x2.dtype, device=x2.device) for _ in range(2))
         stats = torch.empty((rows, 2), dtype=torch.float32, device=x2.device)
         g = gamma.to(x2.dtype) if gamma.dtype != x2.dtype else gamma
         b = None if beta is None else (beta.to(x2.dtype) if beta.dtype != x2.dtype else beta)
@@ -178,18 +178,19 @@ class _AddNormFn(torch.autograd.Function):
             call(1, x2, d2)                      # writes h and the partial row sums
             dist.all_reduce(stats, group=group)
             call(3, h, None)                     # finishes (mean, rstd) in place and applies them
-        ctx.save_for_backward(h, g, stats)
-        return _shaped(h, shape), _shaped(y, shape)
+        ctx.save_for_backward(h, g, stats, *(() if g is gamma else (gamma,)))
+        return h, y
 
     @staticmethod
+    @first_derivative_only
     def backward(ctx, dh, dy):
         rms, group, n = ctx.rms, ctx.group, ctx.n
         H = ctx.shape[-1]
         if not dy.is_cuda:
             dy2 = dy.reshape(-1, H).contiguous()
             dh2 = None if dh is None else dh.reshape(-1, H).contiguous()
-            x2, gamma, mean, rstd = ctx.saved_tensors
-            xh = (x2.float() - mean) * rstd
+            h, gamma, mean, rstd = ctx.saved_tensors
+            xh = (h.reshape(-1, H).float() - mean) * rstd
             gd = dy2.float() * gamma.float()
             s1 = torch.zeros_like(mean) if rms else gd.sum(-1, keepdim=True)
             s2 = (gd * xh).sum(-1, keepdim=True)
@@ -205,7 +206,7 @@ class _AddNormFn(torch.autograd.Function):
             dbeta = dy2.float().sum(0).to(gamma.dtype) if ctx.has_beta else None
             dx = dx.to(dy.dtype).reshape(ctx.shape)
             return dx, dx, dgamma, dbeta, None, None, None
-        x2, g, stats = ctx.saved_tensors
+        x2, g, stats = ctx.saved_tensors[:3]
         dy2 = _dense_rows(dy, H)
         dh2 = None if dh is None else _dense_rows(dh, H)
         rows = stats.shape[0]
@@ -272,7 +273,8 @@ def _norm(x, delta, gamma, beta, eps, rms, group):
     direct = _norm_direct(x, delta, gamma, beta, eps, rms, group)
     if delta is not None:
         return direct or _AddNormFn.apply(x, delta, gamma, beta, eps, rms, group)
-    return _NormFn.apply(x, gamma, beta, eps, rms, group) if direct is None else direct[1]
+    # dense outside of the function: what it saves is its input then
+    return _NormFn.apply(x.contiguous(), gamma, beta, eps, rms, group) if direct is None else direct[1]
 
 
 def add_layer_norm(x, delta, gamma, beta, eps=1e-5, group=None):

@@ -127,6 +127,34 @@ def test_norms_are_seen(monkeypatch):
     assert _lib.launch_count == 0
 
 
+@pytest.mark.parametrize("form", ["dense", "strided", "other type"])
+@pytest.mark.parametrize("native", [False, True])
+@pytest.mark.parametrize("residual", [False, True])
+def test_second_derivatives_are_refused(native, residual, form, monkeypatch):
+    """First derivatives with ``create_graph`` are what they are without; one of them, also beside terms that do have a second
+    derivative, is not taken for a constant."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib
+
+    if not native:
+        monkeypatch.setattr(_lib, "_HOST", None)
+    x, d = (torch.randn(3, 5, 64, device=DEV, requires_grad=True) for _ in range(2))
+    g = torch.ones(64, device=DEV, dtype=BF16 if form == "other type" else torch.float32, requires_grad=True)
+    leaves = (x, d, g) if residual else (x, g)
+
+    def loss():
+        a, b = (t.transpose(0, 1) if form == "strided" else t for t in (x, d))
+        y = sum(ops.add_layer_norm(a, b, g, None)) if residual else ops.rms_norm(a, g)
+        return y.sum() + sum((t ** 3).sum() for t in leaves)
+    want = torch.autograd.grad(loss(), leaves)
+    got = torch.autograd.grad(loss(), leaves, create_graph=True)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    for a in got:
+        for leaf in leaves:
+            with pytest.raises(RuntimeError, match="second derivatives"):
+                torch.autograd.grad(a.pow(2).sum(), leaf, allow_unused=True, retain_graph=True)
+
+
 @pytest.mark.parametrize("dtype", [BF16, torch.float16, torch.float32])
 def test_linear_and_attention(dtype, monkeypatch):
     from axonn_b200 import ops

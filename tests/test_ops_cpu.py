@@ -210,3 +210,25 @@ print("alias ok")
     r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300,
                        env=dict(os.environ, CUDA_VISIBLE_DEVICES=""))
     assert r.returncode == 0 and "alias ok" in r.stdout, r.stdout[-1500:] + r.stderr[-1500:]
+
+
+@pytest.mark.parametrize("form", ["dense", "strided", "other type"])
+@pytest.mark.parametrize("residual", [False, True])
+def test_second_derivatives_of_norms_are_refused(residual, form):
+    """First derivatives with ``create_graph`` are what they are without; one of them, also beside terms that do have a second
+    derivative, is not taken for a constant."""
+    x, d = (torch.randn(3, 5, 64).requires_grad_(True) for _ in range(2))
+    g = torch.ones(64, dtype=torch.bfloat16 if form == "other type" else torch.float32, requires_grad=True)
+    leaves = (x, d, g) if residual else (x, g)
+
+    def loss():
+        a, b = (t.transpose(0, 1) if form == "strided" else t for t in (x, d))
+        y = sum(ops.add_layer_norm(a, b, g, None)) if residual else ops.rms_norm(a, g)
+        return y.sum() + sum((t ** 3).sum() for t in leaves)
+    want = torch.autograd.grad(loss(), leaves)
+    got = torch.autograd.grad(loss(), leaves, create_graph=True)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    for a in got:
+        for leaf in leaves:
+            with pytest.raises(RuntimeError, match="second derivatives"):
+                torch.autograd.grad(a.pow(2).sum(), leaf, allow_unused=True, retain_graph=True)
