@@ -56,6 +56,12 @@ int dtype_code(const Tensor& t) {
   return t.scalar_type() == at::kBFloat16 ? 0 : t.scalar_type() == at::kHalf ? 1 : t.scalar_type() == at::kFloat ? 2 : -1;
 }
 const void* addr(const optional<Tensor>& t) { return t ? t->data_ptr() : nullptr; }
+// The norm kernels read 16 bytes at a time.
+bool on_16_bytes(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+Tensor dense(const Tensor& t) {
+  const Tensor d = t.contiguous();
+  return on_16_bytes(d) ? d : d.clone();
+}
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
 // Other Python threads run while this one allocates (the allocator may have to free blocks, which synchronises) and launches (a full
@@ -127,9 +133,9 @@ struct NormNode : torch::autograd::Function<NormNode> {
   static torch::autograd::variable_list gradients(torch::autograd::AutogradContext* ctx, const torch::autograd::variable_list& grads) {
     const auto saved = ctx->get_saved_variables();
     // what hooks (offloading, compression) give back may lie in another layout
-    const Tensor h = saved[0].contiguous(), gamma = saved[1].contiguous(), stats = saved[2].contiguous();
+    const Tensor h = dense(saved[0]), gamma = dense(saved[1]), stats = dense(saved[2]);
     const bool rms = ctx->saved_data["rms"].toBool(), delta = ctx->saved_data["delta"].toBool();
-    const Tensor dy = grads[delta ? 1 : 0].contiguous();
+    const Tensor dy = dense(grads[delta ? 1 : 0]);
     const int H = static_cast<int>(h.size(-1)), rows = static_cast<int>(stats.size(0)), device = h.get_device();
     const int grid = norm_grid(device, rows);
     Tensor dx = at::empty_like(h), part = at::empty({2, grid, H}, stats.options()), dgamma = at::empty_like(gamma), dbeta;
@@ -138,7 +144,7 @@ struct NormNode : torch::autograd::Function<NormNode> {
     float* pb = pa + static_cast<size_t>(grid) * H;
     void* db = rms ? nullptr : dbeta.data_ptr();
     if (delta) {
-      const Tensor dh = grads[0].contiguous();
+      const Tensor dh = dense(grads[0]);
       check(add_norm_bwd(dy.data_ptr(), dh.data_ptr(), h.data_ptr(), gamma.data_ptr(), stats.data_ptr<float>(), dx.data_ptr(), nullptr, pa, pb,
                          dgamma.data_ptr(), db, rows, H, H, rms, 0, dtype_code(h), dtype_code(gamma), device, stream()),
             "axb_add_norm_bwd", 2);
@@ -166,7 +172,8 @@ PyObject* py_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int64_t H = x.size(-1);
   if (H > INT32_MAX || x.numel() / H > INT32_MAX) Py_RETURN_NONE;
   for (const Tensor* v : {&gamma, beta ? &*beta : &gamma})
-    if (v->scalar_type() != type || v->dim() != 1 || v->size(0) != H || !v->is_contiguous() || v->device() != x.device()) Py_RETURN_NONE;
+    if (v->scalar_type() != type || v->dim() != 1 || v->size(0) != H || !v->is_contiguous() || v->device() != x.device() || !on_16_bytes(*v)) Py_RETURN_NONE;
+  if (!on_16_bytes(x) || (delta && !on_16_bytes(*delta))) Py_RETURN_NONE;
   if (delta && (delta->sizes() != x.sizes() || delta->scalar_type() != type || !delta->is_contiguous() || delta->device() != x.device())) Py_RETURN_NONE;
   const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || gamma.requires_grad() || (delta && delta->requires_grad()) ||
                                                    (beta && beta->requires_grad()));

@@ -11,6 +11,8 @@
 //   mode 0  statistics computed locally and applied in one kernel
 //   mode 1  only emit per-row partial sums
 //   mode 2  apply with externally supplied (already reduced) statistics
+#include <initializer_list>
+
 #include "common.cuh"
 
 namespace axb {
@@ -1139,6 +1141,14 @@ static int norm_bwd_t(const void* dy, const void* x, const void* gamma, const fl
 
 }  // namespace axb
 
+// The kernels read and write 16 bytes at a time.
+static bool on_16_bytes(std::initializer_list<const void*> ptrs) {
+  uintptr_t bits = 0;
+  for (const void* p : ptrs) bits |= reinterpret_cast<uintptr_t>(p);
+  if (bits & 15) axb::set_error("operands must be 16-byte aligned");
+  return (bits & 15) == 0;
+}
+
 extern "C" int axb_norm_grid(int device, int rows) {
   int g = 8 * axb::sm_count(device);
   return rows < g ? rows : g;
@@ -1153,6 +1163,7 @@ extern "C" int axb_add_norm_fwd(const void* x, const void* delta, void* hout, co
   if (H % 8 || H > NORM_THREADS * 8 * NORM_MAX_CHUNKS) { set_error("norm: hidden %d unsupported", H); return -1; }
   if (delta && (mode == 2 || !hout)) { set_error("norm: the fused residual add needs an output for x + delta and mode 0 or 1"); return -1; }
   if (rows <= 0) return 0;
+  if (!on_16_bytes({x, delta, hout, gamma, beta, y})) return -1;
   const int grid = axb_norm_grid(device, rows);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == 0) return norm_fwd_t<__nv_bfloat16>(x, gamma, beta, y, stats, rows, H, H_total, eps, rms, mode, grid, s, delta, hout);
@@ -1185,6 +1196,7 @@ extern "C" int axb_add_norm_bwd(const void* dy, const void* dres, const void* x,
   using namespace axb;
   if (H % 8 || H > NORM_THREADS * 8 * NORM_MAX_CHUNKS) { set_error("norm: hidden %d unsupported", H); return -1; }
   if (rows <= 0) return 0;
+  if (!on_16_bytes({dy, dres, x, gamma, dx, dgamma_part, dbeta_part})) return -1;
   const int grid = axb_norm_grid(device, rows);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int rc, nblocks = grid;
@@ -1213,6 +1225,7 @@ extern "C" int axb_colsum(const void* x, float* part, void* out, int rows, int N
                           void* stream) {
   using namespace axb;
   if (N % 8 || rows <= 0) { set_error("colsum: N must be a multiple of 8 and rows positive"); return -1; }
+  if (!on_16_bytes({x})) return -1;
   const int splits = axb_colsum_splits(device, rows, N);
   dim3 grid((N / 8 + 31) / 32, splits);
   cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -22,8 +22,13 @@ def _group_size(group):
 
 
 def _dense_rows(t, H):
-    """``t`` itself when it is dense (the kernels see rows of ``H``), otherwise a dense copy of its rows."""
-    return t if t.is_contiguous() else t.reshape(-1, H).contiguous()
+    """``t`` itself when it is dense (the kernels see rows of ``H``) and on 16 bytes, otherwise a copy of its rows that is."""
+    return _on_16_bytes(t if t.is_contiguous() else t.reshape(-1, H).contiguous())
+
+
+def _on_16_bytes(t):
+    """``t`` where the kernels can read 16 bytes at a time: a view into a buffer at another offset is copied."""
+    return t.clone() if t is not None and t.is_cuda and t.data_ptr() % 16 else t
 
 
 def _shaped(t, shape):
@@ -67,8 +72,8 @@ class _NormFn(torch.autograd.Function):
         dev = x2.device.index
         y = torch.empty_like(x2)
         stats = torch.empty((rows, 2), dtype=torch.float32, device=x2.device)
-        g = gamma.to(x2.dtype) if gamma.dtype != x2.dtype else gamma
-        b = None if beta is None else (beta.to(x2.dtype) if beta.dtype != x2.dtype else beta)
+        g = _on_16_bytes(gamma.to(x2.dtype) if gamma.dtype != x2.dtype else gamma)
+        b = None if beta is None else _on_16_bytes(beta.to(x2.dtype) if beta.dtype != x2.dtype else beta)
 
         def call(mode):
             st = L.axb_norm_fwd(_lib.addr(x2), _lib.addr(g), _lib.addr(b), _lib.addr(y), _lib.addr(stats),
@@ -83,7 +88,7 @@ class _NormFn(torch.autograd.Function):
             call(1)                              # partial (sum x, sum x^2) of my slice of the hidden dimension
             dist.all_reduce(stats, group=group)
             call(3)                              # finishes (mean, rstd) in place and applies them
-        ctx.save_for_backward(x2, g, stats, *(() if g is gamma else (gamma,)))
+        ctx.save_for_backward(x2, g, stats, *(i for i, t in ((x, x2), (gamma, g)) if i is not t))
         return _shaped(y, shape)
 
     @staticmethod
@@ -162,8 +167,8 @@ class _AddNormFn(torch.autograd.Function):
         dev = x2.device.index
         h, y = (torch.empty(shape, dtype=x2.dtype, device=x2.device) for _ in range(2))
         stats = torch.empty((rows, 2), dtype=torch.float32, device=x2.device)
-        g = gamma.to(x2.dtype) if gamma.dtype != x2.dtype else gamma
-        b = None if beta is None else (beta.to(x2.dtype) if beta.dtype != x2.dtype else beta)
+        g = _on_16_bytes(gamma.to(x2.dtype) if gamma.dtype != x2.dtype else gamma)
+        b = None if beta is None else _on_16_bytes(beta.to(x2.dtype) if beta.dtype != x2.dtype else beta)
 
         def call(mode, src, dl):
             st = L.axb_add_norm_fwd(_lib.addr(src), _lib.addr(dl), _lib.addr(h if dl is not None else None), _lib.addr(g),
@@ -245,7 +250,8 @@ def _norm_direct(x, delta, gamma, beta, eps, rms, group):
     if (not no_graph(x, delta, gamma, beta) or x.dtype not in _DT or gamma.dtype != x.dtype or gamma.shape != (H,)
             or (beta is not None and (beta.dtype != x.dtype or beta.shape != (H,) or not beta.is_contiguous()))
             or x.numel() == 0 or _group_size(group) != 1 or not x.is_contiguous() or not gamma.is_contiguous()
-            or (delta is not None and (delta.shape != x.shape or delta.dtype != x.dtype or not delta.is_contiguous()))):
+            or (delta is not None and (delta.shape != x.shape or delta.dtype != x.dtype or not delta.is_contiguous()))
+            or any(t is not None and t.data_ptr() % 16 for t in (x, delta, gamma, beta))):
         return None
     rows = x.numel() // H
     y = torch.empty_like(x)
@@ -273,7 +279,7 @@ def _norm(x, delta, gamma, beta, eps, rms, group):
     direct = _norm_direct(x, delta, gamma, beta, eps, rms, group)
     if delta is not None:
         return direct or _AddNormFn.apply(x, delta, gamma, beta, eps, rms, group)
-    # dense outside of the function: what it saves is its input then
+    # made dense outside of the function: what it saves is its input then
     return _NormFn.apply(x.contiguous(), gamma, beta, eps, rms, group) if direct is None else direct[1]
 
 
@@ -303,7 +309,7 @@ def column_sum(x, out_dtype=torch.float32):
     """``x.sum(0)`` of a 2-D tensor, accumulated in fp32 and returned as ``out_dtype`` (bias gradients).  One
     pass over ``x`` at memory bandwidth on CUDA (partial sums per row split, then a fold that writes the
     requested dtype); plain PyTorch elsewhere."""
-    if not (_lib.use_cuda_kernels(x) and x.dim() == 2 and x.shape[1] % 8 == 0 and x.is_contiguous()
+    if not (_lib.use_cuda_kernels(x) and x.dim() == 2 and x.shape[1] % 8 == 0 and x.is_contiguous() and x.data_ptr() % 16 == 0
             and x.dtype in (torch.bfloat16, torch.float16, torch.float32) and x.shape[0] > 0
             and out_dtype in _DT):
         return x.sum(0, dtype=torch.float32).to(out_dtype)

@@ -127,6 +127,35 @@ def test_norms_are_seen(monkeypatch):
     assert _lib.launch_count == 0
 
 
+@pytest.mark.parametrize("dtype", [BF16, torch.float16, torch.float32])
+@pytest.mark.parametrize("native", [False, True])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norms_of_views_at_any_offset(residual, native, dtype, monkeypatch):
+    """Dense views that do not begin on 16 bytes - input, residual, gain, bias, incoming gradients - are what their copies are; the
+    launchers themselves refuse such addresses."""
+    from axonn_b200 import ops
+    from axonn_b200.ops import _lib
+
+    if not native:
+        monkeypatch.setattr(_lib, "_HOST", None)
+    shapes = [(6, 264), (6, 264), (264,), (264,), (6, 264), (6, 264)]
+    off = [torch.randn(1 + torch.Size(s).numel(), device=DEV).to(dtype)[1:].view(s) for s in shapes]
+    assert all(t.data_ptr() % 16 for t in off)
+
+    def run(tensors, grad):
+        x, d, g, b = (t.detach().requires_grad_(grad) for t in tensors[:4])
+        out = ops.add_layer_norm(x, d, g, b) if residual else (ops.layer_norm(x, g, b),)
+        leaves = (x, d, g, b) if residual else (x, g, b)
+        return [o.detach() for o in out] + list(torch.autograd.grad(out, leaves, tensors[4:4 + len(out)]) if grad else ())
+    for grad in (False, True):
+        for i in range(7):                                                # all, or one at a time
+            mixed = [t if i in (j, 6) else t.clone() for j, t in enumerate(off)]
+            for a, w in zip(run(mixed, grad), run([t.clone() for t in off], grad)):
+                assert torch.equal(a, w)
+    # sums of six values in another order: 6 roundings of 2^-24
+    assert float((ops.column_sum(off[0]) - ops.column_sum(off[0].clone())).abs().max()) <= 6 * 2 ** -24 * float(off[0].float().abs().sum(0).max())
+
+
 @pytest.mark.parametrize("form", ["dense", "strided", "other type"])
 @pytest.mark.parametrize("native", [False, True])
 @pytest.mark.parametrize("residual", [False, True])

@@ -46,6 +46,20 @@ def test_prune_refuses_an_unaligned_workspace():
     assert L.axb_prune_topk(4096, 1 << 20, 0, 1000, 4096 + 4, 0, None) == -1 and "aligned" in _error()
 
 
+@native
+@pytest.mark.parametrize("which", range(6))
+def test_norms_refuse_unaligned_operands(which):
+    """The kernels move 16 bytes at a time (addresses that are never used: the call is refused on the host)."""
+    L, p = _lib.lib(), [4096] * 6
+    p[which] += 2
+    assert L.axb_add_norm_fwd(*p, 4096, 4, 64, 64, 1e-5, 0, 0, 0, 0, None) == -1 and "aligned" in _error()
+    dy, dres, x, gamma, dx, part = p
+    assert L.axb_add_norm_bwd(dy, dres, x, gamma, 4096, dx, None, part, 4096, 4096, 4096, 4, 64, 64, 0, 0, 0, 0, 0, None) == -1
+    assert "aligned" in _error()
+    if which == 0:
+        assert L.axb_colsum(dy, 4096, 4096, 4, 64, 0, 2, 0, None) == -1 and "aligned" in _error()
+
+
 def test_every_status_code_of_the_kernels_has_a_name():
     """A wait that gave up is reported by name: every code that a kernel writes, and no code of a kernel that is gone."""
     csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(_lib.__file__))), "csrc")
