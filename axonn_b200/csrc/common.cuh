@@ -164,7 +164,11 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
 // --- programmatic dependent launch.  A kernel launched with the attribute may start before its predecessor in the stream has
 // ended, once all of that one's CTAs have called pdl_launch_next or ended (at its end, if it never calls it); pdl_wait returns when
 // the predecessor has ended and its writes are visible.  Every thread that reads or writes global memory calls pdl_wait first, and a
-// CTA calls pdl_launch_next after its tensor memory is allocated: a CTA of the next kernel may be given what is left.
+// CTA calls pdl_launch_next after its tensor memory is allocated: a CTA of the next kernel may be given what is left.  Bounded waits
+// start after pdl_wait too: their deadline does not include the predecessor's run.
+// Two kernels touch global memory before pdl_wait.  Split-K products fetch weights into the L2, where every writer's data is.  The later
+// pruning passes load the gradient: all passes before them only read it, and the first one is an ordinary launch, which starts when
+// whatever wrote the gradient has ended.
 // One B200: attention layer of 777 tokens (four launches) 96 -> 90 us, residual LayerNorm forward and backward 104.6 -> 102.7, loss
 // head of 4096 tokens 2057 -> 2016.  The attention backward's kernels are launched without: 1 % slower with (803 / 795 us).
 // While GEMMs are capped nothing is launched ahead: the SMs that the cap leaves are for another stream's kernel, not for blocks that

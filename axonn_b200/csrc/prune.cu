@@ -287,6 +287,8 @@ int prune_topk_launch(void* g, long long n, int dtype, long long k, unsigned int
   const long long bytes = n * (dtype == PR_F32 ? 4 : 2);
   const bool is_long = bytes >= PR_LONG_BYTES && (dtype != PR_F32 || bytes <= PR_LONG_F32_BYTES);
   auto hist = is_long ? prune_hist1_kernel<true> : prune_hist1_kernel<false>;
+  // An ordinary launch, and it has to stay one: the passes after it load the gradient before they wait for their predecessor, and mask
+  // what they have loaded.  Launched ahead itself, this pass could let them do so while the gradient is still being written.
   hist<<<sms, PR_THREADS, PR_BINS1 * 4, s>>>(g, n, dtype, k, hist1, meta);
   AXB_CUDA(cudaGetLastError());
   if (dtype == PR_F32) {
