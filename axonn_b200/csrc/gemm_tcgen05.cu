@@ -1526,7 +1526,7 @@ __host__ __device__ inline int pair_whole_tiles(long long total, int pairs) {
 }
 
 // Work of a CTA pair: tiles, dealt in turn.  When the last wave would leave half of the pairs or more without a tile, its tiles
-// are cut into two halves of 128 columns, one for each of two pairs: the same MMAs with N = 128, half the time.
+// are cut into two halves of their columns (p.bn / 2), one for each of two pairs: the same MMAs with half of N, half the time.
 // One B200, bf16, whole tiles / with halves: 777 x 6144 x 4096 (96 tiles on 74 pairs) 46.7 / 38.8 us, 1024 x 6144 x 2048 26.9 /
 // 22.3, 1024 x 6144 x 512 14.8 / 10.5, 8192 x 2048 x 4096 111 / 103; no difference within the noise of the power cap for the
 // weight gradients 8192 x 2048 x 16384.  More than half of the pairs busy: halves would need a second round, nothing gained.
@@ -1820,6 +1820,10 @@ struct SplitKSmem {
   __host__ __device__ static constexpr int ring(bool small) { return small ? 100 * 1024 : 192 * 1024; }
   __host__ __device__ static constexpr int total(bool small) { return ring(small) + BAR_BYTES + 1024 /* alignment slack */; }
 };
+static_assert(BM * SplitKSmem::PART_LD * 4 <= SplitKSmem::ring(true) && SplitKSmem::ring(true) < SplitKSmem::ring(false),
+              "the partial tile lies in the operand ring");
+static_assert(SplitKSmem::total(false) <= 232448 && 2 * (SplitKSmem::total(true) + 1024) <= 233472,
+              "shared memory of a CTA, and of two on an SM");
 
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t local_smem_addr, uint32_t cta) {
   uint32_t a;
@@ -2126,12 +2130,12 @@ int sm_count_current() {
   return sm_count(dev);
 }
 
-// Communicating GEMM on CTA pairs: the kernel above with PAIR = true, launched as clusters of two.
 static inline int usable_sms(int device) {
   const int sms = sm_count(device), cap = max_ctas();
   return (cap >= 2 && cap < sms) ? cap : sms;
 }
 
+// Communicating GEMM on CTA pairs: the kernel above with PAIR = true, launched as clusters of two.
 template <int A_MN, int B_MN>
 static int launch_comm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmParams& p, int device, cudaStream_t stream) {
   using S = GemmSmem<256, true>;
@@ -2507,7 +2511,6 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
 // Milliseconds the fused GEMM kernels spent stalled on peers since the last reset (sum over launches of the mean
 // over each launch's CTAs).  Synchronises the device; `device` must be current.  A diagnostic for reporting exposed
 // communication, not for use inside a timed region.
-
 extern "C" double axb_comm_stall_ms(int device, int reset) {
   (void)device;
   unsigned long long v = 0;
