@@ -208,11 +208,31 @@ def test_linear_and_attention(dtype, monkeypatch):
                 assert torch.equal(ops.flash_attention_packed(qkv), _python(monkeypatch, lambda: ops.flash_attention_packed(qkv)))
 
 
-def test_launch_errors_keep_their_type():
-    """A launcher's status becomes the error that the Python paths raise (a device that the library does not know)."""
+def test_launch_errors_keep_their_type(monkeypatch):
+    """A launcher that refuses a call: the error and its text are those of the Python paths.  What is not for the native paths is left
+    to the general ones."""
+    from axonn_b200 import ops
+    from axonn_b200.intra_layer import Linear
     from axonn_b200.ops import _lib
 
     assert issubclass(_lib.KernelError, RuntimeError)
+    layer = Linear(64, 64, bias=False, expert_mode=True, dtype=BF16)
+    flat, narrow = torch.randn(65, device=DEV, dtype=BF16), torch.randn(2, 12, device=DEV, dtype=BF16)
+    gain = torch.ones(12, device=DEV, dtype=BF16)
+
+    def refused(call):
+        before = _lib.launch_count
+        with torch.no_grad(), pytest.raises(_lib.KernelError) as e:
+            call()
+        assert _lib.launch_count == before
+        return str(e.value)
+    for call, text in ((lambda: layer(flat[1:].view(1, 64)), "axb_gemm failed (status -1): TMA base address must be 16-byte aligned"),
+                       (lambda: ops.rms_norm(narrow, gain), "axb_norm_fwd failed (status -1): norm: hidden 12 unsupported"),
+                       (lambda: ops.add_rms_norm(narrow, narrow, gain), "axb_add_norm_fwd failed (status -1): norm: hidden 12 unsupported")):
+        assert refused(call) == text == _python(monkeypatch, lambda: refused(call))
+    x = narrow.clone().requires_grad_(True)
+    with pytest.raises(_lib.KernelError):
+        ops.rms_norm(x, gain)
     host = _lib.host()
     x, w = torch.randn(8, device=DEV, dtype=BF16), torch.ones(8, device=DEV, dtype=BF16)
     assert host.norm(x.cpu(), None, w, None, 1e-5, True) is None and host.norm(x, None, w.cpu(), None, 1e-5, True) is None
