@@ -2322,32 +2322,36 @@ struct PairTiles { int bn; bool swap; };
 
 // Time of a product on `pairs` CTA pairs in columns of work: waves of tiles, the last one in halves where it is small.  A tile
 // costs 80 columns beside its own (its 256 rows are loaded whatever its width, and loads from the L2 bound narrow tiles), and 2 %
-// more where half of its width is an odd multiple of 8.
-static float pair_cost(unsigned tile_rows, unsigned cols, unsigned bn, unsigned pairs) {
+// more where half of its width is an odd multiple of 8.  `column`: cost of a column; with exchanged roles it also passes through
+// shared memory once, which takes as long as 2.5 of its K blocks.
+static float pair_cost(unsigned tile_rows, unsigned cols, unsigned bn, unsigned pairs, float column) {
   const unsigned total = tile_rows * ((cols + bn - 1) / bn), waves = total / pairs, rest = total - waves * pairs;
-  float cost = static_cast<float>(waves * (bn + 80));
-  if (rest != 0) cost += bn % 32 == 0 && 2 * rest <= pairs ? bn / 2 + 80 : bn + 80;
+  float cost = static_cast<float>(waves) * (column * bn + 80);
+  if (rest != 0) cost += (bn % 32 == 0 && 2 * rest <= pairs ? column * (bn / 2) : column * bn) + 80;
   return bn % 32 == 0 ? cost : 1.02f * cost;
 }
+static float pair_column(bool swap, int K) { return swap ? 1.f + 2.5f * BK / K : 1.f; }
 
 // Widths from 96 to 256 columns in either orientation; 256 with the roles as they are unless another one saves 2 % or more.
-// Exchanged roles take a little longer at the end of the launch (300 columns of one K block).  A B whose columns are
-// contiguous (layouts 1 and 2) is loaded in blocks of 64 that have to start on 128 bytes: other widths made it slower.
+// A B whose columns are contiguous (layouts 1 and 2) is loaded in blocks of 64 that have to start on 128 bytes: other widths made
+// it slower.
 // One B200, bf16, 256 / chosen (M x N x K): 777 x 6144 x 4096 41.9 / 35.4 us (144, exchanged), 777 x 4096 x 4096 26.8 / 23.9 (208,
 // exchanged), 777 x 3072 x 1024 10.9 / 6.5 (144, exchanged), 1300 x 50304 x 2048 215 / 184 (224, exchanged), 4096 x 2048 x 50304 in layout
 // 1 663 / 635 (240, exchanged).  Over 243 shapes of M 300 .. 4096, N 1024 .. 50304, K 1024 .. 50304, layouts 0 (plain, bias, GELU)
 // and 1 on average 0.916 of the time, at best 0.60, at worst 1.023 (4096 x 2048 x 2048, layout 1); the best widths of
-// each shape would give 0.910.
+// each shape would give 0.910.  Over 882 shapes of M 300 .. 16384, N 768 .. 8192, K 128 .. 4096, where the pass through shared memory
+// shows: 0.976, at worst 1.04, the best widths 0.969 (with exchanged roles at the price of the others 0.983, at worst 1.26: 16500 x
+// 2048 x 256 26.4 us with 256 columns, 32.9 with 224 exchanged, which is what it took for the better one).
 static PairTiles pair_tiles(int M, int N, int K, int layout, bool can_swap, int pairs) {
   PairTiles best = {PAIR_BN, false};
   const unsigned rows_m = (M + 2 * BM - 1) / (2 * BM), rows_n = (N + 2 * BM - 1) / (2 * BM);
   if (layout > 1 || static_cast<long long>(rows_m) * rows_n > (1 << 20)) return best;
-  float least = 0.98f * pair_cost(rows_m, N, PAIR_BN, pairs);
+  float least = 0.98f * pair_cost(rows_m, N, PAIR_BN, pairs, 1.f);
   // no width can do better than full waves of the widest tiles without a padded row: the search costs 0.3 us of host time
   if (static_cast<float>(M) * static_cast<float>(N) * (PAIR_BN + 80) >= least * (2.f * BM * PAIR_BN) * pairs) return best;
   for (int swap = layout == 0 ? 0 : 1; swap <= (can_swap ? 1 : 0); ++swap) {
     for (int bn = PAIR_BN; bn >= 96; bn -= 16) {
-      const float cost = swap ? pair_cost(rows_n, M, bn, pairs) + 300.f * BK / K : pair_cost(rows_m, N, bn, pairs);
+      const float cost = pair_cost(swap ? rows_n : rows_m, swap ? M : N, bn, pairs, pair_column(swap, K));
       if (cost < least) { least = cost; best = {bn, swap != 0}; }
     }
   }
@@ -2665,7 +2669,7 @@ extern "C" int axb_gemm_ce_pays(int M, int N, int K, int device) {
   // the plain product's tiles may fit a ragged M better (pair_tiles): 1.2 ns a column and K block against the pass over the logits
   const axb::PairTiles best = axb::pair_tiles(M, N, K, 0, true, pairs);
   const unsigned rows = ((best.swap ? N : M) + 255) / 256, cols = best.swap ? M : N;
-  const float saved = static_cast<float>((tiles + pairs - 1) / pairs) * (axb::PAIR_BN + 80) - axb::pair_cost(rows, cols, best.bn, pairs);
+  const float saved = static_cast<float>((tiles + pairs - 1) / pairs) * (axb::PAIR_BN + 80) - axb::pair_cost(rows, cols, best.bn, pairs, axb::pair_column(best.swap, K));
   if (saved * (K / axb::BK) * 1.2e-3f > 0.4e-6f * M * N) return 0;
   if (M >= 2048) return !(halved && tiles < 2ll * pairs && K > 2048);
   if (M <= 512 || K < 512) return 0;

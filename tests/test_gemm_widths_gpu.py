@@ -10,7 +10,9 @@ DEV = "cuda:0"
 # rows off 32 bytes (N % 16 == 8), tiles of 64 and 128 columns for the small ones
 SHAPES = [(777, 6144, 256), (777, 3072, 1024), (769, 4104, 264), (1300, 2056, 328), (300, 8200, 136), (2500, 1032, 512), (513, 14344, 72),
           (3000, 1024, 200), (1024, 3080, 128), (1, 264, 64), (65, 8, 1024), (308, 1000, 256), (1000, 1024, 1024), (129, 4096, 520),
-          (1531, 1032, 264), (640, 1000, 8)]
+          (1531, 1032, 264), (640, 1000, 8),
+          # long enough along K for exchanged roles to pay
+          (777, 6144, 1032), (769, 4104, 1032), (300, 8200, 1032), (2500, 1032, 1032), (1300, 2056, 2056)]
 
 
 def _check(got, want, bound):
