@@ -2240,17 +2240,19 @@ static int splitk_rows(int M) { return M <= 96 ? (M + 31) / 32 * 32 : BM; }
 
 // CTAs per output tile of the split-K kernel (z 1: do not split) and whether their rings are the small ones.  All clusters have to
 // be in flight at once, every CTA needs 2 K blocks to work on, and the blocks that it does not walk have to outweigh the exchange of
-// its partial rows (25 rows cost as much as one block).  One CTA per SM with the large ring is as fast as or faster than two
-// with small ones at the same or half the split; only where one per SM leaves nothing to split, tiles of few rows are halved.
+// its partial rows: 25 of them cost as much as one block.  Where narrow tiles on pairs would run instead (pair_tiles_small) and fill
+// their columns, 9 do: with 25 there too, 1000 x 512 x 512 took 6.4 us (6.1 before the split, 4.9 on pairs), 304 x 3072 x 768 7.4 (6.9,
+// 5.9).  One CTA per SM with the large ring is as fast as or faster than two with small ones at the same or half the split; only
+// where one per SM leaves nothing to split, tiles of few rows are halved.
 // One B200, bf16 with bias, graph replay, weights from DRAM / from the L2, before (at most 6 stages, exchange by columns, no
 // programmatic launch) / now: 24 x 1024 x 512 6.7 / 3.8 us, 24 x 2048 x 2048 7.7 / 5.8 and 7.4 / 5.0, 24 x 8192 x 2048 13.4 / 9.4 and 12.3 /
 // 6.9, 24 x 2048 x 8192 13.6 / 10.5 and 10.5 / 8.7, 64 x 1024 x 8192 12.4 / 9.0, 128 x 1024 x 2048 11.7 / 7.3, 24 x 16384 x 2048 22.5 / 14.5.
 struct SplitK { int z; bool small; };
-static SplitK splitk_ctas(int layout, int M, int N, int K, int sms, int device) {
-  const int rows = M < BM ? M : BM, num_kb = (K + BK - 1) / BK;
+static SplitK splitk_ctas(int layout, int M, int N, int K, bool narrow_pairs, int sms, int device) {
+  const int rows = M < BM ? M : BM, num_kb = (K + BK - 1) / BK, rows_per_block = narrow_pairs && N > 64 ? 9 : 25;
   const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + SplitKSmem::BN - 1) / SplitKSmem::BN);
   for (int z = 8; z >= 2; z /= 2)
-    if (num_kb >= 2 * z && 25 * (num_kb - num_kb / z) > rows && tiles * z <= sms && tiles <= splitk_max_clusters(z, device))
+    if (num_kb >= 2 * z && rows_per_block * (num_kb - num_kb / z) > rows && tiles * z <= sms && tiles <= splitk_max_clusters(z, device))
       return {z, false};
   if (layout != 2 && M <= 32 && num_kb >= 4 && tiles <= sms && splitk_max_clusters(2, device) > 0) return {2, true};
   return {1, false};
@@ -2405,12 +2407,17 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
   // K-major operand [R, K]: box 64(K) x tile rows.  MN-major operand [K, R]: box 64(R) x 64(K).
   const bool wide_pair = !comm && plain_on_pairs(M, N, device);
   if (wide_pair) BN = 256;
-  const SplitK split = comm || wide_pair || BN != 128 ? SplitK{1, false} : splitk_ctas(layout, M, N, K, usable_sms(device), device);
   const bool can_swap = out_dtype != 2 && !accumulate && (layout == 0 || (layout == 1 && epilogue < 2));
   const int sms = usable_sms(device);
   PairTiles tiles = {0, false};
-  if (wide_pair) tiles = pair_tiles(M, N, K, layout, can_swap, sms / 2);
-  else if (!comm && split.z == 1) tiles = pair_tiles_small(M, N, K, layout, can_swap, sms / 2);
+  SplitK split = {1, false};
+  if (wide_pair) {
+    tiles = pair_tiles(M, N, K, layout, can_swap, sms / 2);
+  } else if (!comm) {
+    tiles = pair_tiles_small(M, N, K, layout, can_swap, sms / 2);
+    if (BN == 128) split = splitk_ctas(layout, M, N, K, tiles.bn != 0, sms, device);
+    if (split.z > 1) tiles = {0, false};
+  }
   const bool pair = tiles.bn != 0;
   // rows of A that a split-K stage holds
   const int arows = split.z > 1 && a_mn == 0 ? splitk_rows(M) : BM;
