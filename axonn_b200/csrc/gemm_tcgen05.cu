@@ -2254,7 +2254,8 @@ static SplitK splitk_ctas(int layout, int M, int N, int K, bool narrow_pairs, in
   for (int z = 8; z >= 2; z /= 2)
     if (num_kb >= 2 * z && rows_per_block * (num_kb - num_kb / z) > rows && tiles * z <= sms && tiles <= splitk_max_clusters(z, device))
       return {z, false};
-  if (layout != 2 && M <= 32 && num_kb >= 4 && tiles <= sms && splitk_max_clusters(2, device) > 0) return {2, true};
+  if (layout != 2 && M <= 32 && num_kb >= 4 && tiles <= sms && (!narrow_pairs || 2 * tiles > sms) && splitk_max_clusters(2, device) > 0)
+    return {2, true};
   return {1, false};
 }
 
