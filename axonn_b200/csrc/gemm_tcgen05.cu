@@ -1977,7 +1977,11 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (++stage == stages) { stage = 0; phase ^= 1; }
       }
       if (ok) umma_commit(acc_full);
-      else report_status(p.status, 0x152u);
+      else {
+        const uint64_t t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 50000ull) {}   // let MMAs in flight finish before TMEM is released
+        report_status(p.status, 0x152u);
+      }
     }
   } else {
     // the accumulator is complete: every MMA has read its operands, the ring now holds this CTA's partial tile
@@ -2004,12 +2008,6 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   }
   tcgen05_fence_before();
   __syncthreads();
-  if (*abort_flag != 0) {
-    // Whoever gave up, the producer may have issued its last copies long before: they land, and the MMAs on them end, before
-    // the CTA gives its shared and tensor memory back.
-    const uint64_t t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 200000ull) {}
-  }
   if (warp == 1) { __syncwarp(); tcgen05_fence_after(); tmem_dealloc(tmem_base, BN); }
   __syncwarp();
   cluster_sync_all();                 // all partials of the tile are in shared memory
@@ -2018,6 +2016,10 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     if (z_ctas == 2) splitk_finish<2>(p, smem_u32(smem), z, tm, tn);
     else if (z_ctas == 4) splitk_finish<4>(p, smem_u32(smem), z, tm, tn);
     else splitk_finish<8>(p, smem_u32(smem), z, tm, tn);
+  } else {
+    // Whoever gave up, the producer may have issued its last copies just before: they land before the CTA ends.
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) {}
   }
   __syncwarp();
   cluster_sync_all();                 // a CTA's partial stays valid until its peers have read it
