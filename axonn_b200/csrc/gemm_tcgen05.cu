@@ -2243,15 +2243,16 @@ static int splitk_rows(int M) { return M <= 96 ? (M + 31) / 32 * 32 : BM; }
 // CTAs per output tile of the split-K kernel (z 1: do not split) and whether their rings are the small ones.  All clusters have to
 // be in flight at once, every CTA needs 2 K blocks to work on, and the blocks that it does not walk have to outweigh the exchange of
 // its partial rows: 25 of them cost as much as one block.  Where narrow tiles on pairs would run instead (pair_tiles_small) and fill
-// their columns, 9 do: with 25 there too, 1000 x 512 x 512 took 6.4 us (6.1 before the split, 4.9 on pairs), 304 x 3072 x 768 7.4 (6.9,
-// 5.9).  One CTA per SM with the large ring is as fast as or faster than two with small ones at the same or half the split; only
-// where one per SM leaves nothing to split, tiles of few rows are halved.
+// their columns, 11 do: with 25 there too, 1000 x 512 x 512 took 6.4 us (6.1 before the split, 4.9 on pairs), 304 x 3072 x 768 7.4 (6.9,
+// 5.9); with 9, products of 64 rows, or of K 1024 with a GELU behind them, were up to 3 % slower (174 x 1024 x 1024 6.1 / 6.2).  One CTA
+// per SM with the large ring is as fast as or faster than two with small ones at the same or half the split; only where one per SM
+// leaves nothing to split, tiles of few rows are halved.
 // One B200, bf16 with bias, graph replay, weights from DRAM / from the L2, before (at most 6 stages, exchange by columns, no
 // programmatic launch) / now: 24 x 1024 x 512 6.7 / 3.8 us, 24 x 2048 x 2048 7.7 / 5.8 and 7.4 / 5.0, 24 x 8192 x 2048 13.4 / 9.4 and 12.3 /
 // 6.9, 24 x 2048 x 8192 13.6 / 10.5 and 10.5 / 8.7, 64 x 1024 x 8192 12.4 / 9.0, 128 x 1024 x 2048 11.7 / 7.3, 24 x 16384 x 2048 22.5 / 14.5.
 struct SplitK { int z; bool small; };
 static SplitK splitk_ctas(int layout, int M, int N, int K, bool narrow_pairs, int sms, int device) {
-  const int rows = M < BM ? M : BM, num_kb = (K + BK - 1) / BK, rows_per_block = narrow_pairs && N > 64 ? 9 : 25;
+  const int rows = M < BM ? M : BM, num_kb = (K + BK - 1) / BK, rows_per_block = narrow_pairs && N > 64 ? 11 : 25;
   const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + SplitKSmem::BN - 1) / SplitKSmem::BN);
   for (int z = 8; z >= 2; z /= 2)
     if (num_kb >= 2 * z && rows_per_block * (num_kb - num_kb / z) > rows && tiles * z <= sms && tiles <= splitk_max_clusters(z, device))
