@@ -2243,8 +2243,8 @@ static int splitk_rows(int M) { return M <= 96 ? (M + 31) / 32 * 32 : BM; }
 // CTAs per output tile of the split-K kernel (z 1: do not split) and whether their rings are the small ones.  All clusters have to
 // be in flight at once, every CTA needs 2 K blocks to work on, and the blocks that it does not walk have to outweigh the exchange of
 // its partial rows: 25 of them cost as much as one block.  Where narrow tiles on pairs would run instead (pair_tiles_small) and fill
-// their columns, 11 do: with 25 there too, 1000 x 512 x 512 took 6.4 us (6.1 before the split, 4.9 on pairs), 304 x 3072 x 768 7.4 (6.9,
-// 5.9); with 9, products of 64 rows, or of K 1024 with a GELU behind them, were up to 3 % slower (174 x 1024 x 1024 6.1 / 6.2).  One CTA
+// their columns, 11 do: with 25 there too, in layout 1, 1000 x 512 x 512 took 6.4 us (6.1 unsplit on single CTAs, 4.9 on pairs), 304 x
+// 3072 x 768 7.4 (6.9, 5.9); with 9, products of 64 rows, or of K 1024 with a GELU behind them, were up to 3 % slower (174 x 1024 x 1024 6.1 / 6.2).  One CTA
 // per SM with the large ring is as fast as or faster than two with small ones at the same or half the split; only where one per SM
 // leaves nothing to split, tiles of few rows are halved.
 // One B200, bf16 with bias, graph replay, weights from DRAM / from the L2, before (at most 6 stages, exchange by columns, no
@@ -2368,7 +2368,9 @@ static PairTiles pair_tiles(int M, int N, int K, int layout, bool can_swap, int 
 // Their kernel has six warps instead of the sixteen of the single CTAs' (which serves the fused collectives), and a
 // tile of half the width has its epilogue done sooner.  One B200, bf16, single CTAs / pairs: 308 x 768 x 256 5.5 / 4.6 us,
 // 308 x 1024 x 1024 7.6 / 6.8, 1000 x 1024 x 1024 7.8 / 7.2, layout 1 308 x 1024 x 256 5.3 / 4.7.  Over M 64 .. 1531, N 256 .. 6144, K 256 ..
-// 1024 0.82 - 1.0; with K 2048 and 4096 0.92 - 1.4.
+// 1024 0.82 - 1.0; with K 2048 and 4096 0.92 - 1.4.  With all that came since (overlapped launches among it) against single CTAs:
+// M 1 .. 100, N 64 .. 8192, K 64 .. 248 0.47 - 0.86 over 1200 shapes; M 1304 and 2048, N 64, K 384 in layout 1, where a pair's tile has 64
+// rows of 256, 1.07.
 static PairTiles pair_tiles_small(int M, int N, int K, int layout, bool can_swap, int pairs) {
   if (!pair_mode_enabled() || K > 1024 || layout > 1 || (layout == 1 && !can_swap)) return {0, false};
   // up to 128 rows the features go on the rows of the tiles: the second CTA of a pair would have none of A's
@@ -2419,7 +2421,8 @@ static int gemm_common(int layout, const void* A, const void* B, void* C, const 
     tiles = pair_tiles(M, N, K, layout, can_swap, sms / 2);
   } else if (!comm) {
     tiles = pair_tiles_small(M, N, K, layout, can_swap, sms / 2);
-    if (BN == 128) split = splitk_ctas(layout, M, N, K, tiles.bn != 0, sms, device);
+    // 32-bit results are split wherever single CTAs are the measure: shorter sums round less
+    if (BN == 128) split = splitk_ctas(layout, M, N, K, tiles.bn != 0 && out_dtype != 2, sms, device);
     if (split.z > 1) tiles = {0, false};
   }
   const bool pair = tiles.bn != 0;
