@@ -35,7 +35,8 @@ int axb_gemm_batched(int layout, const void* A, const void* B, void* C, int nb, 
                      int a_batch_rows, int b_batch_rows, int c_batch_rows, int in_dtype, int out_dtype,
                      int accumulate, const int* seg_counts /* device int32 [nb, nseg] or NULL */, int seg_rows,
                      int nseg, int device, void* stream);
-/* cap on the CTAs of the following GEMM launches (0: one per SM), for GEMMs that share the GPU from two streams */
+/* cap on the CTAs of the following GEMM launches (0: one per SM), for GEMMs that share the GPU from two streams; while it is in
+   force no launch begins before its predecessor in the stream has ended */
 void axb_gemm_set_max_ctas(int n);
 int axb_gemm_swiglu(int backward, const void* A, const void* B, void* out, void* saved, int nb, int M, int N, int K,
                     const int* seg_counts, int seg_rows, int nseg, int device, void* stream);

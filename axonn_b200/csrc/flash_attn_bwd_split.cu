@@ -12,8 +12,8 @@
 //                      dQ is scaled and written once, as bf16, into the packed gradient tensor.
 //   fa_bwd_dkv_kernel  one 128-row key tile per work item, walks the query tiles from the diagonal down (and the
 //                      query heads of the group) in steps of 64 queries: S^T = K Q^T and dP^T = V dO^T into
-//                      double-buffered 64-column score buffers (a thread owns a key row), P^T and dS^T go back as
-//                      bf16, dV += P^T dO and dK += dS^T Q accumulate in tensor memory; one MMA warp per
+//                      double-buffered 64-column score buffers (a thread has 4 keys x 8 queries), P^T and dS^T go back
+//                      as bf16, dV += P^T dO and dK += dS^T Q accumulate in tensor memory; one MMA warp per
 //                      accumulator.
 //
 // Both recompute S, so the pair does 7 MMA units per tile against 5 of the one-kernel form, but neither has a
