@@ -137,7 +137,7 @@ def build_library(force=False, verbose=True):
         return LIB_PATH
     os.makedirs(OBJ_DIR, exist_ok=True)
     with ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 2)) as ex:
-        ex.submit(_build_host_if_possible, force)
+        host = ex.submit(_build_host_if_possible, force)
         results = list(ex.map(lambda s: _compile(s, verbose), sources()))
     objs = [o for o, _ in results]
     log = "\n".join(l for _, l in results if l)
@@ -150,6 +150,7 @@ def build_library(force=False, verbose=True):
     os.replace(LIB_PATH + ".tmp", LIB_PATH)
     if verbose:
         print(f"built {LIB_PATH} from {len(objs)} sources", file=sys.stderr)
+    host.result()                  # what is not one of the reasons to do without is an error, after the library is there
     return LIB_PATH
 
 

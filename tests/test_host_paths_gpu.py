@@ -88,6 +88,14 @@ def test_norms_are_seen(monkeypatch):
     with torch.autograd.graph.saved_tensors_hooks(lambda t: turned(t.detach()), lambda t: t):
         y = ops.add_rms_norm(x, d, g)[1]
     assert torch.equal(torch.autograd.grad(y, x, dy)[0], want)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: 1 / 0, lambda t: t), pytest.raises(ZeroDivisionError):
+        ops.add_rms_norm(x, d, g)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: 1 / 0):
+        y = ops.add_rms_norm(x, d, g)[1]
+    with pytest.raises(ZeroDivisionError):
+        torch.autograd.grad(y, x, dy)
+    with torch.autograd.detect_anomaly(check_nan=False):
+        assert torch.equal(torch.autograd.grad(ops.add_rms_norm(x, d, g)[1], x, dy)[0], want)
     y = ops.rms_norm(x, g)
     torch.autograd.grad(y, x, dy)
     with pytest.raises(RuntimeError):
@@ -271,4 +279,4 @@ def test_other_threads_run_while_a_launch_waits(path, grad):
     other.join()
     torch.cuda.synchronize()
     assert longest > 0.2                                               # the queue was full
-    assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.1
+    assert max(b - a for a, b in zip(ticks, ticks[1:])) < longest / 2
