@@ -1,6 +1,7 @@
 """The native host paths (csrc/host_ops.cpp) against the Python code that launches the same kernels: same bits over all forms
 that either takes, refused where it was refused, seen by everything that looks at an operation."""
 
+import gc
 import threading
 import time
 
@@ -271,12 +272,16 @@ def test_other_threads_run_while_a_launch_waits(path, grad):
     other.start()
     longest = 0.0
     torch.cuda._sleep(10 ** 9)
-    for _ in range(3000):
-        t = time.perf_counter()
-        call()
-        longest = max(longest, time.perf_counter() - t)
-    done.set()
-    other.join()
+    gc.disable()                                                       # a collection stops both threads
+    try:
+        for _ in range(3000):
+            t = time.perf_counter()
+            call()
+            longest = max(longest, time.perf_counter() - t)
+    finally:
+        gc.enable()
+        done.set()
+        other.join()
     torch.cuda.synchronize()
     assert longest > 0.2                                               # the queue was full
     assert max(b - a for a, b in zip(ticks, ticks[1:])) < longest / 2

@@ -184,11 +184,17 @@ def test_a_cap_leaves_its_sms_to_the_other_stream():
 
     a, b = (torch.randn(4096, 8192, device=DEV).to(BF16) for _ in range(2))
     x, y = torch.randn(65536, 4096, device=DEV).to(BF16), torch.randn(1 << 24, device=DEV)
-    want = ops.column_sum(x)
     y.mul_(1.0)
-    side, behind = torch.cuda.Stream(), torch.cuda.Event()
+    side, (start, done, behind) = torch.cuda.Stream(), (torch.cuda.Event(enable_timing=True) for _ in range(3))
     L = _lib.lib()
     torch.cuda.synchronize()
+    with torch.cuda.stream(side):                      # kernels loaded, the stream's memory allocated: neither waits for the GPU below
+        gemm.matmul_nt(a, b)
+        want = ops.column_sum(x)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(2 * 10 ** 8)                     # 0.1 s: everything is launched before anything runs
+    start.record()
+    side.wait_event(start)
     with torch.cuda.stream(side):
         try:
             L.axb_gemm_set_max_ctas(2)
@@ -197,11 +203,9 @@ def test_a_cap_leaves_its_sms_to_the_other_stream():
         finally:
             L.axb_gemm_set_max_ctas(0)
         behind.record()
-    done = torch.cuda.Event()
     for _ in range(20):
         y.mul_(1.0)
     done.record()
-    done.synchronize()
-    assert not behind.query()                            # the product is still at work
     torch.cuda.synchronize()
+    assert start.elapsed_time(behind) > 6 and start.elapsed_time(done) < start.elapsed_time(behind) / 2
     assert torch.equal(got, want)
